@@ -160,6 +160,8 @@ int enqueue_mgpoisl(Ctx* c) {
     // converged flag and outer count; the error flag ctl[2] is cleared when
     // the stage (or the solve) starts
     MG_CUDA(cudaMemsetAsync(m->d_ctl, 0, 2 * sizeof(int), c->stream));
+    if (sip_on_tiles(s))   // the outer step takes its maxima into these
+        MG_CUDA(cudaMemsetAsync(c->d_gridred, 0, (size_t)c->ngrid * sizeof(double), c->stream));
     if (int rc = sip_divcal(c, s, m->d_sprm + 2)) return rc;
     int* ctl = m->d_ctl;
     // pressuresolver_mod.F90:196-199: the divergence restricted into the
@@ -219,7 +221,7 @@ int enqueue_mgpoisl(Ctx* c) {
                 if (int rc = mx_ftoc(c, s, lv, l, true, ctl)) return rc;
             if (int rc = mx_gridmax(c, s, ctl)) return rc;
         }
-        if (int rc = sip_conv(c, m->d_ctl, m->d_maxrhs, m->d_sprm)) return rc;
+        if (int rc = sip_conv(c, s, m->d_ctl, m->d_maxrhs, m->d_sprm)) return rc;
     }
     if (int rc = sip_scatter_dp(c, s)) return rc;
     // dp ghosts (the reference accumulates the connected hilf ghosts into dp)
@@ -513,11 +515,14 @@ int mixed_init(Ctx* c) {
     // the defaults)
     const char* tune = std::getenv("MGLET_TUNE");
     if (!(tune && tune[0] == '0')) {
-        if (int rc2 = sip_tune(c, m->sip, m->cf, m->d_gcls, m->d_ctl)) return rc2;
-        if (int rc2 = sip_tune_outer(c, m->sip, m->apx, m->d_gcls, m->d_ctl)) return rc2;
-        if (int rc2 = sip_tune_solve(c, m->sip, m->cf, m->apx, m->d_gcls, m->d_ctl, m->d_maxrhs,
-                                     m->d_sprm))
-            return rc2;
+        // (the solver on tiles has nothing to pick)
+        if (!sip_on_tiles(m->sip)) {
+            if (int rc2 = sip_tune(c, m->sip, m->cf, m->d_gcls, m->d_ctl)) return rc2;
+            if (int rc2 = sip_tune_outer(c, m->sip, m->apx, m->d_gcls, m->d_ctl)) return rc2;
+            if (int rc2 = sip_tune_solve(c, m->sip, m->cf, m->apx, m->d_gcls, m->d_ctl, m->d_maxrhs,
+                                         m->d_sprm))
+                return rc2;
+        }
         if (int rc2 = mx_flux_tune(c, m->du32, m->dv32, m->dw32, m->sx, m->sy, m->sz, m->d_sprm,
                                    m->d_ctl + 2))
             return rc2;
@@ -589,6 +594,7 @@ int mixed_force_variant(Ctx* c, const char* kernel, int v) {
             return MGLET_ERR_ARG;
         }
         m->sip.outer_variant = v;
+        m->sip.outer_forced = v >= 0;
         if (m->graph) {
             cudaGraphExecDestroy(m->graph);
             m->graph = nullptr;
@@ -645,6 +651,7 @@ int mixed_force_variant(Ctx* c, const char* kernel, int v) {
             return MGLET_ERR_ARG;
         }
         m->sip.sweep_variant = v;
+        m->sip.sweep_forced = v >= 0;
         if (m->graph) {
             cudaGraphExecDestroy(m->graph);
             m->graph = nullptr;
@@ -668,6 +675,7 @@ int mixed_force_variant(Ctx* c, const char* kernel, int v) {
         return MGLET_ERR_UNSUPPORTED;
     }
     m->sip.pre_variant = v;
+    m->sip.pre_forced = v >= 0;
     if (m->graph) {          // the captured stage holds the old launch
         cudaGraphExecDestroy(m->graph);
         m->graph = nullptr;

@@ -28,14 +28,7 @@
 namespace mg {
 namespace {
 
-// Plane-order geometry of the (common) grid shape
-struct PlaneMap {
-    const int* tpos;            // [nm][ni]: position of (io, jo) in plane m is tpos[m*ni+io] + jo
-    int ni, nj, nk, npp, fs;
-    __device__ __forceinline__ int pos(int io, int jo, int ko) const {
-        return tpos[(io + jo + ko) * ni + io] + jo;
-    }
-};
+using PlaneMap = PosMap;
 
 __device__ __forceinline__ int fidx(const PlaneMap& m, int axis, int ko, int jo, int io) {
     return axis == 0 ? ko + jo * m.nk : (axis == 1 ? ko + io * m.nk : jo + io * m.nj);
@@ -382,9 +375,7 @@ __global__ void k_mx_rk_par(const DevGrid* __restrict__ grids, const unsigned ch
     UO[c] = 0.0; VO[c] = 0.0; WO[c] = 0.0;
 }
 
-PlaneMap plane_map(const SipState& st) {
-    return PlaneMap{st.d_tpos, st.ni, st.nj, st.nk, st.npp, st.fs};
-}
+PlaneMap plane_map(const SipState& st) { return sip_posmap(st); }
 
 int upload(Ctx* c, const std::vector<int>& h, int** d) {
     if (h.empty()) return 0;
@@ -483,7 +474,7 @@ int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, co
     A.hier = c->d_hier;
     A.list = lv.d_pars[l];
     A.fnbr = st.d_fnbr;
-    A.facepos = st.d_facepos;
+    A.facepos = sip_facepos(st);
     A.m = plane_map(st);
     A.H = st.h32;
     A.PG = st.pg;
@@ -514,7 +505,7 @@ int mx_ftoc(Ctx* c, SipState& st, const LevelState& lv, int ilevel, bool rhs, co
 
 int mx_gridmax(Ctx* c, SipState& st, const int* ctl) {
     ProfScope ps_(c, "mx_gridmax");
-    k_mx_gridmax<<<c->ngrid, 256, 0, c->stream>>>(st.npp, st.rhs32, c->d_gridred, ctl);
+    k_mx_gridmax<<<c->ngrid, 256, 0, c->stream>>>(plane_map(st).npp, st.rhs32, c->d_gridred, ctl);
     MG_LAUNCHED(c);
     return 0;
 }

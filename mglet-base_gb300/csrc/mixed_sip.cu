@@ -45,10 +45,29 @@
 
 #include "internal.h"
 #include "mixed_sip.h"
+#include "sip_tile.cuh"
 
 namespace mg {
 namespace {
 
+#ifndef TFEW
+#define TFEW 304
+#endif
+#ifndef TDF
+#define TDF 3
+#endif
+#ifndef TDM
+#define TDM 2
+#endif
+#ifndef TBM
+#define TBM 4
+#endif
+#ifndef TPB
+#define TPB 5
+#endif
+#ifndef TOB
+#define TOB 4
+#endif
 constexpr int kMaxCols = 1024; // longest hyperplane (points)
 // A wait gives up after this many SM clock cycles (about one second); a
 // healthy wait lasts microseconds.
@@ -1016,15 +1035,16 @@ __global__ void __launch_bounds__(512, kMinBlocks) k_sip_outer_direct(OuterArgs 
 // flag.  The maximum is exact, so the result does not depend on the CTA size.
 template <bool kCoh>
 __device__ __forceinline__ void conv_step(const DevGrid* grids, int ngrid, int maxlevel,
-                                          const double* gridmax, int* ctl, double* maxrhs,
+                                          double* gridmax, int* ctl, double* maxrhs,
                                           const double* sprm, double epcorr, int nouter_min,
-                                          double* sh) {
+                                          double* sh, bool reset) {
     const double prefak = sprm[2];
     double m = 0.0;
     for (int g = threadIdx.x; g < ngrid; g += blockDim.x) {
         double gm;
         if constexpr (kCoh) gm = __ldcg(gridmax + g);
         else gm = gridmax[g];
+        if (reset) gridmax[g] = 0.0;
         m = fmax(fabs(gm * ldexp(1.0, maxlevel - grids[g].level)), m);
     }
     m = block_max2(m, sh);
@@ -1037,11 +1057,11 @@ __device__ __forceinline__ void conv_step(const DevGrid* grids, int ngrid, int m
 }
 
 __global__ void k_mx_conv(const DevGrid* __restrict__ grids, int ngrid, int maxlevel,
-                          const double* __restrict__ gridmax, int* ctl, double* maxrhs,
-                          const double* __restrict__ sprm, double epcorr, int nouter_min) {
+                          double* __restrict__ gridmax, int* ctl, double* maxrhs,
+                          const double* __restrict__ sprm, double epcorr, int nouter_min, int reset) {
     if (ctl[0]) return;
     __shared__ double sh[32];
-    conv_step<false>(grids, ngrid, maxlevel, gridmax, ctl, maxrhs, sprm, epcorr, nouter_min, sh);
+    conv_step<false>(grids, ngrid, maxlevel, gridmax, ctl, maxrhs, sprm, epcorr, nouter_min, sh, reset != 0);
 }
 
 // ---- Persistent solve -------------------------------------------------------
@@ -1185,7 +1205,7 @@ __global__ void __launch_bounds__(kSolveThreads, kMinBlocks) k_sip_solve(const _
             }
         } else if (!a.noconv && blockIdx.x == 0) {
             conv_step<true>(a.out.grids, ng, a.maxlevel, a.out.gridmax, a.ctl, a.maxrhs, a.sprm,
-                            a.epcorr, a.nouter_min, sh);
+                            a.epcorr, a.nouter_min, sh, false);
         }
         if (!grid_sync(a.bar, a.ctl + 2, (unsigned)ph + 1)) return;
         if (r == per - 1 && !a.noconv && __ldcg(a.ctl) != 0) break;
@@ -1238,8 +1258,7 @@ __device__ __forceinline__ void nat_point(int t, int ni, int nj, int nk, int& io
     io = t / (nk * nj);
 }
 
-__global__ void k_sip_divcal_nat(const DevGrid* __restrict__ grids, int ni, int nj, int nk,
-                                 const int* __restrict__ tpos, int npp, float* __restrict__ RHS,
+__global__ void k_sip_divcal_nat(const DevGrid* __restrict__ grids, PosMap m, float* __restrict__ RHS,
                                  float* __restrict__ RHSL, const double* __restrict__ U,
                                  const double* __restrict__ V, const double* __restrict__ W,
                                  const double* __restrict__ RDDX, const double* __restrict__ RDDY,
@@ -1247,9 +1266,9 @@ __global__ void k_sip_divcal_nat(const DevGrid* __restrict__ grids, int ni, int 
                                  const double* __restrict__ SDIV, const double* __restrict__ BP) {
     const int g = blockIdx.y;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ni * nj * nk) return;
+    if (t >= m.ni * m.nj * m.nk) return;
     int io, jo, ko;
-    nat_point(t, ni, nj, nk, io, jo, ko);
+    nat_point(t, m.ni, m.nj, m.nk, io, jo, ko);
     const DevGrid G = grids[g];
     const int kk = G.kk, jj = G.jj;
     const int k = ko + 3, j = jo + 3, i = io + 3;
@@ -1264,22 +1283,21 @@ __global__ void k_sip_divcal_nat(const DevGrid* __restrict__ grids, int ni, int 
         d = BP[G.ip3 + id] * d;
     }
     const float dh = (float)d;
-    const long long o = (long long)g * npp + tpos[(io + jo + ko) * ni + io] + jo;
+    const long long o = (long long)g * m.npp + m.pos(io, jo, ko);
     RHS[o] = dh;
     RHSL[o] = (float)(d - (double)dh);
 }
 
-__global__ void k_sip_scatter_nat(const DevGrid* __restrict__ grids, int ni, int nj, int nk,
-                                  const int* __restrict__ tpos, int npp, const float* __restrict__ DPH,
+__global__ void k_sip_scatter_nat(const DevGrid* __restrict__ grids, PosMap m, const float* __restrict__ DPH,
                                   const float* __restrict__ DPL, double* __restrict__ DP) {
     const int g = blockIdx.y;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ni * nj * nk) return;
+    if (t >= m.ni * m.nj * m.nk) return;
     int io, jo, ko;
-    nat_point(t, ni, nj, nk, io, jo, ko);
+    nat_point(t, m.ni, m.nj, m.nk, io, jo, ko);
     const DevGrid G = grids[g];
     const int id = (io + 2) * G.kk * G.jj + (jo + 2) * G.kk + (ko + 2);
-    const long long o = (long long)g * npp + tpos[(io + jo + ko) * ni + io] + jo;
+    const long long o = (long long)g * m.npp + m.pos(io, jo, ko);
     DP[G.ip3 + id] = (double)DPH[o] + (double)DPL[o];
 }
 
@@ -1364,6 +1382,140 @@ __global__ void k_sip_extract(const DevGrid* __restrict__ grids, const int* __re
     const double apv = ap[G.ip3 + id];
     aph[qp] = (float)apv;
     aph[npp + qp] = (float)(apv - (double)(float)apv);
+}
+
+// ---- on tiles ---------------------------------------------------------------
+// class coefficients on tiles from the FP64 fields of the representative grids:
+// {lw, ls, lb, lpr}, {ue, un, ut}, the operator's seven (with the couplings BP
+// closes masked) and ap as two floats
+__global__ void k_tile_extract(const DevGrid* __restrict__ grids, const int* __restrict__ reps, TileShape s,
+                               int planeorder, const double* __restrict__ lw, const double* __restrict__ ls,
+                               const double* __restrict__ lb, const double* __restrict__ lpr,
+                               const double* __restrict__ ue, const double* __restrict__ un,
+                               const double* __restrict__ ut, const double* __restrict__ ap,
+                               const float* __restrict__ AW, const float* __restrict__ AE,
+                               const float* __restrict__ AS, const float* __restrict__ AN,
+                               const float* __restrict__ AB, const float* __restrict__ AT,
+                               const unsigned char* __restrict__ BM, float* CF, float* CB, float* LAP,
+                               float* APX) {
+    const long long cls = blockIdx.y;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= s.npp) return;
+    const int rep = reps[cls];
+    const DevGrid G = grids[rep];
+    const int id = s.cell[p];
+    const long long src = G.ip3 + (planeorder ? s.plane[p] : id);
+    const float f[4] = {(float)lw[src], (float)ls[src], (float)lb[src], (float)lpr[src]};
+    const float b[3] = {(float)ue[src], (float)un[src], (float)ut[src]};
+    const double apv = ap[G.ip3 + id];
+    for (int q = 0; q < 4; ++q) CF[(cls * 4 + q) * s.npp + p] = f[q];
+    for (int q = 0; q < 3; ++q) CB[(cls * 3 + q) * s.npp + p] = b[q];
+    const int kk = G.kk, jj = G.jj;
+    const int ix = G.ipx + id / (kk * jj), iy = G.ipy + (id / kk) % jj, iz = G.ipz + id % kk;
+    const unsigned mk = BM ? BM[(long long)rep * s.npp + p] : 0x3Fu;
+    auto on = [mk](int q, float x) { return (mk >> q) & 1u ? x : 0.f; };
+    const float l[7] = {on(0, AW[ix]), on(1, AE[ix]), on(2, AS[iy]), on(3, AN[iy]),
+                        on(4, AB[iz]), on(5, AT[iz]), (float)apv};
+    for (int q = 0; q < 7; ++q) LAP[(cls * 7 + q) * s.npp + p] = l[q];
+    APX[cls * 2 * s.npp + p] = (float)apv;
+    APX[(cls * 2 + 1) * s.npp + p] = (float)(apv - (double)(float)apv);
+}
+
+struct TileOuterArgs {
+    TileArgs<float> t;
+    const unsigned char* BM;
+    float *RHS, *RHSL, *DPH, *DPL;
+    const float* APX;
+    const float* A1[6];
+    const float* A1L[6];
+    const DevGrid* grids;
+    double* gridmax;
+};
+
+// The outer step on tiles (laplacephi + rescal + maxabscal_grid +
+// accumulate_pcorr, see k_sip_outer): one thread a tile, the tiles of a grid in
+// gridDim.x CTAs; gridmax takes the maximum over them (a maximum of non-negative
+// numbers, as integers).
+__global__ void __launch_bounds__(128, TOB) k_tile_outer(const __grid_constant__ TileOuterArgs a) {
+    if (a.t.ctl[0]) return;
+    __shared__ float shm[4];
+    const TileShape& s = a.t.s;
+    const int g = a.t.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
+    const long long base = (long long)g * s.npp;
+    const DevGrid* G = a.grids + g;
+    const int ipx = G->ipx + 2, ipy = G->ipy + 2, ipz = G->ipz + 2;
+    const float* APX = a.APX + (long long)a.t.gcls[g] * 2 * s.npp;
+    float mx = 0.f;
+    for (int tile = blockIdx.x * 128 + threadIdx.x; tile < s.ntile; tile += gridDim.x * 128) {
+        const int p = 8 * tile;
+        TileHalo<float> o;
+        tile_halo(a.t, g, tile, o);
+        const int org = __ldg(s.nbr + 2 * tile + 1).z;
+        const int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
+        Vec8<float> aph, apl, rh8, rl8, dh8, dl8;
+        ld8(true, APX + p, aph);
+        ld8(true, APX + s.npp + p, apl);
+        ld8_rw(true, a.RHS + base + p, rh8);
+        ld8_rw(true, a.RHSL + base + p, rl8);
+        ld8_rw(true, a.DPH + base + p, dh8);
+        ld8_rw(true, a.DPL + base + p, dl8);
+        uint2 bm = make_uint2(0x3f3f3f3fu, 0x3f3f3f3fu);
+        if (a.BM) bm = *reinterpret_cast<const uint2*>(a.BM + base + p);
+        float ch[6][2], cl[6][2];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            const int x = f < 2 ? ipx + io : (f < 4 ? ipy + jo : ipz + ko);
+#pragma unroll
+            for (int d = 0; d < 2; ++d) {
+                ch[f][d] = __ldg(a.A1[f] + x + d);
+                cl[f][d] = __ldg(a.A1L[f] + x + d);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float n[6];
+            tile_nbrs(o, i, n);
+            const unsigned mk = ((i < 4 ? bm.x : bm.y) >> (8 * (i & 3))) & 0xffu;
+            const int d[3] = {i >> 2, (i >> 1) & 1, i & 1};
+            float sum = 0.f, comp = 0.f;
+#pragma unroll
+            for (int f = 0; f < 6; ++f) {
+                const float h = a.BM ? ((mk >> f) & 1u ? n[f] : 0.f) : n[f];
+                ff_acc(ch[f][d[f / 2]], cl[f][d[f / 2]], h, sum, comp);
+            }
+            const float hc = o.h.v[i];
+            ff_acc(aph.v[i], apl.v[i], hc, sum, comp);
+            // (rh + rl) - (sum + comp)
+            float rh, e;
+            two_sum(rh8.v[i], -sum, rh, e);
+            e = e + (rl8.v[i] - comp);
+            float rl;
+            two_sum(rh, e, rh, rl);
+            rh8.v[i] = rh;
+            rl8.v[i] = rl;
+            // (dh + dl) + hc
+            float dh, de;
+            two_sum(dh8.v[i], hc, dh, de);
+            de = de + dl8.v[i];
+            float dl;
+            two_sum(dh, de, dh, dl);
+            dh8.v[i] = dh;
+            dl8.v[i] = dl;
+            mx = fmaxf(mx, fabsf(rh));
+        }
+        st8(a.RHS + base + p, rh8);
+        st8(a.RHSL + base + p, rl8);
+        st8(a.DPH + base + p, dh8);
+        st8(a.DPL + base + p, dl8);
+    }
+    for (int q = 16; q > 0; q >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, q));
+    if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mx = fmaxf(fmaxf(shm[0], shm[1]), fmaxf(shm[2], shm[3]));
+        atomicMax(reinterpret_cast<unsigned long long*>(a.gridmax) + g,
+                  (unsigned long long)__double_as_longlong((double)mx));
+    }
 }
 
 Shape shape(const SipState& st) {
@@ -1808,6 +1960,59 @@ int sip_tune_outer(Ctx* c, SipState& st, const float* apx, const int* gcls, int*
     return 0;
 }
 
+// ---- on tiles ---------------------------------------------------------------
+static TileArgs<float> tile_args(SipState& st, const int* gcls, const int* ctl, const int* glist) {
+    TileArgs<float> a{};
+    a.s = st.tile->s;
+    a.glist = glist;
+    a.fnbr = st.d_fnbr;
+    a.gcls = gcls;
+    a.H = st.h32;
+    a.RHS = st.rhs32;
+    a.PG = st.pg;
+    a.LAP = st.tlap;
+    a.UNI = st.uni;
+    a.ctl = ctl;
+    a.rev = next_order(st);
+    return a;
+}
+
+static int tile_threads(const SipState& st) { return (st.tile->s.maxt + 31) / 32 * 32 + 32; }
+
+// CTAs a grid of the kernels with one thread a tile
+static int tile_parts(const SipState& st, int threads) { return (st.tile->s.ntile + threads - 1) / threads; }
+
+template <bool kFwd, bool kHz>
+static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
+    const unsigned smem = tile_layout<float>(a.s).bytes;
+    auto go = [&](auto* k) -> int {
+        if (smem > 48 * 1024)
+            MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        k<<<ng, tile_threads(st), smem, s>>>(a);
+        return 0;
+    };
+    if (tile_threads(st) <= 160) {
+        if (ng <= TFEW) return go(k_tile_sweep<float, kFwd, kHz, TDF, 160, 1>);
+        return go(k_tile_sweep<float, kFwd, kHz, TDM, 160, TBM>);
+    }
+    return go(k_tile_sweep<float, kFwd, kHz, 2, 544, 1>);
+}
+
+bool sip_on_tiles(const SipState& st) {
+    return st.tile && st.natural && !st.pre_forced && !st.sweep_forced && !st.outer_forced &&
+           !st.fuse_pre && st.solve_variant < 0;
+}
+
+PosMap sip_posmap(const SipState& st) {
+    if (sip_on_tiles(st)) {
+        const TileShape& s = st.tile->s;
+        return PosMap{s.tpos, s.ni, s.nj, s.nk, s.npp, s.fs, s.NI};
+    }
+    return PosMap{st.d_tpos, st.ni, st.nj, st.nk, st.npp, st.fs, 0};
+}
+
+const int* sip_facepos(const SipState& st) { return sip_on_tiles(st) ? st.tile->s.facepos : st.d_facepos; }
+
 int sip_init(Ctx* c, SipState& st) {
     const DevGrid& G0 = c->grids[0];
     st.kk = G0.kk; st.jj = G0.jj; st.ii = G0.ii;
@@ -1983,6 +2188,14 @@ int sip_init(Ctx* c, SipState& st) {
     MG_CUDA(cudaMalloc(&st.d_rowoff, rowoff.size() * sizeof(short)));
     MG_CUDA(copy_on(c->stream, st.d_rowoff, rowoff.data(), rowoff.size() * sizeof(short),
                        cudaMemcpyHostToDevice));
+    // the tables of the solver on tiles, for the shapes it takes
+    st.tile = new TileDev();
+    if (int rc = tile_init(c, st.ni, st.nj, st.nk, *st.tile)) return rc;
+    if (!st.tile->ok || tile_layout<float>(st.tile->s).bytes > 200 * 1024) {
+        tile_free(*st.tile);
+        delete st.tile;
+        st.tile = nullptr;
+    }
     // face neighbours from the connection table (regular periodic tiling)
     std::vector<int> fn((size_t)6 * c->ngrid, -1);
     for (size_t r = 0; r < c->conns.size(); r += 4) {
@@ -2039,7 +2252,8 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
     const size_t n = (size_t)nclass * st.npp;
     // a second extraction (new classes after the ghost-cell set-up) replaces
     // the records of the first
-    for (void** p : {(void**)&st.swf, (void**)&st.swb, (void**)&st.spr, (void**)&st.uni}) {
+    for (void** p : {(void**)&st.swf, (void**)&st.swb, (void**)&st.spr, (void**)&st.uni, (void**)&st.tcf,
+                     (void**)&st.tcb, (void**)&st.tlap, (void**)&st.tap}) {
         cudaFree(*p);
         *p = nullptr;
     }
@@ -2048,6 +2262,19 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
     MG_CUDA(cudaMalloc(cb, 3 * n * sizeof(float)));
     MG_CUDA(cudaMalloc(apx, 2 * n * sizeof(float)));
     dim3 grid((st.npp + 255) / 256, nclass);
+    if (st.tile) {
+        const TileShape& ts = st.tile->s;
+        const size_t nt = (size_t)nclass * ts.npp * sizeof(float);
+        MG_CUDA(cudaMalloc(&st.tcf, 4 * nt));
+        MG_CUDA(cudaMalloc(&st.tcb, 3 * nt));
+        MG_CUDA(cudaMalloc(&st.tlap, 7 * nt));
+        MG_CUDA(cudaMalloc(&st.tap, 2 * nt));
+        k_tile_extract<<<dim3((ts.npp + 255) / 256, nclass), 256, 0, c->stream>>>(
+            c->d_grids, d_reps, ts, planeorder ? 1 : 0, c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"),
+            c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), st.a1[0], st.a1[1],
+            st.a1[2], st.a1[3], st.a1[4], st.a1[5], st.tbm, st.tcf, st.tcb, st.tlap, st.tap);
+        MG_LAUNCHED(c);
+    }
     k_sip_extract<<<grid, 256, 0, c->stream>>>(
         c->d_grids, d_reps, st.d_qmap, d_idx, st.d_pst, st.nm, st.npp, planeorder ? 1 : 0,
         c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"), c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"),
@@ -2109,8 +2336,13 @@ void sip_release(SipState& st) {
                     (void*)st.d_pcode, (void*)st.spr, (void*)st.uni, (void*)st.a1[0], (void*)st.a1[1],
                     (void*)st.a1[2], (void*)st.a1[3], (void*)st.a1[4], (void*)st.a1[5],
                     (void*)st.a1lo[0], (void*)st.a1lo[1], (void*)st.a1lo[2], (void*)st.a1lo[3],
-                    (void*)st.a1lo[4], (void*)st.a1lo[5], (void*)st.pg, (void*)st.bm, (void*)st.d_bar})
+                    (void*)st.a1lo[4], (void*)st.a1lo[5], (void*)st.pg, (void*)st.bm, (void*)st.d_bar,
+                    (void*)st.tcf, (void*)st.tcb, (void*)st.tlap, (void*)st.tap, (void*)st.tbm})
         cudaFree(p);
+    if (st.tile) {
+        tile_free(*st.tile);
+        delete st.tile;
+    }
 }
 
 int sip_divcal(Ctx* c, SipState& st, const double* fak) {
@@ -2118,7 +2350,7 @@ int sip_divcal(Ctx* c, SipState& st, const double* fak) {
     if (st.natural) {
         dim3 grid((st.npts + 255) / 256, c->ngrid);
         k_sip_divcal_nat<<<grid, 256, 0, c->stream>>>(
-            c->d_grids, st.ni, st.nj, st.nk, st.d_tpos, st.npp, st.rhs32, st.rhsl, c->F("U"),
+            c->d_grids, sip_posmap(st), st.rhs32, st.rhsl, c->F("U"),
             c->F("V"), c->F("W"), c->L("RDDX"), c->L("RDDY"), c->L("RDDZ"), fak,
             c->ibtype == 1 ? c->F("SDIV") : nullptr, c->ibtype == 1 ? c->F("BP") : nullptr);
         MG_LAUNCHED(c);
@@ -2137,6 +2369,30 @@ int sip_divcal(Ctx* c, SipState& st, const double* fak) {
 int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl, int rlow,
                 int rwrite, bool hzero, const int* glist, int nlist, bool skip_pre) {
     const int ng = glist ? nlist : c->ngrid;
+    if (sip_on_tiles(st)) {
+        const TileShape& ts = st.tile->s;
+        {
+            ProfScope ps_(c, "mx_sip_pre");
+            TileArgs<float> a = tile_args(st, gcls, ctl, glist);
+            a.R = st.rs[rwrite];
+            a.LPR = st.tcf + 3 * ts.npp;
+            a.lprcls = 4 * ts.npp;
+            a.hzero = hzero ? 1 : 0;
+            const dim3 grid(tile_parts(st, 128), ng);
+            if (st.unicls) k_tile_pre<float, true, 128, TPB><<<grid, 128, 0, c->stream>>>(a);
+            else k_tile_pre<float, false, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            MG_LAUNCHED(c);
+        }
+        ProfScope ps_(c, "mx_sip_fwd");
+        TileArgs<float> a = tile_args(st, gcls, ctl, glist);
+        a.R = st.rs[rwrite];
+        a.G = rlow >= 0 ? st.rs[rlow] : nullptr;
+        a.CF = st.tcf;
+        a.cfcls = 4 * ts.npp;
+        if (int rc = launch_tile_sweep<true, false>(st, a, ng, c->stream)) return rc;
+        MG_LAUNCHED(c);
+        return 0;
+    }
     if (!skip_pre) {
         ProfScope ps_(c, "mx_sip_pre");
         PreArgs p = pre_args(c, st, cf, gcls, ctl, rwrite, hzero);
@@ -2185,6 +2441,18 @@ int sip_backward(Ctx* c, SipState& st, const float* cb, const int* gcls, int* ct
                  bool hzero, const int* glist, int nlist) {
     ProfScope ps_(c, "mx_sip_bwd");
     const int ng = glist ? nlist : c->ngrid;
+    if (sip_on_tiles(st)) {
+        TileArgs<float> a = tile_args(st, gcls, ctl, glist);
+        a.R = st.rs[rhi];
+        a.G = st.rs[rhi];
+        a.CF = st.tcb;
+        a.cfcls = 3 * st.tile->s.npp;
+        if (int rc = hzero ? launch_tile_sweep<false, true>(st, a, ng, c->stream)
+                           : launch_tile_sweep<false, false>(st, a, ng, c->stream))
+            return rc;
+        MG_LAUNCHED(c);
+        return 0;
+    }
     BwdArgs a{};
     a.s = shape(st);
     a.glist = glist;
@@ -2217,6 +2485,21 @@ int sip_backward(Ctx* c, SipState& st, const float* cb, const int* gcls, int* ct
 int sip_outer(Ctx* c, SipState& st, const float* apx, const int* gcls, const int* ctl,
               float* pre_next) {
     ProfScope ps_(c, "mx_outer");
+    if (sip_on_tiles(st)) {
+        TileOuterArgs a{};
+        a.t = tile_args(st, gcls, ctl, nullptr);
+        a.BM = st.tbm;
+        a.RHS = st.rhs32; a.RHSL = st.rhsl; a.DPH = st.dph; a.DPL = st.dpl; a.APX = st.tap;
+        for (int q = 0; q < 6; ++q) {
+            a.A1[q] = st.a1[q];
+            a.A1L[q] = st.a1lo[q];
+        }
+        a.grids = c->d_grids;
+        a.gridmax = c->d_gridred;
+        k_tile_outer<<<dim3(tile_parts(st, 128), c->ngrid), 128, 0, c->stream>>>(a);
+        MG_LAUNCHED(c);
+        return 0;
+    }
     OuterArgs a{};
     a.s = shape(st);
     a.PG = st.pg;
@@ -2245,6 +2528,13 @@ int sip_bpmask(Ctx* c, SipState& st) {
     dim3 grid((st.npp + 255) / 256, c->ngrid);
     k_sip_bpmask<<<grid, 256, 0, c->stream>>>(c->d_grids, st.npp, st.d_idxp, c->F("BP"), st.bm);
     MG_LAUNCHED(c);
+    if (st.tile) {
+        const TileShape& ts = st.tile->s;
+        if (!st.tbm) MG_CUDA(cudaMalloc(&st.tbm, (size_t)c->ngrid * ts.npp));
+        k_sip_bpmask<<<dim3((ts.npp + 255) / 256, c->ngrid), 256, 0, c->stream>>>(c->d_grids, ts.npp, ts.cell,
+                                                                                  c->F("BP"), st.tbm);
+        MG_LAUNCHED(c);
+    }
     return 0;
 }
 
@@ -2252,8 +2542,8 @@ int sip_scatter_dp(Ctx* c, SipState& st) {
     ProfScope ps_(c, "mx_scatter");
     if (st.natural) {
         dim3 grid((st.npts + 255) / 256, c->ngrid);
-        k_sip_scatter_nat<<<grid, 256, 0, c->stream>>>(c->d_grids, st.ni, st.nj, st.nk, st.d_tpos,
-                                                       st.npp, st.dph, st.dpl, c->F("DP"));
+        k_sip_scatter_nat<<<grid, 256, 0, c->stream>>>(c->d_grids, sip_posmap(st), st.dph, st.dpl,
+                                                       c->F("DP"));
         MG_LAUNCHED(c);
         return 0;
     }
@@ -2264,10 +2554,11 @@ int sip_scatter_dp(Ctx* c, SipState& st) {
     return 0;
 }
 
-int sip_conv(Ctx* c, int* ctl, double* maxrhs, const double* sprm) {
+int sip_conv(Ctx* c, const SipState& st, int* ctl, double* maxrhs, const double* sprm) {
     ProfScope ps_(c, "mx_conv");
     k_mx_conv<<<1, 1024, 0, c->stream>>>(c->d_grids, c->ngrid, c->maxlevel, c->d_gridred, ctl,
-                                         maxrhs, sprm, c->prm.epcorr, c->prm.nouter_min);
+                                         maxrhs, sprm, c->prm.epcorr, c->prm.nouter_min,
+                                         sip_on_tiles(st) ? 1 : 0);
     MG_LAUNCHED(c);
     return 0;
 }

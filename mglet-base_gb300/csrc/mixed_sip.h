@@ -5,6 +5,8 @@
 
 namespace mg {
 
+struct TileDev;   // sip_tile.cuh
+
 struct SipState {
     int kk = 0, jj = 0, ii = 0, ni = 0, nj = 0, nk = 0, npts = 0, fs = 0;
     int nm = 0;                 // hyperplanes per grid
@@ -36,6 +38,13 @@ struct SipState {
     int* d_wb = nullptr;
     float4* swf = nullptr;      // [ncls][npp]
     float4* swb = nullptr;
+    // grids of even dimensions: the solver on 2x2x2 tiles (sip_tile.cuh): tables,
+    // and per class {lw, ls, lb, lpr}, {ue, un, ut}, the seven operator
+    // coefficients and ap in two floats, npp values each; tbm the open couplings of
+    // the ghost-cell IB
+    TileDev* tile = nullptr;
+    float *tcf = nullptr, *tcb = nullptr, *tlap = nullptr, *tap = nullptr;
+    unsigned char* tbm = nullptr;
     // packed pre-pass (npp + 6 fs < 32768): neighbour codes [npp][3] and per
     // class the records [ncls][3][npp]
     bool prepk = false;
@@ -49,6 +58,8 @@ struct SipState {
     // launch variant of the pre-pass (index into the variant table), picked by
     // the tuner or forced by the caller; -1 = default
     int pre_variant = -1;
+    // a plane-order variant was forced: the solve runs in the cell hyperplane order
+    bool pre_forced = false, sweep_forced = false, outer_forced = false;
     double pre_ms = 0.0;        // its measured time per launch (tuner)
     // launch variant of the packed sweeps (points per thread, CTAs per SM),
     // -1 = default; the tuner's time of one forward + backward pair
@@ -86,6 +97,26 @@ struct SipState {
     float* a1lo[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}; // FP32 of the remainders
 };
 
+// The layout of the solver's arrays (hilf, res, rhs, dp): on tiles, unless the
+// shape or a forced variant asks for the cell hyperplane order.  The arrays are
+// written and read within one pressure solve, so the layout may change between
+// solves.
+bool sip_on_tiles(const SipState& st);
+// position of a cell in the layout in use
+struct PosMap {
+    const int* tpos;            // [planes][ni or NI], see mixed_sip.cu and sip_tile.cuh
+    int ni, nj, nk, npp, fs;
+    int NI;                     // tiles along i; 0: the cell hyperplane order
+    __device__ __forceinline__ int pos(int io, int jo, int ko) const {
+        if (NI) {
+            const int I = io >> 1, J = jo >> 1, K = ko >> 1;
+            return ((tpos[(I + J + K) * NI + I] + J) << 3) | ((io & 1) << 2) | ((jo & 1) << 1) | (ko & 1);
+        }
+        return tpos[(io + jo + ko) * ni + io] + jo;
+    }
+};
+PosMap sip_posmap(const SipState& st);
+const int* sip_facepos(const SipState& st);
 int sip_init(Ctx* c, SipState& st);
 // Class coefficients: FP32 blocks [lw|ls|lb|lpr|ap] and [ue|un|ut] per padded
 // plane, and ap split in two floats [hi npp | lo npp], from the representative
@@ -122,7 +153,7 @@ const char* sip_sweep_variant_name(int v);
 int sip_outer_variants();
 const char* sip_outer_variant_name(int v);
 // maxabscal over the grids and the outer-loop stopping test (one CTA)
-int sip_conv(Ctx* c, int* ctl, double* maxrhs, const double* sprm);
+int sip_conv(Ctx* c, const SipState& st, int* ctl, double* maxrhs, const double* sprm);
 // The persistent solve: every inner iteration, outer step and stopping test
 // of one single-level mgpoisl in one cooperative launch, the same bits as the
 // per-phase kernels.  fits: variant v can run on this case (one level, the
