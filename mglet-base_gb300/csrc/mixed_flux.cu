@@ -874,8 +874,8 @@ static int encode_plane_map(Ctx* c, const double* base, CUtensorMap* m) {
 
 // Checks the launch limits of the flux kernel for this grid shape and opts
 // in to the dynamic shared memory it needs; where a grid's k x j interior
-// fits one CTA and its planes meet the TMA rules (16-byte rows, boxes of at
-// most 256 points per side), also builds the TMA variant's tensor maps.
+// fits one CTA and its planes meet the TMA rules (16-byte rows, whole 128-byte
+// lines, boxes of at most 256 points per side), also builds the TMA variant's tensor maps.
 int mx_flux_prepare(Ctx* c) {
     const DevGrid& G0 = c->grids[0];
     if (G0.kk - 4 > 576) {
@@ -894,7 +894,10 @@ int mx_flux_prepare(Ctx* c) {
     for (const DevGrid& g : c->grids)
         for (int f = 0; f < 6; ++f) fs.walls |= g.bc[f] != MGLET_BC_CON;
     const size_t tsm = flux_tma_smem(G0);
-    if (flux_slabs(G0) == 1 && (G0.kk * sizeof(double)) % 16 == 0 && G0.kk <= 256 &&
+    // the four planes of a staging slot follow each other in shared memory, and a
+    // tensor copy's destination has to start on a 128-byte line there
+    const bool lines = ((size_t)G0.kk * G0.jj * sizeof(double)) % 128 == 0;
+    if (flux_slabs(G0) == 1 && lines && (G0.kk * sizeof(double)) % 16 == 0 && G0.kk <= 256 &&
         G0.jj <= 256 && tsm <= 113 * 1024) {
         const char* names[4] = {"U", "V", "W", "P"};
         for (int f = 0; f < 4; ++f)
