@@ -50,24 +50,11 @@
 namespace mg {
 namespace {
 
-#ifndef TFEW
-#define TFEW 304
-#endif
-#ifndef TDF
-#define TDF 3
-#endif
-#ifndef TDM
-#define TDM 2
-#endif
-#ifndef TBM
-#define TBM 4
-#endif
-#ifndef TPB
-#define TPB 5
-#endif
-#ifndef TOB
-#define TOB 4
-#endif
+// Up to this many grids -- two CTAs of the ping-pong sweep on each of the 152 SMs
+// -- a sweep is bound by the chain of its steps and that form runs: 9.5 us for 8
+// grids of 24^3 against 12 us, but 46 against 29 us for 512 grids, whose CTAs
+// already fill each other's waits.
+constexpr int kTileFew = 304;
 constexpr int kMaxCols = 1024; // longest hyperplane (points)
 // A wait gives up after this many SM clock cycles (about one second); a
 // healthy wait lasts microseconds.
@@ -1436,7 +1423,7 @@ struct TileOuterArgs {
 // accumulate_pcorr, see k_sip_outer): one thread a tile, the tiles of a grid in
 // gridDim.x CTAs; gridmax takes the maximum over them (a maximum of non-negative
 // numbers, as integers).
-__global__ void __launch_bounds__(128, TOB) k_tile_outer(const __grid_constant__ TileOuterArgs a) {
+__global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ TileOuterArgs a) {
     if (a.t.ctl[0]) return;
     __shared__ float shm[4];
     const TileShape& s = a.t.s;
@@ -1991,10 +1978,17 @@ static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int n
         k<<<ng, tile_threads(st), smem, s>>>(a);
         return 0;
     };
-    if (tile_threads(st) <= 160) {
-        if (ng <= TFEW) return go(k_tile_sweep<float, kFwd, kHz, TDF, 160, 1>);
-        return go(k_tile_sweep<float, kFwd, kHz, TDM, 160, TBM>);
+    if (ng <= kTileFew) {
+        auto few = [&](auto* k) -> int {
+            if (smem > 48 * 1024)
+                MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            k<<<ng, 2 * tile_threads(st) - 32, smem, s>>>(a);
+            return 0;
+        };
+        if (tile_threads(st) <= 160) return few(k_tile_sweep_few<float, kFwd, kHz, 2, 288>);
+        if (tile_threads(st) <= 288) return few(k_tile_sweep_few<float, kFwd, kHz, 1, 544>);
     }
+    if (tile_threads(st) <= 160) return go(k_tile_sweep<float, kFwd, kHz, 2, 160, 4>);
     return go(k_tile_sweep<float, kFwd, kHz, 2, 544, 1>);
 }
 
@@ -2379,8 +2373,9 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
             a.lprcls = 4 * ts.npp;
             a.hzero = hzero ? 1 : 0;
             const dim3 grid(tile_parts(st, 128), ng);
-            if (st.unicls) k_tile_pre<float, true, 128, TPB><<<grid, 128, 0, c->stream>>>(a);
-            else k_tile_pre<float, false, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            if (st.unicls) k_tile_pre<float, true, 0, 128, 5><<<grid, 128, 0, c->stream>>>(a);
+            else if (st.prepk) k_tile_pre<float, false, 0, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            else k_tile_pre<float, false, 1, 128, 4><<<grid, 128, 0, c->stream>>>(a);
             MG_LAUNCHED(c);
         }
         ProfScope ps_(c, "mx_sip_fwd");

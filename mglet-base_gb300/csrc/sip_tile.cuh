@@ -36,7 +36,7 @@ struct TileShape {
     int w, slots;                   // NJ + 1; (NI + 1)(NJ + 1)
     int nside;                      // ghost tiles on the three low (or high) faces
     const int* tst;                 // [NT+1] first tile of each hyperplane
-    const unsigned short* slot;     // [ntile] slot of the tile
+    const unsigned short* slot;     // [ntile, padded to 4] slot of the tile
     // [ntile][2]: tiles at i-1, i+1, j-1, j+1 | k-1, k+1, cell (io, jo, ko) of the
     // tile's first cell (10 bits each), 0; a negative entry -1-t is tile t of the
     // grid across that face
@@ -127,6 +127,19 @@ __device__ __forceinline__ void st8(double* a, const Vec8<double>& r) {
         : "memory");
 }
 
+// a += r: one writer per value, so the reduction (round to nearest) is the plain
+// sum without a load
+__device__ __forceinline__ void add8(float* a, const Vec8<float>& r) {
+    asm volatile(
+        "red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n red.global.add.v4.f32 [%0 + 16], {%5, %6, %7, %8};" ::"l"(a),
+        "f"(r.v[0]), "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]), "f"(r.v[7])
+        : "memory");
+}
+__device__ __forceinline__ void add8(double* a, const Vec8<double>& r) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) atomicAdd(a + i, r.v[i]);
+}
+
 // The quad of a tile that faces its neighbour: on axis 0, 1, 2 the cells with
 // offset hi along that axis; in the order of the other two offsets.
 template <int kAxis, int kHi, typename T>
@@ -182,11 +195,30 @@ __host__ __device__ inline TileLayout tile_layout(const TileShape& s) {
 }
 
 // A tile's loads of one step
-template <typename T, bool kH>
+template <typename T>
 struct TileSet {
     int tile, x;                    // tile (-1: none) and slot
-    Vec8<T> c[3], v, h[kH ? 1 : 1];
+    Vec8<T> c[3], v;
 };
+
+// The predecessor recurrence of a tile's 8 cells (see k_tile_sweep)
+template <bool kFwd, typename T>
+__device__ __forceinline__ Vec8<T> tile_solve(const Vec8<T>& v, const Vec8<T>& ci, const Vec8<T>& cj,
+                                              const Vec8<T>& ck, const Vec4<T>& fi, const Vec4<T>& fj,
+                                              const Vec4<T>& fk) {
+    Vec8<T> r;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int i = kFwd ? m : 7 - m;          // di dj dk
+        const int di = i >> 2, dj = (i >> 1) & 1, dk = i & 1;
+        constexpr int in = kFwd ? 1 : 0;         // offset of a cell whose predecessor is in the tile
+        const T rk = dk == in ? r.v[i ^ 1] : fk.v[2 * di + dj];
+        const T rj = dj == in ? r.v[i ^ 2] : fj.v[2 * di + dk];
+        const T ri = di == in ? r.v[i ^ 4] : fi.v[2 * dj + dk];
+        r.v[i] = v.v[i] - ck.v[i] * rk - cj.v[i] * rj - ci.v[i] * ri;
+    }
+    return r;
+}
 
 // One sweep of a grid.  kFwd: tile hyperplanes in order, res = v - lb res(k-1) -
 // ls res(j-1) - lw res(i-1) (sip_hyperplane_mod.F90:491-495); else in reverse,
@@ -265,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
         }
         return;
     }
-    using Set = TileSet<T, !kFwd && !kHz>;
+    using Set = TileSet<T>;
     auto fetch = [&](int t, Set& q) {
         const int ta = tst[t], tb = tst[t + 1];
         const int tile = (kFwd ? ta : tb) + tid;
@@ -278,7 +310,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
         ld8(on, C + 2 * s.npp + p, q.c[2]);
         if constexpr (kFwd) ld8_rw(on, R + p, q.v);
         else ld8(on, R + p, q.v);
-        if constexpr (!kFwd && !kHz) ld8_rw(on, H + p, q.h[0]);
     };
     Set q[kD];
 #pragma unroll
@@ -289,17 +320,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
             Vec4<T>* cur = face + (t & 1) * 3 * s.slots + c.x;
             const Vec4<T>* prv = face + ((t + 1) & 1) * 3 * s.slots + c.x;
             const Vec4<T> fi = prv[W], fj = prv[s.slots + one], fk = prv[2 * s.slots];
-            Vec8<T> r;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) {
-                const int i = kFwd ? m : 7 - m;          // di dj dk
-                const int di = i >> 2, dj = (i >> 1) & 1, dk = i & 1;
-                constexpr int in = kFwd ? 1 : 0;         // offset of a cell whose predecessor is in the tile
-                const T rk = dk == in ? r.v[i ^ 1] : fk.v[2 * di + dj];
-                const T rj = dj == in ? r.v[i ^ 2] : fj.v[2 * di + dk];
-                const T ri = di == in ? r.v[i ^ 4] : fi.v[2 * dj + dk];
-                r.v[i] = c.v.v[i] - c.c[2].v[i] * rk - c.c[1].v[i] * rj - c.c[0].v[i] * ri;
-            }
+            const Vec8<T> r = tile_solve<kFwd>(c.v, c.c[0], c.c[1], c.c[2], fi, fj, fk);
             constexpr int out = kFwd ? 1 : 0;
             cur[0] = quad<0, out>(r);
             cur[s.slots] = quad<1, out>(r);
@@ -309,10 +330,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
             } else if constexpr (kHz) {
                 st8(H + 8 * c.tile, r);
             } else {
-                Vec8<T> h;
-#pragma unroll
-                for (int m = 0; m < 8; ++m) h.v[m] = c.h[0].v[m] + r.v[m];
-                st8(H + 8 * c.tile, h);
+                add8(H + 8 * c.tile, r);
             }
         }
         fetch(t + kD, c);
@@ -323,6 +341,145 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
         for (int d = 0; d < kD; ++d) {
             if (t + d >= NT) break;
             step(t + d, q[d]);
+        }
+    }
+}
+
+// The sweep of few grids (at most two on an SM), where nothing else runs while a
+// step waits: the time is the chain of one warp's instructions through all
+// steps.  Two sets of warps take the steps in turn, so that the chain of a step is
+// three face loads, the recurrence and three face stores; a set stores its results
+// and issues its next loads while the other set works.  The tables, the ghosts and
+// the first tiles are loaded at once.
+template <typename T, bool kFwd, bool kHz, int kD, int kThreads>
+__global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_constant__ TileArgs<T> a) {
+    extern __shared__ __align__(32) unsigned char tsm[];
+    const TileShape& s = a.s;
+    const int b = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const int g = a.glist ? a.glist[b] : b;
+    const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT;
+    const int set = tid >= ncomp ? 1 : 0, lane = tid - set * ncomp;   // (the last warp: neither)
+    const int W = kFwd ? -s.w : s.w, one = kFwd ? -1 : 1, back = kFwd ? 0 : s.w + 1;
+    const TileLayout l = tile_layout<T>(s);
+    int *tst = reinterpret_cast<int*>(tsm), *gst = reinterpret_cast<int*>(tsm + l.gst),
+        *gent = reinterpret_cast<int*>(tsm + l.gent);
+    Vec4<T>*gval = reinterpret_cast<Vec4<T>*>(tsm + l.gval), *face = reinterpret_cast<Vec4<T>*>(tsm + l.face);
+    const long long base = (long long)g * s.npp;
+    const T* C = a.CF + (long long)a.gcls[g] * a.cfcls;
+    T* R = a.R + base;
+    T* H = a.H + base;
+    constexpr int side = kFwd ? 0 : 1;
+    const int converged = __ldg(a.ctl);
+    TileSet<T> q[kD];
+    // the loads of a step whose tiles are t0 .. t1
+    auto fetch = [&](TileSet<T>& c, int t0, int t1) {
+        const int tile = t0 + lane;
+        const bool on = tile < t1;
+        c.tile = on ? tile : -1;
+        const int p = 8 * tile;
+        if (on) c.x = (int)__ldg(s.slot + tile) - back;
+        ld8(on, C + p, c.c[0]);
+        ld8(on, C + s.npp + p, c.c[1]);
+        ld8(on, C + 2 * s.npp + p, c.c[2]);
+        if constexpr (kFwd) ld8_rw(on, R + p, c.v);
+        else ld8(on, R + p, c.v);
+    };
+    // first tile of step t's hyperplane and the one past its last, from global memory
+    auto first = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t : NT - 1 - t)) : 0; };
+    auto past = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t + 1 : NT - t)) : 0; };
+    constexpr int kU = 4;
+    int nb[3];
+    for (int d = 0; d < 3; ++d) nb[d] = a.G ? a.fnbr[6 * g + 2 * d + side] : -1;
+    int2 e[kU];
+#pragma unroll
+    for (int i = 0; i < kU; ++i)
+        e[i] = __ldg(s.gent[side] + min(tid + i * (int)blockDim.x, s.nside - 1));
+    if (tid < 2 * ncomp)
+#pragma unroll
+        for (int d = 0; d < kD; ++d) fetch(q[d], first(set + 2 * d), past(set + 2 * d));
+    for (int t = tid; t < NT + 1 + kTilePad; t += blockDim.x) {
+        // step t covers tiles tst[t] .. tst[t+1] forward, tst[t+1] .. tst[t] backward
+        tst[t] = t <= NT ? s.tst[kFwd ? t : NT - t] : (kFwd ? s.ntile : 0);
+        if (t < NT + 3) gst[t] = s.gst[side][t];
+    }
+    // the ghosts: the facing quads of the grids across
+    for (int q0 = tid; q0 < s.nside; q0 += kU * blockDim.x) {
+        Vec8<T> v[kU];
+#pragma unroll
+        for (int i = 0; i < kU; ++i) {
+            const int d = e[i].x >> 16, n = d == 0 ? nb[0] : (d == 1 ? nb[1] : nb[2]);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[i].v[m] = T(0);
+            ld8(n >= 0, a.G + ((long long)max(n, 0) * s.npp + 8 * e[i].y), v[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kU; ++i) {
+            const int m = q0 + i * (int)blockDim.x;
+            if (m < s.nside) {
+                const int d = e[i].x >> 16;
+                constexpr int hi = kFwd ? 1 : 0;   // the neighbour's high cells are my low ghosts
+                gval[m] = d == 0 ? quad<0, hi>(v[i]) : (d == 1 ? quad<1, hi>(v[i]) : quad<2, hi>(v[i]));
+                gent[m] = e[i].x;
+            }
+            e[i] = __ldg(s.gent[side] + min(m + kU * (int)blockDim.x, s.nside - 1));
+        }
+    }
+    if (converged) return;
+    __syncthreads();
+    const int steps = (NT + 1) & ~1;
+    if (tid >= 2 * ncomp) {
+        // the ghosts of step t (-1: those before the first) into their faces
+        auto ghosts = [&](int t) {
+            Vec4<T>* f = face + (t & 1) * 3 * s.slots;
+            const int p = kFwd ? t : NT - 1 - t;
+            const int g0 = gst[p + 1], n = gst[p + 2];
+            for (int m = g0 + (tid & 31); m < n; m += 32)
+                f[(gent[m] >> 16) * s.slots + (gent[m] & 0xffff)] = gval[m];
+        };
+        ghosts(-1);
+        __syncthreads();
+        for (int t = 0; t < steps; ++t) {
+            if (t < NT) ghosts(t);
+            __syncthreads();
+        }
+        return;
+    }
+    __syncthreads();
+    // step t of this set
+    auto work = [&](int t, TileSet<T>& c, Vec8<T>& r) {
+        if (c.tile >= 0) {
+            Vec4<T>* cur = face + (t & 1) * 3 * s.slots + c.x;
+            const Vec4<T>* prv = face + ((t + 1) & 1) * 3 * s.slots + c.x;
+            r = tile_solve<kFwd>(c.v, c.c[0], c.c[1], c.c[2], prv[W], prv[s.slots + one], prv[2 * s.slots]);
+            constexpr int out = kFwd ? 1 : 0;
+            cur[0] = quad<0, out>(r);
+            cur[s.slots] = quad<1, out>(r);
+            cur[2 * s.slots] = quad<2, out>(r);
+        }
+    };
+    // while the other set works: the results of step t to memory, the loads of the
+    // step kD turns on
+    auto rest = [&](int t, TileSet<T>& c, const Vec8<T>& r) {
+        if (c.tile >= 0) {
+            if constexpr (kFwd) st8(R + 8 * c.tile, r);
+            else if constexpr (kHz) st8(H + 8 * c.tile, r);
+            else add8(H + 8 * c.tile, r);
+        }
+        const int n = min(t + 2 * kD, NT + 1);
+        const int ta = tst[n], tb = tst[n + 1];
+        fetch(c, kFwd ? ta : tb, kFwd ? tb : ta);
+    };
+    Vec8<T> r;
+    if (set) __syncthreads();   // step 0
+    for (int t = set; t < steps; t += 2 * kD) {
+#pragma unroll
+        for (int d = 0; d < kD; ++d) {
+            const int m = t + 2 * d;
+            if (m >= steps) break;
+            work(m, q[d], r);
+            __syncthreads();
+            rest(m, q[d], r);
+            if (m + 1 < steps) __syncthreads();   // the other set's step
         }
     }
 }
@@ -395,8 +552,10 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<T>& o, int i, T n[6]) {
 // The part of sipiter1 outside the recurrence, (rhs + laplacephi(hilf)) lpr
 // (sip_hyperplane_mod.F90:491, laplacephi_mod.F90:153-160), one thread a tile;
 // the tiles of a grid in gridDim.x CTAs.  kUni: one value of each operator
-// coefficient a class.
-template <typename T, bool kUni, int kThreads, int kMinBlocks>
+// coefficient a class.  Of the first two products one rounds by itself and the
+// other is contracted with it: the first in kOrder 0, the second in kOrder 1, as the
+// compiler does it in the packed and in the table-driven cell pre-pass.
+template <typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_constant__ TileArgs<T> a) {
     if (a.ctl[0]) return;
     const TileShape& s = a.s;
@@ -428,13 +587,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
             for (int i = 0; i < 8; ++i) {
                 T n[6];
                 tile_nbrs(o, i, n);
-                T lap;
-                if constexpr (kUni)
-                    lap = -u[0] * n[0] - u[1] * n[1] - u[2] * n[2] - u[3] * n[3] - u[4] * n[4] -
-                          u[5] * n[5] - u[6] * o.h.v[i];
-                else
-                    lap = -c[0].v[i] * n[0] - c[1].v[i] * n[1] - c[2].v[i] * n[2] - c[3].v[i] * n[3] -
-                          c[4].v[i] * n[4] - c[5].v[i] * n[5] - c[6].v[i] * o.h.v[i];
+                T w[7];
+#pragma unroll
+                for (int f = 0; f < 7; ++f) w[f] = kUni ? u[f] : c[kUni ? 0 : f].v[i];
+                T lap = mul_rounded(-w[kOrder], n[kOrder]);
+                lap = lap - w[1 - kOrder] * n[1 - kOrder] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] -
+                      w[5] * n[5] - w[6] * o.h.v[i];
                 out.v[i] = mul_rounded(rh.v[i] + lap, lp.v[i]);
             }
         }
@@ -469,7 +627,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, TileDev& d) {
     s.slots = (NI + 1) * (NJ + 1);
     s.nside = NI * NJ + NI * NK + NJ * NK;
     std::vector<int> tst(s.NT + 1, 0), tpos((size_t)s.NT * NI, 0);
-    std::vector<unsigned short> slot(s.ntile);
+    std::vector<unsigned short> slot((s.ntile + 3) & ~3, 0);
     std::vector<int> ti(s.ntile), tj(s.ntile), tk(s.ntile);
     for (int t = 0, p = 0; t < s.NT; ++t) {
         for (int I = 0; I < NI; ++I) {

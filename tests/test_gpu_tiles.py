@@ -1,0 +1,61 @@
+"""The pressure solver on 2x2x2 tiles (the default for grids of even dimensions)
+against the same solver in the cell hyperplane order (forced by a sweep
+variant): the same bits on every shape, at the edges of the tile hyperplanes, with
+few and many grids, walls on graded grids and a hierarchy."""
+import numpy as np
+import pytest
+
+from mglet_gb300 import abi, cases
+from test_oracle_levels import prepare_levels
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(gpu_lib, case, plane_order, nouter=3):
+    prm = abi.make_flow_params(gmol=1e-3, epcorr=1e-10, nouter=nouter, ninner=3, form=abi.FORM_MIXED)
+    g = gpu_lib.Solver(case, prm)
+    if plane_order:
+        g.force_variant("mx_sip_sweep", 0)
+    u, v, w, p = cases.taylor_green(case)
+    u, v, w = cases.add_noise(case, (u, v, w), amplitude=1e-2, seed=5)
+    for nm, a in zip("UVWP", (u, v, w, p)):
+        g.set(nm, a)
+    if case.iparent is not None:
+        g.set_hierarchy(case.iparent, case.position)
+        for lvl in (1, 2):
+            g.connect(lvl, 2, v1="U", v2="V", v3="W", s1="P", corners=True)
+        prepare_levels(g, case)
+    else:
+        g.connect(0, 2, "U", "V", "W", "P", corners=True)
+    rk = gpu_lib.rk_scheme("williamson")
+    st = [g.timeintegrate_flow(1, 1, 0.0, 5e-4, irk, rk) for irk in (1, 2, 3)]
+    out = [g.get(nm) for nm in ("U", "V", "W", "P", "DP")]
+    g.close()
+    return [(s.nouter_done, s.maxrhs) for s in st], out
+
+
+def _same(gpu_lib, case):
+    (sa, a), (sb, b) = _run(gpu_lib, case, False), _run(gpu_lib, case, True)
+    assert sa == sb
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+
+
+# the smallest tile grid, one tile wide in each direction, hyperplanes of one to
+# three warps, shapes beyond the packed cell tables, two sets of warps and one
+@pytest.mark.parametrize("tiles,shape", [
+    ((2, 1, 1), (2, 2, 2)), ((1, 2, 2), (2, 16, 6)), ((2, 1, 2), (12, 2, 8)), ((2, 2, 1), (6, 10, 2)),
+    ((2, 2, 2), (24, 24, 24)), ((1, 2, 1), (32, 28, 36)), ((7, 7, 7), (8, 10, 12)),
+    ((8, 7, 6), (20, 24, 16))])
+def test_tiles_match_the_cell_order(gpu_lib, tiles, shape):
+    ni, nj, nk = shape
+    _same(gpu_lib, cases.periodic_box(*tiles, n=ni, nj=nj, nk=nk))
+
+
+def test_tiles_match_with_walls_on_graded_grids(gpu_lib):
+    walls = {1: abi.BC_FIX, 2: abi.BC_OP1, 3: abi.BC_NOS, 4: abi.BC_SLI}
+    _same(gpu_lib, cases.stretch(cases.periodic_box(3, 2, 2, n=10, length=(2.0, 2.0, 1.0), walls=walls)))
+
+
+def test_tiles_match_on_a_hierarchy(gpu_lib):
+    _same(gpu_lib, cases.refined_box(2, 2, 2, n=8, refine=(1,)))
