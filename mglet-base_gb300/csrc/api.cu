@@ -19,6 +19,7 @@
 
 #include "internal.h"
 #include "mixed.h"
+#include "plain_tile.h"
 
 namespace mg {
 
@@ -365,7 +366,8 @@ int solve_pressure_system(Ctx* c, double prefak, mglet_stage_stats* st, bool zer
     const size_t bytes = (size_t)c->idim3d * sizeof(double);
     if (zero_work)
         for (double* a : {dp, hilf, res}) MG_CUDA(cudaMemsetAsync(a, 0, bytes, c->stream));
-    if (int rc = launch_bp_ones(c)) return rc;
+    if (!plain_tile_ready(c))
+        if (int rc = launch_bp_ones(c)) return rc;
     if (prefak <= 0.0) {
         if (int rc = MG_PLAIN_FN(c, launch_rescal_maxabs)(c, rhs, nullptr)) return rc;
         MG_CUDA(cudaMemcpyAsync(c->h_scalar, c->d_scalar, sizeof(double), cudaMemcpyDeviceToHost,
@@ -378,6 +380,7 @@ int solve_pressure_system(Ctx* c, double prefak, mglet_stage_stats* st, bool zer
             return 0;
         }
     }
+    if (plain_tile_ready(c)) return MG_PLAIN_FN(c, plain_tile_solve)(c, prefak, st);
     const bool multi = c->minlevel != c->maxlevel;
     const char* const none[3] = {nullptr, nullptr, nullptr};
     const char* const shilf[3] = {"HILF", nullptr, nullptr};
@@ -768,6 +771,7 @@ int mglet_gpu_create(const mglet_grid_desc* d, const mglet_flow_params* prm, int
     }
     if (prm->form == MGLET_FORM_MIXED)
         if (int rc2 = mixed_init(c)) return bail(rc2);
+    if (int rc2 = plain_tile_init(c, d)) return bail(rc2);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return bail(cuda_fail(e, "create"));
     *out = c;
@@ -785,6 +789,7 @@ int mglet_gpu_destroy(mglet_ctx* c) {
             cudaEventDestroy(ev.second);
         }
     mixed_release(c);
+    plain_tile_release(c);
     release_tables(c);
     contract::release_tables(c);
     for (auto& kv : c->f3) cudaFree(kv.second);
@@ -840,6 +845,9 @@ int mglet_gpu_set_field(mglet_ctx* c, const char* name, const double* host, int6
     MG_CUDA(cudaMemcpyAsync(p, host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     MG_CUDA(cudaStreamSynchronize(c->stream));
     if (std::strcmp(name, "G") == 0) c->g_user = true;
+    // the solve on tiles keeps copies of these
+    if (!std::strcmp(name, "BP") || !std::strcmp(name, "GSAP") || !std::strncmp(name, "SIP", 3))
+        c->coef_user = true;
     if (c->prm.form == MGLET_FORM_MIXED) mixed_field_changed(c, name);
     return 0;
 }

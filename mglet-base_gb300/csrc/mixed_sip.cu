@@ -1372,6 +1372,8 @@ __global__ void k_sip_extract(const DevGrid* __restrict__ grids, const int* __re
 }
 
 // ---- on tiles ---------------------------------------------------------------
+using T8 = Tile<2, 2, 2>;
+
 // class coefficients on tiles from the FP64 fields of the representative grids:
 // {lw, ls, lb, lpr}, {ue, un, ut}, the operator's seven (with the couplings BP
 // closes masked) and ap as two floats
@@ -1435,17 +1437,17 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
     float mx = 0.f;
     for (int tile = blockIdx.x * 128 + threadIdx.x; tile < s.ntile; tile += gridDim.x * 128) {
         const int p = 8 * tile;
-        TileHalo<float> o;
+        TileHalo<T8, float> o;
         tile_halo(a.t, g, tile, o);
         const int org = __ldg(s.nbr + 2 * tile + 1).z;
         const int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
-        Vec8<float> aph, apl, rh8, rl8, dh8, dl8;
-        ld8(true, APX + p, aph);
-        ld8(true, APX + s.npp + p, apl);
-        ld8_rw(true, a.RHS + base + p, rh8);
-        ld8_rw(true, a.RHSL + base + p, rl8);
-        ld8_rw(true, a.DPH + base + p, dh8);
-        ld8_rw(true, a.DPL + base + p, dl8);
+        Vec<float, 8> aph, apl, rh8, rl8, dh8, dl8;
+        ldt(true, APX + p, aph);
+        ldt(true, APX + s.npp + p, apl);
+        ldt_rw(true, a.RHS + base + p, rh8);
+        ldt_rw(true, a.RHSL + base + p, rl8);
+        ldt_rw(true, a.DPH + base + p, dh8);
+        ldt_rw(true, a.DPL + base + p, dl8);
         uint2 bm = make_uint2(0x3f3f3f3fu, 0x3f3f3f3fu);
         if (a.BM) bm = *reinterpret_cast<const uint2*>(a.BM + base + p);
         float ch[6][2], cl[6][2];
@@ -1461,7 +1463,7 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             float n[6];
-            tile_nbrs(o, i, n);
+            tile_nbrs<T8>(o, i, n);
             const unsigned mk = ((i < 4 ? bm.x : bm.y) >> (8 * (i & 3))) & 0xffu;
             const int d[3] = {i >> 2, (i >> 1) & 1, i & 1};
             float sum = 0.f, comp = 0.f;
@@ -1490,10 +1492,10 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
             dl8.v[i] = dl;
             mx = fmaxf(mx, fabsf(rh));
         }
-        st8(a.RHS + base + p, rh8);
-        st8(a.RHSL + base + p, rl8);
-        st8(a.DPH + base + p, dh8);
-        st8(a.DPL + base + p, dl8);
+        stt(a.RHS + base + p, rh8);
+        stt(a.RHSL + base + p, rl8);
+        stt(a.DPH + base + p, dh8);
+        stt(a.DPL + base + p, dl8);
     }
     for (int q = 16; q > 0; q >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, q));
     if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
@@ -1971,7 +1973,7 @@ static int tile_parts(const SipState& st, int threads) { return (st.tile->s.ntil
 
 template <bool kFwd, bool kHz>
 static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
-    const unsigned smem = tile_layout<float>(a.s).bytes;
+    const unsigned smem = tile_layout<T8, float>(a.s).bytes;
     auto go = [&](auto* k) -> int {
         if (smem > 48 * 1024)
             MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1985,11 +1987,11 @@ static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int n
             k<<<ng, 2 * tile_threads(st) - 32, smem, s>>>(a);
             return 0;
         };
-        if (tile_threads(st) <= 160) return few(k_tile_sweep_few<float, kFwd, kHz, 2, 288>);
-        if (tile_threads(st) <= 288) return few(k_tile_sweep_few<float, kFwd, kHz, 1, 544>);
+        if (tile_threads(st) <= 160) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 2, 288>);
+        if (tile_threads(st) <= 288) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 1, 544>);
     }
-    if (tile_threads(st) <= 160) return go(k_tile_sweep<float, kFwd, kHz, 2, 160, 4>);
-    return go(k_tile_sweep<float, kFwd, kHz, 2, 544, 1>);
+    if (tile_threads(st) <= 160) return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 160, 4>);
+    return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 544, 1>);
 }
 
 bool sip_on_tiles(const SipState& st) {
@@ -2184,8 +2186,8 @@ int sip_init(Ctx* c, SipState& st) {
                        cudaMemcpyHostToDevice));
     // the tables of the solver on tiles, for the shapes it takes
     st.tile = new TileDev();
-    if (int rc = tile_init(c, st.ni, st.nj, st.nk, *st.tile)) return rc;
-    if (!st.tile->ok || tile_layout<float>(st.tile->s).bytes > 200 * 1024) {
+    if (int rc = tile_init(c, st.ni, st.nj, st.nk, 1, 1, 1, 512, *st.tile)) return rc;
+    if (!st.tile->ok || tile_layout<T8, float>(st.tile->s).bytes > 200 * 1024) {
         tile_free(*st.tile);
         delete st.tile;
         st.tile = nullptr;
@@ -2373,9 +2375,9 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
             a.lprcls = 4 * ts.npp;
             a.hzero = hzero ? 1 : 0;
             const dim3 grid(tile_parts(st, 128), ng);
-            if (st.unicls) k_tile_pre<float, true, 0, 128, 5><<<grid, 128, 0, c->stream>>>(a);
-            else if (st.prepk) k_tile_pre<float, false, 0, 128, 4><<<grid, 128, 0, c->stream>>>(a);
-            else k_tile_pre<float, false, 1, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            if (st.unicls) k_tile_pre<T8, float, true, 0, 128, 6><<<grid, 128, 0, c->stream>>>(a);
+            else if (st.prepk) k_tile_pre<T8, float, false, 0, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            else k_tile_pre<T8, float, false, 1, 128, 4><<<grid, 128, 0, c->stream>>>(a);
             MG_LAUNCHED(c);
         }
         ProfScope ps_(c, "mx_sip_fwd");

@@ -25,3 +25,5 @@ int launch_accumulate(Ctx* c, double* dp, double* hilf);
 int launch_mgpcorr(Ctx* c, double* u, double* v, double* w, double* p, const double* dp,
                    double rfak);
 void release_tables(Ctx* c);
+// the outer loop of mgpoisl on RHS into DP, on tiles (plain_tile.cu)
+int plain_tile_solve(Ctx* c, double prefak, mglet_stage_stats* st);

@@ -1,0 +1,452 @@
+// plain_tile.cu -- the outer loop of mgpoisl (pressuresolver_mod.F90:203-305) of
+// the plain FP64 form on one level, on tiles (sip_tile.cuh).
+//
+// The values and their order are those of the per-operator kernels
+// (plain_poisson.cu): laplacephi, sipiter1, sipiter2, accumulate and rescal per
+// point, the halos of conn(res) and conn(dp) read from the neighbours' arrays at
+// the iterations the reference exchanges them.  What falls away is the traffic
+// between the operators (res written by laplacephi and read by sipiter1, hilf and
+// rhs passed over by accumulate and rescal), the connect launches, the per-grid
+// copies of the SIP factors (grids with equal spacing and faces share a set, which
+// stays in L2), and the host round trip of every outer iteration: the stopping
+// test sets a flag the following kernels return on.  A time step of three stages
+// (per-operator kernels before): one grid of 32^3 23.8 ms (50.3), 64 of 24^3 21.4
+// (38.5), 512 of 24^3 contracted 72 (103).  What bounds the sweeps is the FP64 pipe
+// (432 warps of points of 24^3, 7 instructions a point uncontracted, 64 clocks each
+// on four pipes: 25 us on one SM) and, with fewer grids than SMs, the chain of the
+// hyperplanes.
+//
+// Compiled twice like plain_poisson.cu (-fmad=false and, in namespace contract,
+// with contraction).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <map>
+
+#include "internal.h"
+#include "plain_tile.h"
+
+namespace mg {
+MG_PLAIN_BEGIN
+namespace {
+
+using T2 = Tile<1, 1, 2>;
+using T1 = Tile<1, 1, 1>;
+
+// RHS (natural layout) into tiles
+__global__ void k_pt_gather(const DevGrid* __restrict__ grids, TileShape s, const double* __restrict__ F,
+                            double* __restrict__ X) {
+    const int g = blockIdx.y, p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= s.npp) return;
+    X[(long long)g * s.npp + p] = F[grids[g].ip3 + s.cell[p]];
+}
+
+struct PtOuterArgs {
+    TileArgs<double> t;
+    double *RHS, *DP;
+    double* gridmax;
+};
+
+// the laplacian coefficients of a tile's cells (kUni: one value each over a class)
+template <class L, bool kUni>
+__device__ __forceinline__ void tile_lap_coefs(const TileArgs<double>& a, int cls, int p,
+                                               Vec<double, L::N> (&c)[kUni ? 1 : 7]) {
+    if constexpr (!kUni)
+#pragma unroll
+        for (int f = 0; f < 7; ++f) ldt(true, a.LAP + ((long long)cls * 7 + f) * a.s.npp + p, c[f]);
+}
+
+// laplacephi at cell i of a tile
+template <class L, bool kUni>
+__device__ __forceinline__ double tile_lap(const TileArgs<double>& a, int cls, const TileHalo<L, double>& o,
+                                           const Vec<double, L::N> (&c)[kUni ? 1 : 7], int i) {
+    double n[6], w[7];
+    tile_nbrs<L>(o, i, n);
+#pragma unroll
+    for (int f = 0; f < 7; ++f) w[f] = kUni ? a.UNI[8 * cls + f] : c[kUni ? 0 : f].v[i];
+    const double lap = mul_rounded(-w[0], n[0]);
+    return lap - w[1] * n[1] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] - w[5] * n[5] - w[6] * o.h.v[i];
+}
+
+// laplacephi of hilf, rescal (rhs += res) with maxabscal_grid, accumulate (dp +=
+// hilf): one thread a tile; gridmax takes the maximum over the CTAs of a grid (of
+// non-negative numbers, as integers).
+template <class L, bool kUni>
+__global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOuterArgs a) {
+    if (a.t.ctl[0]) return;
+    constexpr int N = L::N;
+    __shared__ double shm[4];
+    const TileShape& s = a.t.s;
+    const int g = blockIdx.y, cls = a.t.gcls[g];
+    const long long base = (long long)g * s.npp;
+    const int tile = blockIdx.x * 128 + threadIdx.x, p = N * tile;
+    double mx = 0.0;
+    if (tile < s.ntile) {
+        TileHalo<L, double> o;
+        tile_halo(a.t, g, tile, o);
+        Vec<double, N> rh, dp, c[kUni ? 1 : 7];
+        ldt_rw(true, a.RHS + base + p, rh);
+        ldt_rw(true, a.DP + base + p, dp);
+        tile_lap_coefs<L, kUni>(a.t, cls, p, c);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const double r = rh.v[i] + tile_lap<L, kUni>(a.t, cls, o, c, i);
+            rh.v[i] = r;
+            dp.v[i] = dp.v[i] + o.h.v[i];
+            mx = fmax(fabs(r), mx);
+        }
+        stt(a.RHS + base + p, rh);
+        stt(a.DP + base + p, dp);
+    }
+    for (int q = 16; q > 0; q >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, q));
+    if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        mx = fmax(fmax(shm[0], shm[1]), fmax(shm[2], shm[3]));
+        atomicMax(reinterpret_cast<unsigned long long*>(a.gridmax) + g,
+                  (unsigned long long)__double_as_longlong(mx));
+    }
+}
+
+// the residual and the accumulated correction back into RHS and DP, and the
+// laplacian of the last correction into RES
+template <class L, bool kUni>
+__global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOuterArgs a,
+                                                    const DevGrid* __restrict__ grids,
+                                                    double* __restrict__ RHS, double* __restrict__ DP,
+                                                    double* __restrict__ RES) {
+    constexpr int N = L::N;
+    const TileShape& s = a.t.s;
+    const int g = blockIdx.y, cls = a.t.gcls[g];
+    const int tile = blockIdx.x * 128 + threadIdx.x, p = N * tile;
+    if (tile >= s.ntile) return;
+    const long long base = (long long)g * s.npp, ip3 = grids[g].ip3;
+    TileHalo<L, double> o;
+    tile_halo(a.t, g, tile, o);
+    Vec<double, N> c[kUni ? 1 : 7];
+    tile_lap_coefs<L, kUni>(a.t, cls, p, c);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const long long q = ip3 + s.cell[p + i];
+        RHS[q] = a.RHS[base + p + i];
+        DP[q] = a.DP[base + p + i];
+        RES[q] = tile_lap<L, kUni>(a.t, cls, o, c, i);
+    }
+}
+
+// maxabscal over the grids (one level: no level scale) and the stopping test; the
+// maxima are cleared for the next outer iteration.  stat: {max |rhs|, converged,
+// outer iterations done}.
+__global__ void k_pt_conv(int ngrid, double* __restrict__ gridmax, double* stat, double prefak, double epcorr,
+                          int nouter_min) {
+    int* ctl = reinterpret_cast<int*>(stat + 1);
+    if (ctl[0]) return;
+    __shared__ double sh[32];
+    double m = 0.0;
+    for (int g = threadIdx.x; g < ngrid; g += blockDim.x) {
+        m = fmax(gridmax[g], m);
+        gridmax[g] = 0.0;
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) sh[w] = m;
+    __syncthreads();
+    if (w == 0) {
+        m = l < (int)(blockDim.x >> 5) ? sh[l] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (l == 0) {
+            const int done = ctl[1] + 1;
+            ctl[1] = done;
+            stat[0] = m;
+            if (done >= nouter_min && m / prefak < epcorr) ctl[0] = 1;
+        }
+    }
+}
+
+// Up to one grid an SM the step chain of a sweep bounds it, and two sets of warps
+// take the steps in turn (24^3: 49 us a sweep on 64 grids, 53 with one set); past
+// that a CTA's registers would leave SMs with one grid where two fit (216 grids of
+// 20^3: 54 us with one set, 60 with two).
+constexpr int kFew = 152;
+
+template <class L, bool kFwd, bool kHz>
+int launch_sweep(Ctx* c, const TileArgs<double>& a) {
+    const unsigned smem = tile_layout<L, double>(a.s).bytes;
+    const int threads = (a.s.maxt + 31) / 32 * 32 + 32;
+    auto go = [&](auto* k) -> int {
+        if (smem > 48 * 1024)
+            MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        k<<<c->ngrid, threads, smem, c->stream>>>(a);
+        return 0;
+    };
+    int rc;
+    if (c->ngrid <= kFew && 2 * threads - 32 <= 1024) {
+        auto few = [&](auto* k) -> int {
+            if (smem > 48 * 1024)
+                MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            k<<<c->ngrid, 2 * threads - 32, smem, c->stream>>>(a);
+            return 0;
+        };
+        rc = 2 * threads - 32 <= 544 ? few(k_tile_sweep_few<L, double, kFwd, kHz, 2, 544>)
+                                     : few(k_tile_sweep_few<L, double, kFwd, kHz, 1, 1024>);
+    } else if (threads <= 160) rc = go(k_tile_sweep<L, double, kFwd, kHz, 2, 160, 4>);
+    else if (threads <= 320) rc = go(k_tile_sweep<L, double, kFwd, kHz, 2, 320, 2>);
+    else if (threads <= 544) rc = go(k_tile_sweep<L, double, kFwd, kHz, 2, 544, 1>);
+    else rc = go(k_tile_sweep<L, double, kFwd, kHz, 1, 1024, 1>);
+    if (rc) return rc;
+    MG_LAUNCHED(c);
+    return 0;
+}
+
+template <class L>
+int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
+    PlainTile& p = *c->ptile;
+    const TileShape& s = p.t.s;
+    const size_t bytes = (size_t)c->ngrid * s.npp * sizeof(double);
+    const dim3 cells((s.npp + 255) / 256, c->ngrid), tiles((s.ntile + 127) / 128, c->ngrid);
+    int* ctl = reinterpret_cast<int*>(p.stat + 1);
+    MG_CUDA(cudaMemsetAsync(p.stat, 0, 2 * sizeof(double), c->stream));
+    MG_CUDA(cudaMemsetAsync(p.gridmax, 0, c->ngrid * sizeof(double), c->stream));
+    MG_CUDA(cudaMemsetAsync(p.dp, 0, bytes, c->stream));
+    k_pt_gather<<<cells, 256, 0, c->stream>>>(c->d_grids, s, c->F("RHS"), p.rhs);
+    MG_LAUNCHED(c);
+    TileArgs<double> a{};
+    a.s = s;
+    a.fnbr = p.fnbr;
+    a.gcls = p.gcls;
+    a.H = p.h;
+    a.RHS = p.rhs;
+    a.LPR = p.cf + 3 * s.npp;
+    a.lprcls = 4 * s.npp;
+    a.LAP = p.lap;
+    a.UNI = p.uni;
+    a.ctl = ctl;
+    PtOuterArgs o{};
+    o.RHS = p.rhs;
+    o.DP = p.dp;
+    o.gridmax = p.gridmax;
+    const int ninner = c->prm.ninner;
+    // inner iteration gi writes res slot gi % 3 and takes its low ghosts from the
+    // last iteration whose exchange covered every face (every inner iteration but
+    // the last of an outer one)
+    int gi = 0, lastfull = 0;
+    for (int ip = 1; ip <= c->prm.nouter; ++ip) {
+        for (int il = 1; il <= ninner; ++il) {
+            ++gi;
+            const bool hz = il == 1;
+            a.R = p.rs[gi % 3];
+            a.hzero = hz;
+            a.rev = 0;
+            {
+                ProfScope ps_(c, "laplacephi");
+                if (p.unicls) k_tile_pre<L, double, true, 0, 128, 4><<<tiles, 128, 0, c->stream>>>(a);
+                else k_tile_pre<L, double, false, 0, 128, 4><<<tiles, 128, 0, c->stream>>>(a);
+                MG_LAUNCHED(c);
+            }
+            {
+                ProfScope ps_(c, "sipiter1");
+                a.G = lastfull > 0 ? p.rs[lastfull % 3] : nullptr;
+                a.CF = p.cf;
+                a.cfcls = 4 * s.npp;
+                a.rev = 1;
+                if (int rc = launch_sweep<L, true, false>(c, a)) return rc;
+            }
+            {
+                ProfScope ps_(c, "sipiter2");
+                a.G = a.R;
+                a.CF = p.cb;
+                a.cfcls = 3 * s.npp;
+                a.rev = 0;
+                if (int rc = hz ? launch_sweep<L, false, true>(c, a) : launch_sweep<L, false, false>(c, a))
+                    return rc;
+            }
+            if (il < ninner) lastfull = gi;
+        }
+        {
+            ProfScope ps_(c, "rescal_maxabs");
+            o.t = a;
+            if (p.unicls) k_pt_outer<L, true><<<tiles, 128, 0, c->stream>>>(o);
+            else k_pt_outer<L, false><<<tiles, 128, 0, c->stream>>>(o);
+            MG_LAUNCHED(c);
+            k_pt_conv<<<1, 256, 0, c->stream>>>(c->ngrid, p.gridmax, p.stat, prefak, c->prm.epcorr,
+                                                c->prm.nouter_min);
+            MG_LAUNCHED(c);
+        }
+        // a long outer loop looks now and then whether it has converged
+        if (ip % 12 == 0 && ip < c->prm.nouter) {
+            MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+            MG_CUDA(cudaStreamSynchronize(c->stream));
+            if (reinterpret_cast<const int*>(p.h_stat + 1)[0]) break;
+        }
+    }
+    o.t = a;
+    if (p.unicls)
+        k_pt_scatter<L, true><<<tiles, 128, 0, c->stream>>>(o, c->d_grids, c->F("RHS"), c->F("DP"), c->F("RES"));
+    else
+        k_pt_scatter<L, false><<<tiles, 128, 0, c->stream>>>(o, c->d_grids, c->F("RHS"), c->F("DP"), c->F("RES"));
+    MG_LAUNCHED(c);
+    MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    // dp ghosts: the reference accumulates the connected hilf ghosts into dp
+    if (int rc = connect(c, 0, 1, nullptr, nullptr, nullptr, c->F("DP"), nullptr, nullptr, false, false, 0))
+        return rc;
+    MG_CUDA(cudaStreamSynchronize(c->stream));
+    if (st) {
+        st->nouter_done = reinterpret_cast<const int*>(p.h_stat + 1)[1];
+        st->ipc = st->nouter_done * ninner;
+        st->maxrhs = p.h_stat[0];
+        st->prefak = prefak;
+    }
+    return 0;
+}
+
+}  // namespace
+
+int plain_tile_solve(Ctx* c, double prefak, mglet_stage_stats* st) {
+    return c->ptile->pair ? solve<T2>(c, prefak, st) : solve<T1>(c, prefak, st);
+}
+
+MG_PLAIN_END
+
+#ifndef MG_FMA_BUILD
+// class coefficients from the FP64 fields of the representative grids
+__global__ void k_pt_extract(const DevGrid* __restrict__ grids, const int* __restrict__ reps, TileShape s,
+                             const double* __restrict__ lw, const double* __restrict__ ls,
+                             const double* __restrict__ lb, const double* __restrict__ lpr,
+                             const double* __restrict__ ue, const double* __restrict__ un,
+                             const double* __restrict__ ut, const double* __restrict__ ap,
+                             const double* __restrict__ AW, const double* __restrict__ AE,
+                             const double* __restrict__ AS, const double* __restrict__ AN,
+                             const double* __restrict__ AB, const double* __restrict__ AT, double* CF,
+                             double* CB, double* LAP) {
+    const long long cls = blockIdx.y;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= s.npp) return;
+    const DevGrid G = grids[reps[cls]];
+    const int id = s.cell[p];
+    const long long src = G.ip3 + s.plane[p];
+    const double f[4] = {lw[src], ls[src], lb[src], lpr[src]};
+    const double b[3] = {ue[src], un[src], ut[src]};
+    const int kk = G.kk, jj = G.jj;
+    const int ix = G.ipx + id / (kk * jj), iy = G.ipy + (id / kk) % jj, iz = G.ipz + id % kk;
+    const double l[7] = {AW[ix], AE[ix], AS[iy], AN[iy], AB[iz], AT[iz], ap[G.ip3 + id]};
+    for (int q = 0; q < 4; ++q) CF[(cls * 4 + q) * s.npp + p] = f[q];
+    for (int q = 0; q < 3; ++q) CB[(cls * 3 + q) * s.npp + p] = b[q];
+    for (int q = 0; q < 7; ++q) LAP[(cls * 7 + q) * s.npp + p] = l[q];
+}
+
+// per class {1, seven coefficients} when each is one value over the class, else {0}
+__global__ void k_pt_uniform(TileShape s, const double* __restrict__ LAP, double* UNI) {
+    const long long cls = blockIdx.x;
+    int bad = 0;
+    for (int q = 0; q < 7; ++q) {
+        const double* l = LAP + (cls * 7 + q) * s.npp;
+        for (int p = threadIdx.x; p < s.npp; p += blockDim.x) bad |= !(l[p] == l[0]);
+        if (threadIdx.x == 0) UNI[8 * cls + q] = l[0];
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) UNI[8 * cls + 7] = bad ? 0.0 : 1.0;
+}
+
+int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
+    if (c->minlevel != c->maxlevel || !c->uniform || c->prm.psolver == MGLET_PSOLVER_CLASSIC ||
+        c->prm.form != MGLET_FORM_PLAIN || c->prm.ninner < 1 || c->prm.nouter < 1)
+        return 0;
+    const DevGrid& G0 = c->grids[0];
+    std::vector<int> fn((size_t)6 * c->ngrid, -1);
+    for (size_t r = 0; r < c->conns.size(); r += 4) {
+        const int rf = c->conns[r + 2], sf = c->conns[r + 3];
+        if (rf > 6) continue;
+        if (sf != (rf % 2 ? rf + 1 : rf - 1)) return 0;
+        fn[(size_t)6 * (c->conns[r] - 1) + rf - 1] = c->conns[r + 1] - 1;
+    }
+    PlainTile* p = new PlainTile();
+    c->ptile = p;
+    auto give_up = [&]() {
+        plain_tile_release(c);
+        return 0;
+    };
+    const int ni = G0.ii - 4, nj = G0.jj - 4, nk = G0.kk - 4;
+    p->pair = nk % 2 == 0;
+    if (int rc = tile_init(c, ni, nj, nk, 0, 0, p->pair, 992, p->t)) return rc;
+    if (!p->t.ok) return give_up();
+    const TileShape& s = p->t.s;
+    const unsigned smem = p->pair ? tile_layout<Tile<1, 1, 2>, double>(s).bytes
+                                  : tile_layout<Tile<1, 1, 1>, double>(s).bytes;
+    if (smem > 220 * 1024) return give_up();
+    // grids with the same faces and spacing share a set of coefficients
+    std::map<std::vector<double>, int> seen;
+    std::vector<int> gcls(c->ngrid), reps;
+    for (int g = 0; g < c->ngrid; ++g) {
+        const DevGrid& G = c->grids[g];
+        std::vector<double> key;
+        for (int f = 0; f < 6; ++f) key.push_back(G.bc[f]);
+        key.insert(key.end(), d->dx + G.ipx, d->dx + G.ipx + G.ii);
+        key.insert(key.end(), d->dy + G.ipy, d->dy + G.ipy + G.jj);
+        key.insert(key.end(), d->dz + G.ipz, d->dz + G.ipz + G.kk);
+        auto it = seen.find(key);
+        if (it == seen.end()) {
+            it = seen.emplace(std::move(key), (int)reps.size()).first;
+            reps.push_back(g);
+        }
+        gcls[g] = it->second;
+    }
+    p->ncls = (int)reps.size();
+    auto up = [&](int** q, const std::vector<int>& h) -> int {
+        MG_CUDA(cudaMalloc(q, h.size() * sizeof(int)));
+        MG_CUDA(copy_on(c->stream, *q, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
+        return 0;
+    };
+    if (int rc = up(&p->gcls, gcls)) return rc;
+    if (int rc = up(&p->fnbr, fn)) return rc;
+    // one allocation for the FP64 arrays (each a multiple of 256 bytes)
+    auto pad = [](size_t n) { return (n + 31) & ~(size_t)31; };
+    const size_t n = pad((size_t)c->ngrid * s.npp), m = (size_t)p->ncls * s.npp;
+    const size_t cls[3] = {pad(4 * m), pad(3 * m), pad(7 * m)};
+    const size_t all = 6 * n + cls[0] + cls[1] + cls[2] + pad(8 * p->ncls) + pad(c->ngrid) + pad(2);
+    MG_CUDA(cudaMalloc(&p->mem, all * sizeof(double)));
+    double* q = p->mem;
+    auto take = [&](double** d, size_t len) {
+        *d = q;
+        q += len;
+    };
+    for (double** d : {&p->h, &p->rhs, &p->dp, &p->rs[0], &p->rs[1], &p->rs[2]}) take(d, n);
+    take(&p->cf, cls[0]);
+    take(&p->cb, cls[1]);
+    take(&p->lap, cls[2]);
+    take(&p->uni, pad(8 * p->ncls));
+    take(&p->gridmax, pad(c->ngrid));
+    take(&p->stat, pad(2));
+    MG_CUDA(cudaMallocHost(&p->h_stat, 2 * sizeof(double)));
+    int* d_reps = nullptr;
+    if (int rc = up(&d_reps, reps)) return rc;
+    k_pt_extract<<<dim3((s.npp + 255) / 256, p->ncls), 256, 0, c->stream>>>(
+        c->d_grids, d_reps, s, c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"), c->F("SIPLPR"), c->F("SIPUE"),
+        c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), c->L("GSAW"), c->L("GSAE"), c->L("GSAS"), c->L("GSAN"),
+        c->L("GSAB"), c->L("GSAT"), p->cf, p->cb, p->lap);
+    k_pt_uniform<<<p->ncls, 256, 0, c->stream>>>(s, p->lap, p->uni);
+    c->launches += 2;
+    std::vector<double> uni((size_t)8 * p->ncls);
+    cudaError_t e = copy_on(c->stream, uni.data(), p->uni, uni.size() * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(d_reps);
+    if (e != cudaSuccess) return cuda_fail(e, "plain tiles");
+    p->unicls = true;
+    for (int q = 0; q < p->ncls; ++q) p->unicls = p->unicls && uni[(size_t)8 * q + 7] != 0.0;
+    return 0;
+}
+
+void plain_tile_release(Ctx* c) {
+    PlainTile* p = c->ptile;
+    if (!p) return;
+    tile_free(p->t);
+    for (void* q : {(void*)p->gcls, (void*)p->fnbr, (void*)p->mem}) cudaFree(q);
+    if (p->h_stat) cudaFreeHost(p->h_stat);
+    delete p;
+    c->ptile = nullptr;
+}
+
+bool plain_tile_ready(const Ctx* c) {
+    return c->ptile && !c->part && c->ibtype == 0 && !c->coef_user;
+}
+#endif
+
+}  // namespace mg

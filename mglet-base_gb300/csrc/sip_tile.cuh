@@ -1,23 +1,26 @@
-// sip_tile.cuh -- the SIP solver on 2x2x2 tiles, in FP32 (mixed form) and FP64
-// (plain form).
+// sip_tile.cuh -- the SIP solver on small tiles of cells, in FP32 (mixed form,
+// 2x2x2) and FP64 (plain form, 1x1x2 or single cells).
 //
-// A grid of even dimensions is cut into tiles of 2x2x2 cells, stored tile after
-// tile in the order of the hyperplanes I+J+K of the tile lattice, the 8 values of
-// a tile (k fastest) in one 32-byte (64-byte) line.  A sweep walks the tile
-// hyperplanes, one thread a tile, one CTA a grid: 34 steps for 24^3 cells where
-// the cell hyperplanes take 70, and a step's 8 points pass their values in
-// registers.  Between tiles only faces travel: a thread reads the three facing
-// quads of its predecessors from shared memory and leaves its own three, six
-// 16-byte accesses for 8 points (cell by cell it takes 32 of 4 bytes, and the
+// A grid is cut into tiles of TI x TJ x TK cells (its dimensions must divide),
+// stored tile after tile in the order of the hyperplanes I+J+K of the tile
+// lattice, the values of a tile together, k fastest.  A sweep walks the tile
+// hyperplanes, one thread a tile, one CTA a grid: 34 steps for 24^3 cells in tiles
+// of 2x2x2 where the cell hyperplanes take 70, and the points of a tile pass their
+// values in registers.  Between tiles only faces travel: a thread reads the three
+// facing quads of its predecessors from shared memory and leaves its own three --
+// six 16-byte accesses for 8 points (cell by cell it takes 32 of 4 bytes, and the
 // index of each).  In shared memory a face of tile (I, J, K) of hyperplane t sits
 // in slot (I+1)(NJ+1) + (J+1), which no other tile of that hyperplane shares, so
 // the predecessors are at the constant offsets -(NJ+1), -1 and 0 of the plane
 // before.  The arithmetic of a point and its order are those of the cell sweeps
 // (sip_hyperplane_mod.F90:450-569), so the results are the same bits.
 //
-// The sweeps are bound by the chain of their steps (few grids) and by the
-// issue of their loads (many); all global loads of a step are 32 bytes wide and
-// are issued kD steps ahead.
+// What bounds it: FP32, the chain of the steps (few grids) and the issue of the
+// loads (many); all global loads of a step are issued kD steps ahead.  FP64, the
+// FP64 pipe: an instruction of a warp takes it 64 clocks whatever the number of
+// active lanes, so there the lanes have to be full and the four pipes of an SM
+// evenly used -- 2-cell tiles (12 instructions a step, 119 tiles a step on 24^3)
+// cost 52 k clocks a sweep, 2x2x2 tiles (48 a step, 51 tiles) 104 k.
 #pragma once
 
 #include <algorithm>
@@ -30,6 +33,7 @@ namespace mg {
 // Tables of one grid shape (device pointers)
 struct TileShape {
     int ni, nj, nk;                 // cells
+    int si, sj, sk;                 // log2 of the tile's extents (0 or 1)
     int NI, NJ, NK, NT, ntile;      // tiles; tile hyperplanes; tiles in all
     int npp, fs;                    // cells of a grid's array; length of a face array
     int maxt;                       // tiles of the largest hyperplane
@@ -53,9 +57,11 @@ struct TileShape {
 };
 
 // position of a cell
-__host__ __device__ inline int tile_pos(const int* tpos, int NI, int io, int jo, int ko) {
-    const int I = io >> 1, J = jo >> 1, K = ko >> 1;
-    return ((tpos[(I + J + K) * NI + I] + J) << 3) | ((io & 1) << 2) | ((jo & 1) << 1) | (ko & 1);
+__host__ __device__ inline int tile_pos(const TileShape& s, const int* tpos, int io, int jo, int ko) {
+    const int I = io >> s.si, J = jo >> s.sj, K = ko >> s.sk;
+    const int di = io & s.si, dj = jo & s.sj, dk = ko & s.sk;   // (extents are 1 or 2)
+    return ((tpos[(I + J + K) * s.NI + I] + J) << (s.si + s.sj + s.sk)) |
+           (((di << s.sj) | dj) << s.sk | dk);
 }
 
 struct TileDev {
@@ -66,88 +72,108 @@ struct TileDev {
 
 namespace {
 
-template <typename T>
-struct alignas(16) Vec4 {
-    T v[4];
-};
-template <typename T>
-struct Vec8 {
-    T v[8];
+template <typename T, int N>
+struct alignas(sizeof(T) * N < 16 ? sizeof(T) * N : 16) Vec {
+    T v[N];
 };
 
-// 8 values of a tile.  kNc: through the read-only path (nothing in the launch
-// writes them); p: a predicate, without a branch (a load inside a branch is
-// waited for where the branch ends).
-__device__ __forceinline__ void ld8(bool p, const float* a, Vec8<float>& r) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
-        " @q ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"
-        : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]), "+f"(r.v[4]), "+f"(r.v[5]),
-          "+f"(r.v[6]), "+f"(r.v[7])
-        : "l"(a), "r"((int)p));
-}
-__device__ __forceinline__ void ld8(bool p, const double* a, Vec8<double>& r) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
-        " @q ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%8];\n"
-        " @q ld.global.nc.v4.f64 {%4, %5, %6, %7}, [%8 + 32];\n}"
-        : "+d"(r.v[0]), "+d"(r.v[1]), "+d"(r.v[2]), "+d"(r.v[3]), "+d"(r.v[4]), "+d"(r.v[5]),
-          "+d"(r.v[6]), "+d"(r.v[7])
-        : "l"(a), "r"((int)p));
-}
-// values this CTA writes later in the same launch
-__device__ __forceinline__ void ld8_rw(bool p, const float* a, Vec8<float>& r) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
-        " @q ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"
-        : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]), "+f"(r.v[4]), "+f"(r.v[5]),
-          "+f"(r.v[6]), "+f"(r.v[7])
-        : "l"(a), "r"((int)p)
-        : "memory");
-}
-__device__ __forceinline__ void ld8_rw(bool p, const double* a, Vec8<double>& r) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n"
-        " @q ld.global.v4.f64 {%0, %1, %2, %3}, [%8];\n"
-        " @q ld.global.v4.f64 {%4, %5, %6, %7}, [%8 + 32];\n}"
-        : "+d"(r.v[0]), "+d"(r.v[1]), "+d"(r.v[2]), "+d"(r.v[3]), "+d"(r.v[4]), "+d"(r.v[5]),
-          "+d"(r.v[6]), "+d"(r.v[7])
-        : "l"(a), "r"((int)p)
-        : "memory");
-}
-__device__ __forceinline__ void st8(float* a, const Vec8<float>& r) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a), "f"(r.v[0]),
-                 "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]), "f"(r.v[7])
-                 : "memory");
-}
-__device__ __forceinline__ void st8(double* a, const Vec8<double>& r) {
-    asm volatile(
-        "st.global.v4.f64 [%0], {%1, %2, %3, %4};\n st.global.v4.f64 [%0 + 32], {%5, %6, %7, %8};" ::"l"(a),
-        "d"(r.v[0]), "d"(r.v[1]), "d"(r.v[2]), "d"(r.v[3]), "d"(r.v[4]), "d"(r.v[5]), "d"(r.v[6]), "d"(r.v[7])
-        : "memory");
-}
+// The N values of a tile.  ldt: through the read-only path (nothing in the launch
+// writes them); ldt_rw: values this CTA writes later in the same launch; p: a
+// predicate, without a branch (a load inside a branch is waited for where the
+// branch ends).
+#define MG_LD(SUF, CLOB)                                                                                 \
+    template <int N>                                                                                     \
+    __device__ __forceinline__ void ldt##SUF(bool p, const float* a, Vec<float, N>& r) {                 \
+        if constexpr (N == 8)                                                                            \
+            asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %9, 0;\n @q ld.global" MG_NC                 \
+                         ".v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n}"                            \
+                         : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]), "+f"(r.v[4]),         \
+                           "+f"(r.v[5]), "+f"(r.v[6]), "+f"(r.v[7])                                      \
+                         : "l"(a), "r"((int)p) CLOB);                                                    \
+        else if constexpr (N == 2)                                                                       \
+            asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q ld.global" MG_NC                 \
+                         ".v2.f32 {%0, %1}, [%2];\n}"                                                    \
+                         : "+f"(r.v[0]), "+f"(r.v[1])                                                    \
+                         : "l"(a), "r"((int)p) CLOB);                                                    \
+        else                                                                                             \
+            asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.global" MG_NC                 \
+                         ".f32 %0, [%1];\n}"                                                             \
+                         : "+f"(r.v[0])                                                                  \
+                         : "l"(a), "r"((int)p) CLOB);                                                    \
+    }                                                                                                    \
+    template <int N>                                                                                     \
+    __device__ __forceinline__ void ldt##SUF(bool p, const double* a, Vec<double, N>& r) {               \
+        if constexpr (N == 2)                                                                            \
+            asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %3, 0;\n @q ld.global" MG_NC                 \
+                         ".v2.f64 {%0, %1}, [%2];\n}"                                                    \
+                         : "+d"(r.v[0]), "+d"(r.v[1])                                                    \
+                         : "l"(a), "r"((int)p) CLOB);                                                    \
+        else                                                                                             \
+            asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %2, 0;\n @q ld.global" MG_NC                 \
+                         ".f64 %0, [%1];\n}"                                                             \
+                         : "+d"(r.v[0])                                                                  \
+                         : "l"(a), "r"((int)p) CLOB);                                                    \
+    }
+#define MG_NC ".nc"
+MG_LD(, )
+#undef MG_NC
+#define MG_NC ""
+MG_LD(_rw, : "memory")
+#undef MG_NC
+#undef MG_LD
 
+template <typename T, int N>
+__device__ __forceinline__ void stt(T* a, const Vec<T, N>& r) {
+    static_assert(N <= 2 || N == 8, "tile sizes");
+    if constexpr (N == 8 && sizeof(T) == 4)
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(a), "f"(r.v[0]),
+                     "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]),
+                     "f"(r.v[7])
+                     : "memory");
+    else
+        *reinterpret_cast<Vec<T, N>*>(a) = r;
+}
 // a += r: one writer per value, so the reduction (round to nearest) is the plain
 // sum without a load
-__device__ __forceinline__ void add8(float* a, const Vec8<float>& r) {
-    asm volatile(
-        "red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n red.global.add.v4.f32 [%0 + 16], {%5, %6, %7, %8};" ::"l"(a),
-        "f"(r.v[0]), "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]), "f"(r.v[7])
-        : "memory");
-}
-__device__ __forceinline__ void add8(double* a, const Vec8<double>& r) {
+template <typename T, int N>
+__device__ __forceinline__ void addt(T* a, const Vec<T, N>& r) {
+    if constexpr (N == 8 && sizeof(T) == 4) {
+        asm volatile(
+            "red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n"
+            " red.global.add.v4.f32 [%0 + 16], {%5, %6, %7, %8};" ::"l"(a),
+            "f"(r.v[0]), "f"(r.v[1]), "f"(r.v[2]), "f"(r.v[3]), "f"(r.v[4]), "f"(r.v[5]), "f"(r.v[6]),
+            "f"(r.v[7])
+            : "memory");
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) atomicAdd(a + i, r.v[i]);
+        for (int i = 0; i < N; ++i) atomicAdd(a + i, r.v[i]);
+    }
 }
 
-// The quad of a tile that faces its neighbour: on axis 0, 1, 2 the cells with
-// offset hi along that axis; in the order of the other two offsets.
-template <int kAxis, int kHi, typename T>
-__device__ __forceinline__ Vec4<T> quad(const Vec8<T>& r) {
-    if constexpr (kAxis == 0) return Vec4<T>{r.v[4 * kHi], r.v[4 * kHi + 1], r.v[4 * kHi + 2], r.v[4 * kHi + 3]};
-    else if constexpr (kAxis == 1)
-        return Vec4<T>{r.v[2 * kHi], r.v[2 * kHi + 1], r.v[4 + 2 * kHi], r.v[5 + 2 * kHi]};
-    else return Vec4<T>{r.v[kHi], r.v[2 + kHi], r.v[4 + kHi], r.v[6 + kHi]};
+// The extents of a tile, and the cells of its faces: on axis A the cells with the
+// lowest or highest offset along it, in the order of the other two offsets.
+template <int TI_, int TJ_, int TK_>
+struct Tile {
+    static constexpr int TI = TI_, TJ = TJ_, TK = TK_, N = TI * TJ * TK;
+    static constexpr int FI = TJ * TK, FJ = TI * TK, FK = TI * TJ;
+    template <int A>
+    static constexpr int F = A == 0 ? FI : (A == 1 ? FJ : FK);
+    // cell q of the face on axis A, at the high end when hi
+    template <int A>
+    __host__ __device__ static constexpr int cell(int q, bool hi) {
+        if (A == 0) return (hi ? (TI - 1) * TJ * TK : 0) + q;
+        if (A == 1) return (q / TK) * TJ * TK + (hi ? (TJ - 1) * TK : 0) + q % TK;
+        return q * TK + (hi ? TK - 1 : 0);
+    }
+};
+
+// (kM: the size of the result, the face's cells first)
+template <class L, int A, bool kHi, typename T, int kM = L::template F<A>>
+__device__ __forceinline__ Vec<T, kM> tile_part(const Vec<T, L::N>& r) {
+    Vec<T, kM> o;
+#pragma unroll
+    for (int q = 0; q < kM; ++q) o.v[q] = q < L::template F<A> ? r.v[L::template cell<A>(q, kHi) % L::N] : T(0);
+    return o;
 }
 
 // a product that is rounded before anything is added to it
@@ -177,170 +203,203 @@ struct TileArgs {
 
 constexpr int kTilePad = 8;         // empty hyperplanes past the last in the table of starts
 
-// Shared memory of a sweep: [tst] [gst] [ghost entries] [ghost quads] [2][3][slots] quads
+// Shared memory of a sweep: [tst] [gst] [ghost entries] [ghost faces] [2][3][slots]
+// faces (of equal size for the three axes, so that a ghost is one copy)
+template <class L>
+struct TileFace {   // values of the largest face
+    static constexpr int M = L::FI > L::FJ ? (L::FI > L::FK ? L::FI : L::FK) : (L::FJ > L::FK ? L::FJ : L::FK);
+};
 struct TileLayout {
     unsigned gst, gent, gval, face, bytes;
 };
-template <typename T>
+template <class L, typename T>
 __host__ __device__ inline TileLayout tile_layout(const TileShape& s) {
     auto up = [](unsigned v) { return (v + 31u) & ~31u; };
+    constexpr unsigned fb = TileFace<L>::M * sizeof(T);
     TileLayout l;
     unsigned o = (s.NT + 1 + kTilePad) * 4;
     l.gst = o; o = up(o + (s.NT + 3) * 4);
     l.gent = o; o = up(o + s.nside * 4);
-    l.gval = o; o = up(o + s.nside * (unsigned)sizeof(Vec4<T>));
-    l.face = o; o += 6 * s.slots * (unsigned)sizeof(Vec4<T>);
+    l.gval = o; o = up(o + s.nside * fb);
+    l.face = o; o += 6 * s.slots * fb;
     l.bytes = o;
     return l;
 }
 
 // A tile's loads of one step
-template <typename T>
+template <class L, typename T>
 struct TileSet {
     int tile, x;                    // tile (-1: none) and slot
-    Vec8<T> c[3], v;
+    Vec<T, L::N> c[3], v;
 };
 
-// The predecessor recurrence of a tile's 8 cells (see k_tile_sweep)
-template <bool kFwd, typename T>
-__device__ __forceinline__ Vec8<T> tile_solve(const Vec8<T>& v, const Vec8<T>& ci, const Vec8<T>& cj,
-                                              const Vec8<T>& ck, const Vec4<T>& fi, const Vec4<T>& fj,
-                                              const Vec4<T>& fk) {
-    Vec8<T> r;
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-        const int i = kFwd ? m : 7 - m;          // di dj dk
-        const int di = i >> 2, dj = (i >> 1) & 1, dk = i & 1;
-        constexpr int in = kFwd ? 1 : 0;         // offset of a cell whose predecessor is in the tile
-        const T rk = dk == in ? r.v[i ^ 1] : fk.v[2 * di + dj];
-        const T rj = dj == in ? r.v[i ^ 2] : fj.v[2 * di + dk];
-        const T ri = di == in ? r.v[i ^ 4] : fi.v[2 * dj + dk];
-        r.v[i] = v.v[i] - ck.v[i] * rk - cj.v[i] * rj - ci.v[i] * ri;
+// What the two sweep kernels share: a CTA's grid and its tables.
+template <class L, typename T, bool kFwd>
+struct TileSweep {
+    const TileArgs<T>& a;
+    const TileShape& s;
+    int g, W, one, back;
+    int *tst, *gst, *gent;
+    using Face = Vec<T, TileFace<L>::M>;
+    Face *gval, *face;
+    const T* C;
+    T *R, *H;
+    static constexpr int side = kFwd ? 0 : 1;
+
+    __device__ __forceinline__ TileSweep(const TileArgs<T>& args, unsigned char* sm) : a(args), s(args.s) {
+        const int b = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+        g = a.glist ? a.glist[b] : b;
+        W = kFwd ? -s.w : s.w;
+        one = kFwd ? -1 : 1;
+        back = kFwd ? 0 : s.w + 1;
+        const TileLayout l = tile_layout<L, T>(s);
+        tst = reinterpret_cast<int*>(sm);
+        gst = reinterpret_cast<int*>(sm + l.gst);
+        gent = reinterpret_cast<int*>(sm + l.gent);
+        gval = reinterpret_cast<Face*>(sm + l.gval);
+        face = reinterpret_cast<Face*>(sm + l.face);
+        const long long base = (long long)g * s.npp;
+        C = a.CF + (long long)a.gcls[g] * a.cfcls;
+        R = a.R + base;
+        H = a.H + base;
     }
-    return r;
-}
+    // step t covers tiles tst[t] .. tst[t+1] forward, tst[t+1] .. tst[t] backward
+    __device__ __forceinline__ void tables() {
+        for (int t = threadIdx.x; t < s.NT + 1 + kTilePad; t += blockDim.x) {
+            tst[t] = t <= s.NT ? s.tst[kFwd ? t : s.NT - t] : (kFwd ? s.ntile : 0);
+            if (t < s.NT + 3) gst[t] = s.gst[side][t];
+        }
+    }
+    // the facing cells of the grids across (e0: the thread's first entries, loaded
+    // by the caller)
+    static constexpr int kU = 4;
+    __device__ __forceinline__ void entries(int2 e[kU], int q0) {
+#pragma unroll
+        for (int i = 0; i < kU; ++i) e[i] = __ldg(s.gent[side] + min(q0 + i * (int)blockDim.x, s.nside - 1));
+    }
+    __device__ __forceinline__ void ghosts(int2 e[kU]) {
+        int nb[3];
+        for (int d = 0; d < 3; ++d) nb[d] = a.G ? a.fnbr[6 * g + 2 * d + side] : -1;
+        for (int q0 = threadIdx.x; q0 < s.nside; q0 += kU * blockDim.x) {
+            Vec<T, L::N> v[kU];
+#pragma unroll
+            for (int i = 0; i < kU; ++i) {
+                const int d = e[i].x >> 16, n = d == 0 ? nb[0] : (d == 1 ? nb[1] : nb[2]);
+#pragma unroll
+                for (int m = 0; m < L::N; ++m) v[i].v[m] = T(0);
+                ldt(n >= 0, a.G + ((long long)max(n, 0) * s.npp + L::N * e[i].y), v[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < kU; ++i) {
+                const int m = q0 + i * (int)blockDim.x;
+                if (m < s.nside) {
+                    const int d = e[i].x >> 16;
+                    // the neighbour's high cells are my low ghosts
+                    const Face x = tile_part<L, 0, kFwd, T, TileFace<L>::M>(v[i]), y = tile_part<L, 1, kFwd, T, TileFace<L>::M>(v[i]),
+                               z = tile_part<L, 2, kFwd, T, TileFace<L>::M>(v[i]);
+                    gval[m] = d == 0 ? x : (d == 1 ? y : z);
+                    gent[m] = e[i].x;
+                }
+            }
+            entries(e, q0 + kU * (int)blockDim.x);
+        }
+    }
+    // one warp: the ghosts of step t (-1: those before the first) into their faces
+    __device__ __forceinline__ void stage(int t) {
+        const int p = kFwd ? t : s.NT - 1 - t;
+        Face* f = face + (t & 1) * 3 * s.slots;
+        const int g0 = gst[p + 1], n = gst[p + 2];
+        for (int m = g0 + (threadIdx.x & 31); m < n; m += 32)
+            f[(gent[m] >> 16) * s.slots + (gent[m] & 0xffff)] = gval[m];
+    }
+    // thread lane's loads of a step whose tiles are t0 .. t1
+    __device__ __forceinline__ void fetch(TileSet<L, T>& q, int lane, int t0, int t1) {
+        const int tile = t0 + lane;
+        const bool on = tile < t1;
+        q.tile = on ? tile : -1;
+        const int p = L::N * tile;
+        if (on) q.x = (int)__ldg(s.slot + tile);
+        ldt(on, C + p, q.c[0]);
+        ldt(on, C + s.npp + p, q.c[1]);
+        ldt(on, C + 2 * s.npp + p, q.c[2]);
+        if constexpr (kFwd) ldt_rw(on, R + p, q.v);
+        else ldt(on, R + p, q.v);
+    }
+    // the recurrence of a tile's cells in step t
+    __device__ __forceinline__ void solve(int t, const TileSet<L, T>& q, Vec<T, L::N>& r) {
+        const int x = q.x - back;
+        Face* cur = face + (t & 1) * 3 * s.slots + x;
+        const Face* prv = face + ((t + 1) & 1) * 3 * s.slots + x;
+        const Face fi = prv[W], fj = prv[s.slots + one], fk = prv[2 * s.slots];
+#pragma unroll
+        for (int m = 0; m < L::N; ++m) {
+            const int i = kFwd ? m : L::N - 1 - m;
+            const int di = i / (L::TJ * L::TK), dj = (i / L::TK) % L::TJ, dk = i % L::TK;
+            const bool ik = kFwd ? dk > 0 : dk < L::TK - 1, ij = kFwd ? dj > 0 : dj < L::TJ - 1,
+                       ii = kFwd ? di > 0 : di < L::TI - 1;
+            constexpr int o = kFwd ? -1 : 1;
+            const T rk = ik ? r.v[(i + o) & (L::N - 1)] : fk.v[di * L::TJ + dj];
+            const T rj = ij ? r.v[(i + o * L::TK) & (L::N - 1)] : fj.v[di * L::TK + dk];
+            const T ri = ii ? r.v[(i + o * L::TJ * L::TK) & (L::N - 1)] : fi.v[dj * L::TK + dk];
+            r.v[i] = q.v.v[i] - q.c[2].v[i] * rk - q.c[1].v[i] * rj - q.c[0].v[i] * ri;
+        }
+        cur[0] = tile_part<L, 0, kFwd, T, TileFace<L>::M>(r);
+        cur[s.slots] = tile_part<L, 1, kFwd, T, TileFace<L>::M>(r);
+        cur[2 * s.slots] = tile_part<L, 2, kFwd, T, TileFace<L>::M>(r);
+    }
+    template <bool kHz>
+    __device__ __forceinline__ void store(int tile, const Vec<T, L::N>& r) {
+        if constexpr (kFwd) stt(R + L::N * tile, r);
+        else if constexpr (kHz) stt(H + L::N * tile, r);
+        else addt(H + L::N * tile, r);
+    }
+};
 
 // One sweep of a grid.  kFwd: tile hyperplanes in order, res = v - lb res(k-1) -
 // ls res(j-1) - lw res(i-1) (sip_hyperplane_mod.F90:491-495); else in reverse,
 // res = res - ut res(k+1) - un res(j+1) - ue res(i+1), hilf += res (:546-547,
 // 559-567; kHz: hilf = res).  The last warp stages the ghosts.
-template <typename T, bool kFwd, bool kHz, int kD, int kThreads, int kMinBlocks>
+template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __grid_constant__ TileArgs<T> a) {
     if (a.ctl[0]) return;
     extern __shared__ __align__(32) unsigned char tsm[];
-    const TileShape& s = a.s;
-    const int b = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-    const int g = a.glist ? a.glist[b] : b;
-    const int tid = threadIdx.x, ncomp = blockDim.x - 32, NT = s.NT;
-    const int W = kFwd ? -s.w : s.w, one = kFwd ? -1 : 1, back = kFwd ? 0 : s.w + 1;
-    const TileLayout l = tile_layout<T>(s);
-    int *tst = reinterpret_cast<int*>(tsm), *gst = reinterpret_cast<int*>(tsm + l.gst),
-        *gent = reinterpret_cast<int*>(tsm + l.gent);
-    Vec4<T>*gval = reinterpret_cast<Vec4<T>*>(tsm + l.gval), *face = reinterpret_cast<Vec4<T>*>(tsm + l.face);
-    const long long base = (long long)g * s.npp;
-    const T* C = a.CF + (long long)a.gcls[g] * a.cfcls;
-    T* R = a.R + base;
-    T* H = a.H + base;
-    constexpr int side = kFwd ? 0 : 1;
-    for (int q = tid; q < NT + 1 + kTilePad; q += blockDim.x) {
-        // step t covers tiles tst[t] .. tst[t+1] forward, tst[t+1] .. tst[t] backward
-        tst[q] = q <= NT ? s.tst[kFwd ? q : NT - q] : (kFwd ? s.ntile : 0);
-        if (q < NT + 3) gst[q] = s.gst[side][q];
-    }
-    // the ghosts: the facing quads of the grids across
-    {
-        const int* fn = a.fnbr + 6 * g;
-        int nb[3];
-        for (int d = 0; d < 3; ++d) nb[d] = a.G ? fn[2 * d + side] : -1;
-        constexpr int kU = 4;
-        for (int q0 = tid; q0 < s.nside; q0 += kU * blockDim.x) {
-            int2 e[kU];
-            Vec8<T> v[kU];
-#pragma unroll
-            for (int i = 0; i < kU; ++i) {
-                e[i] = make_int2(0, 0);
-                if (q0 + i * (int)blockDim.x < s.nside) e[i] = __ldg(s.gent[side] + q0 + i * blockDim.x);
-            }
-#pragma unroll
-            for (int i = 0; i < kU; ++i) {
-                const int d = e[i].x >> 16, n = d == 0 ? nb[0] : (d == 1 ? nb[1] : nb[2]);
-#pragma unroll
-                for (int m = 0; m < 8; ++m) v[i].v[m] = T(0);
-                ld8(n >= 0, a.G + ((long long)max(n, 0) * s.npp + 8 * e[i].y), v[i]);
-            }
-#pragma unroll
-            for (int i = 0; i < kU; ++i) {
-                const int q = q0 + i * (int)blockDim.x;
-                if (q >= s.nside) break;
-                const int d = e[i].x >> 16;
-                constexpr int hi = kFwd ? 1 : 0;   // the neighbour's high cells are my low ghosts
-                gval[q] = d == 0 ? quad<0, hi>(v[i]) : (d == 1 ? quad<1, hi>(v[i]) : quad<2, hi>(v[i]));
-                gent[q] = e[i].x;
-            }
-        }
-    }
+    TileSweep<L, T, kFwd> w(a, tsm);
+    const int tid = threadIdx.x, ncomp = blockDim.x - 32, NT = a.s.NT;
+    int2 e[w.kU];
+    w.entries(e, tid);
+    w.tables();
+    w.ghosts(e);
     __syncthreads();
     if (tid >= ncomp) {
-        // the ghosts of step t (-1: those before the first) into their faces
-        auto ghosts = [&](int t) {
-            Vec4<T>* f = face + (t & 1) * 3 * s.slots;
-            const int p = kFwd ? t : NT - 1 - t;
-            const int g0 = gst[p + 1], n = gst[p + 2];
-            for (int q = g0 + (tid & 31); q < n; q += 32)
-                f[(gent[q] >> 16) * s.slots + (gent[q] & 0xffff)] = gval[q];
-        };
-        ghosts(-1);
+        w.stage(-1);
         __syncthreads();
         for (int t = 0; t < NT; ++t) {
-            ghosts(t);
+            w.stage(t);
             __syncthreads();
         }
         return;
     }
-    using Set = TileSet<T>;
-    auto fetch = [&](int t, Set& q) {
-        const int ta = tst[t], tb = tst[t + 1];
-        const int tile = (kFwd ? ta : tb) + tid;
-        const bool on = tile < (kFwd ? tb : ta);
-        q.tile = on ? tile : -1;
-        const int p = 8 * tile;
-        if (on) q.x = (int)__ldg(s.slot + tile) - back;
-        ld8(on, C + p, q.c[0]);
-        ld8(on, C + s.npp + p, q.c[1]);
-        ld8(on, C + 2 * s.npp + p, q.c[2]);
-        if constexpr (kFwd) ld8_rw(on, R + p, q.v);
-        else ld8(on, R + p, q.v);
+    // kD steps of loads in flight: a step issues the loads of kD steps on before it
+    // computes, into the set the step before has left
+    TileSet<L, T> q[kD + 1];
+    auto fetch = [&](int t, TileSet<L, T>& c) {
+        const int ta = w.tst[t], tb = w.tst[t + 1];
+        w.fetch(c, tid, kFwd ? ta : tb, kFwd ? tb : ta);
     };
-    Set q[kD];
 #pragma unroll
     for (int d = 0; d < kD; ++d) fetch(d, q[d]);
     __syncthreads();
-    auto step = [&](int t, Set& c) {
-        if (c.tile >= 0) {
-            Vec4<T>* cur = face + (t & 1) * 3 * s.slots + c.x;
-            const Vec4<T>* prv = face + ((t + 1) & 1) * 3 * s.slots + c.x;
-            const Vec4<T> fi = prv[W], fj = prv[s.slots + one], fk = prv[2 * s.slots];
-            const Vec8<T> r = tile_solve<kFwd>(c.v, c.c[0], c.c[1], c.c[2], fi, fj, fk);
-            constexpr int out = kFwd ? 1 : 0;
-            cur[0] = quad<0, out>(r);
-            cur[s.slots] = quad<1, out>(r);
-            cur[2 * s.slots] = quad<2, out>(r);
-            if constexpr (kFwd) {
-                st8(R + 8 * c.tile, r);
-            } else if constexpr (kHz) {
-                st8(H + 8 * c.tile, r);
-            } else {
-                add8(H + 8 * c.tile, r);
-            }
-        }
-        fetch(t + kD, c);
-        __syncthreads();
-    };
-    for (int t = 0; t < NT; t += kD) {
+    for (int t = 0; t < NT; t += kD + 1) {
 #pragma unroll
-        for (int d = 0; d < kD; ++d) {
+        for (int d = 0; d <= kD; ++d) {
             if (t + d >= NT) break;
-            step(t + d, q[d]);
+            fetch(t + d + kD, q[(d + kD) % (kD + 1)]);
+            if (q[d].tile >= 0) {
+                Vec<T, L::N> r;
+                w.solve(t + d, q[d], r);
+                w.template store<kHz>(q[d].tile, r);
+            }
+            __syncthreads();
         }
     }
 }
@@ -351,202 +410,131 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
 // three face loads, the recurrence and three face stores; a set stores its results
 // and issues its next loads while the other set works.  The tables, the ghosts and
 // the first tiles are loaded at once.
-template <typename T, bool kFwd, bool kHz, int kD, int kThreads>
+template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads>
 __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_constant__ TileArgs<T> a) {
     extern __shared__ __align__(32) unsigned char tsm[];
+    TileSweep<L, T, kFwd> w(a, tsm);
     const TileShape& s = a.s;
-    const int b = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-    const int g = a.glist ? a.glist[b] : b;
     const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT;
     const int set = tid >= ncomp ? 1 : 0, lane = tid - set * ncomp;   // (the last warp: neither)
-    const int W = kFwd ? -s.w : s.w, one = kFwd ? -1 : 1, back = kFwd ? 0 : s.w + 1;
-    const TileLayout l = tile_layout<T>(s);
-    int *tst = reinterpret_cast<int*>(tsm), *gst = reinterpret_cast<int*>(tsm + l.gst),
-        *gent = reinterpret_cast<int*>(tsm + l.gent);
-    Vec4<T>*gval = reinterpret_cast<Vec4<T>*>(tsm + l.gval), *face = reinterpret_cast<Vec4<T>*>(tsm + l.face);
-    const long long base = (long long)g * s.npp;
-    const T* C = a.CF + (long long)a.gcls[g] * a.cfcls;
-    T* R = a.R + base;
-    T* H = a.H + base;
-    constexpr int side = kFwd ? 0 : 1;
     const int converged = __ldg(a.ctl);
-    TileSet<T> q[kD];
-    // the loads of a step whose tiles are t0 .. t1
-    auto fetch = [&](TileSet<T>& c, int t0, int t1) {
-        const int tile = t0 + lane;
-        const bool on = tile < t1;
-        c.tile = on ? tile : -1;
-        const int p = 8 * tile;
-        if (on) c.x = (int)__ldg(s.slot + tile) - back;
-        ld8(on, C + p, c.c[0]);
-        ld8(on, C + s.npp + p, c.c[1]);
-        ld8(on, C + 2 * s.npp + p, c.c[2]);
-        if constexpr (kFwd) ld8_rw(on, R + p, c.v);
-        else ld8(on, R + p, c.v);
-    };
+    int2 e[w.kU];
+    w.entries(e, tid);
+    TileSet<L, T> q[kD];
     // first tile of step t's hyperplane and the one past its last, from global memory
     auto first = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t : NT - 1 - t)) : 0; };
     auto past = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t + 1 : NT - t)) : 0; };
-    constexpr int kU = 4;
-    int nb[3];
-    for (int d = 0; d < 3; ++d) nb[d] = a.G ? a.fnbr[6 * g + 2 * d + side] : -1;
-    int2 e[kU];
-#pragma unroll
-    for (int i = 0; i < kU; ++i)
-        e[i] = __ldg(s.gent[side] + min(tid + i * (int)blockDim.x, s.nside - 1));
     if (tid < 2 * ncomp)
 #pragma unroll
-        for (int d = 0; d < kD; ++d) fetch(q[d], first(set + 2 * d), past(set + 2 * d));
-    for (int t = tid; t < NT + 1 + kTilePad; t += blockDim.x) {
-        // step t covers tiles tst[t] .. tst[t+1] forward, tst[t+1] .. tst[t] backward
-        tst[t] = t <= NT ? s.tst[kFwd ? t : NT - t] : (kFwd ? s.ntile : 0);
-        if (t < NT + 3) gst[t] = s.gst[side][t];
-    }
-    // the ghosts: the facing quads of the grids across
-    for (int q0 = tid; q0 < s.nside; q0 += kU * blockDim.x) {
-        Vec8<T> v[kU];
-#pragma unroll
-        for (int i = 0; i < kU; ++i) {
-            const int d = e[i].x >> 16, n = d == 0 ? nb[0] : (d == 1 ? nb[1] : nb[2]);
-#pragma unroll
-            for (int m = 0; m < 8; ++m) v[i].v[m] = T(0);
-            ld8(n >= 0, a.G + ((long long)max(n, 0) * s.npp + 8 * e[i].y), v[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < kU; ++i) {
-            const int m = q0 + i * (int)blockDim.x;
-            if (m < s.nside) {
-                const int d = e[i].x >> 16;
-                constexpr int hi = kFwd ? 1 : 0;   // the neighbour's high cells are my low ghosts
-                gval[m] = d == 0 ? quad<0, hi>(v[i]) : (d == 1 ? quad<1, hi>(v[i]) : quad<2, hi>(v[i]));
-                gent[m] = e[i].x;
-            }
-            e[i] = __ldg(s.gent[side] + min(m + kU * (int)blockDim.x, s.nside - 1));
-        }
-    }
+        for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(set + 2 * d), past(set + 2 * d));
+    w.tables();
+    w.ghosts(e);
     if (converged) return;
     __syncthreads();
     const int steps = (NT + 1) & ~1;
     if (tid >= 2 * ncomp) {
-        // the ghosts of step t (-1: those before the first) into their faces
-        auto ghosts = [&](int t) {
-            Vec4<T>* f = face + (t & 1) * 3 * s.slots;
-            const int p = kFwd ? t : NT - 1 - t;
-            const int g0 = gst[p + 1], n = gst[p + 2];
-            for (int m = g0 + (tid & 31); m < n; m += 32)
-                f[(gent[m] >> 16) * s.slots + (gent[m] & 0xffff)] = gval[m];
-        };
-        ghosts(-1);
+        w.stage(-1);
         __syncthreads();
         for (int t = 0; t < steps; ++t) {
-            if (t < NT) ghosts(t);
+            if (t < NT) w.stage(t);
             __syncthreads();
         }
         return;
     }
     __syncthreads();
-    // step t of this set
-    auto work = [&](int t, TileSet<T>& c, Vec8<T>& r) {
-        if (c.tile >= 0) {
-            Vec4<T>* cur = face + (t & 1) * 3 * s.slots + c.x;
-            const Vec4<T>* prv = face + ((t + 1) & 1) * 3 * s.slots + c.x;
-            r = tile_solve<kFwd>(c.v, c.c[0], c.c[1], c.c[2], prv[W], prv[s.slots + one], prv[2 * s.slots]);
-            constexpr int out = kFwd ? 1 : 0;
-            cur[0] = quad<0, out>(r);
-            cur[s.slots] = quad<1, out>(r);
-            cur[2 * s.slots] = quad<2, out>(r);
-        }
-    };
-    // while the other set works: the results of step t to memory, the loads of the
-    // step kD turns on
-    auto rest = [&](int t, TileSet<T>& c, const Vec8<T>& r) {
-        if (c.tile >= 0) {
-            if constexpr (kFwd) st8(R + 8 * c.tile, r);
-            else if constexpr (kHz) st8(H + 8 * c.tile, r);
-            else add8(H + 8 * c.tile, r);
-        }
-        const int n = min(t + 2 * kD, NT + 1);
-        const int ta = tst[n], tb = tst[n + 1];
-        fetch(c, kFwd ? ta : tb, kFwd ? tb : ta);
-    };
-    Vec8<T> r;
+    Vec<T, L::N> r;
     if (set) __syncthreads();   // step 0
     for (int t = set; t < steps; t += 2 * kD) {
 #pragma unroll
         for (int d = 0; d < kD; ++d) {
             const int m = t + 2 * d;
             if (m >= steps) break;
-            work(m, q[d], r);
+            if (q[d].tile >= 0) w.solve(m, q[d], r);
             __syncthreads();
-            rest(m, q[d], r);
+            // while the other set works: the results to memory, the loads of the
+            // step kD turns on
+            if (q[d].tile >= 0) w.template store<kHz>(q[d].tile, r);
+            const int n = min(m + 2 * kD, NT + 1);
+            const int ta = w.tst[n], tb = w.tst[n + 1];
+            w.fetch(q[d], lane, kFwd ? ta : tb, kFwd ? tb : ta);
             if (m + 1 < steps) __syncthreads();   // the other set's step
         }
     }
 }
 
-// hilf of a tile and the facing quads around it (f = -i, +i, -j, +j, -k, +k)
-template <typename T>
+// hilf of a tile and the facing cells around it
+template <class L, typename T>
 struct TileHalo {
-    Vec8<T> h;
-    Vec4<T> f[6];
+    Vec<T, L::N> h;
+    Vec<T, L::FI> im, ip;
+    Vec<T, L::FJ> jm, jp;
+    Vec<T, L::FK> km, kp;
 };
 
-// The quad across face kF of a tile: of tile nb of the same grid (>= 0), of tile
-// -1-nb of the grid across that face, of the grid's own ghost plane, or zero.
-template <int kF, typename T>
-__device__ __forceinline__ Vec4<T> tile_face(const TileArgs<T>& a, int g, int nb, int org) {
+// The cells across face kF (-i, +i, -j, +j, -k, +k) of a tile: of tile nb of the
+// same grid (>= 0), of tile -1-nb of the grid across that face, of the grid's own
+// ghost plane, or zero.
+template <class L, int kF, typename T>
+__device__ __forceinline__ Vec<T, L::template F<kF / 2>> tile_face(const TileArgs<T>& a, int g, int nb,
+                                                                   int org) {
     const TileShape& s = a.s;
-    constexpr int ax = kF / 2, hi = kF % 2 == 0 ? 1 : 0;
+    constexpr int ax = kF / 2, nf = L::template F<ax>;
+    constexpr bool hi = kF % 2 == 0;
     int n = g;
     if (nb < 0) {
         n = a.fnbr[6 * g + kF];
         nb = -1 - nb;
         if (n < 0) {
-            Vec4<T> z{T(0), T(0), T(0), T(0)};
+            Vec<T, nf> z;
+#pragma unroll
+            for (int q = 0; q < nf; ++q) z.v[q] = T(0);
             if (a.PG) {
                 const T* P = a.PG + ((long long)g * 6 + kF) * s.fs;
                 const int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
-                const int st = ax == 2 ? s.nj : s.nk;   // stride of the second index
-                const int q = ax == 0 ? ko + jo * s.nk : (ax == 1 ? ko + io * s.nk : jo + io * s.nj);
-                // a quad runs over (dj, dk), (di, dk), (di, dj)
-                z = Vec4<T>{P[q], P[q + 1], P[q + st], P[q + st + 1]};
+                // a face runs over (dj, dk), (di, dk), (di, dj)
+                constexpr int n2 = ax == 2 ? L::TJ : L::TK;
+                const int st = ax == 2 ? s.nj : s.nk;
+                const int q0 = ax == 0 ? ko + jo * s.nk : (ax == 1 ? ko + io * s.nk : jo + io * s.nj);
+#pragma unroll
+                for (int q = 0; q < nf; ++q) z.v[q] = P[q0 + (q / n2) * st + q % n2];
             }
             return z;
         }
     }
-    const T* p = a.H + ((long long)n * s.npp + 8 * nb);
-    if constexpr (ax == 0) {
-        const Vec4<T> v = *reinterpret_cast<const Vec4<T>*>(p + 4 * hi);
-        return v;
+    const T* p = a.H + ((long long)n * s.npp + L::N * nb);
+    if constexpr (ax == 0 || nf == 1) {
+        // the face's cells are contiguous
+        return *reinterpret_cast<const Vec<T, nf>*>(p + L::template cell<ax>(0, hi));
     } else {
-        Vec8<T> v;
-        ld8(true, p, v);
-        return quad<ax, hi>(v);
+        Vec<T, L::N> v;
+        ldt(true, p, v);
+        return tile_part<L, ax, hi>(v);
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void tile_halo(const TileArgs<T>& a, int g, int tile, TileHalo<T>& o) {
+template <class L, typename T>
+__device__ __forceinline__ void tile_halo(const TileArgs<T>& a, int g, int tile, TileHalo<L, T>& o) {
     const int4 n0 = __ldg(a.s.nbr + 2 * tile), n1 = __ldg(a.s.nbr + 2 * tile + 1);
-    ld8(true, a.H + ((long long)g * a.s.npp + 8 * tile), o.h);
-    o.f[0] = tile_face<0>(a, g, n0.x, n1.z);
-    o.f[1] = tile_face<1>(a, g, n0.y, n1.z);
-    o.f[2] = tile_face<2>(a, g, n0.z, n1.z);
-    o.f[3] = tile_face<3>(a, g, n0.w, n1.z);
-    o.f[4] = tile_face<4>(a, g, n1.x, n1.z);
-    o.f[5] = tile_face<5>(a, g, n1.y, n1.z);
+    ldt(true, a.H + ((long long)g * a.s.npp + L::N * tile), o.h);
+    o.im = tile_face<L, 0>(a, g, n0.x, n1.z);
+    o.ip = tile_face<L, 1>(a, g, n0.y, n1.z);
+    o.jm = tile_face<L, 2>(a, g, n0.z, n1.z);
+    o.jp = tile_face<L, 3>(a, g, n0.w, n1.z);
+    o.km = tile_face<L, 4>(a, g, n1.x, n1.z);
+    o.kp = tile_face<L, 5>(a, g, n1.y, n1.z);
 }
 
-// the neighbours of cell i (di dj dk) of a tile: i-1, i+1, j-1, j+1, k-1, k+1
-template <typename T>
-__device__ __forceinline__ void tile_nbrs(const TileHalo<T>& o, int i, T n[6]) {
-    const int di = i >> 2, dj = (i >> 1) & 1, dk = i & 1;
-    n[0] = di ? o.h.v[i ^ 4] : o.f[0].v[2 * dj + dk];
-    n[1] = di ? o.f[1].v[2 * dj + dk] : o.h.v[i ^ 4];
-    n[2] = dj ? o.h.v[i ^ 2] : o.f[2].v[2 * di + dk];
-    n[3] = dj ? o.f[3].v[2 * di + dk] : o.h.v[i ^ 2];
-    n[4] = dk ? o.h.v[i ^ 1] : o.f[4].v[2 * di + dj];
-    n[5] = dk ? o.f[5].v[2 * di + dj] : o.h.v[i ^ 1];
+// the neighbours of cell i of a tile: i-1, i+1, j-1, j+1, k-1, k+1
+template <class L, typename T>
+__device__ __forceinline__ void tile_nbrs(const TileHalo<L, T>& o, int i, T n[6]) {
+    const int di = i / (L::TJ * L::TK), dj = (i / L::TK) % L::TJ, dk = i % L::TK;
+    constexpr int M = L::N - 1, J = L::TK, I = L::TJ * L::TK;
+    n[0] = di > 0 ? o.h.v[(i - I) & M] : o.im.v[dj * L::TK + dk];
+    n[1] = di < L::TI - 1 ? o.h.v[(i + I) & M] : o.ip.v[dj * L::TK + dk];
+    n[2] = dj > 0 ? o.h.v[(i - J) & M] : o.jm.v[di * L::TK + dk];
+    n[3] = dj < L::TJ - 1 ? o.h.v[(i + J) & M] : o.jp.v[di * L::TK + dk];
+    n[4] = dk > 0 ? o.h.v[(i - 1) & M] : o.km.v[di * L::TJ + dj];
+    n[5] = dk < L::TK - 1 ? o.h.v[(i + 1) & M] : o.kp.v[di * L::TJ + dj];
 }
 
 // The part of sipiter1 outside the recurrence, (rhs + laplacephi(hilf)) lpr
@@ -555,9 +543,10 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<T>& o, int i, T n[6]) {
 // coefficient a class.  Of the first two products one rounds by itself and the
 // other is contracted with it: the first in kOrder 0, the second in kOrder 1, as the
 // compiler does it in the packed and in the table-driven cell pre-pass.
-template <typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks>
+template <class L, typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_constant__ TileArgs<T> a) {
     if (a.ctl[0]) return;
+    constexpr int N = L::N;
     const TileShape& s = a.s;
     const int b = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
     const int g = a.glist ? a.glist[b] : b;
@@ -569,25 +558,24 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
 #pragma unroll
     for (int f = 0; f < 7; ++f) u[f] = kUni ? a.UNI[8 * cls + f] : T(0);
     for (int tile = blockIdx.x * kThreads + threadIdx.x; tile < s.ntile; tile += gridDim.x * kThreads) {
-        const int p = 8 * tile;
-        Vec8<T> rh, lp, out;
-        ld8(true, a.RHS + base + p, rh);
-        ld8(true, LPR + p, lp);
+        const int p = N * tile;
+        Vec<T, N> rh, lp, out;
+        ldt(true, a.RHS + base + p, rh);
+        ldt(true, LPR + p, lp);
         if (a.hzero) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
+            for (int i = 0; i < N; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
         } else {
-            TileHalo<T> o;
+            TileHalo<L, T> o;
             tile_halo(a, g, tile, o);
-            Vec8<T> c[kUni ? 1 : 7];
+            Vec<T, N> c[kUni ? 1 : 7];
             if constexpr (!kUni)
 #pragma unroll
-                for (int f = 0; f < 7; ++f) ld8(true, LAP + f * s.npp + p, c[f]);
+                for (int f = 0; f < 7; ++f) ldt(true, LAP + f * s.npp + p, c[f]);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                T n[6];
-                tile_nbrs(o, i, n);
-                T w[7];
+            for (int i = 0; i < N; ++i) {
+                T n[6], w[7];
+                tile_nbrs<L>(o, i, n);
 #pragma unroll
                 for (int f = 0; f < 7; ++f) w[f] = kUni ? u[f] : c[kUni ? 0 : f].v[i];
                 T lap = mul_rounded(-w[kOrder], n[kOrder]);
@@ -596,7 +584,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
                 out.v[i] = mul_rounded(rh.v[i] + lap, lp.v[i]);
             }
         }
-        st8(a.R + base + p, out);
+        stt(a.R + base + p, out);
     }
 }
 
@@ -611,17 +599,18 @@ int tile_up(Ctx* c, TileDev& d, const V** p, const std::vector<V>& h) {
     return 0;
 }
 
-// Tables of a grid of ni x nj x nk cells with kk, jj points a line (ghosts
-// included).  d.ok stays false for odd dimensions, hyperplanes of more than 512
-// tiles and shapes beyond the 10-bit cells or 16-bit slots.
-inline int tile_init(Ctx* c, int ni, int nj, int nk, TileDev& d) {
+// Tables of a grid of ni x nj x nk cells in tiles of 2^si x 2^sj x 2^sk.  d.ok
+// stays false when the tiles do not divide it, for hyperplanes of more than
+// maxtiles tiles and shapes beyond the 10-bit cells or 16-bit slots.
+inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int maxtiles, TileDev& d) {
     TileShape& s = d.s;
     s.ni = ni; s.nj = nj; s.nk = nk;
-    if (ni % 2 || nj % 2 || nk % 2 || ni > 1023 || nj > 1023 || nk > 1023) return 0;
-    const int NI = s.NI = ni / 2, NJ = s.NJ = nj / 2, NK = s.NK = nk / 2;
+    s.si = si; s.sj = sj; s.sk = sk;
+    if (ni & si || nj & sj || nk & sk || ni > 1023 || nj > 1023 || nk > 1023) return 0;
+    const int NI = s.NI = ni >> si, NJ = s.NJ = nj >> sj, NK = s.NK = nk >> sk;
     s.NT = NI + NJ + NK - 2;
     s.ntile = NI * NJ * NK;
-    s.npp = 8 * s.ntile;
+    s.npp = s.ntile << (si + sj + sk);
     s.fs = (std::max(nj * nk, std::max(ni * nk, ni * nj)) + 3) & ~3;
     s.w = NJ + 1;
     s.slots = (NI + 1) * (NJ + 1);
@@ -641,7 +630,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, TileDev& d) {
         tst[t + 1] = p;
         s.maxt = std::max(s.maxt, p - tst[t]);
     }
-    if (tst[s.NT] != s.ntile || s.maxt > 512 || s.slots > 0xffff) return 0;
+    if (tst[s.NT] != s.ntile || s.maxt > maxtiles || s.slots > 0xffff) return 0;
     auto tile = [&](int I, int J, int K) { return tpos[(size_t)(I + J + K) * NI + I] + J; };
     std::vector<int4> nbr((size_t)2 * s.ntile);
     for (int p = 0; p < s.ntile; ++p) {
@@ -653,7 +642,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, TileDev& d) {
         const int km = K > 0 ? tile(I, J, K - 1) : -1 - tile(I, J, NK - 1);
         const int kp = K < NK - 1 ? tile(I, J, K + 1) : -1 - tile(I, J, 0);
         nbr[2 * p] = make_int4(im, ip, jm, jp);
-        nbr[2 * p + 1] = make_int4(km, kp, (2 * I) | (2 * J) << 10 | (2 * K) << 20, 0);
+        nbr[2 * p + 1] = make_int4(km, kp, (I << si) | (J << sj) << 10 | (K << sk) << 20, 0);
     }
     for (int sd = 0; sd < 2; ++sd) {
         struct Entry {
@@ -702,14 +691,14 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, TileDev& d) {
             for (int io = 0; io < ni; ++io) {
                 const int jlo = std::max(0, m - io - (nk - 1)), jhi = std::min(nj - 1, m - io);
                 for (int jo = jlo; jo <= jhi; ++jo, ++q) {
-                    const int ko = m - io - jo, p = tile_pos(tpos.data(), NI, io, jo, ko);
+                    const int ko = m - io - jo, p = tile_pos(s, tpos.data(), io, jo, ko);
                     cell[p] = (ko + 2) + (jo + 2) * kk + (io + 2) * kk * jj;
                     plane[p] = q;
                 }
             }
     }
     std::vector<int> facepos((size_t)6 * s.fs, -1);
-    auto pos = [&](int io, int jo, int ko) { return tile_pos(tpos.data(), NI, io, jo, ko); };
+    auto pos = [&](int io, int jo, int ko) { return tile_pos(s, tpos.data(), io, jo, ko); };
     for (int jo = 0; jo < nj; ++jo)
         for (int ko = 0; ko < nk; ++ko) {
             facepos[0 * s.fs + ko + jo * nk] = pos(0, jo, ko);

@@ -2,7 +2,7 @@
 
 Each translation unit is compiled in parallel with nvcc; the FP64 parity
 kernels (plain_*.cu) get -fmad=false so no multiply-add is contracted, the
-mixed-precision kernels keep FMA.  The plain flux and Poisson units are
+mixed-precision kernels keep FMA.  The plain flux, Poisson and tile-solve units are
 compiled a second time with contraction (-DMG_FMA_BUILD, namespace mg::contract),
 the plain form's performance build.  Output goes next to the sources, into
 mglet-base_gb300/_build/ (git-ignored), so the library stays in-tree.
@@ -21,16 +21,16 @@ LIB = os.path.join(OUT, "libmglet_gpu.so")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 BASE = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]
-SOURCES = ["api.cu", "plain_flux.cu", "plain_poisson.cu", "plain_misc.cu", "plain_bound.cu",
+SOURCES = ["api.cu", "plain_flux.cu", "plain_poisson.cu", "plain_tile.cu", "plain_misc.cu", "plain_bound.cu",
            "plain_gc.cu", "plain_level.cu", "mixed.cu", "mixed_flux.cu", "mixed_sip.cu", "noalloc.cu",
            "adjoint.cu", "les.cu", "scalar.cu", "diag.cu", "gc_create.cu", "dist.cu", "mesh_sdf.cu",
            "mixed_level.cu"]
 # translation units whose FP64 arithmetic must not be contracted into FMAs
-NO_FMA = {"plain_flux.cu", "plain_poisson.cu", "plain_misc.cu", "plain_bound.cu", "plain_gc.cu",
+NO_FMA = {"plain_flux.cu", "plain_poisson.cu", "plain_tile.cu", "plain_misc.cu", "plain_bound.cu", "plain_gc.cu",
           "plain_level.cu", "noalloc.cu", "les.cu", "scalar.cu"}
 # compiled a second time with contraction, into namespace mg::contract (the plain
 # form's performance build, MGLET_FORM_PLAIN_FMA)
-FMA_TWINS = ["plain_flux.cu", "plain_poisson.cu"]
+FMA_TWINS = ["plain_flux.cu", "plain_poisson.cu", "plain_tile.cu"]
 
 
 def nvcc():
