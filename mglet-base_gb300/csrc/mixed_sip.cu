@@ -2186,7 +2186,7 @@ int sip_init(Ctx* c, SipState& st) {
                        cudaMemcpyHostToDevice));
     // the tables of the solver on tiles, for the shapes it takes
     st.tile = new TileDev();
-    if (int rc = tile_init(c, st.ni, st.nj, st.nk, 1, 1, 1, 512, *st.tile)) return rc;
+    if (int rc = tile_init(c, st.ni, st.nj, st.nk, 1, 1, 1, 1, 512, *st.tile)) return rc;
     if (!st.tile->ok || tile_layout<T8, float>(st.tile->s).bytes > 200 * 1024) {
         tile_free(*st.tile);
         delete st.tile;

@@ -169,6 +169,29 @@ __global__ void k_pt_conv(int ngrid, double* __restrict__ gridmax, double* stat,
 // 20^3: 54 us with one set, 60 with two).
 constexpr int kFew = 152;
 
+// Clusters of 8, 4 or 2 CTAs a grid while every CTA has an SM of its own (us a sweep):
+// one grid of 32^3 41 / 51 / 83 on 8 / 4 / 2 SMs, 84 on one; 27 grids of 24^3 34 on 4,
+// 40 on 2, 49 on one; 64 grids 40 on 2, 49 on one.
+constexpr int kRankThreads = 672, kDepth = 2;
+
+// the launch of a sweep by clusters of s.nc CTAs
+template <class K>
+int rank_config(K* k, Ctx* c, const TileShape& s, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+    const unsigned smem = tile_layout<T1, double>(s).bytes;
+    if (smem > 48 * 1024)
+        MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = s.nc;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg->gridDim = dim3(c->ngrid * s.nc);
+    cfg->blockDim = dim3(2 * ((s.maxt + 31) / 32 * 32) + 32);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = c->stream;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+    return 0;
+}
+
 template <class L, bool kFwd, bool kHz>
 int launch_sweep(Ctx* c, const TileArgs<double>& a) {
     const unsigned smem = tile_layout<L, double>(a.s).bytes;
@@ -179,6 +202,19 @@ int launch_sweep(Ctx* c, const TileArgs<double>& a) {
         k<<<c->ngrid, threads, smem, c->stream>>>(a);
         return 0;
     };
+    if constexpr (L::N == 1)
+        if (a.s.nc > 1) {
+            auto ranks = [&](auto* k) -> int {
+                cudaLaunchConfig_t cfg = {};
+                cudaLaunchAttribute at = {};
+                if (int e = rank_config(k, c, a.s, &cfg, &at)) return e;
+                MG_CUDA(cudaLaunchKernelEx(&cfg, k, a));
+                return 0;
+            };
+            if (int rc = ranks(k_tile_sweep_few<L, double, kFwd, kHz, kDepth, kRankThreads, true>)) return rc;
+            MG_LAUNCHED(c);
+            return 0;
+        }
     int rc;
     if (c->ngrid <= kFew && 2 * threads - 32 <= 1024) {
         auto few = [&](auto* k) -> int {
@@ -205,7 +241,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     const size_t bytes = (size_t)c->ngrid * s.npp * sizeof(double);
     const dim3 cells((s.npp + 255) / 256, c->ngrid), tiles((s.ntile + 127) / 128, c->ngrid);
     int* ctl = reinterpret_cast<int*>(p.stat + 1);
-    MG_CUDA(cudaMemsetAsync(p.stat, 0, 2 * sizeof(double), c->stream));
+    MG_CUDA(cudaMemsetAsync(p.stat, 0, 3 * sizeof(double), c->stream));
     MG_CUDA(cudaMemsetAsync(p.gridmax, 0, c->ngrid * sizeof(double), c->stream));
     MG_CUDA(cudaMemsetAsync(p.dp, 0, bytes, c->stream));
     k_pt_gather<<<cells, 256, 0, c->stream>>>(c->d_grids, s, c->F("RHS"), p.rhs);
@@ -221,6 +257,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     a.LAP = p.lap;
     a.UNI = p.uni;
     a.ctl = ctl;
+    a.err = ctl + 2;
     PtOuterArgs o{};
     o.RHS = p.rhs;
     o.DP = p.dp;
@@ -274,7 +311,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
         }
         // a long outer loop looks now and then whether it has converged
         if (ip % 12 == 0 && ip < c->prm.nouter) {
-            MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+            MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
             MG_CUDA(cudaStreamSynchronize(c->stream));
             if (reinterpret_cast<const int*>(p.h_stat + 1)[0]) break;
         }
@@ -285,11 +322,15 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     else
         k_pt_scatter<L, false><<<tiles, 128, 0, c->stream>>>(o, c->d_grids, c->F("RHS"), c->F("DP"), c->F("RES"));
     MG_LAUNCHED(c);
-    MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     // dp ghosts: the reference accumulates the connected hilf ghosts into dp
     if (int rc = connect(c, 0, 1, nullptr, nullptr, nullptr, c->F("DP"), nullptr, nullptr, false, false, 0))
         return rc;
     MG_CUDA(cudaStreamSynchronize(c->stream));
+    if (reinterpret_cast<const int*>(p.h_stat + 2)[0]) {
+        set_error("mgpoisl: a sweep waited for another CTA in vain");
+        return MGLET_ERR_CUDA;
+    }
     if (st) {
         st->nouter_done = reinterpret_cast<const int*>(p.h_stat + 1)[1];
         st->ipc = st->nouter_done * ninner;
@@ -366,8 +407,24 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
         return 0;
     };
     const int ni = G0.ii - 4, nj = G0.jj - 4, nk = G0.kk - 4;
-    p->pair = nk % 2 == 0;
-    if (int rc = tile_init(c, ni, nj, nk, 0, 0, p->pair, 992, p->t)) return rc;
+    // few grids: as many SMs to a grid as there are, if the clusters fit at once
+    for (int nc = 8; nc > 1 && !p->t.ok; nc /= 2) {
+        if (nc * c->ngrid > 152 || nc > ni) continue;
+        if (int rc = tile_init(c, ni, nj, nk, 0, 0, 0, nc, (kRankThreads - 32) / 2, p->t)) return rc;
+        int fit = 0;
+        if (p->t.ok && tile_layout<T1, double>(p->t.s).bytes <= 220 * 1024) {
+            auto* k = k_tile_sweep_few<T1, double, true, false, kDepth, kRankThreads, true>;
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at = {};
+            if (int rc = rank_config(k, c, p->t.s, &cfg, &at)) return rc;
+            MG_CUDA(cudaOccupancyMaxActiveClusters(&fit, k, &cfg));
+        }
+        if (fit < c->ngrid) tile_free(p->t);
+    }
+    if (!p->t.ok) {
+        p->pair = nk % 2 == 0;
+        if (int rc = tile_init(c, ni, nj, nk, 0, 0, p->pair, 1, 992, p->t)) return rc;
+    }
     if (!p->t.ok) return give_up();
     const TileShape& s = p->t.s;
     const unsigned smem = p->pair ? tile_layout<Tile<1, 1, 2>, double>(s).bytes
@@ -402,7 +459,7 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
     auto pad = [](size_t n) { return (n + 31) & ~(size_t)31; };
     const size_t n = pad((size_t)c->ngrid * s.npp), m = (size_t)p->ncls * s.npp;
     const size_t cls[3] = {pad(4 * m), pad(3 * m), pad(7 * m)};
-    const size_t all = 6 * n + cls[0] + cls[1] + cls[2] + pad(8 * p->ncls) + pad(c->ngrid) + pad(2);
+    const size_t all = 6 * n + cls[0] + cls[1] + cls[2] + pad(8 * p->ncls) + pad(c->ngrid) + pad(3);
     MG_CUDA(cudaMalloc(&p->mem, all * sizeof(double)));
     double* q = p->mem;
     auto take = [&](double** d, size_t len) {
@@ -415,8 +472,8 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
     take(&p->lap, cls[2]);
     take(&p->uni, pad(8 * p->ncls));
     take(&p->gridmax, pad(c->ngrid));
-    take(&p->stat, pad(2));
-    MG_CUDA(cudaMallocHost(&p->h_stat, 2 * sizeof(double)));
+    take(&p->stat, pad(3));
+    MG_CUDA(cudaMallocHost(&p->h_stat, 3 * sizeof(double)));
     int* d_reps = nullptr;
     if (int rc = up(&d_reps, reps)) return rc;
     k_pt_extract<<<dim3((s.npp + 255) / 256, p->ncls), 256, 0, c->stream>>>(

@@ -36,18 +36,19 @@ struct TileShape {
     int si, sj, sk;                 // log2 of the tile's extents (0 or 1)
     int NI, NJ, NK, NT, ntile;      // tiles; tile hyperplanes; tiles in all
     int npp, fs;                    // cells of a grid's array; length of a face array
-    int maxt;                       // tiles of the largest hyperplane
+    int nc;                         // CTAs of a sweep (a cluster); rank I nc / NI takes the tiles of row I
+    int maxt;                       // most tiles of a rank in a hyperplane
     int w, slots;                   // NJ + 1; (NI + 1)(NJ + 1)
-    int nside;                      // ghost tiles on the three low (or high) faces
-    const int* tst;                 // [NT+1] first tile of each hyperplane
+    int nside;                      // most ghost tiles of a rank on the three low (or high) faces
+    const int* tst;                 // [NT*nc+1] first tile of each hyperplane and rank
     const unsigned short* slot;     // [ntile, padded to 4] slot of the tile
     // [ntile][2]: tiles at i-1, i+1, j-1, j+1 | k-1, k+1, cell (io, jo, ko) of the
     // tile's first cell (10 bits each), 0; a negative entry -1-t is tile t of the
     // grid across that face
     const int4* nbr;
-    // ghost tiles on the low and high faces by extended hyperplane: gst[s][p+1] ..
-    // gst[s][p+2] those of hyperplane p (-1 .. NT); {slot | axis << 16, tile of the
-    // grid across the face}
+    // ghost tiles on the low and high faces by rank and extended hyperplane: of the
+    // rank's, gst[s][p+1] .. gst[s][p+2] those of hyperplane p (-1 .. NT), [NT+3] the
+    // rank's first ([nc][NT+4]); {slot | axis << 16, tile of the grid across the face}
     const int* gst[2];
     const int2* gent[2];
     const int* tpos;                // [NT][NI] tile (I, J) of hyperplane T is tpos[T*NI+I] + J
@@ -197,31 +198,38 @@ struct TileArgs {
     const T* UNI;                   // [ncls][8] operator coefficients of uniform classes
     const int* ctl;                 // [0] converged: nothing to do
     int cfcls, lprcls;              // values between the classes of CF and of LPR
+    int* err;                       // set when a rank waited in vain
     int hzero;                      // hilf is zero
     int rev;                        // walk the grids in reverse block order
 };
 
 constexpr int kTilePad = 8;         // empty hyperplanes past the last in the table of starts
 
-// Shared memory of a sweep: [tst] [gst] [ghost entries] [ghost faces] [2][3][slots]
-// faces (of equal size for the three axes, so that a ghost is one copy)
+// Shared memory of a sweep: [tst] [ends, if ranks share the hyperplanes] [gst] [ghost entries] [ghost faces] [2][3][slots]
+// faces (of equal size for the three axes, so that a ghost is one copy) [faces of the
+// row before the rank's, [NJ][NK]] [their mbarriers]
 template <class L>
 struct TileFace {   // values of the largest face
     static constexpr int M = L::FI > L::FJ ? (L::FI > L::FK ? L::FI : L::FK) : (L::FJ > L::FK ? L::FJ : L::FK);
 };
 struct TileLayout {
-    unsigned gst, gent, gval, face, bytes;
+    unsigned tend, gst, gent, gval, face, bnd, mbar, bytes;
 };
 template <class L, typename T>
 __host__ __device__ inline TileLayout tile_layout(const TileShape& s) {
     auto up = [](unsigned v) { return (v + 31u) & ~31u; };
     constexpr unsigned fb = TileFace<L>::M * sizeof(T);
-    TileLayout l;
+    TileLayout l{};
     unsigned o = (s.NT + 1 + kTilePad) * 4;
+    l.tend = o; if (s.nc > 1) o += (s.NT + 1 + kTilePad) * 4;
     l.gst = o; o = up(o + (s.NT + 3) * 4);
     l.gent = o; o = up(o + s.nside * 4);
     l.gval = o; o = up(o + s.nside * fb);
     l.face = o; o += 6 * s.slots * fb;
+    if (s.nc > 1) {
+        l.bnd = o; o = up(o + s.NJ * s.NK * fb);
+        l.mbar = o; o += (s.NJ + s.NK - 1) * 8;
+    }
     l.bytes = o;
     return l;
 }
@@ -233,31 +241,79 @@ struct TileSet {
     Vec<T, L::N> c[3], v;
 };
 
-// What the two sweep kernels share: a CTA's grid and its tables.
-template <class L, typename T, bool kFwd>
+// the shared memory of another CTA of the cluster
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+template <int N>
+__device__ __forceinline__ void cluster_put(unsigned a, unsigned mbar, const Vec<double, N>& v) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(a + 8 * i),
+                     "d"(v.v[i]), "r"(mbar)
+                     : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// What the sweep kernels share: a CTA's grid and its tables (kRanks: its rank's part).
+template <class L, typename T, bool kFwd, bool kRanks = false>
 struct TileSweep {
     const TileArgs<T>& a;
     const TileShape& s;
     int g, W, one, back;
-    int *tst, *gst, *gent;
+    int rank, nent, ent0;           // rank in the cluster; its ghosts and the first of them
+    int t0, t1;                     // its steps
+    int i0, i1;                     // its rows
+    bool up, down;                  // does a rank before, after it take part?
+    int *tst, *tend, *gst, *gent;
     using Face = Vec<T, TileFace<L>::M>;
-    Face *gval, *face;
+    Face *gval, *face, *bnd;
+    unsigned mbar, bndto, mbarto;   // its mbarriers; bnd and mbarriers of the rank after
     const T* C;
     T *R, *H;
     static constexpr int side = kFwd ? 0 : 1;
 
     __device__ __forceinline__ TileSweep(const TileArgs<T>& args, unsigned char* sm) : a(args), s(args.s) {
-        const int b = a.rev ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+        const int nb = kRanks ? gridDim.x / s.nc : gridDim.x, b0 = kRanks ? blockIdx.x / s.nc : blockIdx.x;
+        const int b = a.rev ? nb - 1 - b0 : b0;
+        rank = kRanks ? blockIdx.x % s.nc : 0;
         g = a.glist ? a.glist[b] : b;
         W = kFwd ? -s.w : s.w;
         one = kFwd ? -1 : 1;
         back = kFwd ? 0 : s.w + 1;
         const TileLayout l = tile_layout<L, T>(s);
         tst = reinterpret_cast<int*>(sm);
+        tend = reinterpret_cast<int*>(sm + l.tend);
         gst = reinterpret_cast<int*>(sm + l.gst);
         gent = reinterpret_cast<int*>(sm + l.gent);
         gval = reinterpret_cast<Face*>(sm + l.gval);
         face = reinterpret_cast<Face*>(sm + l.face);
+        t0 = 0;
+        t1 = s.NT;
+        nent = s.nside;
+        ent0 = 0;
+        if constexpr (kRanks) {
+            const int* gr = s.gst[side] + rank * (s.NT + 4);
+            nent = __ldg(gr + s.NT + 2);
+            ent0 = __ldg(gr + s.NT + 3);
+            i0 = (rank * s.NI + s.nc - 1) / s.nc;
+            i1 = ((rank + 1) * s.NI + s.nc - 1) / s.nc - 1;
+            const int last = i1 + s.NJ + s.NK - 2;   // hyperplane
+            t0 = kFwd ? i0 : s.NT - 1 - last;
+            t1 = (kFwd ? last : s.NT - 1 - i0) + 1;
+            up = kFwd ? rank > 0 : rank < s.nc - 1;
+            down = kFwd ? rank < s.nc - 1 : rank > 0;
+            bnd = reinterpret_cast<Face*>(sm + l.bnd);
+            mbar = (unsigned)__cvta_generic_to_shared(sm + l.mbar);
+            const int to = down ? (kFwd ? rank + 1 : rank - 1) : rank;
+            bndto = cluster_addr(bnd, to);
+            mbarto = cluster_addr(sm + l.mbar, to);
+        }
         const long long base = (long long)g * s.npp;
         C = a.CF + (long long)a.gcls[g] * a.cfcls;
         R = a.R + base;
@@ -266,8 +322,14 @@ struct TileSweep {
     // step t covers tiles tst[t] .. tst[t+1] forward, tst[t+1] .. tst[t] backward
     __device__ __forceinline__ void tables() {
         for (int t = threadIdx.x; t < s.NT + 1 + kTilePad; t += blockDim.x) {
-            tst[t] = t <= s.NT ? s.tst[kFwd ? t : s.NT - t] : (kFwd ? s.ntile : 0);
-            if (t < s.NT + 3) gst[t] = s.gst[side][t];
+            if constexpr (kRanks) {
+                const int* x = s.tst + (kFwd ? t : s.NT - 1 - t) * s.nc + rank;
+                tst[t] = t < s.NT ? x[0] : 0;
+                tend[t] = t < s.NT ? x[1] : 0;
+            } else {
+                tst[t] = t <= s.NT ? s.tst[kFwd ? t : s.NT - t] : (kFwd ? s.ntile : 0);
+            }
+            if (t < s.NT + 3) gst[t] = s.gst[side][rank * (s.NT + 4) + t];
         }
     }
     // the facing cells of the grids across (e0: the thread's first entries, loaded
@@ -275,12 +337,12 @@ struct TileSweep {
     static constexpr int kU = 4;
     __device__ __forceinline__ void entries(int2 e[kU], int q0) {
 #pragma unroll
-        for (int i = 0; i < kU; ++i) e[i] = __ldg(s.gent[side] + min(q0 + i * (int)blockDim.x, s.nside - 1));
+        for (int i = 0; i < kU; ++i) e[i] = __ldg(s.gent[side] + ent0 + max(min(q0 + i * (int)blockDim.x, nent - 1), 0));
     }
     __device__ __forceinline__ void ghosts(int2 e[kU]) {
         int nb[3];
         for (int d = 0; d < 3; ++d) nb[d] = a.G ? a.fnbr[6 * g + 2 * d + side] : -1;
-        for (int q0 = threadIdx.x; q0 < s.nside; q0 += kU * blockDim.x) {
+        for (int q0 = threadIdx.x; q0 < nent; q0 += kU * blockDim.x) {
             Vec<T, L::N> v[kU];
 #pragma unroll
             for (int i = 0; i < kU; ++i) {
@@ -292,7 +354,7 @@ struct TileSweep {
 #pragma unroll
             for (int i = 0; i < kU; ++i) {
                 const int m = q0 + i * (int)blockDim.x;
-                if (m < s.nside) {
+                if (m < nent) {
                     const int d = e[i].x >> 16;
                     // the neighbour's high cells are my low ghosts
                     const Face x = tile_part<L, 0, kFwd, T, TileFace<L>::M>(v[i]), y = tile_part<L, 1, kFwd, T, TileFace<L>::M>(v[i]),
@@ -311,6 +373,46 @@ struct TileSweep {
         const int g0 = gst[p + 1], n = gst[p + 2];
         for (int m = g0 + (threadIdx.x & 31); m < n; m += 32)
             f[(gent[m] >> 16) * s.slots + (gent[m] & 0xffff)] = gval[m];
+    }
+    // The faces of the row before arrive with their own completion: one mbarrier for
+    // each of the row's hyperplanes J + K, armed once for the bytes of its faces.
+    __device__ __forceinline__ int row_lo(int h) const { return max(0, h - (s.NK - 1)); }
+    __device__ __forceinline__ int row_hi(int h) const { return min(s.NJ - 1, h); }
+    __device__ __forceinline__ void arm() {
+        if (up)
+            for (int h = threadIdx.x; h < s.NJ + s.NK - 1; h += blockDim.x) {
+                const unsigned m = mbar + 8 * h;
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(m) : "memory");
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(m),
+                             "r"((row_hi(h) - row_lo(h) + 1) * (int)sizeof(Face))
+                             : "memory");
+            }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // one warp, in step t: stages the faces the rank before has put in step t.  The wait
+    // for them ends after kSpin looks: then the error flag is set and nothing waits
+    // any more.
+    static constexpr int kSpin = 1 << 20;
+    __device__ __forceinline__ void boundary(int t, bool& lost) {
+        if (!up) return;
+        const int I = kFwd ? i0 - 1 : i1 + 1, h = (kFwd ? t : s.NT - 1 - t) - I;
+        const int lo = row_lo(h), hi = row_hi(h);
+        if (lo > hi) return;
+        for (int n = 0; !lost; ++n) {
+            int ok;
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+                         " selp.s32 %0, 1, 0, p;\n}"
+                         : "=r"(ok)
+                         : "r"(mbar + 8 * h)
+                         : "memory");
+            if (__all_sync(0xffffffffu, ok)) break;
+            if (n >= kSpin) {
+                lost = true;
+                if ((threadIdx.x & 31) == 0) *a.err = 1;
+            }
+        }
+        Face* f = face + (t & 1) * 3 * s.slots + (kFwd ? (I + 1) * s.w + 1 : I * s.w);
+        for (int J = lo + (threadIdx.x & 31); J <= hi; J += 32) f[J] = bnd[J * s.NK + h - J];
     }
     // thread lane's loads of a step whose tiles are t0 .. t1
     __device__ __forceinline__ void fetch(TileSet<L, T>& q, int lane, int t0, int t1) {
@@ -344,6 +446,13 @@ struct TileSweep {
             r.v[i] = q.v.v[i] - q.c[2].v[i] * rk - q.c[1].v[i] * rj - q.c[0].v[i] * ri;
         }
         cur[0] = tile_part<L, 0, kFwd, T, TileFace<L>::M>(r);
+        if constexpr (kRanks) {
+            // the row the next rank starts from
+            const int I = kFwd ? i1 : i0, J = q.x - (I + 1) * s.w - 1;
+            const int h = (kFwd ? t : s.NT - 1 - t) - I;
+            if (down && J >= 0 && J < s.NJ)
+                cluster_put(bndto + (J * s.NK + h - J) * (unsigned)sizeof(Face), mbarto + 8 * h, cur[0]);
+        }
         cur[s.slots] = tile_part<L, 1, kFwd, T, TileFace<L>::M>(r);
         cur[2 * s.slots] = tile_part<L, 2, kFwd, T, TileFace<L>::M>(r);
     }
@@ -410,56 +519,76 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
 // three face loads, the recurrence and three face stores; a set stores its results
 // and issues its next loads while the other set works.  The tables, the ghosts and
 // the first tiles are loaded at once.
-template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads>
+//
+// kRanks: the rows of a grid's tile lattice are shared by the CTAs of a cluster, so
+// that a step has the FP64 pipes of nc SMs.  A rank puts the faces of its last row
+// into a plane in the next rank's shared memory, where they complete an mbarrier; it
+// never waits for that rank, so the way from SM to SM delays the start of a rank once and
+// not every step.  Us a sweep of one grid of 32^3 on 8 SMs: 41; with a cluster barrier
+// in every step 63; with a released step counter in place of the mbarriers 72.
+template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, bool kRanks = false>
 __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_constant__ TileArgs<T> a) {
     extern __shared__ __align__(32) unsigned char tsm[];
-    TileSweep<L, T, kFwd> w(a, tsm);
+    TileSweep<L, T, kFwd, kRanks> w(a, tsm);
     const TileShape& s = a.s;
-    const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT;
+    const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT, t0 = w.t0, t1 = w.t1;
     const int set = tid >= ncomp ? 1 : 0, lane = tid - set * ncomp;   // (the last warp: neither)
     const int converged = __ldg(a.ctl);
     int2 e[w.kU];
     w.entries(e, tid);
     TileSet<L, T> q[kD];
     // first tile of step t's hyperplane and the one past its last, from global memory
-    auto first = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t : NT - 1 - t)) : 0; };
-    auto past = [&](int t) { return t < NT ? __ldg(s.tst + (kFwd ? t + 1 : NT - t)) : 0; };
+    const int nc = kRanks ? s.nc : 1;
+    auto first = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank) : 0; };
+    auto past = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank + 1) : 0; };
     if (tid < 2 * ncomp)
 #pragma unroll
-        for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(set + 2 * d), past(set + 2 * d));
+        for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(t0 + set + 2 * d), past(t0 + set + 2 * d));
     w.tables();
+    if constexpr (kRanks) w.arm();
     w.ghosts(e);
-    if (converged) return;
-    __syncthreads();
-    const int steps = (NT + 1) & ~1;
+    if (converged) return;   // (every rank of a cluster or none)
+    if constexpr (kRanks) cluster_barrier();
+    else __syncthreads();
+    const int end = t0 + ((t1 - t0 + 1) & ~1);
     if (tid >= 2 * ncomp) {
-        w.stage(-1);
+        bool lost = false;
+        w.stage(t0 - 1);
+        if constexpr (kRanks) w.boundary(t0 - 1, lost);
         __syncthreads();
-        for (int t = 0; t < steps; ++t) {
-            if (t < NT) w.stage(t);
+        for (int t = t0; t < end; ++t) {
+            if (t < t1) w.stage(t);
+            if constexpr (kRanks)
+                if (t < t1 - 1) w.boundary(t, lost);
             __syncthreads();
         }
+        if constexpr (kRanks) cluster_barrier();   // no rank ends while another may put into it
         return;
     }
     __syncthreads();
     Vec<T, L::N> r;
-    if (set) __syncthreads();   // step 0
-    for (int t = set; t < steps; t += 2 * kD) {
+    if (set) __syncthreads();   // the first step
+    for (int t = t0 + set; t < end; t += 2 * kD) {
 #pragma unroll
         for (int d = 0; d < kD; ++d) {
             const int m = t + 2 * d;
-            if (m >= steps) break;
+            if (m >= end) break;
             if (q[d].tile >= 0) w.solve(m, q[d], r);
             __syncthreads();
             // while the other set works: the results to memory, the loads of the
             // step kD turns on
             if (q[d].tile >= 0) w.template store<kHz>(q[d].tile, r);
             const int n = min(m + 2 * kD, NT + 1);
-            const int ta = w.tst[n], tb = w.tst[n + 1];
-            w.fetch(q[d], lane, kFwd ? ta : tb, kFwd ? tb : ta);
-            if (m + 1 < steps) __syncthreads();   // the other set's step
+            if constexpr (kRanks) {
+                w.fetch(q[d], lane, w.tst[n], w.tend[n]);
+            } else {
+                const int ta = w.tst[n], tb = w.tst[n + 1];
+                w.fetch(q[d], lane, kFwd ? ta : tb, kFwd ? tb : ta);
+            }
+            if (m + 1 < end) __syncthreads();   // the other set's step
         }
     }
+    if constexpr (kRanks) cluster_barrier();
 }
 
 // hilf of a tile and the facing cells around it
@@ -602,8 +731,9 @@ int tile_up(Ctx* c, TileDev& d, const V** p, const std::vector<V>& h) {
 // Tables of a grid of ni x nj x nk cells in tiles of 2^si x 2^sj x 2^sk.  d.ok
 // stays false when the tiles do not divide it, for hyperplanes of more than
 // maxtiles tiles and shapes beyond the 10-bit cells or 16-bit slots.
-inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int maxtiles, TileDev& d) {
+inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int nc, int maxtiles, TileDev& d) {
     TileShape& s = d.s;
+    s.nc = nc;
     s.ni = ni; s.nj = nj; s.nk = nk;
     s.si = si; s.sj = sj; s.sk = sk;
     if (ni & si || nj & sj || nk & sk || ni > 1023 || nj > 1023 || nk > 1023) return 0;
@@ -614,12 +744,11 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
     s.fs = (std::max(nj * nk, std::max(ni * nk, ni * nj)) + 3) & ~3;
     s.w = NJ + 1;
     s.slots = (NI + 1) * (NJ + 1);
-    s.nside = NI * NJ + NI * NK + NJ * NK;
-    std::vector<int> tst(s.NT + 1, 0), tpos((size_t)s.NT * NI, 0);
+    std::vector<int> tst(1, 0), tpos((size_t)s.NT * NI, 0);
     std::vector<unsigned short> slot((s.ntile + 3) & ~3, 0);
     std::vector<int> ti(s.ntile), tj(s.ntile), tk(s.ntile);
-    for (int t = 0, p = 0; t < s.NT; ++t) {
-        for (int I = 0; I < NI; ++I) {
+    for (int t = 0, p = 0; t < s.NT; ++t) for (int r = 0; r < nc; ++r) {
+        for (int I = (r * NI + nc - 1) / nc; I < ((r + 1) * NI + nc - 1) / nc; ++I) {
             const int jlo = std::max(0, t - I - (NK - 1)), jhi = std::min(NJ - 1, t - I);
             tpos[(size_t)t * NI + I] = p - jlo;
             for (int J = jlo; J <= jhi; ++J, ++p) {
@@ -627,10 +756,10 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
                 slot[p] = (unsigned short)((I + 1) * s.w + J + 1);
             }
         }
-        tst[t + 1] = p;
-        s.maxt = std::max(s.maxt, p - tst[t]);
+        s.maxt = std::max(s.maxt, p - tst.back());
+        tst.push_back(p);
     }
-    if (tst[s.NT] != s.ntile || s.maxt > maxtiles || s.slots > 0xffff) return 0;
+    if (tst.back() != s.ntile || s.maxt > maxtiles || s.slots > 0xffff) return 0;
     auto tile = [&](int I, int J, int K) { return tpos[(size_t)(I + J + K) * NI + I] + J; };
     std::vector<int4> nbr((size_t)2 * s.ntile);
     for (int p = 0; p < s.ntile; ++p) {
@@ -646,7 +775,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
     }
     for (int sd = 0; sd < 2; ++sd) {
         struct Entry {
-            int p;
+            int r, p;
             int2 e;
         };
         std::vector<Entry> gs;
@@ -654,7 +783,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
         // I w + J the backward sweep uses
         auto add = [&](int ax, int I, int J, int K, int t) {
             const int x = sd == 0 ? (I + 1) * s.w + J + 1 : I * s.w + J;
-            gs.push_back(Entry{I + J + K, make_int2(x | (ax << 16), t)});
+            gs.push_back(Entry{(ax > 0 ? I : (sd ? NI - 1 : 0)) * nc / NI, I + J + K, make_int2(x | (ax << 16), t)});
         };
         for (int J = 0; J < NJ; ++J)
             for (int K = 0; K < NK; ++K)
@@ -666,19 +795,25 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
             for (int J = 0; J < NJ; ++J)
                 add(2, I, J, sd ? NK : -1, sd ? tile(I, J, 0) : tile(I, J, NK - 1));
         std::stable_sort(gs.begin(), gs.end(), [](const Entry& a, const Entry& b) {
+            if (a.r != b.r) return a.r < b.r;
             if (a.p != b.p) return a.p < b.p;
             if ((a.e.x >> 16) != (b.e.x >> 16)) return (a.e.x >> 16) < (b.e.x >> 16);
             return a.e.y < b.e.y;
         });
-        std::vector<int> gst(s.NT + 3, 0);
+        std::vector<int> gst;
         std::vector<int2> gent;
         size_t q = 0;
-        for (int p = -1; p <= s.NT; ++p) {
-            gst[p + 1] = (int)q;
-            for (; q < gs.size() && gs[q].p == p; ++q) gent.push_back(gs[q].e);
+        for (int r = 0; r < nc; ++r) {
+            const int first = (int)q;
+            for (int p = -1; p <= s.NT; ++p) {
+                gst.push_back((int)q - first);
+                for (; q < gs.size() && gs[q].r == r && gs[q].p == p; ++q) gent.push_back(gs[q].e);
+            }
+            gst.push_back((int)q - first);
+            gst.push_back(first);
+            s.nside = std::max(s.nside, (int)q - first);
         }
-        gst[s.NT + 2] = (int)q;
-        if ((int)q != s.nside) return 0;
+        if (q != gs.size()) return 0;
         if (int rc = tile_up(c, d, &s.gst[sd], gst)) return rc;
         if (int rc = tile_up(c, d, &s.gent[sd], gent)) return rc;
     }

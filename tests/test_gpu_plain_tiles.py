@@ -1,7 +1,8 @@
 """The plain form's pressure solve on tiles (the default on one level) against the
 per-operator kernels (taken when the caller sets a coefficient field, here BP to the
 ones it holds anyway): the same bits at the edges of the tile hyperplanes, in pairs
-(even k extents) and single cells, with few and many grids, on walls and graded
+(even k extents) and single cells, with grids on one SM and shared by 2, 4 and 8 (row
+counts that do not divide), on walls and graded
 grids, and when the outer loop stops early or runs past a look at its flag."""
 import numpy as np
 import pytest
@@ -40,7 +41,7 @@ def _same(gpu_lib, case, form, **kw):
 SHAPES = [
     ((2, 1, 1), (2, 2, 2)), ((1, 1, 1), (2, 3, 5)), ((1, 2, 2), (2, 16, 6)), ((2, 1, 2), (11, 2, 7)),
     ((2, 2, 2), (24, 24, 24)), ((1, 1, 2), (33, 29, 31)), ((1, 1, 1), (40, 36, 44)),
-    ((6, 6, 5), (8, 10, 12)), ((6, 6, 5), (9, 8, 7))]
+    ((3, 3, 3), (10, 9, 8)), ((4, 4, 4), (5, 6, 8)), ((6, 6, 5), (8, 10, 12)), ((6, 6, 5), (9, 8, 7))]
 
 
 @pytest.mark.parametrize("tiles,shape", SHAPES)
