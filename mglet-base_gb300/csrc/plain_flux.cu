@@ -256,6 +256,12 @@ __device__ double wo_point(int k, int j, int i, int kk, int jj, const double* u,
     return wo;
 }
 
+__device__ __forceinline__ bool all_connected(const DevGrid& G) {
+    bool r = true;
+    for (int f = 0; f < 6; ++f) r = r && G.bc[f] == 7;
+    return r;
+}
+
 // tstle4 over the full box of every grid: points outside the reference's
 // loop ranges get 0, as tstle4 zeroes uo, vo, wo before its loops.
 __global__ void __launch_bounds__(256) k_tstle4(const DevGrid* __restrict__ grids, Spacing sp,
@@ -267,9 +273,11 @@ __global__ void __launch_bounds__(256) k_tstle4(const DevGrid* __restrict__ grid
                                                 const double* __restrict__ P, const double* __restrict__ Gf,
                                                 Wall wl, double iles, double gx, double gy, double gz,
                                                 const double* __restrict__ FX, const double* __restrict__ FY,
-                                                const double* __restrict__ FZ, const double* __restrict__ GU) {
+                                                const double* __restrict__ FZ, const double* __restrict__ GU,
+                                                const double* __restrict__ redo) {
     const int gi = blockIdx.y;
     const DevGrid G = grids[gi];
+    if (redo && redo[gi] == 0.0) return;   // k_tstle4_march has done it
     const int kk = G.kk, jj = G.jj, ii = G.ii;
     const int npts = kk * jj * ii;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -328,6 +336,250 @@ __global__ void __launch_bounds__(256) k_tstle4(const DevGrid* __restrict__ grid
     wo[o + t] = rw;
 }
 
+// ---- tstle4 of grids between other grids -------------------------------------
+// Most grids have six connected faces, one value of G and no model term.  There a
+// face flux of one cell is, operation for operation, that of its neighbour across the
+// face (qe(i) = qw(i+1), ...), so each is computed once: a thread keeps a column
+// (k, j) and marches in i, the fluxes through its i face stay in registers, those
+// through its j and k faces reach the neighbours through shared memory.  The model
+// term st*0 is zero for finite fields and falls away; a grid with a result that is not
+// finite is left to k_tstle4, as one with several values of G is.
+// Bound by the FP64 pipe (ncu: busy all the time on the SMs with a CTA): 526
+// instructions a point and its faces in k_tstle4, about 150 here.  512 grids of 24^3
+// contracted 6.15 -> 2.72 ms, 64 grids uncontracted 0.95 -> 0.45, 216 of 20^3 1.84 ->
+// 0.74.
+
+// (a comparison of doubles is an FP64 instruction, one of their words is not)
+__device__ __forceinline__ bool is_zero(double x) {
+    return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+
+// x / 2: the exponent less one, an integer operation, where that is exact
+__device__ __forceinline__ double half_of(double x) {
+    const int hi = __double2hiint(x), lo = __double2loint(x), e = hi & 0x7ff00000;
+    if (e > 0x00100000 && e < 0x7ff00000) return __hiloint2double(hi - 0x00100000, lo);
+    return is_zero(x) ? x : x * 0.5;
+}
+
+// x / d with r = RN(1 / d): Markstein's correction (P. Markstein, IBM J. Res. Dev. 34,
+// 1990) -- after one step the quotient is within an ulp, after the second it is the
+// correctly rounded one, for operands whose products stay normal.  mid: d is one of
+// them.
+__device__ __forceinline__ bool mid_range(double x) {
+    return (unsigned)((__double2hiint(x) >> 20) & 0x7ff) - 523u < 1000u;   // 2^-500 .. 2^499
+}
+__device__ __forceinline__ double div_by(double x, double d, double r, bool mid) {
+    if (is_zero(x)) return x;   // (d > 0)
+    if (!mid || !mid_range(x)) return x / d;
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-d, q, x), r, q);
+    return __fma_rn(__fma_rn(-d, q, x), r, q);
+}
+
+struct MarchArgs {
+    const DevGrid* grids;
+    Spacing sp;
+    double *uo, *vo, *wo;
+    const double *U, *V, *W, *P, *G, *FX, *FY, *FZ, *GU;
+    Wall wl;
+    double* redo;                  // [ngrid] not 0: k_tstle4 does the grid
+    double gx, gy, gz;
+    int rows, nrow, len, nchunk;   // rows and planes of a CTA; CTAs along j and i
+};
+
+// what a plane of constant i needs
+struct MarchPlane {
+    double dx, ddx, rdx, rddx;
+    double ddxe, rddxe, rcp;       // ddx and rddx at i+1, 1 / ddx(i+1)
+    double pu, gdx;                // 1/(rho dx), gpx dx
+};
+// products of a plane with a row k or j: face areas, and with the viscosity
+struct MarchK {
+    double ayu, ayv, ayw, nyu, nyv, nyw;
+};
+struct MarchJ {
+    double azu, azv, azw, nzu, nzv, nzw, fu, fv, fw;   // f: 1/rho and the spacings but k's
+};
+
+constexpr int kMarchThreads = 640;
+
+__device__ __forceinline__ GridPtrs march_spacing(const MarchArgs& a, const DevGrid& G) {
+    GridPtrs s;
+    s.kk = G.kk; s.jj = G.jj; s.ii = G.ii;
+    s.dx = a.sp.dx + G.ipx - 1; s.dy = a.sp.dy + G.ipy - 1; s.dz = a.sp.dz + G.ipz - 1;
+    s.ddx = a.sp.ddx + G.ipx - 1; s.ddy = a.sp.ddy + G.ipy - 1; s.ddz = a.sp.ddz + G.ipz - 1;
+    s.rdx = a.sp.rdx + G.ipx - 1; s.rdy = a.sp.rdy + G.ipy - 1; s.rdz = a.sp.rdz + G.ipz - 1;
+    s.rddx = a.sp.rddx + G.ipx - 1; s.rddy = a.sp.rddy + G.ipy - 1; s.rddz = a.sp.rddz + G.ipz - 1;
+    return s;
+}
+
+__global__ void __launch_bounds__(kMarchThreads) k_tstle4_march(const __grid_constant__ MarchArgs a) {
+    const int gi = blockIdx.y;
+    const DevGrid G = a.grids[gi];
+    if (!all_connected(G) || a.GU[2 * gi] == 0.0) return;
+    extern __shared__ __align__(16) unsigned char msm[];
+    const int kk = G.kk, jj = G.jj, ii = G.ii, nt = blockDim.x, tid = threadIdx.x;
+    const int row = blockIdx.x % a.nrow, chunk = blockIdx.x / a.nrow;
+    const int ja = 3 + row * a.rows, je = min(ja + a.rows - 1, jj - 2);
+    const int ia = 3 + chunk * a.len, ie = min(ia + a.len - 1, ii - 2);
+    const long long o = G.ip3;
+    double *uo = a.uo + o, *vo = a.vo + o, *wo = a.wo + o;
+    const double *u = a.U + o, *v = a.V + o, *w = a.W + o, *p = a.P + o;
+    const GridPtrs s = march_spacing(a, G);
+    const double gfl = (double)G.gradpflag, rho = a.wl.rho;
+    const double gx = a.gx * gfl, gy = a.gy * gfl, gz = a.gz * gfl;
+    // the ghost layers: zero (tstle4 zeroes uo, vo, wo before its loops)
+    {
+        const int j0 = ja == 3 ? 1 : ja, j1 = je == jj - 2 ? jj : je;
+        const int i0 = ia == 3 ? 1 : ia, i1 = ie == ii - 2 ? ii : ie;
+        for (int t = tid; t < (j1 - j0 + 1) * kk; t += nt) {
+            const int k = t % kk + 1, j = t / kk + j0;
+            const bool shell = k < 3 || k > kk - 2 || j < 3 || j > jj - 2;
+            for (int i = i0; i <= i1; ++i)
+                if (shell || i < 3 || i > ii - 2) {
+                    const long long c = IX(k, j, i);
+                    uo[c] = 0.0;
+                    vo[c] = 0.0;
+                    wo[c] = 0.0;
+                }
+        }
+    }
+    const int nk1 = kk - 3;
+    const int k = 2 + tid % nk1, j = ja - 1 + tid / nk1;
+    const bool on = j <= je, out = on && k >= 3 && j >= ja;
+    const double g0 = A((a.G + o), 3, 3, 3), h2 = a.GU[2 * gi + 1], ir = 1.0 / rho;
+    // faces: [2][12][nt]; planes ia-1 .. ie
+    double* face = reinterpret_cast<double*>(msm);
+    MarchPlane* pl = reinterpret_cast<MarchPlane*>(face + 24 * nt);
+    bool mid = true;
+    for (int q = tid; q <= ie - ia + 1; q += nt) {
+        const int i = ia - 1 + q;
+        MarchPlane m;
+        m.dx = s.dx[i]; m.ddx = s.ddx[i]; m.rdx = s.rdx[i]; m.rddx = s.rddx[i];
+        m.ddxe = s.ddx[i + 1]; m.rddxe = s.rddx[i + 1];
+        m.rcp = 1.0 / m.ddxe;
+        m.pu = 1.0 / (rho * m.dx);
+        m.gdx = gx * m.dx;
+        mid = mid && mid_range(m.ddxe);
+        pl[q] = m;
+    }
+    MarchK* pk = reinterpret_cast<MarchK*>(pl + a.len + 1);
+    MarchJ* pj = reinterpret_cast<MarchJ*>(pk + (a.len + 1) * nk1);
+    const int nj1 = je - ja + 2;
+    for (int t = tid; t < (ie - ia + 2) * nk1; t += nt) {
+        const int i = ia - 1 + t / nk1, kq = 2 + t % nk1;
+        MarchK m;
+        m.ayu = s.dx[i] * s.ddz[kq]; m.nyu = -h2 * m.ayu;
+        m.ayv = s.ddx[i] * s.ddz[kq]; m.nyv = -g0 * m.ayv;
+        m.ayw = s.ddx[i] * s.dz[kq]; m.nyw = -h2 * m.ayw;
+        pk[t] = m;
+    }
+    for (int t = tid; t < (ie - ia + 2) * nj1; t += nt) {
+        const int i = ia - 1 + t / nj1, jq = ja - 1 + t % nj1;
+        MarchJ m;
+        m.azu = s.dx[i] * s.ddy[jq]; m.nzu = -h2 * m.azu;
+        m.azv = s.ddx[i] * s.dy[jq]; m.nzv = -h2 * m.azv;
+        m.azw = s.ddx[i] * s.ddy[jq]; m.nzw = -g0 * m.azw;
+        m.fu = ir * s.rddy[jq] * s.rdx[i];
+        m.fv = ir * s.rddx[i] * s.rdy[jq];
+        m.fw = ir * s.rddx[i] * s.rddy[jq];
+        pj[t] = m;
+    }
+    double dy = 1.0, ddy = 1.0, rdy = 1.0, rddy = 1.0, ddyn = 1.0, rddyn = 1.0;
+    double dz = 1.0, ddz = 1.0, rdz = 1.0, rddz = 1.0, ddzt = 1.0, rddzt = 1.0;
+    if (on) {
+        dy = s.dy[j]; ddy = s.ddy[j]; rdy = s.rdy[j]; rddy = s.rddy[j]; ddyn = s.ddy[j + 1]; rddyn = s.rddy[j + 1];
+        dz = s.dz[k]; ddz = s.ddz[k]; rdz = s.rdz[k]; rddz = s.rddz[k]; ddzt = s.ddz[k + 1]; rddzt = s.rddz[k + 1];
+        mid = mid && mid_range(ddyn) && mid_range(ddzt);
+    }
+    mid = __syncthreads_and(mid);
+    const double rcpy = 1.0 / ddyn, rcpz = 1.0 / ddzt;
+    const double pv = 1.0 / (rho * dy), pw = 1.0 / (rho * dz), gdy = gy * dy, gdz = gz * dz;
+    const double axu = ddy * ddz, axv = dy * ddz, axw = ddy * dz;
+    const double eu = -g0 * axu, ev = -h2 * axv, ew = -h2 * axw;
+    double u0 = 0.0, v0 = 0.0, w0 = 0.0, p0 = 0.0;
+    long long c = IX(k, j, ia - 1);
+    const int sj = kk, si = kk * jj;
+    if (on) {
+        u0 = u[c]; v0 = v[c]; w0 = w[c];
+        p0 = p[c + si];
+    }
+    double cw[3] = {0.0, 0.0, 0.0}, dw[3] = {0.0, 0.0, 0.0};   // through the face before
+    for (int q = 0; q <= ie - ia + 1; ++q) {
+        const MarchPlane& m = pl[q];
+        const MarchK& mk = pk[q * nk1 + k - 2];
+        const MarchJ& mj = pj[q * nj1 + min(j - ja + 1, nj1 - 1)];
+        double ce[3], de[3], u1 = 0.0, v1 = 0.0, w1 = 0.0;
+        if (on) {
+            const double un = u[c + sj], uk = u[c + 1], vk = v[c + 1], vn = v[c + sj], wn = w[c + sj], wk = w[c + 1];
+            u1 = u[c + si]; v1 = v[c + si]; w1 = w[c + si];
+            double f;
+            // i face
+            f = axu * (u0 + div_by(half_of(u1 - u0) * m.dx, m.ddxe, m.rcp, mid));
+            ce[0] = half_of(f) * (u0 + u1);
+            f = half_of(axv * (u0 + un));
+            ce[1] = half_of(f) * (v0 + v1);
+            f = half_of(axw * (u0 + uk));
+            ce[2] = half_of(f) * (w0 + w1);
+            de[0] = eu * m.rddxe * (u1 - u0);
+            de[1] = ev * m.rdx * (v1 - v0);
+            de[2] = ew * m.rdx * (w1 - w0);
+            if (q > 0) {
+                double* x = face + (q & 1) * 12 * nt + tid;
+                f = half_of(mk.ayu * (v0 + v1));
+                x[0] = half_of(f) * (u0 + un);
+                x[nt] = mk.nyu * rdy * (un - u0);
+                f = half_of(mj.azu * (w0 + w1));
+                x[2 * nt] = half_of(f) * (u0 + uk);
+                x[3 * nt] = mj.nzu * rdz * (uk - u0);
+                f = mk.ayv * (v0 + div_by(half_of(vn - v0) * dy, ddyn, rcpy, mid));
+                x[4 * nt] = half_of(f) * (v0 + vn);
+                x[5 * nt] = mk.nyv * rddyn * (vn - v0);
+                f = half_of(mj.azv * (w0 + wn));
+                x[6 * nt] = half_of(f) * (v0 + vk);
+                x[7 * nt] = mj.nzv * rdz * (vk - v0);
+                f = half_of(mk.ayw * (v0 + vk));
+                x[8 * nt] = half_of(f) * (w0 + wn);
+                x[9 * nt] = mk.nyw * rdy * (wn - w0);
+                f = mj.azw * (w0 + div_by(half_of(wk - w0) * dz, ddzt, rcpz, mid));
+                x[10 * nt] = half_of(f) * (w0 + wk);
+                x[11 * nt] = mj.nzw * rddzt * (wk - w0);
+            }
+        }
+        __syncthreads();
+        if (out && q > 0) {
+            const double* x = face + (q & 1) * 12 * nt + tid;
+            // fluxes through the faces: e w (this thread), n s (row before), t b (k before)
+            auto sum = [&](int f, double e, double ww) {
+                return e - ww + x[f * nt] - x[f * nt - nk1] + x[(f + 2) * nt] - x[(f + 2) * nt - 1];
+            };
+            double ru = -sum(0, ce[0], cw[0]) * m.rdx * rddy * rddz;
+            ru = ru - mj.fu * rddz * sum(1, de[0], dw[0]);
+            ru = ru - m.pu * (p[c + si] - p0 + m.gdx);
+            double rv = -sum(4, ce[1], cw[1]) * m.rddx * rdy * rddz;
+            rv = rv - mj.fv * rddz * sum(5, de[1], dw[1]);
+            rv = rv - pv * (p[c + sj] - p0 + gdy);
+            double rw = -sum(8, ce[2], cw[2]) * m.rddx * rddy * rdz;
+            rw = rw - mj.fw * rdz * sum(9, de[2], dw[2]);
+            rw = rw - pw * (p[c + 1] - p0 + gdz);
+            if (!is_finite(ru) || !is_finite(rv) || !is_finite(rw)) a.redo[gi] = 1.0;
+            // the steady body force (when set) follows gradp
+            uo[c] = a.FX ? ru + a.FX[o + c] : ru;
+            vo[c] = a.FY ? rv + a.FY[o + c] : rv;
+            wo[c] = a.FZ ? rw + a.FZ[o + c] : rw;
+            p0 = p[c + si];
+        }
+        u0 = u1; v0 = v1; w0 = w1;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) {
+            cw[f] = ce[f];
+            dw[f] = de[f];
+        }
+        c += si;
+    }
+}
+
 // rkstep: dp = frhs*dp + rhs; p = p + dtfu*dp over the whole flat array.
 __global__ void k_rkstep(double* __restrict__ p, double* __restrict__ dp,
                          const double* __restrict__ rhs, double frhs, double dtfu, long long n) {
@@ -358,7 +610,7 @@ static Spacing spacing(Ctx* c) {
 // bits.  Without an LES model G is gmol there on grids without walls.
 __global__ void k_g_uniform(const DevGrid* __restrict__ grids, const double* __restrict__ Gf, double gmol,
                             double* __restrict__ out) {
-    const DevGrid G = grids[blockIdx.x];
+    const DevGrid G = grids[blockIdx.x];   // (behind the pairs: 1 where k_tstle4 has to run)
     const int kk = G.kk, jj = G.jj, ii = G.ii;
     const int nk = kk - 2, nj = jj - 2, ni = ii - 2;
     const double* g = Gf + G.ip3;
@@ -371,6 +623,7 @@ __global__ void k_g_uniform(const DevGrid* __restrict__ grids, const double* __r
     bad = __syncthreads_or(bad);
     if (threadIdx.x == 0) {
         const double h = hm(g0, g0, gmol);
+        out[2 * gridDim.x + blockIdx.x] = bad || !all_connected(G) ? 1.0 : 0.0;
         out[2 * blockIdx.x] = bad ? 0.0 : 1.0;
         out[2 * blockIdx.x + 1] = bad ? 0.0 : h + h;
     }
@@ -390,6 +643,49 @@ static int max_points(Ctx* c) {
     return m;
 }
 
+// Threads of k_tstle4_march: rows + 1 rows of k = 2 .. kk-2
+static int march_threads(int rows, int kk) { return ((rows + 1) * (kk - 3) + 31) / 32 * 32; }
+
+static size_t march_smem(int rows, int len, int kk) {
+    return (size_t)24 * march_threads(rows, kk) * sizeof(double) +
+           (len + 1) * (sizeof(MarchPlane) + (kk - 3) * sizeof(MarchK) + (rows + 1) * sizeof(MarchJ));
+}
+constexpr size_t kMarchSmem = 220 * 1024;
+
+// How k_tstle4_march cuts the grids: as many rows a CTA as its threads hold (the row
+// before the first is computed twice), and planes so that the CTAs fill the SMs
+// evenly (the fluxes through the first i face twice).  Returns the grids it takes:
+// equal dimensions, all six faces connected.
+static int march_shape(Ctx* c, MarchArgs* m) {
+    int n = 0;
+    for (const DevGrid& G : c->grids) {
+        bool con = true;
+        for (int f = 0; f < 6; ++f) con = con && G.bc[f] == 7;
+        n += con;
+    }
+    const DevGrid& G = c->grids[0];
+    const int nk1 = G.kk - 3, nj = G.jj - 4, ni = G.ii - 4;
+    if (!c->uniform || n == 0 || 2 * nk1 > kMarchThreads) return 0;
+    const int most = kMarchThreads / nk1 - 1;
+    m->nrow = (nj + most - 1) / most;
+    m->rows = (nj + m->nrow - 1) / m->nrow;
+    double best = 0.0;
+    for (int len = 1; len <= ni; ++len) {
+        if (march_smem(m->rows, len, G.kk) > kMarchSmem) break;
+        const int nchunk = (ni + len - 1) / len;
+        const long long waves = ((long long)n * m->nrow * nchunk + 151) / 152;
+        const double t = (double)waves * (len + 0.5);
+        if (best == 0.0 || t <= best) {
+            best = t;
+            m->len = len;
+            m->nchunk = nchunk;
+        }
+    }
+    // the last rows and planes of the cut may be empty
+    m->nrow = (nj + m->rows - 1) / m->rows;
+    return n;
+}
+
 int launch_tstle4(Ctx* c, double* uo, double* vo, double* wo, const double* u, const double* v,
                   const double* w, const double* ut, const double* vt, const double* wt,
                   const double* p, const double* g) {
@@ -407,12 +703,31 @@ int launch_tstle4(Ctx* c, double* uo, double* vo, double* wo, const double* u, c
     wl.cpo5 = 0.5 * cpo1 * std::pow(cwa, cpo2 / cpo1) * std::pow(gmol / rho, cpo2);
     wl.cpo6 = 0.5 * gmol / rho * std::pow(cwa, 2.0 / cpo1);
     wl.cpo8 = 2.0 / cpo2;
+    MarchArgs m{};
+    if (int n = march_shape(c, &m); n > 0 && u == ut && v == vt && w == wt && !c->ilesmodel) {
+        m.grids = c->d_grids;
+        m.sp = spacing(c);
+        m.uo = uo; m.vo = vo; m.wo = wo;
+        m.U = u; m.V = v; m.W = w; m.P = p; m.G = g;
+        if (c->bodyforce) {
+            m.FX = c->F("FBX"); m.FY = c->F("FBY"); m.FZ = c->F("FBZ");
+        }
+        m.GU = c->d_guni;
+        m.redo = c->d_guni + 2 * c->ngrid;
+        m.wl = wl;
+        m.gx = c->prm.gradp[0]; m.gy = c->prm.gradp[1]; m.gz = c->prm.gradp[2];
+        const int threads = march_threads(m.rows, c->grids[0].kk);
+        const size_t smem = march_smem(m.rows, m.len, c->grids[0].kk);
+        MG_CUDA(cudaFuncSetAttribute(k_tstle4_march, cudaFuncAttributeMaxDynamicSharedMemorySize, kMarchSmem));
+        k_tstle4_march<<<dim3(m.nrow * m.nchunk, c->ngrid), threads, smem, c->stream>>>(m);
+        MG_LAUNCHED(c);
+    }
     k_tstle4<<<grid, 256, 0, c->stream>>>(c->d_grids, spacing(c), uo, vo, wo, u, v, w, ut, vt, wt, p, g,
                                           wl, c->ilesmodel ? 1.0 : 0.0, c->prm.gradp[0], c->prm.gradp[1],
                                           c->prm.gradp[2],
                                           c->bodyforce ? c->F("FBX") : nullptr,
                                           c->bodyforce ? c->F("FBY") : nullptr,
-                                          c->bodyforce ? c->F("FBZ") : nullptr, c->d_guni);
+                                          c->bodyforce ? c->F("FBZ") : nullptr, c->d_guni, m.redo);
     MG_LAUNCHED(c);
     // tstle4_mod.F90:114: tstle4_par after kon, diff and gradp (PAR faces)
     return launch_tstle4_par(c, uo, vo, wo, u, v, w, ut, vt, wt);
