@@ -155,8 +155,8 @@ int enqueue_mgpoisl(Ctx* c) {
     const LevelState& lv = m->lv;
     const bool multi = c->minlevel != c->maxlevel;
     double *U = c->F("U"), *V = c->F("V"), *W = c->F("W"), *P = c->F("P"), *dp = c->F("DP");
-    MG_CUDA(cudaMemsetAsync(s.dph, 0, (size_t)c->ngrid * s.npp * sizeof(float), c->stream));
-    MG_CUDA(cudaMemsetAsync(s.dpl, 0, (size_t)c->ngrid * s.npp * sizeof(float), c->stream));
+    MG_CUDA(cudaMemsetAsync(s.dph, 0, (size_t)c->ngrid * sip_npp(s) * sizeof(float), c->stream));
+    MG_CUDA(cudaMemsetAsync(s.dpl, 0, (size_t)c->ngrid * sip_npp(s) * sizeof(float), c->stream));
     // converged flag and outer count; the error flag ctl[2] is cleared when
     // the stage (or the solve) starts
     MG_CUDA(cudaMemsetAsync(m->d_ctl, 0, 2 * sizeof(int), c->stream));

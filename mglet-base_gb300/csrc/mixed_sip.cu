@@ -1393,6 +1393,13 @@ __global__ void k_tile_extract(const DevGrid* __restrict__ grids, const int* __r
     const int rep = reps[cls];
     const DevGrid G = grids[rep];
     const int id = s.cell[p];
+    if (id < 0) {   // a pad
+        for (int q = 0; q < 4; ++q) CF[(cls * 4 + q) * s.npp + p] = 0.f;
+        for (int q = 0; q < 3; ++q) CB[(cls * 3 + q) * s.npp + p] = 0.f;
+        for (int q = 0; q < 7; ++q) LAP[(cls * 7 + q) * s.npp + p] = 0.f;
+        APX[cls * 2 * s.npp + p] = APX[(cls * 2 + 1) * s.npp + p] = 0.f;
+        return;
+    }
     const long long src = G.ip3 + (planeorder ? s.plane[p] : id);
     const float f[4] = {(float)lw[src], (float)ls[src], (float)lb[src], (float)lpr[src]};
     const float b[3] = {(float)ue[src], (float)un[src], (float)ut[src]};
@@ -1425,6 +1432,7 @@ struct TileOuterArgs {
 // accumulate_pcorr, see k_sip_outer): one thread a tile, the tiles of a grid in
 // gridDim.x CTAs; gridmax takes the maximum over them (a maximum of non-negative
 // numbers, as integers).
+template <bool kPad>
 __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ TileOuterArgs a) {
     if (a.t.ctl[0]) return;
     __shared__ float shm[4];
@@ -1438,7 +1446,7 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
     for (int tile = blockIdx.x * 128 + threadIdx.x; tile < s.ntile; tile += gridDim.x * 128) {
         const int p = 8 * tile;
         TileHalo<T8, float> o;
-        tile_halo(a.t, g, tile, o);
+        tile_halo<kPad>(a.t, g, tile, o);
         const int org = __ldg(s.nbr + 2 * tile + 1).z;
         const int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
         Vec<float, 8> aph, apl, rh8, rl8, dh8, dl8;
@@ -1490,6 +1498,12 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
             two_sum(dh, de, dh, dl);
             dh8.v[i] = dh;
             dl8.v[i] = dl;
+            if constexpr (kPad) {
+                if (io + d[0] >= s.ni || jo + d[1] >= s.nj || ko + d[2] >= s.nk) {
+                    rh8.v[i] = rl8.v[i] = 0.f;
+                    continue;
+                }
+            }
             mx = fmaxf(mx, fabsf(rh));
         }
         stt(a.RHS + base + p, rh8);
@@ -1899,8 +1913,8 @@ int sip_tune(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl) {
     }
     // the timing launches wrote the inner solver's arrays; leave them zeroed
     for (int r = 0; r < 3; ++r)
-        MG_CUDA(cudaMemsetAsync(st.rs[r], 0, (size_t)c->ngrid * st.npp * sizeof(float), c->stream));
-    MG_CUDA(cudaMemsetAsync(st.h32, 0, (size_t)c->ngrid * st.npp * sizeof(float), c->stream));
+        MG_CUDA(cudaMemsetAsync(st.rs[r], 0, (size_t)c->ngrid * sip_npp(st) * sizeof(float), c->stream));
+    MG_CUDA(cudaMemsetAsync(st.h32, 0, (size_t)c->ngrid * sip_npp(st) * sizeof(float), c->stream));
     return 0;
 }
 
@@ -1971,8 +1985,8 @@ static int tile_threads(const SipState& st) { return (st.tile->s.maxt + 31) / 32
 // CTAs a grid of the kernels with one thread a tile
 static int tile_parts(const SipState& st, int threads) { return (st.tile->s.ntile + threads - 1) / threads; }
 
-template <bool kFwd, bool kHz>
-static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
+template <bool kFwd, bool kHz, bool kPad>
+static int launch_tile_sweep_of(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
     const unsigned smem = tile_layout<T8, float>(a.s).bytes;
     auto go = [&](auto* k) -> int {
         if (smem > 48 * 1024)
@@ -1987,11 +2001,25 @@ static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int n
             k<<<ng, 2 * tile_threads(st) - 32, smem, s>>>(a);
             return 0;
         };
-        if (tile_threads(st) <= 160) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 2, 288>);
-        if (tile_threads(st) <= 288) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 1, 544>);
+        if (tile_threads(st) <= 160) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 2, 288, false, kPad>);
+        if (tile_threads(st) <= 288) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 1, 544, false, kPad>);
     }
-    if (tile_threads(st) <= 160) return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 160, 4>);
-    return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 544, 1>);
+    if (tile_threads(st) <= 160) return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 160, 4, kPad>);
+    return go(k_tile_sweep<T8, float, kFwd, kHz, 1, 544, 1, kPad>);
+}
+
+template <bool kFwd, bool kHz>
+static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
+    return a.s.pad ? launch_tile_sweep_of<kFwd, kHz, true>(st, a, ng, s)
+                   : launch_tile_sweep_of<kFwd, kHz, false>(st, a, ng, s);
+}
+
+template <bool kPad>
+static void launch_tile_pre(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
+    const dim3 grid(tile_parts(st, 128), ng);
+    if (st.unicls) k_tile_pre<T8, float, true, 0, 128, 6, kPad><<<grid, 128, 0, s>>>(a);
+    else if (st.prepk) k_tile_pre<T8, float, false, 0, 128, 4, kPad><<<grid, 128, 0, s>>>(a);
+    else k_tile_pre<T8, float, false, 1, 128, 4, kPad><<<grid, 128, 0, s>>>(a);
 }
 
 bool sip_on_tiles(const SipState& st) {
@@ -2008,6 +2036,8 @@ PosMap sip_posmap(const SipState& st) {
 }
 
 const int* sip_facepos(const SipState& st) { return sip_on_tiles(st) ? st.tile->s.facepos : st.d_facepos; }
+
+int sip_npp(const SipState& st) { return st.tile ? std::max(st.npp, st.tile->s.npp) : st.npp; }
 
 int sip_init(Ctx* c, SipState& st) {
     const DevGrid& G0 = c->grids[0];
@@ -2208,7 +2238,7 @@ int sip_init(Ctx* c, SipState& st) {
     // -1: its hilf and res ghosts read as zero, as the reference's ghost
     // layers that no exchange writes stay zero through mgpoisl
     if (int rc = up(&st.d_fnbr, fn)) return rc;
-    const size_t n = (size_t)c->ngrid * st.npp;
+    const size_t n = (size_t)c->ngrid * sip_npp(st);
     for (float** p : {&st.h32, &st.rs[0], &st.rs[1], &st.rs[2], &st.rhs32}) {
         MG_CUDA(cudaMalloc(p, n * sizeof(float)));
         MG_CUDA(zero_on(c->stream, *p, n * sizeof(float)));
@@ -2374,10 +2404,8 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
             a.LPR = st.tcf + 3 * ts.npp;
             a.lprcls = 4 * ts.npp;
             a.hzero = hzero ? 1 : 0;
-            const dim3 grid(tile_parts(st, 128), ng);
-            if (st.unicls) k_tile_pre<T8, float, true, 0, 128, 6><<<grid, 128, 0, c->stream>>>(a);
-            else if (st.prepk) k_tile_pre<T8, float, false, 0, 128, 4><<<grid, 128, 0, c->stream>>>(a);
-            else k_tile_pre<T8, float, false, 1, 128, 4><<<grid, 128, 0, c->stream>>>(a);
+            if (ts.pad) launch_tile_pre<true>(st, a, ng, c->stream);
+            else launch_tile_pre<false>(st, a, ng, c->stream);
             MG_LAUNCHED(c);
         }
         ProfScope ps_(c, "mx_sip_fwd");
@@ -2493,7 +2521,9 @@ int sip_outer(Ctx* c, SipState& st, const float* apx, const int* gcls, const int
         }
         a.grids = c->d_grids;
         a.gridmax = c->d_gridred;
-        k_tile_outer<<<dim3(tile_parts(st, 128), c->ngrid), 128, 0, c->stream>>>(a);
+        const dim3 grid(tile_parts(st, 128), c->ngrid);
+        if (st.tile->s.pad) k_tile_outer<true><<<grid, 128, 0, c->stream>>>(a);
+        else k_tile_outer<false><<<grid, 128, 0, c->stream>>>(a);
         MG_LAUNCHED(c);
         return 0;
     }
@@ -2699,7 +2729,7 @@ int sip_tune_solve(Ctx* c, SipState& st, const float* cf, const float* apx, cons
                   std::vector<double>(st.solve_var_ms, st.solve_var_ms + kNumSolve)};
     // the timing runs wrote the solver's arrays; leave them zeroed
     for (float* p : {st.rs[0], st.rs[1], st.rs[2], st.h32, st.rhs32, st.rhsl, st.dph, st.dpl})
-        MG_CUDA(cudaMemsetAsync(p, 0, (size_t)c->ngrid * st.npp * sizeof(float), c->stream));
+        MG_CUDA(cudaMemsetAsync(p, 0, (size_t)c->ngrid * sip_npp(st) * sizeof(float), c->stream));
     MG_CUDA(cudaMemsetAsync(ctl, 0, 3 * sizeof(int), c->stream));
     return done(cudaSuccess, "");
 }

@@ -38,7 +38,7 @@ struct SipState {
     int* d_wb = nullptr;
     float4* swf = nullptr;      // [ncls][npp]
     float4* swb = nullptr;
-    // grids of even dimensions: the solver on 2x2x2 tiles (sip_tile.cuh): tables,
+    // the solver on 2x2x2 tiles (sip_tile.cuh): tables,
     // and per class {lw, ls, lb, lpr}, {ue, un, ut}, the seven operator
     // coefficients and ap in two floats, npp values each; tbm the open couplings of
     // the ghost-cell IB
@@ -117,6 +117,7 @@ struct PosMap {
 };
 PosMap sip_posmap(const SipState& st);
 const int* sip_facepos(const SipState& st);
+int sip_npp(const SipState& st);   // length of a grid's array, for either order
 int sip_init(Ctx* c, SipState& st);
 // Class coefficients: FP32 blocks [lw|ls|lb|lpr|ap] and [ue|un|ut] per padded
 // plane, and ap split in two floats [hi npp | lo npp], from the representative

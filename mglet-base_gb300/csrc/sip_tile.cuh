@@ -1,8 +1,7 @@
 // sip_tile.cuh -- the SIP solver on small tiles of cells, in FP32 (mixed form,
 // 2x2x2) and FP64 (plain form, 1x1x2 or single cells).
 //
-// A grid is cut into tiles of TI x TJ x TK cells (its dimensions must divide),
-// stored tile after tile in the order of the hyperplanes I+J+K of the tile
+// A grid is cut into tiles of TI x TJ x TK cells, stored tile after tile in the order of the hyperplanes I+J+K of the tile
 // lattice, the values of a tile together, k fastest.  A sweep walks the tile
 // hyperplanes, one thread a tile, one CTA a grid: 34 steps for 24^3 cells in tiles
 // of 2x2x2 where the cell hyperplanes take 70, and the points of a tile pass their
@@ -14,6 +13,12 @@
 // the predecessors are at the constant offsets -(NJ+1), -1 and 0 of the plane
 // before.  The arithmetic of a point and its order are those of the cell sweeps
 // (sip_hyperplane_mod.F90:450-569), so the results are the same bits.
+//
+// An odd dimension leaves pads in the last tiles.  Their coefficients are zero, so a
+// sweep passes through a pad what its array holds there: the backward sweep first
+// writes the ghosts of that side into the pads of res, the pre-pass and the outer
+// step take them for the pads of hilf, and the forward sweep has no successor that
+// reads a pad.
 //
 // What bounds it: FP32, the chain of the steps (few grids) and the issue of the
 // loads (many); all global loads of a step are issued kD steps ahead.  FP64, the
@@ -34,6 +39,7 @@ namespace mg {
 struct TileShape {
     int ni, nj, nk;                 // cells
     int si, sj, sk;                 // log2 of the tile's extents (0 or 1)
+    int pad;                        // axes (bit 0: i) where the last tile holds one cell and a pad
     int NI, NJ, NK, NT, ntile;      // tiles; tile hyperplanes; tiles in all
     int npp, fs;                    // cells of a grid's array; length of a face array
     int nc;                         // CTAs of a sweep (a cluster); rank I nc / NI takes the tiles of row I
@@ -52,8 +58,8 @@ struct TileShape {
     const int* gst[2];
     const int2* gent[2];
     const int* tpos;                // [NT][NI] tile (I, J) of hyperplane T is tpos[T*NI+I] + J
-    const int* cell;                // [npp] natural local index of each position
-    const int* plane;               // [npp] its position in the cell hyperplane order
+    const int* cell;                // [npp] natural local index of each position, -1 in pads
+    const int* plane;               // [npp] its position in the cell hyperplane order, -1 in pads
     const int* facepos;             // [6][fs] position of the boundary cell of each face index
 };
 
@@ -261,7 +267,7 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 
 // What the sweep kernels share: a CTA's grid and its tables (kRanks: its rank's part).
-template <class L, typename T, bool kFwd, bool kRanks = false>
+template <class L, typename T, bool kFwd, bool kRanks = false, bool kPad = false>
 struct TileSweep {
     const TileArgs<T>& a;
     const TileShape& s;
@@ -334,7 +340,7 @@ struct TileSweep {
     }
     // the facing cells of the grids across (e0: the thread's first entries, loaded
     // by the caller)
-    static constexpr int kU = 4;
+    static constexpr int kU = 4, M = TileFace<L>::M;
     __device__ __forceinline__ void entries(int2 e[kU], int q0) {
 #pragma unroll
         for (int i = 0; i < kU; ++i) e[i] = __ldg(s.gent[side] + ent0 + max(min(q0 + i * (int)blockDim.x, nent - 1), 0));
@@ -349,7 +355,10 @@ struct TileSweep {
                 const int d = e[i].x >> 16, n = d == 0 ? nb[0] : (d == 1 ? nb[1] : nb[2]);
 #pragma unroll
                 for (int m = 0; m < L::N; ++m) v[i].v[m] = T(0);
-                ldt(n >= 0, a.G + ((long long)max(n, 0) * s.npp + L::N * e[i].y), v[i]);
+                // (in the launches that write pads, the arrays' other cells are read here)
+                const T* src = a.G + ((long long)max(n, 0) * s.npp + L::N * (kPad ? e[i].y & 0xffff : e[i].y));
+                if constexpr (kPad && !kFwd) ldt_rw(n >= 0, src, v[i]);
+                else ldt(n >= 0, src, v[i]);
             }
 #pragma unroll
             for (int i = 0; i < kU; ++i) {
@@ -357,8 +366,32 @@ struct TileSweep {
                 if (m < nent) {
                     const int d = e[i].x >> 16;
                     // the neighbour's high cells are my low ghosts
-                    const Face x = tile_part<L, 0, kFwd, T, TileFace<L>::M>(v[i]), y = tile_part<L, 1, kFwd, T, TileFace<L>::M>(v[i]),
-                               z = tile_part<L, 2, kFwd, T, TileFace<L>::M>(v[i]);
+                    Face x = tile_part<L, 0, kFwd, T, M>(v[i]), y = tile_part<L, 1, kFwd, T, M>(v[i]),
+                         z = tile_part<L, 2, kFwd, T, M>(v[i]);
+                    if constexpr (kPad) {
+                        const bool last = s.pad >> d & 1;
+                        if (kFwd) {
+                            // the last cells are the low ones of their tile
+                            if (last) {
+                                x = tile_part<L, 0, false, T, M>(v[i]);
+                                y = tile_part<L, 1, false, T, M>(v[i]);
+                                z = tile_part<L, 2, false, T, M>(v[i]);
+                            }
+                        } else if (last) {
+                            // the ghosts are pads of res; nothing is behind them
+                            T* r = R + L::N * (int)((unsigned)e[i].y >> 16);
+#pragma unroll
+                            for (int c = 0; c < M; ++c) {
+                                const Face f = d == 0 ? x : (d == 1 ? y : z);
+                                const int o = d == 0 ? L::template cell<0>(c, true)
+                                                     : (d == 1 ? L::template cell<1>(c, true)
+                                                               : L::template cell<2>(c, true));
+                                r[o] = f.v[c];
+                            }
+#pragma unroll
+                            for (int c = 0; c < M; ++c) x.v[c] = y.v[c] = z.v[c] = T(0);
+                        }
+                    }
                     gval[m] = d == 0 ? x : (d == 1 ? y : z);
                     gent[m] = e[i].x;
                 }
@@ -424,7 +457,7 @@ struct TileSweep {
         ldt(on, C + p, q.c[0]);
         ldt(on, C + s.npp + p, q.c[1]);
         ldt(on, C + 2 * s.npp + p, q.c[2]);
-        if constexpr (kFwd) ldt_rw(on, R + p, q.v);
+        if constexpr (kFwd || kPad) ldt_rw(on, R + p, q.v);
         else ldt(on, R + p, q.v);
     }
     // the recurrence of a tile's cells in step t
@@ -468,11 +501,11 @@ struct TileSweep {
 // ls res(j-1) - lw res(i-1) (sip_hyperplane_mod.F90:491-495); else in reverse,
 // res = res - ut res(k+1) - un res(j+1) - ue res(i+1), hilf += res (:546-547,
 // 559-567; kHz: hilf = res).  The last warp stages the ghosts.
-template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, int kMinBlocks>
+template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, int kMinBlocks, bool kPad = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __grid_constant__ TileArgs<T> a) {
     if (a.ctl[0]) return;
     extern __shared__ __align__(32) unsigned char tsm[];
-    TileSweep<L, T, kFwd> w(a, tsm);
+    TileSweep<L, T, kFwd, false, kPad> w(a, tsm);
     const int tid = threadIdx.x, ncomp = blockDim.x - 32, NT = a.s.NT;
     int2 e[w.kU];
     w.entries(e, tid);
@@ -526,10 +559,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
 // never waits for that rank, so the way from SM to SM delays the start of a rank once and
 // not every step.  Us a sweep of one grid of 32^3 on 8 SMs: 41; with a cluster barrier
 // in every step 63; with a released step counter in place of the mbarriers 72.
-template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, bool kRanks = false>
+template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, bool kRanks = false, bool kPad = false>
 __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_constant__ TileArgs<T> a) {
     extern __shared__ __align__(32) unsigned char tsm[];
-    TileSweep<L, T, kFwd, kRanks> w(a, tsm);
+    TileSweep<L, T, kFwd, kRanks, kPad> w(a, tsm);
+    constexpr bool kLate = kPad && !kFwd;   // loads see the pads written first
     const TileShape& s = a.s;
     const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT, t0 = w.t0, t1 = w.t1;
     const int set = tid >= ncomp ? 1 : 0, lane = tid - set * ncomp;   // (the last warp: neither)
@@ -541,15 +575,19 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     const int nc = kRanks ? s.nc : 1;
     auto first = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank) : 0; };
     auto past = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank + 1) : 0; };
-    if (tid < 2 * ncomp)
+    auto start = [&]() {
+        if (tid < 2 * ncomp)
 #pragma unroll
-        for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(t0 + set + 2 * d), past(t0 + set + 2 * d));
+            for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(t0 + set + 2 * d), past(t0 + set + 2 * d));
+    };
+    if constexpr (!kLate) start();
     w.tables();
     if constexpr (kRanks) w.arm();
     w.ghosts(e);
     if (converged) return;   // (every rank of a cluster or none)
     if constexpr (kRanks) cluster_barrier();
     else __syncthreads();
+    if constexpr (kLate) start();
     const int end = t0 + ((t1 - t0 + 1) & ~1);
     if (tid >= 2 * ncomp) {
         bool lost = false;
@@ -603,14 +641,16 @@ struct TileHalo {
 // The cells across face kF (-i, +i, -j, +j, -k, +k) of a tile: of tile nb of the
 // same grid (>= 0), of tile -1-nb of the grid across that face, of the grid's own
 // ghost plane, or zero.
-template <class L, int kF, typename T>
+template <class L, int kF, bool kPad, typename T>
 __device__ __forceinline__ Vec<T, L::template F<kF / 2>> tile_face(const TileArgs<T>& a, int g, int nb,
                                                                    int org) {
     const TileShape& s = a.s;
     constexpr int ax = kF / 2, nf = L::template F<ax>;
     constexpr bool hi = kF % 2 == 0;
     int n = g;
+    bool last = false;   // across a low face: the neighbour's last cells are the low ones of their tile
     if (nb < 0) {
+        if constexpr (kPad && hi) last = s.pad >> ax & 1;
         n = a.fnbr[6 * g + kF];
         nb = -1 - nb;
         if (n < 0) {
@@ -625,7 +665,14 @@ __device__ __forceinline__ Vec<T, L::template F<kF / 2>> tile_face(const TileArg
                 const int st = ax == 2 ? s.nj : s.nk;
                 const int q0 = ax == 0 ? ko + jo * s.nk : (ax == 1 ? ko + io * s.nk : jo + io * s.nj);
 #pragma unroll
-                for (int q = 0; q < nf; ++q) z.v[q] = P[q0 + (q / n2) * st + q % n2];
+                for (int q = 0; q < nf; ++q) {
+                    const int u = q / n2, v = q % n2;   // (offsets; a pad has no ghost)
+                    bool in = true;
+                    if constexpr (kPad)
+                        in = (ax == 0 ? jo : io) + u < (ax == 0 ? s.nj : s.ni) &&
+                             (ax == 2 ? jo : ko) + v < (ax == 2 ? s.nj : s.nk);
+                    if (in) z.v[q] = P[q0 + u * st + v];
+                }
             }
             return z;
         }
@@ -633,24 +680,38 @@ __device__ __forceinline__ Vec<T, L::template F<kF / 2>> tile_face(const TileArg
     const T* p = a.H + ((long long)n * s.npp + L::N * nb);
     if constexpr (ax == 0 || nf == 1) {
         // the face's cells are contiguous
-        return *reinterpret_cast<const Vec<T, nf>*>(p + L::template cell<ax>(0, hi));
+        return *reinterpret_cast<const Vec<T, nf>*>(p + (last ? L::template cell<ax>(0, false) : L::template cell<ax>(0, hi)));
     } else {
         Vec<T, L::N> v;
         ldt(true, p, v);
+        if (kPad && last) return tile_part<L, ax, false>(v);
         return tile_part<L, ax, hi>(v);
     }
 }
 
-template <class L, typename T>
+template <bool kPad = false, class L, typename T>
 __device__ __forceinline__ void tile_halo(const TileArgs<T>& a, int g, int tile, TileHalo<L, T>& o) {
     const int4 n0 = __ldg(a.s.nbr + 2 * tile), n1 = __ldg(a.s.nbr + 2 * tile + 1);
     ldt(true, a.H + ((long long)g * a.s.npp + L::N * tile), o.h);
-    o.im = tile_face<L, 0>(a, g, n0.x, n1.z);
-    o.ip = tile_face<L, 1>(a, g, n0.y, n1.z);
-    o.jm = tile_face<L, 2>(a, g, n0.z, n1.z);
-    o.jp = tile_face<L, 3>(a, g, n0.w, n1.z);
-    o.km = tile_face<L, 4>(a, g, n1.x, n1.z);
-    o.kp = tile_face<L, 5>(a, g, n1.y, n1.z);
+    o.im = tile_face<L, 0, kPad>(a, g, n0.x, n1.z);
+    o.ip = tile_face<L, 1, kPad>(a, g, n0.y, n1.z);
+    o.jm = tile_face<L, 2, kPad>(a, g, n0.z, n1.z);
+    o.jp = tile_face<L, 3, kPad>(a, g, n0.w, n1.z);
+    o.km = tile_face<L, 4, kPad>(a, g, n1.x, n1.z);
+    o.kp = tile_face<L, 5, kPad>(a, g, n1.y, n1.z);
+    if constexpr (kPad) {
+        // pads of the last tiles: the ghosts behind them
+        const int pad = (n0.y < 0 ? 1 : 0) | (n0.w < 0 ? 2 : 0) | (n1.y < 0 ? 4 : 0);
+        if (a.s.pad & pad & 1)
+#pragma unroll
+            for (int q = 0; q < L::FI; ++q) o.h.v[L::template cell<0>(q, true)] = o.ip.v[q];
+        if (a.s.pad & pad & 2)
+#pragma unroll
+            for (int q = 0; q < L::FJ; ++q) o.h.v[L::template cell<1>(q, true)] = o.jp.v[q];
+        if (a.s.pad & pad & 4)
+#pragma unroll
+            for (int q = 0; q < L::FK; ++q) o.h.v[L::template cell<2>(q, true)] = o.kp.v[q];
+    }
 }
 
 // the neighbours of cell i of a tile: i-1, i+1, j-1, j+1, k-1, k+1
@@ -672,7 +733,7 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<L, T>& o, int i, T n[6]
 // coefficient a class.  Of the first two products one rounds by itself and the
 // other is contracted with it: the first in kOrder 0, the second in kOrder 1, as the
 // compiler does it in the packed and in the table-driven cell pre-pass.
-template <class L, typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks>
+template <class L, typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks, bool kPad = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_constant__ TileArgs<T> a) {
     if (a.ctl[0]) return;
     constexpr int N = L::N;
@@ -696,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
             for (int i = 0; i < N; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
         } else {
             TileHalo<L, T> o;
-            tile_halo(a, g, tile, o);
+            tile_halo<kPad>(a, g, tile, o);
             Vec<T, N> c[kUni ? 1 : 7];
             if constexpr (!kUni)
 #pragma unroll
@@ -729,15 +790,16 @@ int tile_up(Ctx* c, TileDev& d, const V** p, const std::vector<V>& h) {
 }
 
 // Tables of a grid of ni x nj x nk cells in tiles of 2^si x 2^sj x 2^sk.  d.ok
-// stays false when the tiles do not divide it, for hyperplanes of more than
-// maxtiles tiles and shapes beyond the 10-bit cells or 16-bit slots.
+// stays false for hyperplanes of more than maxtiles tiles and shapes beyond the
+// 10-bit cells or 16-bit slots.
 inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int nc, int maxtiles, TileDev& d) {
     TileShape& s = d.s;
     s.nc = nc;
     s.ni = ni; s.nj = nj; s.nk = nk;
     s.si = si; s.sj = sj; s.sk = sk;
-    if (ni & si || nj & sj || nk & sk || ni > 1023 || nj > 1023 || nk > 1023) return 0;
-    const int NI = s.NI = ni >> si, NJ = s.NJ = nj >> sj, NK = s.NK = nk >> sk;
+    if (ni > 1023 || nj > 1023 || nk > 1023) return 0;
+    s.pad = (ni & si) | (nj & sj) << 1 | (nk & sk) << 2;
+    const int NI = s.NI = (ni + si) >> si, NJ = s.NJ = (nj + sj) >> sj, NK = s.NK = (nk + sk) >> sk;
     s.NT = NI + NJ + NK - 2;
     s.ntile = NI * NJ * NK;
     s.npp = s.ntile << (si + sj + sk);
@@ -759,7 +821,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
         s.maxt = std::max(s.maxt, p - tst.back());
         tst.push_back(p);
     }
-    if (tst.back() != s.ntile || s.maxt > maxtiles || s.slots > 0xffff) return 0;
+    if (tst.back() != s.ntile || s.maxt > maxtiles || s.slots > 0xffff || (s.pad && s.ntile > 0xffff)) return 0;
     auto tile = [&](int I, int J, int K) { return tpos[(size_t)(I + J + K) * NI + I] + J; };
     std::vector<int4> nbr((size_t)2 * s.ntile);
     for (int p = 0; p < s.ntile; ++p) {
@@ -781,7 +843,9 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
         std::vector<Entry> gs;
         // low: coordinate -1, the slot (I+1)w + J+1; high: coordinate N, the slot
         // I w + J the backward sweep uses
+        // (with pads a high entry names the grid's own last tile as well)
         auto add = [&](int ax, int I, int J, int K, int t) {
+            if (s.pad && sd) t |= tile(std::min(I, NI - 1), std::min(J, NJ - 1), std::min(K, NK - 1)) * 65536u;
             const int x = sd == 0 ? (I + 1) * s.w + J + 1 : I * s.w + J;
             gs.push_back(Entry{(ax > 0 ? I : (sd ? NI - 1 : 0)) * nc / NI, I + J + K, make_int2(x | (ax << 16), t)});
         };
@@ -819,7 +883,7 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
     }
     // cells: natural local index and place in the cell hyperplane order
     const int kk = nk + 4, jj = nj + 4;
-    std::vector<int> cell(s.npp), plane(s.npp);
+    std::vector<int> cell(s.npp, -1), plane(s.npp, -1);
     {
         int q = 0;
         for (int m = 0; m < ni + nj + nk - 2; ++m)

@@ -1,5 +1,4 @@
-"""The pressure solver on 2x2x2 tiles (the default for grids of even dimensions)
-against the same solver in the cell hyperplane order (forced by a sweep
+"""The pressure solver on 2x2x2 tiles (the default; odd dimensions leave pads) against the same solver in the cell hyperplane order (forced by a sweep
 variant): the same bits on every shape, at the edges of the tile hyperplanes, with
 few and many grids, walls on graded grids and a hierarchy."""
 import numpy as np
@@ -46,15 +45,21 @@ def _same(gpu_lib, case):
 @pytest.mark.parametrize("tiles,shape", [
     ((2, 1, 1), (2, 2, 2)), ((1, 2, 2), (2, 16, 6)), ((2, 1, 2), (12, 2, 8)), ((2, 2, 1), (6, 10, 2)),
     ((2, 2, 2), (24, 24, 24)), ((1, 2, 1), (32, 28, 36)), ((7, 7, 7), (8, 10, 12)),
-    ((8, 7, 6), (20, 24, 16))])
+    ((8, 7, 6), (20, 24, 16)),
+    # pads on one axis, two and all; last tiles that are also first ones
+    ((2, 2, 1), (3, 2, 2)), ((1, 2, 2), (2, 5, 4)), ((2, 1, 2), (4, 2, 7)), ((2, 2, 2), (21, 26, 19)),
+    ((1, 1, 1), (3, 3, 3)), ((2, 1, 1), (33, 31, 35)), ((7, 7, 7), (9, 8, 11)), ((3, 2, 3), (5, 25, 13))])
 def test_tiles_match_the_cell_order(gpu_lib, tiles, shape):
     ni, nj, nk = shape
     _same(gpu_lib, cases.periodic_box(*tiles, n=ni, nj=nj, nk=nk))
 
 
-def test_tiles_match_with_walls_on_graded_grids(gpu_lib):
+@pytest.mark.parametrize("shape", [(10, 10, 10), (9, 10, 11), (7, 9, 5)])
+def test_tiles_match_with_walls_on_graded_grids(gpu_lib, shape):
     walls = {1: abi.BC_FIX, 2: abi.BC_OP1, 3: abi.BC_NOS, 4: abi.BC_SLI}
-    _same(gpu_lib, cases.stretch(cases.periodic_box(3, 2, 2, n=10, length=(2.0, 2.0, 1.0), walls=walls)))
+    ni, nj, nk = shape
+    box = cases.periodic_box(3, 2, 2, n=ni, nj=nj, nk=nk, length=(2.0, 2.0, 1.0), walls=walls)
+    _same(gpu_lib, cases.stretch(box))
 
 
 def test_tiles_match_on_a_hierarchy(gpu_lib):
