@@ -163,6 +163,8 @@ int enqueue_mgpoisl(Ctx* c) {
     if (sip_on_tiles(s))   // the outer step takes its maxima into these
         MG_CUDA(cudaMemsetAsync(c->d_gridred, 0, (size_t)c->ngrid * sizeof(double), c->stream));
     if (int rc = sip_divcal(c, s, m->d_sprm + 2)) return rc;
+    if (multi)
+        if (int rc = mx_bound_pressure_begin(c, s, lv)) return rc;
     int* ctl = m->d_ctl;
     // pressuresolver_mod.F90:196-199: the divergence restricted into the
     // coarse grids, finest level first

@@ -64,19 +64,20 @@ struct BpArgs {
     const int* ctl;
 };
 
-// hilf of the parent p at its interior point (io, jo, ko), one coordinate of
-// which may lie on the ghost layer (-1 or n): there the value the reference's
-// coarse ghost holds -- the face neighbour's boundary plane (connect), the
-// parent's own PAR ghost plane, or zero (walls, inflow, outflow).
-__device__ float coarse_hilf(const BpArgs& A, int p, int io, int jo, int ko) {
+// Where hilf of the parent p at its interior point (io, jo, ko) stands, one
+// coordinate of which may lie on the ghost layer (-1 or n): there the value the
+// reference's coarse ghost holds -- the face neighbour's boundary plane (connect),
+// the parent's own PAR ghost plane, or zero (walls, inflow, outflow).  >= 0: an
+// index of hilf, -1: zero, -2 - x: index x of the PAR ghost planes.
+__device__ long long coarse_src(const BpArgs& A, int p, int io, int jo, int ko) {
     const PlaneMap& m = A.m;
     const bool xi = io < 0 || io >= m.ni, xj = jo < 0 || jo >= m.nj, xk = ko < 0 || ko >= m.nk;
-    if (!xi && !xj && !xk) return A.H[(long long)p * m.npp + m.pos(io, jo, ko)];
+    if (!xi && !xj && !xk) return (long long)p * m.npp + m.pos(io, jo, ko);
     // one coordinate on the ghost layer, the others inside (properly nested
     // grids); anything else reads zero rather than outside the arrays
     if ((int)xi + (int)xj + (int)xk != 1 || io < -1 || io > m.ni || jo < -1 || jo > m.nj || ko < -1 ||
         ko > m.nk)
-        return 0.f;
+        return -1;
     const int axis = xi ? 0 : (xj ? 1 : 2);
     const int hi = xi ? io >= m.ni : (xj ? jo >= m.nj : ko >= m.nk);
     const int f = 2 * axis + hi;
@@ -86,21 +87,27 @@ __device__ float coarse_hilf(const BpArgs& A, int p, int io, int jo, int ko) {
         if (axis == 0) io = hi ? 0 : m.ni - 1;
         else if (axis == 1) jo = hi ? 0 : m.nj - 1;
         else ko = hi ? 0 : m.nk - 1;
-        return A.H[(long long)nb * m.npp + m.pos(io, jo, ko)];
+        return (long long)nb * m.npp + m.pos(io, jo, ko);
     }
-    if (A.grids[p].bc[f] == MGLET_BC_PAR) return A.PG[((long long)p * 6 + f) * m.fs + fidx(m, axis, ko, jo, io)];
-    return 0.f;
+    if (A.grids[p].bc[f] == MGLET_BC_PAR) return -2 - (((long long)p * 6 + f) * m.fs + fidx(m, axis, ko, jo, io));
+    return -1;
+}
+__device__ __forceinline__ float coarse_value(const BpArgs& A, long long src) {
+    return src >= 0 ? A.H[src] : (src == -1 ? 0.f : A.PG[-2 - src]);
 }
 
-// parent + bound_pressure of hilf for the PAR faces of one level: one thread
-// per 2x2 block of a face (bound_pressure's blocks), grid = list[blockIdx.y],
-// face = blockIdx.z.
-__global__ void k_mx_bound_pressure(BpArgs A) {
-    if (A.ctl[0]) return;
-    const int g = A.list[blockIdx.y];
-    const int f = blockIdx.z;
+// parent + bound_pressure of hilf for the PAR faces: the weights of a 2x2 block of a
+// face that do not change within a solve.  w: the eight cells' weights in the (BP
+// weighted) volume mean next to the face, their sum (0: the mean is the parent's
+// value) and the factor of the difference to the parent; src: the parent's value
+// (coarse_src), pos: the first of the eight cells.
+struct BpBlock {
+    double w[8], sum, fac;
+    long long src, pos;
+};
+
+__device__ void bp_block(const BpArgs& A, int g, int f, int a, int b, BpBlock& r) {
     const DevGrid G = A.grids[g];
-    if (G.bc[f] != MGLET_BC_PAR) return;
     const PlaneMap& m = A.m;
     const int axis = f / 2;
     const bool lo = (f % 2) == 0;
@@ -108,67 +115,41 @@ __global__ void k_mx_bound_pressure(BpArgs A) {
     const int n2 = lo ? 2 : nn - 1, n3 = lo ? 3 : nn - 2, n4 = lo ? 4 : nn - 3;
     const int st2 = lo ? 2 : nn - 2;
     const int nmin = n3 < n4 ? n3 : n4;
-    const int na = axis == 2 ? G.jj : G.kk, nb = axis == 0 ? G.jj : G.ii;
-    const int nba = (na - 4) / 2, nbb = (nb - 4) / 2;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nba * nbb) return;
-    const int a = 3 + 2 * (q % nba), b = 3 + 2 * (q / nba);
     const double* ddx = A.ddx + G.ipx - 1;
     const double* ddy = A.ddy + G.ipy - 1;
     const double* ddz = A.ddz + G.ipz - 1;
     const double* dn = axis == 0 ? ddx : (axis == 1 ? ddy : ddz);
     const double* dstag = axis == 0 ? A.dx + G.ipx - 1 : (axis == 1 ? A.dy + G.ipy - 1 : A.dz + G.ipz - 1);
-    const float* Hg = A.H + (long long)g * m.npp;
-    // (a, b, n) in face coordinates -> fine interior (io, jo, ko)
-    auto fine = [&](int aa, int bb, int n) -> float {
-        int k, j, i;
-        if (axis == 0) { k = aa; j = bb; i = n; }
-        else if (axis == 1) { k = aa; j = n; i = bb; }
-        else { k = n; j = aa; i = bb; }
-        return Hg[m.pos(i - 3, j - 3, k - 3)];
-    };
     // pressureftocone_A / _B: the (BP-weighted) volume mean of the 2x2x2
     // interior block next to the face
     int k0, j0, i0;
     if (axis == 0) { k0 = a; j0 = b; i0 = nmin; }
     else if (axis == 1) { k0 = a; j0 = nmin; i0 = b; }
     else { k0 = nmin; j0 = a; i0 = b; }
+    r.pos = (long long)g * m.npp + m.pos(i0 - 3, j0 - 3, k0 - 3);
     const double* bp = A.BP ? A.BP + G.ip3 : nullptr;
     const int kk = G.kk, jj = G.jj;
     auto bix = [&](int kx, int jx, int ix) -> long long {
         return (long long)(ix - 1) * kk * jj + (long long)(jx - 1) * kk + (kx - 1);
     };
-    double pc, bpc = 1.0;
-    if (!bp) {
-        double sump = 0.0, sumvol = 0.0;
-        for (int l = 0; l <= 1; ++l)
-            for (int mm = 0; mm <= 1; ++mm)
-                for (int n = 0; n <= 1; ++n) {
-                    const double vol = ddz[k0 + n] * ddy[j0 + mm] * ddx[i0 + l];
-                    sump = sump + (double)Hg[m.pos(i0 + l - 3, j0 + mm - 3, k0 + n - 3)] * vol;
-                    sumvol = sumvol + vol;
-                }
-        pc = sump / sumvol;
-    } else {
+    double bpc = 1.0;
+    if (bp) {
         double sumbp = 0.0;
         for (int l = 0; l <= 1; ++l)
             for (int mm = 0; mm <= 1; ++mm)
                 for (int n = 0; n <= 1; ++n) sumbp = sumbp + bp[bix(k0 + n, j0 + mm, i0 + l)];
         bpc = fmin(sumbp, 1.0);
-        pc = 0.0;
-        if (bpc >= 0.5) {
-            double sump = 0.0, sumvol = 0.0;
-            for (int l = 0; l <= 1; ++l)
-                for (int mm = 0; mm <= 1; ++mm)
-                    for (int n = 0; n <= 1; ++n) {
-                        const double vol = bp[bix(k0 + n, j0 + mm, i0 + l)] * ddz[k0 + n] * ddy[j0 + mm] *
-                                           ddx[i0 + l];
-                        sump = sump + (double)Hg[m.pos(i0 + l - 3, j0 + mm - 3, k0 + n - 3)] * vol;
-                        sumvol = sumvol + vol;
-                    }
-            pc = sump / sumvol;
-        }
     }
+    r.sum = 0.0;
+    for (int l = 0; l <= 1; ++l)
+        for (int mm = 0; mm <= 1; ++mm)
+            for (int n = 0; n <= 1; ++n) {
+                const double vol = bp ? bp[bix(k0 + n, j0 + mm, i0 + l)] * ddz[k0 + n] * ddy[j0 + mm] * ddx[i0 + l]
+                                      : ddz[k0 + n] * ddy[j0 + mm] * ddx[i0 + l];
+                r.w[4 * l + 2 * mm + n] = vol;
+                r.sum = r.sum + vol;
+            }
+    if (!(bpc >= 0.5)) r.sum = 0.0;
     // the parent's slab cell of this block (parent_core_mod.F90:190-255 for a
     // scalar: both block corners odd, so the slab value itself)
     const int4 h = A.hier[g];
@@ -185,7 +166,7 @@ __global__ void k_mx_bound_pressure(BpArgs A) {
     if (axis == 0) { kc = ks + jc - 1; jcc = js + ic - 1; icc = is; }
     else if (axis == 1) { kc = ks + jc - 1; jcc = js; icc = is + ic - 1; }
     else { kc = ks; jcc = js + jc - 1; icc = is + ic - 1; }
-    const double pbv = (double)coarse_hilf(A, p, icc - 3, jcc - 3, kc - 3);
+    r.src = coarse_src(A, p, icc - 3, jcc - 3, kc - 3);
     double fak = 1.0;
     if (bp) {
         // bound_pressure's open-area factor of the block's four face pairs
@@ -196,7 +177,6 @@ __global__ void k_mx_bound_pressure(BpArgs A) {
             if (axis == 1) return bix(aa, n, bb);
             return bix(n, aa, bb);
         };
-        if (bpc < 0.5) pc = pbv;
         const double s11 = bp[fp(a, b, n2)] * bp[fp(a, b, n3)];
         const double s12 = bp[fp(a, b + 1, n2)] * bp[fp(a, b + 1, n3)];
         const double s13 = bp[fp(a + 1, b, n2)] * bp[fp(a + 1, b, n3)];
@@ -207,17 +187,110 @@ __global__ void k_mx_bound_pressure(BpArgs A) {
         if (fak < (double)0.1f) fak = 1.0;
         fak = 1.0 / fak;
     }
-    const double fac = fak * dstag[st2] / (dn[n3] + dn[n2]);
+    r.fac = fak * dstag[st2] / (dn[n3] + dn[n2]);
+}
+
+// the ghosts of a block; h: hilf of its eight cells, k fastest
+__device__ __forceinline__ void bp_ghosts(const BpArgs& A, int g, int f, int a, int b, const BpBlock& r,
+                                          const float (&h)[8]) {
+    const PlaneMap& m = A.m;
+    const int axis = f / 2, d = f % 2;   // the cells at the face: the high ones of the block at a high face
+    const double pbv = (double)coarse_value(A, r.src);
+    double pc = pbv;
+    if (r.sum != 0.0) {
+        double sump = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) sump = sump + (double)h[q] * r.w[q];
+        pc = sump / r.sum;
+    }
     float* pg = A.PG + ((long long)g * 6 + f) * m.fs;
+    const int st = axis == 2 ? m.nj : m.nk;
+#pragma unroll
     for (int l = 0; l <= 1; ++l)
+#pragma unroll
         for (int n = 0; n <= 1; ++n) {
-            const double v = (double)fine(a + n, b + l, n3) + fac * (pbv - pc);
-            int ko, jo, io;
-            if (axis == 0) { ko = a + n - 3; jo = b + l - 3; io = 0; }
-            else if (axis == 1) { ko = a + n - 3; jo = 0; io = b + l - 3; }
-            else { ko = 0; jo = a + n - 3; io = b + l - 3; }
-            pg[fidx(m, axis, ko, jo, io)] = (float)v;
+            const float hc = axis == 0 ? (d ? h[4 + 2 * l + n] : h[2 * l + n])
+                                       : (axis == 1 ? (d ? h[4 * l + 2 + n] : h[4 * l + n])
+                                                    : (d ? h[4 * l + 2 * n + 1] : h[4 * l + 2 * n]));
+            const double v = (double)hc + r.fac * (pbv - pc);
+            pg[(b + l - 3) * st + a + n - 3] = (float)v;
         }
+}
+
+// one thread per 2x2 block of a face (bound_pressure's blocks), grid =
+// list[blockIdx.y], face = blockIdx.z
+__global__ void k_mx_bound_pressure(BpArgs A) {
+    if (A.ctl[0]) return;
+    const int g = A.list[blockIdx.y];
+    const int f = blockIdx.z;
+    if (A.grids[g].bc[f] != MGLET_BC_PAR) return;
+    const PlaneMap& m = A.m;
+    const int nba = (f / 2 == 2 ? m.nj : m.nk) / 2, nbb = (f / 2 == 0 ? m.nj : m.ni) / 2;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nba * nbb) return;
+    const int a = 3 + 2 * (q % nba), b = 3 + 2 * (q / nba);
+    BpBlock r;
+    bp_block(A, g, f, a, b, r);
+    const int axis = f / 2, lo = f % 2 == 0;
+    const int n = lo ? 0 : (axis == 0 ? m.ni : (axis == 1 ? m.nj : m.nk)) - 2;
+    const int io = axis == 0 ? n : b - 3, jo = axis == 0 ? b - 3 : (axis == 1 ? n : a - 3), ko = axis == 2 ? n : a - 3;
+    float h[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        h[c] = A.H[(long long)g * m.npp + m.pos(io + (c >> 2), jo + ((c >> 1) & 1), ko + (c & 1))];
+    bp_ghosts(A, g, f, a, b, r, h);
+}
+
+// The same from a table of the blocks (on tiles, where a block is one tile): the
+// chain of lookups and the weights with their three divisions are taken once a solve
+// for its 36 and more launches a level.  448 + 256 PAR grids of 16^3 with BP, us a
+// launch: 19.6 without, 8.9 with the table.
+struct BpTable {
+    const int2* face;           // [nface] grid, face
+    double* w;                  // [10][nface * nb]
+    long long* idx;             // [2][nface * nb]: src, pos
+    long long n;                // nface * nb
+    int nb;                     // blocks of the largest face
+};
+
+__global__ void k_mx_bp_table(BpArgs A, BpTable T) {
+    const int2 gf = T.face[blockIdx.y];
+    const PlaneMap& m = A.m;
+    const int nba = (gf.y / 2 == 2 ? m.nj : m.nk) / 2, nbb = (gf.y / 2 == 0 ? m.nj : m.ni) / 2;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= nba * nbb) return;
+    BpBlock r;
+    bp_block(A, gf.x, gf.y, 3 + 2 * (q % nba), 3 + 2 * (q / nba), r);
+    const long long t = (long long)blockIdx.y * T.nb + q;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) T.w[c * T.n + t] = r.w[c];
+    T.w[8 * T.n + t] = r.sum;
+    T.w[9 * T.n + t] = r.fac;
+    T.idx[t] = r.src;
+    T.idx[T.n + t] = r.pos;
+}
+
+__global__ void __launch_bounds__(64) k_mx_bp_apply(BpArgs A, BpTable T, int face0) {
+    const int fc = face0 + blockIdx.y, q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int2 gf = T.face[fc];
+    const PlaneMap& m = A.m;
+    const int nba = (gf.y / 2 == 2 ? m.nj : m.nk) / 2, nbb = (gf.y / 2 == 0 ? m.nj : m.ni) / 2;
+    if (q >= nba * nbb) return;
+    const long long t = (long long)fc * T.nb + q;
+    BpBlock r;
+    r.src = T.idx[t];
+    r.pos = T.idx[T.n + t];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) r.w[c] = T.w[c * T.n + t];
+    r.sum = T.w[8 * T.n + t];
+    r.fac = T.w[9 * T.n + t];
+    if (A.ctl[0]) return;
+    float h[8];
+    const float4 x = *reinterpret_cast<const float4*>(A.H + r.pos);
+    const float4 y = *reinterpret_cast<const float4*>(A.H + r.pos + 4);
+    h[0] = x.x; h[1] = x.y; h[2] = x.z; h[3] = x.w;
+    h[4] = y.x; h[5] = y.y; h[6] = y.z; h[7] = y.w;
+    bp_ghosts(A, gf.x, gf.y, 3 + 2 * (q % nba), 3 + 2 * (q / nba), r, h);
 }
 
 // ftoc of a cell-centred field from the fine grids of one level into their
@@ -250,19 +323,31 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
     if (!LO) {
         // the FP32 correction: its mean in FP32 (the FP64 units of this part
         // issue at a small fraction of the FP32 rate)
-        auto Ff = [&](int kx, int jx, int ix) -> float { return H[base + m.pos(ix - 3, jx - 3, kx - 3)]; };
+        float hq[8];   // of the block, k fastest: on tiles one tile
+        if (m.NI) {
+            const float* t = H + base + m.pos(i - 3, j - 3, k - 3);
+            const float4 x = *reinterpret_cast<const float4*>(t), y = *reinterpret_cast<const float4*>(t + 4);
+            hq[0] = x.x; hq[1] = x.y; hq[2] = x.z; hq[3] = x.w;
+            hq[4] = y.x; hq[5] = y.y; hq[6] = y.z; hq[7] = y.w;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) hq[c] = H[base + m.pos(i - 3 + (c >> 2), j - 3 + ((c >> 1) & 1), k - 3 + (c & 1))];
+        }
         const float zx[2] = {(float)ddx[i], (float)ddx[i + 1]}, zy[2] = {(float)ddy[j], (float)ddy[j + 1]};
         const float zz[2] = {(float)ddz[k], (float)ddz[k + 1]};
         const double* bp = BP ? BP + G.ip3 : nullptr;
         const int kk = G.kk, jj = G.jj;
         float spv = 0.f, sv = 0.f;
+#pragma unroll
         for (int l = 0; l < 2; ++l)
+#pragma unroll
             for (int mq = 0; mq < 2; ++mq)
+#pragma unroll
                 for (int n = 0; n < 2; ++n) {
                     float vol = zz[l] * zy[mq] * zx[n];
                     if (bp)
                         vol *= (float)bp[(long long)(i + n - 1) * kk * jj + (long long)(j + mq - 1) * kk + (k + l - 1)];
-                    spv += Ff(k + l, j + mq, i + n) * vol;
+                    spv += hq[4 * n + 2 * mq + l] * vol;
                     sv += vol;
                 }
         const float hv = sv > 0.f ? spv / sv : 0.f;
@@ -419,6 +504,29 @@ int mx_level_prepare(Ctx* c, SipState& st, LevelState& lv) {
         if (int rc = upload(c, lv.pars[l], &lv.d_pars[l])) return rc;
     }
     if (int rc = upload(c, lv.parall, &lv.d_parall)) return rc;
+    // the PAR faces by level, and the table of their blocks
+    if (st.ni % 2 == 0 && st.nj % 2 == 0 && st.nk % 2 == 0) {
+        std::vector<int> gf;
+        lv.face0.assign(1, 0);
+        for (int l = 0; l < nl; ++l) {
+            for (int g : lv.pars[l])
+                for (int f = 0; f < 6; ++f)
+                    if (c->grids[g].bc[f] == MGLET_BC_PAR) {
+                        gf.push_back(g);
+                        gf.push_back(f);
+                    }
+            lv.face0.push_back((int)gf.size() / 2);
+        }
+        const size_t nb = std::max(st.nk * st.nj, std::max(st.nk * st.ni, st.nj * st.ni)) / 4;
+        const size_t n = gf.size() / 2 * nb;
+        if (n && gf.size() / 2 <= 65535) {
+            int* d = nullptr;
+            if (int rc = upload(c, gf, &d)) return rc;
+            lv.d_faces = reinterpret_cast<int2*>(d);
+            MG_CUDA(cudaMalloc(&lv.bpw, 10 * n * sizeof(double)));
+            MG_CUDA(cudaMalloc(&lv.bpidx, 2 * n * sizeof(long long)));
+        }
+    }
     if (!lv.ibflag.empty()) {
         // ghost-cell IB: per-grid flags, set at every stage by k_mx_pwflag
         MG_CUDA(cudaMalloc(&lv.d_skip, (size_t)c->ngrid));
@@ -451,6 +559,9 @@ void mx_level_release(LevelState& lv) {
     for (int* p : lv.d_pars) cudaFree(p);
     cudaFree(lv.d_parall);
     cudaFree(lv.d_skip);
+    cudaFree(lv.d_faces);
+    cudaFree(lv.bpw);
+    cudaFree(lv.bpidx);
     lv = LevelState();
 }
 
@@ -465,14 +576,10 @@ int mx_ctof(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* c
     return 0;
 }
 
-int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* ctl) {
-    const int l = ilevel - c->minlevel;
-    if (lv.pars[l].empty()) return 0;
-    ProfScope ps_(c, "mx_bound_pressure");
+static BpArgs bp_args(Ctx* c, const SipState& st, const int* ctl) {
     BpArgs A{};
     A.grids = c->d_grids;
     A.hier = c->d_hier;
-    A.list = lv.d_pars[l];
     A.fnbr = st.d_fnbr;
     A.facepos = sip_facepos(st);
     A.m = plane_map(st);
@@ -482,6 +589,36 @@ int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, co
     A.ddx = c->L("DDX"); A.ddy = c->L("DDY"); A.ddz = c->L("DDZ");
     A.BP = c->ibtype == 1 ? c->F("BP") : nullptr;
     A.ctl = ctl;
+    return A;
+}
+
+static BpTable bp_table(const SipState& st, const LevelState& lv) {
+    const int nb = std::max(st.nk * st.nj, std::max(st.nk * st.ni, st.nj * st.ni)) / 4;
+    return BpTable{lv.d_faces, lv.bpw, lv.bpidx, (long long)lv.face0.back() * nb, nb};
+}
+
+int mx_bound_pressure_begin(Ctx* c, SipState& st, const LevelState& lv) {
+    if (!sip_on_tiles(st) || !lv.bpw) return 0;
+    ProfScope ps_(c, "mx_bp_table");
+    const BpTable T = bp_table(st, lv);
+    k_mx_bp_table<<<dim3((T.nb + 63) / 64, lv.face0.back()), 64, 0, c->stream>>>(bp_args(c, st, nullptr), T);
+    MG_LAUNCHED(c);
+    return 0;
+}
+
+int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* ctl) {
+    const int l = ilevel - c->minlevel;
+    if (lv.pars[l].empty()) return 0;
+    ProfScope ps_(c, "mx_bound_pressure");
+    BpArgs A = bp_args(c, st, ctl);
+    if (sip_on_tiles(st) && lv.bpw) {
+        const BpTable T = bp_table(st, lv);
+        k_mx_bp_apply<<<dim3((T.nb + 63) / 64, lv.face0[l + 1] - lv.face0[l]), 64, 0, c->stream>>>(A, T,
+                                                                                                    lv.face0[l]);
+        MG_LAUNCHED(c);
+        return 0;
+    }
+    A.list = lv.d_pars[l];
     const int nbmax = std::max(st.nk * st.nj, std::max(st.nk * st.ni, st.nj * st.ni)) / 4;
     const dim3 grid((nbmax + 127) / 128, (unsigned)lv.pars[l].size(), 6);
     k_mx_bound_pressure<<<grid, 128, 0, c->stream>>>(A);

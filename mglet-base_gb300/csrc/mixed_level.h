@@ -20,6 +20,12 @@ struct LevelState {
     int* d_parall = nullptr;
     std::vector<unsigned char> ibflag;
     unsigned char* d_skip = nullptr;
+    // PAR faces (grid, face) by level, face0[l] .. face0[l + 1]; the table of their 2x2
+    // blocks, filled at the start of a solve (null: odd dimensions or no such face)
+    std::vector<int> face0;
+    int2* d_faces = nullptr;
+    double* bpw = nullptr;
+    long long* bpidx = nullptr;
 };
 
 // Lists, the PAR ghost planes of hilf and the level operators' buffers; once,
@@ -28,6 +34,8 @@ int mx_level_prepare(Ctx* c, SipState& st, LevelState& lv);
 void mx_level_release(LevelState& lv);
 // ctof of hilf into the grids of ilevel (nothing on the coarsest level)
 int mx_ctof(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* ctl);
+// what parent + bound_pressure of hilf take from BP and the grids, once a solve
+int mx_bound_pressure_begin(Ctx* c, SipState& st, const LevelState& lv);
 // parent + bound_pressure of hilf: the PAR ghost planes of the grids of ilevel
 int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* ctl);
 // ftoc from the grids of ilevel into their parents: hilf ('P') or the
