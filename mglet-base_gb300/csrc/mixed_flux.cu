@@ -105,6 +105,9 @@ struct FluxArgs {
     int* err;                          // set when a bulk-copy wait gives up
     int skip_plane;                    // test switch: this plane's copy is not issued (0: none)
     int nslab;                         // j-slabs (CTAs) per grid
+    // [grid][border between slabs][0: the row before it, 1: the row after][U V W][ii][kk] as
+    // they were before the launch, which updates U, V, W in place (null: one slab)
+    double* rows;
 };
 
 // j- and k-dependent spacing factors of one thread's (k, j) column
@@ -524,9 +527,19 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
             ring(r, kq, jq);
             const long long c = (long long)(i - 1) * kj + (long long)(jq - 1) * kk + (kq - 1);
             const int q = pl(kq, jq);
-            su[slot3 * plane + q] = split64(U0[c]);
-            sv[slot3 * plane + q] = split64(V0[c]);
-            sw[slot3 * plane + q] = split64(W0[c]);
+            const double *pu = U0 + c, *pv = V0 + c, *pw = W0 + c;
+            // a row of the next slab, which updates it meanwhile
+            const int border = jq < j0 ? slab - 1 : (jq >= j0 + nj ? slab : -1);
+            if (border >= 0 && border < a.nslab - 1) {
+                const long long n = (long long)ii * kk;
+                pu = a.rows + (((long long)(blockIdx.x / a.nslab) * (a.nslab - 1) + border) * 2 + (jq < j0 ? 0 : 1)) * 3 * n +
+                     (long long)(i - 1) * kk + (kq - 1);
+                pv = pu + n;
+                pw = pv + n;
+            }
+            su[slot3 * plane + q] = split64(*pu);
+            sv[slot3 * plane + q] = split64(*pv);
+            sw[slot3 * plane + q] = split64(*pw);
             if (with_p) sp[slot2 * plane + q] = split64(P0[c]);
             if (pwg) {
                 xu[slot3 * plane + q] = split64(a.PU0[o + c]);
@@ -587,6 +600,21 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
         unx = unx2; vnx = vnx2; wnx = wnx2;
         __syncthreads();
     }
+}
+
+// the rows on both sides of the borders between slabs, before k_mx_flux
+__global__ void k_mx_flux_rows(FluxArgs a) {
+    const int nb = 2 * (a.nslab - 1), g = blockIdx.x / nb, b = blockIdx.x % nb;
+    const DevGrid G = a.grids[g];
+    const int kk = G.kk, jj = G.jj, n = G.ii * kk;
+    const int t = blockIdx.y * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int js = (jj - 4 + a.nslab - 1) / a.nslab, j = 2 + (b / 2 + 1) * js + (b & 1);
+    const long long c = G.ip3 + (long long)(t / kk) * kk * jj + (long long)(j - 1) * kk + t % kk;
+    double* r = a.rows + (long long)blockIdx.x * 3 * n + t;
+    r[0] = a.U0[c];
+    r[n] = a.V0[c];
+    r[2LL * n] = a.W0[c];
 }
 
 // ---- the same kernel with the planes staged by TMA -------------------------
@@ -804,18 +832,24 @@ __global__ void __launch_bounds__(576, 2)
 
 }  // namespace
 
-// j-slabs per grid: the fewest for which a slab has at most 576 (k, j) columns
-static int flux_slabs(const DevGrid& G0) {
+// j-slabs per grid: so many that a slab has at most 576 (k, j) columns, and with few
+// grids more, down to two rows a slab, while there are at most 608 in all: a CTA's
+// FP64 conversions and updates of a plane take its SM's pipe, its march in i is a
+// chain.  Us a launch with one slab / up to 608: 8 grids of 24^3 132 / 89, 144 with a
+// model 562 / 447, 210 of 21x26x19 177 / 156, 512 of 24^3 the same.
+static int flux_slabs(const DevGrid& G0, int ngrid) {
     const int nk = G0.kk - 4, nj = G0.jj - 4;
-    for (int s = 1; s <= nj; ++s)
-        if (nk * ((nj + s - 1) / s) <= 576) return s;
-    return 0;
+    int s = 1;
+    while (s < nj && nk * ((nj + s - 1) / s) > 576) ++s;
+    s = std::max(s, std::min(608 / ngrid, nj / 2));
+    const int js = (nj + s - 1) / s;
+    return (nj + js - 1) / js;
 }
 
 // 11 planes of (hi, lo) windows (U, V, W: 3 each; P: 2), 20 with the point
 // values' windows of the ghost-cell IB
-static size_t flux_smem(const DevGrid& G0, bool pw = false) {
-    const int nslab = flux_slabs(G0);
+static size_t flux_smem(const DevGrid& G0, int ngrid, bool pw = false) {
+    const int nslab = flux_slabs(G0, ngrid);
     const int js = (G0.jj - 4 + nslab - 1) / nslab;
     return (size_t)(pw ? 20 : 11) * (G0.kk - 2) * (js + 2) * sizeof(float2);
 }
@@ -830,6 +864,7 @@ struct FluxState {
     // ghost-cell IB: per-grid flags of the grids whose transported velocities
     // are the point values (the plane-load kernel then carries their windows)
     const unsigned char* d_pw = nullptr;
+    double* rows = nullptr;   // the rows on the borders between slabs
     int variant = -1;
     double ms[2] = {0.0, 0.0};
 };
@@ -882,7 +917,7 @@ int mx_flux_prepare(Ctx* c) {
         set_error("mixed form: the flux kernel takes at most 576 cells in k per grid");
         return MGLET_ERR_UNSUPPORTED;
     }
-    const size_t smem = flux_smem(G0);
+    const size_t smem = flux_smem(G0, c->ngrid);
     if (smem > 200 * 1024) {
         set_error("mixed form: grid planes too large for the flux kernel's shared memory");
         return MGLET_ERR_UNSUPPORTED;
@@ -893,11 +928,14 @@ int mx_flux_prepare(Ctx* c) {
     fs = FluxState();
     for (const DevGrid& g : c->grids)
         for (int f = 0; f < 6; ++f) fs.walls |= g.bc[f] != MGLET_BC_CON;
+    const int nslab = flux_slabs(G0, c->ngrid);
+    if (nslab > 1)
+        MG_CUDA(cudaMalloc(&fs.rows, (size_t)c->ngrid * (nslab - 1) * 6 * G0.ii * G0.kk * sizeof(double)));
     const size_t tsm = flux_tma_smem(G0);
     // the four planes of a staging slot follow each other in shared memory, and a
     // tensor copy's destination has to start on a 128-byte line there
     const bool lines = ((size_t)G0.kk * G0.jj * sizeof(double)) % 128 == 0;
-    if (flux_slabs(G0) == 1 && lines && (G0.kk * sizeof(double)) % 16 == 0 && G0.kk <= 256 &&
+    if ((G0.kk - 4) * (G0.jj - 4) <= 576 && lines && (G0.kk * sizeof(double)) % 16 == 0 && G0.kk <= 256 &&
         G0.jj <= 256 && tsm <= 113 * 1024) {
         const char* names[4] = {"U", "V", "W", "P"};
         for (int f = 0; f < 4; ++f)
@@ -911,24 +949,38 @@ int mx_flux_prepare(Ctx* c) {
     return 0;
 }
 
-void mx_flux_release(Ctx* c) { g_flux.erase(c); }
+void mx_flux_release(Ctx* c) {
+    auto it = g_flux.find(c);
+    if (it == g_flux.end()) return;
+    cudaFree(it->second.rows);
+    g_flux.erase(it);
+}
 
 void mx_flux_set_gfield(Ctx* c) { g_flux[c].gfield = true; }
 
 static int launch_variant(Ctx* c, int v, const FluxArgs& a, int threads) {
     const DevGrid& G0 = c->grids[0];
     FluxState& fs = g_flux[c];
-    const size_t tsm = flux_tma_smem(G0), psm = flux_smem(G0, fs.d_pw != nullptr);
+    const size_t tsm = flux_tma_smem(G0), psm = flux_smem(G0, c->ngrid, fs.d_pw != nullptr);
     const unsigned nb = (unsigned)(c->ngrid * a.nslab);
     const bool kw = fs.walls || fs.gfield;
+    // the TMA kernel has one CTA of all columns per grid
+    const int whole = ((G0.kk - 4) * (G0.jj - 4) + 31) / 32 * 32;
     if (v == 1 && fs.tma && !fs.d_pw) {
         if (kw)
-            k_mx_flux_tma<true><<<c->ngrid, threads, tsm, c->stream>>>(a, fs.map[0], fs.map[1],
+            k_mx_flux_tma<true><<<c->ngrid, whole, tsm, c->stream>>>(a, fs.map[0], fs.map[1],
                                                                       fs.map[2], fs.map[3]);
         else
-            k_mx_flux_tma<false><<<c->ngrid, threads, tsm, c->stream>>>(a, fs.map[0], fs.map[1],
+            k_mx_flux_tma<false><<<c->ngrid, whole, tsm, c->stream>>>(a, fs.map[0], fs.map[1],
                                                                        fs.map[2], fs.map[3]);
-    } else if (kw) {
+        MG_LAUNCHED(c);
+        return 0;
+    }
+    if (a.nslab > 1) {
+        k_mx_flux_rows<<<dim3(c->ngrid * 2 * (a.nslab - 1), (G0.ii * G0.kk + 255) / 256), 256, 0, c->stream>>>(a);
+        MG_LAUNCHED(c);
+    }
+    if (kw) {
         k_mx_flux<true><<<nb, threads, psm, c->stream>>>(a);
     } else {
         k_mx_flux<false><<<nb, threads, psm, c->stream>>>(a);
@@ -940,11 +992,11 @@ static int launch_variant(Ctx* c, int v, const FluxArgs& a, int threads) {
 static FluxArgs flux_args(Ctx* c, float* du, float* dv, float* dw, const float* sx, const float* sy,
                           const float* sz, const double* sprm, int* err, int* threads) {
     const DevGrid& G0 = c->grids[0];
-    const int nslab = flux_slabs(G0);
-    const int js = (G0.jj - 4 + nslab - 1) / nslab;
-    *threads = ((G0.kk - 4) * js + 31) / 32 * 32;
+    const int nslab = flux_slabs(G0, c->ngrid);
+    *threads = ((G0.kk - 4) * ((G0.jj - 4 + nslab - 1) / nslab) + 31) / 32 * 32;
     FluxArgs a{};
     a.nslab = nslab;
+    a.rows = g_flux[c].rows;
     a.grids = c->d_grids;
     a.U0 = c->F("U"); a.V0 = c->F("V"); a.W0 = c->F("W"); a.P0 = c->F("P");
     a.U = c->F("U"); a.V = c->F("V"); a.W = c->F("W");
@@ -1065,7 +1117,7 @@ int mx_flux_set_pw(Ctx* c, const unsigned char* d_pw) {
     fs.d_pw = d_pw;
     if (!d_pw) return 0;
     fs.walls = true;
-    const size_t smem = flux_smem(c->grids[0], true);
+    const size_t smem = flux_smem(c->grids[0], c->ngrid, true);
     if (smem > 227 * 1024) {
         set_error("mixed form: grid planes too large for the ghost-cell flux windows");
         return MGLET_ERR_UNSUPPORTED;
