@@ -557,6 +557,7 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
 
     const int q = pl(k, j);
     const float gfl = (float)G.gradpflag;
+    const float frhs = (float)a.sprm[0], fdt = (float)a.sprm[1];
     const bool wg = kW && has_open_face(G);
     const bool pgrid = kW && has_par_face(G);
     const bool wv = (wg || (kW && a.gall)) && !(a.guni && a.guni[2 * (blockIdx.x / a.nslab)] != 0.0);
@@ -585,12 +586,10 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
             if (kW && pgrid) {
                 a.UO[c] = (double)uo; a.VO[c] = (double)vo; a.WO[c] = (double)wo;
             } else {
-                const float frhs = (float)a.sprm[0];
                 const float du = frhs * a.DU[c] + uo;
                 const float dv = frhs * a.DV[c] + vo;
                 const float dw = frhs * a.DW[c] + wo;
                 a.DU[c] = du; a.DV[c] = dv; a.DW[c] = dw;
-                const float fdt = (float)a.sprm[1];
                 a.U[c] = ucur + (double)(fdt * du);
                 a.V[c] = vcur + (double)(fdt * dv);
                 a.W[c] = wcur + (double)(fdt * dw);
@@ -786,6 +785,7 @@ __global__ void __launch_bounds__(576, 2)
 
     const int q = pl(k, j);
     const float gfl = (float)G.gradpflag;
+    const float frhs = (float)a.sprm[0], fdt = (float)a.sprm[1];
     const bool wg = kW && has_open_face(G);
     const bool pgrid = kW && has_par_face(G);
     const bool wv = (wg || (kW && a.gall)) && !(a.guni && a.guni[2 * gid] != 0.0);
@@ -812,12 +812,10 @@ __global__ void __launch_bounds__(576, 2)
             if (kW && pgrid) {
                 a.UO[c] = (double)uo; a.VO[c] = (double)vo; a.WO[c] = (double)wo;
             } else {
-                const float frhs = (float)a.sprm[0];
                 const float du = frhs * a.DU[c] + uo;
                 const float dv = frhs * a.DV[c] + vo;
                 const float dw = frhs * a.DW[c] + wo;
                 a.DU[c] = du; a.DV[c] = dv; a.DW[c] = dw;
-                const float fdt = (float)a.sprm[1];
                 a.U[c] = ucur + (double)(fdt * du);
                 a.V[c] = vcur + (double)(fdt * dv);
                 a.W[c] = wcur + (double)(fdt * dw);

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "cvt64.cuh"
 #include "mixed_level.h"
 
 namespace mg {
@@ -195,12 +196,12 @@ __device__ __forceinline__ void bp_ghosts(const BpArgs& A, int g, int f, int a, 
                                           const float (&h)[8]) {
     const PlaneMap& m = A.m;
     const int axis = f / 2, d = f % 2;   // the cells at the face: the high ones of the block at a high face
-    const double pbv = (double)coarse_value(A, r.src);
+    const double pbv = cvt_double(coarse_value(A, r.src));
     double pc = pbv;
     if (r.sum != 0.0) {
         double sump = 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) sump = sump + (double)h[q] * r.w[q];
+        for (int q = 0; q < 8; ++q) sump = sump + cvt_double(h[q]) * r.w[q];
         pc = sump / r.sum;
     }
     float* pg = A.PG + ((long long)g * 6 + f) * m.fs;
@@ -212,8 +213,8 @@ __device__ __forceinline__ void bp_ghosts(const BpArgs& A, int g, int f, int a, 
             const float hc = axis == 0 ? (d ? h[4 + 2 * l + n] : h[2 * l + n])
                                        : (axis == 1 ? (d ? h[4 * l + 2 + n] : h[4 * l + n])
                                                     : (d ? h[4 * l + 2 * n + 1] : h[4 * l + 2 * n]));
-            const double v = (double)hc + r.fac * (pbv - pc);
-            pg[(b + l - 3) * st + a + n - 3] = (float)v;
+            const double v = cvt_double(hc) + r.fac * (pbv - pc);
+            pg[(b + l - 3) * st + a + n - 3] = cvt_float(v);
         }
 }
 
@@ -317,7 +318,7 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
     const long long base = (long long)g * m.npp;
     auto F = [&](int kx, int jx, int ix) -> double {
         const long long o = base + m.pos(ix - 3, jx - 3, kx - 3);
-        return LO ? (double)H[o] + (double)LO[o] : (double)H[o];
+        return cvt_double(H[o]) + cvt_double(LO[o]);
     };
     double val;
     if (!LO) {
@@ -333,8 +334,8 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
 #pragma unroll
             for (int c = 0; c < 8; ++c) hq[c] = H[base + m.pos(i - 3 + (c >> 2), j - 3 + ((c >> 1) & 1), k - 3 + (c & 1))];
         }
-        const float zx[2] = {(float)ddx[i], (float)ddx[i + 1]}, zy[2] = {(float)ddy[j], (float)ddy[j + 1]};
-        const float zz[2] = {(float)ddz[k], (float)ddz[k + 1]};
+        const float zx[2] = {cvt_float(ddx[i]), cvt_float(ddx[i + 1])}, zy[2] = {cvt_float(ddy[j]), cvt_float(ddy[j + 1])};
+        const float zz[2] = {cvt_float(ddz[k]), cvt_float(ddz[k + 1])};
         const double* bp = BP ? BP + G.ip3 : nullptr;
         const int kk = G.kk, jj = G.jj;
         float spv = 0.f, sv = 0.f;
@@ -346,7 +347,7 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
                 for (int n = 0; n < 2; ++n) {
                     float vol = zz[l] * zy[mq] * zx[n];
                     if (bp)
-                        vol *= (float)bp[(long long)(i + n - 1) * kk * jj + (long long)(j + mq - 1) * kk + (k + l - 1)];
+                        vol *= cvt_float(bp[(long long)(i + n - 1) * kk * jj + (long long)(j + mq - 1) * kk + (k + l - 1)]);
                     spv += hq[4 * n + 2 * mq + l] * vol;
                     sv += vol;
                 }
@@ -390,9 +391,7 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
     const int ioc = h.y + (i - 3) / 2 - 3, joc = h.z + (j - 3) / 2 - 3, koc = h.w + (k - 3) / 2 - 3;
     if (ioc < 0 || ioc >= m.ni || joc < 0 || joc >= m.nj || koc < 0 || koc >= m.nk) return;
     const long long o = (long long)h.x * m.npp + m.pos(ioc, joc, koc);
-    const float hv = (float)val;
-    H[o] = hv;
-    if (LO) LO[o] = (float)(val - (double)hv);
+    cvt_split(val, H[o], LO[o]);
 }
 
 // max |rhs| per grid (maxabscal_grid after the restriction of the residual
@@ -454,9 +453,9 @@ __global__ void k_mx_rk_par(const DevGrid* __restrict__ grids, const unsigned ch
     const float dv = frhs * DV[c] + (float)VO[c];
     const float dw = frhs * DW[c] + (float)WO[c];
     DU[c] = du; DV[c] = dv; DW[c] = dw;
-    U[c] = U[c] + (double)(fdt * du);
-    V[c] = V[c] + (double)(fdt * dv);
-    W[c] = W[c] + (double)(fdt * dw);
+    U[c] = U[c] + cvt_double(fdt * du);
+    V[c] = V[c] + cvt_double(fdt * dv);
+    W[c] = W[c] + cvt_double(fdt * dw);
     UO[c] = 0.0; VO[c] = 0.0; WO[c] = 0.0;
 }
 

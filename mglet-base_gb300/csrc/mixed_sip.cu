@@ -43,6 +43,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cvt64.cuh"
 #include "internal.h"
 #include "mixed_sip.h"
 #include "sip_tile.cuh"
@@ -1269,10 +1270,8 @@ __global__ void k_sip_divcal_nat(const DevGrid* __restrict__ grids, PosMap m, fl
         d = d + fak * SDIV[G.ip3 + id];
         d = BP[G.ip3 + id] * d;
     }
-    const float dh = (float)d;
     const long long o = (long long)g * m.npp + m.pos(io, jo, ko);
-    RHS[o] = dh;
-    RHSL[o] = (float)(d - (double)dh);
+    cvt_split(d, RHS[o], RHSL[o]);
 }
 
 __global__ void k_sip_scatter_nat(const DevGrid* __restrict__ grids, PosMap m, const float* __restrict__ DPH,

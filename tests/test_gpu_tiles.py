@@ -62,5 +62,29 @@ def test_tiles_match_with_walls_on_graded_grids(gpu_lib, shape):
     _same(gpu_lib, cases.stretch(box))
 
 
+@pytest.mark.parametrize("scale", [1.0, 1e-22, 1e-36, 1e-43, 1e-300, 1e30])
+def test_divergence_split_over_the_range(gpu_lib, scale):
+    """The divergence split into two floats by integer arithmetic against the cell
+    order's casts, where the second float is normal, subnormal or lost and where the
+    values leave the floats' range."""
+    case = cases.periodic_box(2, 1, 1, n=6)
+    out = []
+    for plane in (False, True):
+        g = gpu_lib.Solver(case, abi.make_flow_params(gmol=1e-3, epcorr=1e-10, nouter=1, ninner=1,
+                                                      form=abi.FORM_MIXED))
+        if plane:
+            g.force_variant("mx_order", 0)
+        rng = np.random.default_rng(2)
+        for nm in "UVW":
+            a = scale * rng.standard_normal(case.idim3d)
+            a[rng.random(a.size) < 0.3] = 0.0
+            g.set(nm, a)
+        g.timeintegrate_flow(1, 1, 0.0, 5e-4, 1, gpu_lib.rk_scheme("williamson"))
+        out.append([g.get(nm) for nm in ("U", "V", "W", "P", "DP")])
+        g.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y, equal_nan=True)
+
+
 def test_tiles_match_on_a_hierarchy(gpu_lib):
     _same(gpu_lib, cases.refined_box(2, 2, 2, n=8, refine=(1,)))
