@@ -25,6 +25,7 @@
 
 #include "cvt64.cuh"
 #include "mixed_level.h"
+#include "sip_tile.cuh"
 
 namespace mg {
 namespace {
@@ -40,15 +41,18 @@ __device__ __forceinline__ int fidx(const PlaneMap& m, int axis, int ko, int jo,
 // iposition - 1 + (i - 1) / 2).
 __global__ void k_mx_ctof(const DevGrid* __restrict__ grids, const int4* __restrict__ hier,
                           const int* __restrict__ list, PlaneMap m, float* H, const int* ctl) {
-    if (ctl[0]) return;
     const int g = list[blockIdx.y];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m.ni * m.nj * m.nk) return;
     const int ko = t % m.nk, jo = (t / m.nk) % m.nj, io = t / (m.nk * m.nj);
     const int4 h = hier[g];
     const int ioc = h.y - 4 + (io + 2) / 2, joc = h.z - 4 + (jo + 2) / 2, koc = h.w - 4 + (ko + 2) / 2;
-    if (ioc < 0 || ioc >= m.ni || joc < 0 || joc >= m.nj || koc < 0 || koc >= m.nk) return;
-    H[(long long)g * m.npp + m.pos(io, jo, ko)] = H[(long long)h.x * m.npp + m.pos(ioc, joc, koc)];
+    const bool on = t < m.ni * m.nj * m.nk && ioc >= 0 && ioc < m.ni && joc >= 0 && joc < m.nj && koc >= 0 &&
+                    koc < m.nk;
+    const long long to = on ? (long long)g * m.npp + m.pos(io, jo, ko) : 0;
+    const long long from = on ? (long long)h.x * m.npp + m.pos(ioc, joc, koc) : 0;
+    follow_on();
+    if (flag_at(ctl) || !on) return;
+    H[to] = H[from];
 }
 
 struct BpArgs {
@@ -276,8 +280,9 @@ __global__ void __launch_bounds__(64) k_mx_bp_apply(BpArgs A, BpTable T, int fac
     const int2 gf = T.face[fc];
     const PlaneMap& m = A.m;
     const int nba = (gf.y / 2 == 2 ? m.nj : m.nk) / 2, nbb = (gf.y / 2 == 0 ? m.nj : m.ni) / 2;
-    if (q >= nba * nbb) return;
-    const long long t = (long long)fc * T.nb + q;
+    const bool on = q < nba * nbb;
+    // (the table is older than the launch before)
+    const long long t = on ? (long long)fc * T.nb + q : 0;
     BpBlock r;
     r.src = T.idx[t];
     r.pos = T.idx[T.n + t];
@@ -285,7 +290,8 @@ __global__ void __launch_bounds__(64) k_mx_bp_apply(BpArgs A, BpTable T, int fac
     for (int c = 0; c < 8; ++c) r.w[c] = T.w[c * T.n + t];
     r.sum = T.w[8 * T.n + t];
     r.fac = T.w[9 * T.n + t];
-    if (A.ctl[0]) return;
+    follow_on();
+    if (flag_at(A.ctl) || !on) return;
     float h[8];
     const float4 x = *reinterpret_cast<const float4*>(A.H + r.pos);
     const float4 y = *reinterpret_cast<const float4*>(A.H + r.pos + 4);
@@ -305,9 +311,10 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
                           const double* __restrict__ DDX, const double* __restrict__ DDY,
                           const double* __restrict__ DDZ, const double* __restrict__ BP,
                           const int* ctl) {
-    if (ctl[0]) return;
     const int g = list[blockIdx.y];
     const DevGrid G = grids[g];
+    follow_on();
+    if (flag_at(ctl)) return;
     const int nci = m.ni / 2, ncj = m.nj / 2, nck = m.nk / 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nci * ncj * nck) return;
@@ -397,7 +404,8 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
 // max |rhs| per grid (maxabscal_grid after the restriction of the residual
 // into the coarse grids), of its leading float as the outer step forms it
 __global__ void k_mx_gridmax(int npp, const float* __restrict__ H, double* gridmax, const int* ctl) {
-    if (ctl[0]) return;
+    follow_on();
+    if (flag_at(ctl)) return;
     __shared__ float sh[32];
     const long long base = (long long)blockIdx.x * npp;
     float v = 0.f;
@@ -569,8 +577,9 @@ int mx_ctof(Ctx* c, SipState& st, const LevelState& lv, int ilevel, const int* c
     if (l <= 0 || lv.grids[l].empty()) return 0;
     ProfScope ps_(c, "mx_ctof");
     const dim3 grid((st.ni * st.nj * st.nk + 255) / 256, (unsigned)lv.grids[l].size());
-    k_mx_ctof<<<grid, 256, 0, c->stream>>>(c->d_grids, c->d_hier, lv.d_grids[l], plane_map(st),
-                                           st.h32, ctl);
+    if (int rc = launch_follow_on(k_mx_ctof, grid, 256, 0, c->stream, 1, c->d_grids, c->d_hier, lv.d_grids[l],
+                                  plane_map(st), st.h32, ctl))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }
@@ -612,8 +621,9 @@ int mx_bound_pressure(Ctx* c, SipState& st, const LevelState& lv, int ilevel, co
     BpArgs A = bp_args(c, st, ctl);
     if (sip_on_tiles(st) && lv.bpw) {
         const BpTable T = bp_table(st, lv);
-        k_mx_bp_apply<<<dim3((T.nb + 63) / 64, lv.face0[l + 1] - lv.face0[l]), 64, 0, c->stream>>>(A, T,
-                                                                                                    lv.face0[l]);
+        if (int rc = launch_follow_on(k_mx_bp_apply, dim3((T.nb + 63) / 64, lv.face0[l + 1] - lv.face0[l]), 64, 0,
+                                      c->stream, 1, A, T, lv.face0[l]))
+            return rc;
         MG_LAUNCHED(c);
         return 0;
     }
@@ -631,17 +641,19 @@ int mx_ftoc(Ctx* c, SipState& st, const LevelState& lv, int ilevel, bool rhs, co
     ProfScope ps_(c, "mx_ftoc");
     const int nq = (st.ni / 2) * (st.nj / 2) * (st.nk / 2);
     const dim3 grid((nq + 127) / 128, (unsigned)lv.grids[l].size());
-    k_mx_ftoc<<<grid, 128, 0, c->stream>>>(c->d_grids, c->d_hier, lv.d_grids[l], plane_map(st),
-                                           rhs ? st.rhs32 : st.h32, rhs ? st.rhsl : nullptr,
-                                           c->L("DDX"), c->L("DDY"), c->L("DDZ"),
-                                           c->ibtype == 1 ? c->F("BP") : nullptr, ctl);
+    if (int rc = launch_follow_on(k_mx_ftoc, grid, 128, 0, c->stream, 1, c->d_grids, c->d_hier, lv.d_grids[l],
+                                  plane_map(st), rhs ? st.rhs32 : st.h32, rhs ? st.rhsl : nullptr, c->L("DDX"),
+                                  c->L("DDY"), c->L("DDZ"), c->ibtype == 1 ? c->F("BP") : nullptr, ctl))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }
 
 int mx_gridmax(Ctx* c, SipState& st, const int* ctl) {
     ProfScope ps_(c, "mx_gridmax");
-    k_mx_gridmax<<<c->ngrid, 256, 0, c->stream>>>(plane_map(st).npp, st.rhs32, c->d_gridred, ctl);
+    if (int rc = launch_follow_on(k_mx_gridmax, dim3(c->ngrid), 256, 0, c->stream, 1, plane_map(st).npp, st.rhs32,
+                                  c->d_gridred, ctl))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }

@@ -1047,7 +1047,8 @@ __device__ __forceinline__ void conv_step(const DevGrid* grids, int ngrid, int m
 __global__ void k_mx_conv(const DevGrid* __restrict__ grids, int ngrid, int maxlevel,
                           double* __restrict__ gridmax, int* ctl, double* maxrhs,
                           const double* __restrict__ sprm, double epcorr, int nouter_min, int reset) {
-    if (ctl[0]) return;
+    follow_on();
+    if (flag_at(ctl)) return;
     __shared__ double sh[32];
     conv_step<false>(grids, ngrid, maxlevel, gridmax, ctl, maxrhs, sprm, epcorr, nouter_min, sh, reset != 0);
 }
@@ -1433,7 +1434,6 @@ struct TileOuterArgs {
 // numbers, as integers).
 template <bool kPad>
 __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ TileOuterArgs a) {
-    if (a.t.ctl[0]) return;
     __shared__ float shm[4];
     const TileShape& s = a.t.s;
     const int g = a.t.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
@@ -1442,15 +1442,23 @@ __global__ void __launch_bounds__(128, 4) k_tile_outer(const __grid_constant__ T
     const int ipx = G->ipx + 2, ipy = G->ipy + 2, ipz = G->ipz + 2;
     const float* APX = a.APX + (long long)a.t.gcls[g] * 2 * s.npp;
     float mx = 0.f;
-    for (int tile = blockIdx.x * 128 + threadIdx.x; tile < s.ntile; tile += gridDim.x * 128) {
-        const int p = 8 * tile;
+    const int tile = blockIdx.x * 128 + threadIdx.x, p = 8 * tile;
+    const bool on = tile < s.ntile;
+    int4 n0, n1;
+    Vec<float, 8> aph, apl, rh8, rl8, dh8, dl8;
+    if (on) {
+        n0 = __ldg(s.nbr + 2 * tile);
+        n1 = __ldg(s.nbr + 2 * tile + 1);
+    }
+    ldt(on, APX + p, aph);
+    ldt(on, APX + s.npp + p, apl);
+    follow_on();
+    if (flag_at(a.t.ctl)) return;
+    if (on) {
         TileHalo<T8, float> o;
-        tile_halo<kPad>(a.t, g, tile, o);
-        const int org = __ldg(s.nbr + 2 * tile + 1).z;
+        tile_halo<kPad>(a.t, g, tile, n0, n1, o);
+        const int org = n1.z;
         const int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
-        Vec<float, 8> aph, apl, rh8, rl8, dh8, dl8;
-        ldt(true, APX + p, aph);
-        ldt(true, APX + s.npp + p, apl);
         ldt_rw(true, a.RHS + base + p, rh8);
         ldt_rw(true, a.RHSL + base + p, rl8);
         ldt_rw(true, a.DPH + base + p, dh8);
@@ -1990,15 +1998,13 @@ static int launch_tile_sweep_of(const SipState& st, const TileArgs<float>& a, in
     auto go = [&](auto* k) -> int {
         if (smem > 48 * 1024)
             MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        k<<<ng, tile_threads(st), smem, s>>>(a);
-        return 0;
+        return launch_follow_on(k, dim3(ng), tile_threads(st), smem, s, 1, a);
     };
     if (ng <= kTileFew) {
         auto few = [&](auto* k) -> int {
             if (smem > 48 * 1024)
                 MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            k<<<ng, 2 * tile_threads(st) - 32, smem, s>>>(a);
-            return 0;
+            return launch_follow_on(k, dim3(ng), 2 * tile_threads(st) - 32, smem, s, 1, a);
         };
         if (tile_threads(st) <= 160) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 2, 288, false, kPad>);
         if (tile_threads(st) <= 288) return few(k_tile_sweep_few<T8, float, kFwd, kHz, 1, 544, false, kPad>);
@@ -2014,11 +2020,11 @@ static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int n
 }
 
 template <bool kPad>
-static void launch_tile_pre(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
+static int launch_tile_pre(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
     const dim3 grid(tile_parts(st, 128), ng);
-    if (st.unicls) k_tile_pre<T8, float, true, 0, 128, 6, kPad><<<grid, 128, 0, s>>>(a);
-    else if (st.prepk) k_tile_pre<T8, float, false, 0, 128, 4, kPad><<<grid, 128, 0, s>>>(a);
-    else k_tile_pre<T8, float, false, 1, 128, 4, kPad><<<grid, 128, 0, s>>>(a);
+    if (st.unicls) return launch_follow_on(k_tile_pre<T8, float, true, 0, 128, 6, kPad>, grid, 128, 0, s, 1, a);
+    if (st.prepk) return launch_follow_on(k_tile_pre<T8, float, false, 0, 128, 4, kPad>, grid, 128, 0, s, 1, a);
+    return launch_follow_on(k_tile_pre<T8, float, false, 1, 128, 4, kPad>, grid, 128, 0, s, 1, a);
 }
 
 bool sip_on_tiles(const SipState& st) {
@@ -2403,8 +2409,9 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
             a.LPR = st.tcf + 3 * ts.npp;
             a.lprcls = 4 * ts.npp;
             a.hzero = hzero ? 1 : 0;
-            if (ts.pad) launch_tile_pre<true>(st, a, ng, c->stream);
-            else launch_tile_pre<false>(st, a, ng, c->stream);
+            if (int rc = ts.pad ? launch_tile_pre<true>(st, a, ng, c->stream)
+                                : launch_tile_pre<false>(st, a, ng, c->stream))
+                return rc;
             MG_LAUNCHED(c);
         }
         ProfScope ps_(c, "mx_sip_fwd");
@@ -2521,8 +2528,9 @@ int sip_outer(Ctx* c, SipState& st, const float* apx, const int* gcls, const int
         a.grids = c->d_grids;
         a.gridmax = c->d_gridred;
         const dim3 grid(tile_parts(st, 128), c->ngrid);
-        if (st.tile->s.pad) k_tile_outer<true><<<grid, 128, 0, c->stream>>>(a);
-        else k_tile_outer<false><<<grid, 128, 0, c->stream>>>(a);
+        if (int rc = launch_follow_on(st.tile->s.pad ? k_tile_outer<true> : k_tile_outer<false>, grid, 128, 0,
+                                      c->stream, 1, a))
+            return rc;
         MG_LAUNCHED(c);
         return 0;
     }
@@ -2582,9 +2590,10 @@ int sip_scatter_dp(Ctx* c, SipState& st) {
 
 int sip_conv(Ctx* c, const SipState& st, int* ctl, double* maxrhs, const double* sprm) {
     ProfScope ps_(c, "mx_conv");
-    k_mx_conv<<<1, 1024, 0, c->stream>>>(c->d_grids, c->ngrid, c->maxlevel, c->d_gridred, ctl,
-                                         maxrhs, sprm, c->prm.epcorr, c->prm.nouter_min,
-                                         sip_on_tiles(st) ? 1 : 0);
+    if (int rc = launch_follow_on(k_mx_conv, dim3(1), 1024, 0, c->stream, 1, c->d_grids, c->ngrid, c->maxlevel,
+                                  c->d_gridred, ctl, maxrhs, sprm, c->prm.epcorr, c->prm.nouter_min,
+                                  sip_on_tiles(st) ? 1 : 0))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }

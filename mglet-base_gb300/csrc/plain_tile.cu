@@ -73,7 +73,6 @@ __device__ __forceinline__ double tile_lap(const TileArgs<double>& a, int cls, c
 // non-negative numbers, as integers).
 template <class L, bool kUni>
 __global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOuterArgs a) {
-    if (a.t.ctl[0]) return;
     constexpr int N = L::N;
     __shared__ double shm[4];
     const TileShape& s = a.t.s;
@@ -81,9 +80,16 @@ __global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOute
     const long long base = (long long)g * s.npp;
     const int tile = blockIdx.x * 128 + threadIdx.x, p = N * tile;
     double mx = 0.0;
+    int4 n0, n1;
+    if (tile < s.ntile) {
+        n0 = __ldg(s.nbr + 2 * tile);
+        n1 = __ldg(s.nbr + 2 * tile + 1);
+    }
+    follow_on();
+    if (flag_at(a.t.ctl)) return;
     if (tile < s.ntile) {
         TileHalo<L, double> o;
-        tile_halo(a.t, g, tile, o);
+        tile_halo(a.t, g, tile, n0, n1, o);
         Vec<double, N> rh, dp, c[kUni ? 1 : 7];
         ldt_rw(true, a.RHS + base + p, rh);
         ldt_rw(true, a.DP + base + p, dp);
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
     if (tile >= s.ntile) return;
     const long long base = (long long)g * s.npp, ip3 = grids[g].ip3;
     TileHalo<L, double> o;
-    tile_halo(a.t, g, tile, o);
+    tile_halo(a.t, g, tile, __ldg(s.nbr + 2 * tile), __ldg(s.nbr + 2 * tile + 1), o);
     Vec<double, N> c[kUni ? 1 : 7];
     tile_lap_coefs<L, kUni>(a.t, cls, p, c);
 #pragma unroll
@@ -140,7 +146,8 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
 __global__ void k_pt_conv(int ngrid, double* __restrict__ gridmax, double* stat, double prefak, double epcorr,
                           int nouter_min) {
     int* ctl = reinterpret_cast<int*>(stat + 1);
-    if (ctl[0]) return;
+    follow_on();
+    if (flag_at(ctl)) return;
     __shared__ double sh[32];
     double m = 0.0;
     for (int g = threadIdx.x; g < ngrid; g += blockDim.x) {
@@ -174,6 +181,8 @@ constexpr int kFew = 152;
 // 40 on 2, 49 on one; 64 grids 40 on 2, 49 on one.
 constexpr int kRankThreads = 672, kDepth = 2;
 
+static int rank_threads(const TileShape& s) { return 2 * ((s.maxt + 31) / 32 * 32) + 32; }
+
 // the launch of a sweep by clusters of s.nc CTAs
 template <class K>
 int rank_config(K* k, Ctx* c, const TileShape& s, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
@@ -184,7 +193,7 @@ int rank_config(K* k, Ctx* c, const TileShape& s, cudaLaunchConfig_t* cfg, cudaL
     at->val.clusterDim.x = s.nc;
     at->val.clusterDim.y = at->val.clusterDim.z = 1;
     cfg->gridDim = dim3(c->ngrid * s.nc);
-    cfg->blockDim = dim3(2 * ((s.maxt + 31) / 32 * 32) + 32);
+    cfg->blockDim = dim3(rank_threads(s));
     cfg->dynamicSmemBytes = smem;
     cfg->stream = c->stream;
     cfg->attrs = at;
@@ -199,19 +208,15 @@ int launch_sweep(Ctx* c, const TileArgs<double>& a) {
     auto go = [&](auto* k) -> int {
         if (smem > 48 * 1024)
             MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-        k<<<c->ngrid, threads, smem, c->stream>>>(a);
-        return 0;
+        return launch_follow_on(k, dim3(c->ngrid), threads, smem, c->stream, 1, a);
     };
     if constexpr (L::N == 1)
         if (a.s.nc > 1) {
-            auto ranks = [&](auto* k) -> int {
-                cudaLaunchConfig_t cfg = {};
-                cudaLaunchAttribute at = {};
-                if (int e = rank_config(k, c, a.s, &cfg, &at)) return e;
-                MG_CUDA(cudaLaunchKernelEx(&cfg, k, a));
-                return 0;
-            };
-            if (int rc = ranks(k_tile_sweep_few<L, double, kFwd, kHz, kDepth, kRankThreads, true>)) return rc;
+            auto* k = k_tile_sweep_few<L, double, kFwd, kHz, kDepth, kRankThreads, true>;
+            if (smem > 48 * 1024)
+                MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            if (int rc = launch_follow_on(k, dim3(c->ngrid * a.s.nc), rank_threads(a.s), smem, c->stream, a.s.nc, a))
+                return rc;
             MG_LAUNCHED(c);
             return 0;
         }
@@ -220,8 +225,7 @@ int launch_sweep(Ctx* c, const TileArgs<double>& a) {
         auto few = [&](auto* k) -> int {
             if (smem > 48 * 1024)
                 MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            k<<<c->ngrid, 2 * threads - 32, smem, c->stream>>>(a);
-            return 0;
+            return launch_follow_on(k, dim3(c->ngrid), 2 * threads - 32, smem, c->stream, 1, a);
         };
         rc = 2 * threads - 32 <= 544 ? few(k_tile_sweep_few<L, double, kFwd, kHz, 2, 544>)
                                      : few(k_tile_sweep_few<L, double, kFwd, kHz, 1, 1024>);
@@ -276,8 +280,10 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
             a.rev = 0;
             {
                 ProfScope ps_(c, "laplacephi");
-                if (p.unicls) k_tile_pre<L, double, true, 0, 128, 4><<<tiles, 128, 0, c->stream>>>(a);
-                else k_tile_pre<L, double, false, 0, 128, 4><<<tiles, 128, 0, c->stream>>>(a);
+                if (int rc = launch_follow_on(p.unicls ? k_tile_pre<L, double, true, 0, 128, 4>
+                                                       : k_tile_pre<L, double, false, 0, 128, 4>,
+                                              tiles, 128, 0, c->stream, 1, a))
+                    return rc;
                 MG_LAUNCHED(c);
             }
             {
@@ -302,11 +308,13 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
         {
             ProfScope ps_(c, "rescal_maxabs");
             o.t = a;
-            if (p.unicls) k_pt_outer<L, true><<<tiles, 128, 0, c->stream>>>(o);
-            else k_pt_outer<L, false><<<tiles, 128, 0, c->stream>>>(o);
+            if (int rc = launch_follow_on(p.unicls ? k_pt_outer<L, true> : k_pt_outer<L, false>, tiles, 128, 0,
+                                          c->stream, 1, o))
+                return rc;
             MG_LAUNCHED(c);
-            k_pt_conv<<<1, 256, 0, c->stream>>>(c->ngrid, p.gridmax, p.stat, prefak, c->prm.epcorr,
-                                                c->prm.nouter_min);
+            if (int rc = launch_follow_on(k_pt_conv, dim3(1), 256, 0, c->stream, 1, c->ngrid, p.gridmax, p.stat,
+                                          prefak, c->prm.epcorr, c->prm.nouter_min))
+                return rc;
             MG_LAUNCHED(c);
         }
         // a long outer loop looks now and then whether it has converged

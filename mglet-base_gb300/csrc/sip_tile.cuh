@@ -84,9 +84,10 @@ struct alignas(sizeof(T) * N < 16 ? sizeof(T) * N : 16) Vec {
     T v[N];
 };
 
-// The N values of a tile.  ldt: through the read-only path (nothing in the launch
-// writes them); ldt_rw: values this CTA writes later in the same launch; p: a
-// predicate, without a branch (a load inside a branch is waited for where the
+// The N values of a tile.  ldt: through the read-only path (tables and coefficients);
+// ldt_co: values the launch before may still write when this one starts (it waits for
+// them first, see follow_on); ldt_rw: values this CTA writes later in the same launch;
+// p: a predicate, without a branch (a load inside a branch is waited for where the
 // branch ends).
 #define MG_LD(SUF, CLOB)                                                                                 \
     template <int N>                                                                                     \
@@ -125,6 +126,7 @@ struct alignas(sizeof(T) * N < 16 ? sizeof(T) * N : 16) Vec {
 MG_LD(, )
 #undef MG_NC
 #define MG_NC ""
+MG_LD(_co, )
 MG_LD(_rw, : "memory")
 #undef MG_NC
 #undef MG_LD
@@ -186,6 +188,40 @@ __device__ __forceinline__ Vec<T, kM> tile_part(const Vec<T, L::N>& r) {
 // a product that is rounded before anything is added to it
 __device__ __forceinline__ float mul_rounded(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rounded(double a, double b) { return __dmul_rn(a, b); }
+
+// Launches that follow one another in a solve overlap at their ends: a launch may start
+// when every CTA of the one before has passed follow_on(), reads its tables, and waits in
+// follow_on() until the one before is complete.  A kernel calls it before its first look
+// at anything a launch has written.
+__device__ __forceinline__ void follow_on() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ int flag_at(const int* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// A launch of such a kernel; nc > 1: in clusters of nc CTAs.
+template <class... P, class... A>
+int launch_follow_on(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, int nc, A... args) {
+    cudaLaunchAttribute at[2] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = nc;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = nc > 1 ? 2 : 1;
+    MG_CUDA(cudaLaunchKernelEx(&cfg, k, P(args)...));
+    return 0;
+}
 
 template <typename T>
 struct TileArgs {
@@ -358,7 +394,7 @@ struct TileSweep {
                 // (in the launches that write pads, the arrays' other cells are read here)
                 const T* src = a.G + ((long long)max(n, 0) * s.npp + L::N * (kPad ? e[i].y & 0xffff : e[i].y));
                 if constexpr (kPad && !kFwd) ldt_rw(n >= 0, src, v[i]);
-                else ldt(n >= 0, src, v[i]);
+                else ldt_co(n >= 0, src, v[i]);
             }
 #pragma unroll
             for (int i = 0; i < kU; ++i) {
@@ -449,6 +485,10 @@ struct TileSweep {
     }
     // thread lane's loads of a step whose tiles are t0 .. t1
     __device__ __forceinline__ void fetch(TileSet<L, T>& q, int lane, int t0, int t1) {
+        coefs(q, lane, t0, t1);
+        values(q);
+    }
+    __device__ __forceinline__ void coefs(TileSet<L, T>& q, int lane, int t0, int t1) {
         const int tile = t0 + lane;
         const bool on = tile < t1;
         q.tile = on ? tile : -1;
@@ -457,8 +497,11 @@ struct TileSweep {
         ldt(on, C + p, q.c[0]);
         ldt(on, C + s.npp + p, q.c[1]);
         ldt(on, C + 2 * s.npp + p, q.c[2]);
-        if constexpr (kFwd || kPad) ldt_rw(on, R + p, q.v);
-        else ldt(on, R + p, q.v);
+    }
+    __device__ __forceinline__ void values(TileSet<L, T>& q) {
+        const int p = L::N * q.tile;
+        if constexpr (kFwd || kPad) ldt_rw(q.tile >= 0, R + p, q.v);
+        else ldt_co(q.tile >= 0, R + p, q.v);
     }
     // the recurrence of a tile's cells in step t
     __device__ __forceinline__ void solve(int t, const TileSet<L, T>& q, Vec<T, L::N>& r) {
@@ -503,13 +546,14 @@ struct TileSweep {
 // 559-567; kHz: hilf = res).  The last warp stages the ghosts.
 template <class L, typename T, bool kFwd, bool kHz, int kD, int kThreads, int kMinBlocks, bool kPad = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __grid_constant__ TileArgs<T> a) {
-    if (a.ctl[0]) return;
     extern __shared__ __align__(32) unsigned char tsm[];
     TileSweep<L, T, kFwd, false, kPad> w(a, tsm);
     const int tid = threadIdx.x, ncomp = blockDim.x - 32, NT = a.s.NT;
     int2 e[w.kU];
     w.entries(e, tid);
     w.tables();
+    follow_on();
+    if (flag_at(a.ctl)) return;
     w.ghosts(e);
     __syncthreads();
     if (tid >= ncomp) {
@@ -567,7 +611,6 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     const TileShape& s = a.s;
     const int tid = threadIdx.x, ncomp = (blockDim.x - 32) / 2, NT = s.NT, t0 = w.t0, t1 = w.t1;
     const int set = tid >= ncomp ? 1 : 0, lane = tid - set * ncomp;   // (the last warp: neither)
-    const int converged = __ldg(a.ctl);
     int2 e[w.kU];
     w.entries(e, tid);
     TileSet<L, T> q[kD];
@@ -575,14 +618,19 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     const int nc = kRanks ? s.nc : 1;
     auto first = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank) : 0; };
     auto past = [&](int t) { return t < t1 ? __ldg(s.tst + (kFwd ? t : NT - 1 - t) * nc + w.rank + 1) : 0; };
+    if (tid < 2 * ncomp)
+#pragma unroll
+        for (int d = 0; d < kD; ++d) w.coefs(q[d], lane, first(t0 + set + 2 * d), past(t0 + set + 2 * d));
+    w.tables();
+    if constexpr (kRanks) w.arm();
+    follow_on();
+    const int converged = flag_at(a.ctl);
     auto start = [&]() {
         if (tid < 2 * ncomp)
 #pragma unroll
-            for (int d = 0; d < kD; ++d) w.fetch(q[d], lane, first(t0 + set + 2 * d), past(t0 + set + 2 * d));
+            for (int d = 0; d < kD; ++d) w.values(q[d]);
     };
     if constexpr (!kLate) start();
-    w.tables();
-    if constexpr (kRanks) w.arm();
     w.ghosts(e);
     if (converged) return;   // (every rank of a cluster or none)
     if constexpr (kRanks) cluster_barrier();
@@ -683,16 +731,16 @@ __device__ __forceinline__ Vec<T, L::template F<kF / 2>> tile_face(const TileArg
         return *reinterpret_cast<const Vec<T, nf>*>(p + (last ? L::template cell<ax>(0, false) : L::template cell<ax>(0, hi)));
     } else {
         Vec<T, L::N> v;
-        ldt(true, p, v);
+        ldt_co(true, p, v);
         if (kPad && last) return tile_part<L, ax, false>(v);
         return tile_part<L, ax, hi>(v);
     }
 }
 
 template <bool kPad = false, class L, typename T>
-__device__ __forceinline__ void tile_halo(const TileArgs<T>& a, int g, int tile, TileHalo<L, T>& o) {
-    const int4 n0 = __ldg(a.s.nbr + 2 * tile), n1 = __ldg(a.s.nbr + 2 * tile + 1);
-    ldt(true, a.H + ((long long)g * a.s.npp + L::N * tile), o.h);
+__device__ __forceinline__ void tile_halo(const TileArgs<T>& a, int g, int tile, int4 n0, int4 n1,
+                                          TileHalo<L, T>& o) {
+    ldt_co(true, a.H + ((long long)g * a.s.npp + L::N * tile), o.h);
     o.im = tile_face<L, 0, kPad>(a, g, n0.x, n1.z);
     o.ip = tile_face<L, 1, kPad>(a, g, n0.y, n1.z);
     o.jm = tile_face<L, 2, kPad>(a, g, n0.z, n1.z);
@@ -735,47 +783,51 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<L, T>& o, int i, T n[6]
 // compiler does it in the packed and in the table-driven cell pre-pass.
 template <class L, typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks, bool kPad = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_constant__ TileArgs<T> a) {
-    if (a.ctl[0]) return;
     constexpr int N = L::N;
     const TileShape& s = a.s;
     const int b = a.rev ? gridDim.y - 1 - blockIdx.y : blockIdx.y;
     const int g = a.glist ? a.glist[b] : b;
     const int cls = a.gcls[g];
     const long long base = (long long)g * s.npp;
-    const T* LPR = a.LPR + (long long)cls * a.lprcls;
+    const int tile = blockIdx.x * kThreads + threadIdx.x, p = N * tile;
+    const bool on = tile < s.ntile;
     const T* LAP = a.LAP + (long long)cls * 7 * s.npp;
+    Vec<T, N> rh, lp, out;
     T u[7];
 #pragma unroll
     for (int f = 0; f < 7; ++f) u[f] = kUni ? a.UNI[8 * cls + f] : T(0);
-    for (int tile = blockIdx.x * kThreads + threadIdx.x; tile < s.ntile; tile += gridDim.x * kThreads) {
-        const int p = N * tile;
-        Vec<T, N> rh, lp, out;
-        ldt(true, a.RHS + base + p, rh);
-        ldt(true, LPR + p, lp);
-        if (a.hzero) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
-        } else {
-            TileHalo<L, T> o;
-            tile_halo<kPad>(a, g, tile, o);
-            Vec<T, N> c[kUni ? 1 : 7];
-            if constexpr (!kUni)
-#pragma unroll
-                for (int f = 0; f < 7; ++f) ldt(true, LAP + f * s.npp + p, c[f]);
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-                T n[6], w[7];
-                tile_nbrs<L>(o, i, n);
-#pragma unroll
-                for (int f = 0; f < 7; ++f) w[f] = kUni ? u[f] : c[kUni ? 0 : f].v[i];
-                T lap = mul_rounded(-w[kOrder], n[kOrder]);
-                lap = lap - w[1 - kOrder] * n[1 - kOrder] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] -
-                      w[5] * n[5] - w[6] * o.h.v[i];
-                out.v[i] = mul_rounded(rh.v[i] + lap, lp.v[i]);
-            }
-        }
-        stt(a.R + base + p, out);
+    ldt(on, a.LPR + (long long)cls * a.lprcls + p, lp);
+    int4 n0, n1;
+    if (on) {
+        n0 = __ldg(s.nbr + 2 * tile);
+        n1 = __ldg(s.nbr + 2 * tile + 1);
     }
+    follow_on();
+    if (flag_at(a.ctl) || !on) return;
+    ldt_co(true, a.RHS + base + p, rh);
+    if (a.hzero) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
+    } else {
+        TileHalo<L, T> o;
+        tile_halo<kPad>(a, g, tile, n0, n1, o);
+        Vec<T, N> c[kUni ? 1 : 7];
+        if constexpr (!kUni)
+#pragma unroll
+            for (int f = 0; f < 7; ++f) ldt(true, LAP + f * s.npp + p, c[f]);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            T n[6], w[7];
+            tile_nbrs<L>(o, i, n);
+#pragma unroll
+            for (int f = 0; f < 7; ++f) w[f] = kUni ? u[f] : c[kUni ? 0 : f].v[i];
+            T lap = mul_rounded(-w[kOrder], n[kOrder]);
+            lap = lap - w[1 - kOrder] * n[1 - kOrder] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] - w[5] * n[5] -
+                  w[6] * o.h.v[i];
+            out.v[i] = mul_rounded(rh.v[i] + lap, lp.v[i]);
+        }
+    }
+    stt(a.R + base + p, out);
 }
 
 // ---- host tables ------------------------------------------------------------
