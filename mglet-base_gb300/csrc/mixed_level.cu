@@ -403,7 +403,7 @@ __global__ void k_mx_ftoc(const DevGrid* __restrict__ grids, const int4* __restr
 
 // max |rhs| per grid (maxabscal_grid after the restriction of the residual
 // into the coarse grids), of its leading float as the outer step forms it
-__global__ void k_mx_gridmax(int npp, const float* __restrict__ H, double* gridmax, const int* ctl) {
+__global__ void k_mx_gridmax(int npp, const float* H, double* gridmax, const int* ctl) {
     follow_on();
     if (flag_at(ctl)) return;
     __shared__ float sh[32];

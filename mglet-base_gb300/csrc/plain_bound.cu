@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "follow_on.cuh"
 #include "internal.h"
 
 namespace mg {
@@ -68,6 +69,7 @@ struct BoundArgs {
 __global__ void k_bound_vel(BoundArgs a) {
     const int g = a.list[blockIdx.y];
     const DevGrid G = a.grids[g];
+    follow_on();
     if (a.ilevel && G.level != a.ilevel) return;
     const int typ = G.bc[a.iface - 1];
     const Face f = make_face(G, a.iface);
@@ -119,6 +121,7 @@ __global__ void k_bound_vel(BoundArgs a) {
 __global__ void k_bound_p(BoundArgs a) {
     const int g = a.list[blockIdx.y];
     const DevGrid G = a.grids[g];
+    follow_on();
     if (a.ilevel && G.level != a.ilevel) return;
     const int typ = G.bc[a.iface - 1];
     const Face f = make_face(G, a.iface);
@@ -205,10 +208,10 @@ int launch_bound_flow(Ctx* c, double* u, double* v, double* w, double* p, int il
         a.ilevel = ilevel;
         a.rho = c->prm.rho;
         const dim3 grid((maxq + 127) / 128, (unsigned)c->bgrids[f].size());
-        k_bound_vel<<<grid, 128, 0, c->stream>>>(a);
+        if (int rc = launch_follow_on(k_bound_vel, grid, 128, 0, c->stream, 1, a)) return rc;
         MG_LAUNCHED(c);
         if (p) {
-            k_bound_p<<<grid, 128, 0, c->stream>>>(a);
+            if (int rc = launch_follow_on(k_bound_p, grid, 128, 0, c->stream, 1, a)) return rc;
             MG_LAUNCHED(c);
         }
     }

@@ -16,6 +16,7 @@
 #include <limits>
 #include <vector>
 
+#include "follow_on.cuh"
 #include "internal.h"
 
 namespace mg {
@@ -52,6 +53,7 @@ struct ParArgs {
 __global__ void k_bound_par(ParArgs A) {
     const int g = A.list[blockIdx.y];
     const DevGrid G = A.grids[g];
+    follow_on();
     if (A.ilevel && G.level != A.ilevel) return;
     const int axis = (A.iface - 1) / 2;
     const bool lo = (A.iface % 2) == 1;
@@ -132,23 +134,30 @@ __global__ void k_bound_par(ParArgs A) {
 struct ParentArgs {
     const DevGrid* grids;
     const int4* hier;
-    const int* list;            // grids of the level with a PAR face iface
+    // entries first[f] .. first[f + 1] of blockIdx.x: the grids of the level with a PAR
+    // face f + 1 (no face reads what another one's prolongation writes)
+    const int* list[6];
+    int first[7];
     const BFace* bface;
     const double* fc[6];        // coarse fields of the slots
     double* buf[6];             // their boundary buffers
     int comp[6];                // 1..3 vector component (staggered along x/y/z), 0 scalar
-    int iface;
+    int normal;                 // vector components on the faces normal to them only
 };
 
 // One thread per element (j, i) of the fine face buffer (jj2d x ii2d):
 // prolong2 of prolong1 of the parent's slab, evaluated in place.
 __global__ void k_parent(ParentArgs A) {
-    const int g = A.list[blockIdx.y];
+    int face = 0;
+    while ((int)blockIdx.x >= A.first[face + 1]) ++face;
+    const int g = A.list[face][blockIdx.x - A.first[face]];
     const int slot = blockIdx.z;
     const DevGrid G = A.grids[g];
     const int4 H = A.hier[g];
     const DevGrid P = A.grids[H.x];
-    const int iface = A.iface, comp = A.comp[slot];
+    const int iface = face + 1, comp = A.comp[slot];
+    follow_on();
+    if (A.normal && comp > 0 && face / 2 != comp - 1) return;
     const int kk = G.kk, jj = G.jj, ii = G.ii;
     int jj2d, ii2d, st1 = 0, st2 = 0;
     if (iface <= 2) { ii2d = jj; jj2d = kk; }
@@ -157,7 +166,7 @@ __global__ void k_parent(ParentArgs A) {
     if (iface <= 2) { st2 = comp == 2; st1 = comp == 3; }
     else if (iface <= 4) { st2 = comp == 1; st1 = comp == 3; }
     else { st2 = comp == 1; st1 = comp == 2; }
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.y * blockDim.x + threadIdx.x;
     if (q >= jj2d * ii2d) return;
     const int j = q % jj2d + 1, i = q / jj2d + 1;
     // the parent slab (parent_core_mod.F90:190-255)
@@ -205,29 +214,35 @@ __global__ void k_parent(ParentArgs A) {
 // ---- bound_pressure -------------------------------------------------------
 struct BpArgs {
     const DevGrid* grids;
-    const int* list;
+    // entries first[f] .. first[f + 1] of blockIdx.x: the grids with a PAR face f + 1 (a
+    // face reads interior values and writes its own ghosts: the order is free)
+    const int* list[6];
+    int first[7];
     const BFace* bface;
     const double* buf;
     const double* bp;           // null: the no-BP forms
     const double *ddx, *ddy, *ddz, *dx, *dy, *dz;
     double* p;
-    int iface, ilevel;
+    int ilevel;
 };
 
 // One thread per 2x2 block of the face (bfront/bright/bbottom and _bp)
 __global__ void k_bound_pressure(BpArgs A) {
-    const int g = A.list[blockIdx.y];
+    int iface = 1;
+    while ((int)blockIdx.x >= A.first[iface]) ++iface;
+    const int g = A.list[iface - 1][blockIdx.x - A.first[iface - 1]];
     const DevGrid G = A.grids[g];
+    follow_on();
     if (G.level != A.ilevel) return;
-    const int axis = (A.iface - 1) / 2;
-    const bool lo = (A.iface % 2) == 1;
+    const int axis = (iface - 1) / 2;
+    const bool lo = (iface % 2) == 1;
     const int nn = axis == 0 ? G.ii : (axis == 1 ? G.jj : G.kk);
     const int n2 = lo ? 2 : nn - 1, n3 = lo ? 3 : nn - 2, n4 = lo ? 4 : nn - 3;
     const int st2 = lo ? 2 : nn - 2;
     const int nmin = n3 < n4 ? n3 : n4;
     const int na = axis == 2 ? G.jj : G.kk, nb = axis == 0 ? G.jj : G.ii;
     const int nba = (na - 4) / 2, nbb = (nb - 4) / 2;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = blockIdx.y * blockDim.x + threadIdx.x;
     if (q >= nba * nbb) return;
     const int a = 3 + 2 * (q % nba), b = 3 + 2 * (q / nba);
     const FaceIx F{axis, G.kk, G.jj};
@@ -241,7 +256,7 @@ __global__ void k_bound_pressure(BpArgs A) {
     const double* dstag = axis == 0 ? A.dx + G.ipx - 1 : (axis == 1 ? A.dy + G.ipy - 1 : A.dz + G.ipz - 1);
     const double* da = axis == 2 ? ddy : ddz;
     const double* db = axis == 0 ? ddy : ddx;
-    const double pbv = A.buf[A.bface[6 * g + A.iface - 1].off + (long long)(a - 1) + (long long)(b - 1) * na];
+    const double pbv = A.buf[A.bface[6 * g + iface - 1].off + (long long)(a - 1) + (long long)(b - 1) * na];
     int k, j, i;
     if (axis == 0) { k = a; j = b; i = nmin; }
     else if (axis == 1) { k = a; j = nmin; i = b; }
@@ -328,6 +343,7 @@ __global__ void k_ftoc(FtocArgs A) {
     const int g = A.list[blockIdx.y];
     const DevGrid G = A.grids[g];
     const int4 H = A.hier[g];
+    follow_on();
     const DevGrid P = A.grids[H.x];
     const char f = A.flag;
     const double* bp = A.bp + G.ip3;
@@ -1202,48 +1218,47 @@ int launch_bound_par(Ctx* c, int iface, int ilevel, double* u, double* v, double
     A.u = u; A.v = v; A.w = w;
     A.iface = iface;
     A.ilevel = ilevel;
-    k_bound_par<<<dim3((maxq + 127) / 128, (unsigned)c->pgrids[f].size()), 128, 0, c->stream>>>(A);
+    if (int rc = launch_follow_on(k_bound_par, dim3((maxq + 127) / 128, (unsigned)c->pgrids[f].size()), 128, 0,
+                                  c->stream, 1, A))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }
 
 int launch_parent(Ctx* c, int ilevel, const char* const v[3], const char* const s[3], bool normal) {
     ProfScope ps_(c, "parent");
+    ParentArgs A{};
+    A.grids = c->d_grids;
+    A.hier = c->d_hier;
+    A.bface = c->d_bface;
+    A.normal = normal ? 1 : 0;
+    int maxq = 0;
     for (int f = 0; f < 6; ++f) {
         auto it = c->d_plist[f].find(ilevel);
+        A.first[f + 1] = A.first[f];
         if (it == c->d_plist[f].end()) continue;
         const std::vector<int>& list = c->plist[f][ilevel];
-        ParentArgs A{};
-        A.grids = c->d_grids;
-        A.hier = c->d_hier;
-        A.bface = c->d_bface;
-        A.list = it->second;
-        A.iface = f + 1;
-        int nslot = 0;
-        const bool ex[3] = {!normal || f < 2, !normal || (f >= 2 && f < 4), !normal || f >= 4};
-        for (int q = 0; q < 3; ++q)
-            if (v[q] && ex[q]) {
-                A.fc[nslot] = c->F(v[q]);
-                A.buf[nslot] = field_buffer(c, v[q]);
-                if (!A.buf[nslot]) return cuda_fail(cudaErrorMemoryAllocation, "parent buffers");
-                A.comp[nslot++] = q + 1;
-            }
-        for (int q = 0; q < 3; ++q)
-            if (s[q]) {
-                A.fc[nslot] = c->F(s[q]);
-                A.buf[nslot] = field_buffer(c, s[q]);
-                if (!A.buf[nslot]) return cuda_fail(cudaErrorMemoryAllocation, "parent buffers");
-                A.comp[nslot++] = 0;
-            }
-        if (!nslot) continue;
-        int maxq = 0;
+        A.list[f] = it->second;
+        A.first[f + 1] += (int)list.size();
         for (int g : list) {
             const DevGrid& G = c->grids[g];
             maxq = std::max(maxq, (f / 2 == 2 ? G.jj : G.kk) * (f / 2 == 0 ? G.jj : G.ii));
         }
-        k_parent<<<dim3((maxq + 127) / 128, (unsigned)list.size(), nslot), 128, 0, c->stream>>>(A);
-        MG_LAUNCHED(c);
     }
+    if (A.first[6] == 0) return 0;
+    int nslot = 0;
+    for (int q = 0; q < 6; ++q)
+        if (const char* nm = q < 3 ? v[q] : s[q - 3]) {
+            A.fc[nslot] = c->F(nm);
+            A.buf[nslot] = field_buffer(c, nm);
+            if (!A.buf[nslot]) return cuda_fail(cudaErrorMemoryAllocation, "parent buffers");
+            A.comp[nslot++] = q < 3 ? q + 1 : 0;
+        }
+    if (!nslot) return 0;
+    if (int rc = launch_follow_on(k_parent, dim3((unsigned)A.first[6], (maxq + 127) / 128, nslot), 128, 0, c->stream,
+                                  1, A))
+        return rc;
+    MG_LAUNCHED(c);
     return 0;
 }
 
@@ -1278,7 +1293,8 @@ int launch_ftoc(Ctx* c, int ilevel, const double* ff, double* fc, char flag) {
         const DevGrid& G = c->grids[g];
         maxq = std::max(maxq, (G.ii / 2 - 1) * (G.jj / 2 - 1) * (G.kk / 2 - 1));
     }
-    k_ftoc<<<dim3((maxq + 127) / 128, (unsigned)list.size()), 128, 0, c->stream>>>(A);
+    if (int rc = launch_follow_on(k_ftoc, dim3((maxq + 127) / 128, (unsigned)list.size()), 128, 0, c->stream, 1, A))
+        return rc;
     MG_LAUNCHED(c);
     return 0;
 }
@@ -1302,28 +1318,30 @@ int launch_ctof(Ctx* c, int ilevel, double* ff, const double* fc) {
 
 int launch_bound_pressure(Ctx* c, int ilevel, double* p, const double* buf, bool withbp) {
     ProfScope ps_(c, "bound_pressure");
+    BpArgs A{};
+    int maxq = 0;
     for (int f = 0; f < 6; ++f) {
-        if (c->pgrids[f].empty()) continue;
-        int maxq = 0;
+        A.list[f] = c->d_pgrids[f];
+        A.first[f + 1] = A.first[f] + (int)c->pgrids[f].size();
         for (int g : c->pgrids[f]) {
             const DevGrid& G = c->grids[g];
             const int na = f / 2 == 2 ? G.jj : G.kk, nb = f / 2 == 0 ? G.jj : G.ii;
             maxq = std::max(maxq, ((na - 4) / 2) * ((nb - 4) / 2));
         }
-        BpArgs A{};
-        A.grids = c->d_grids;
-        A.list = c->d_pgrids[f];
-        A.bface = c->d_bface;
-        A.buf = buf;
-        A.bp = withbp ? c->F("BP") : nullptr;
-        A.ddx = c->L("DDX"); A.ddy = c->L("DDY"); A.ddz = c->L("DDZ");
-        A.dx = c->L("DX"); A.dy = c->L("DY"); A.dz = c->L("DZ");
-        A.p = p;
-        A.iface = f + 1;
-        A.ilevel = ilevel;
-        k_bound_pressure<<<dim3((maxq + 127) / 128, (unsigned)c->pgrids[f].size()), 128, 0, c->stream>>>(A);
-        MG_LAUNCHED(c);
     }
+    if (A.first[6] == 0 || maxq == 0) return 0;
+    A.grids = c->d_grids;
+    A.bface = c->d_bface;
+    A.buf = buf;
+    A.bp = withbp ? c->F("BP") : nullptr;
+    A.ddx = c->L("DDX"); A.ddy = c->L("DDY"); A.ddz = c->L("DDZ");
+    A.dx = c->L("DX"); A.dy = c->L("DY"); A.dz = c->L("DZ");
+    A.p = p;
+    A.ilevel = ilevel;
+    if (int rc = launch_follow_on(k_bound_pressure, dim3((unsigned)A.first[6], (maxq + 127) / 128), 128, 0,
+                                  c->stream, 1, A))
+        return rc;
+    MG_LAUNCHED(c);
     return 0;
 }
 

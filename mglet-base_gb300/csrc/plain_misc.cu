@@ -12,6 +12,7 @@
 // copy kernel takes one task per CTA.
 #include <algorithm>
 
+#include "follow_on.cuh"
 #include "internal.h"
 
 namespace mg {
@@ -26,6 +27,7 @@ struct FieldSlots {
 __global__ void k_connect(const BoxCopy* __restrict__ tasks, FieldSlots fs) {
     const BoxCopy t = tasks[blockIdx.x];
     double* a = fs.f[t.slot];
+    follow_on();
     const int nkj = t.nk * t.nj;
     for (int q = threadIdx.x; q < t.npts; q += blockDim.x) {
         const int k = q % t.nk, j = (q / t.nk) % t.nj, i = q / nkj;
@@ -145,7 +147,7 @@ int launch_connect(Ctx* c, const ConnectPlan& plan, double* const fields[6]) {
     if (plan.ntasks == 0) return 0;
     FieldSlots fs;
     for (int q = 0; q < 6; ++q) fs.f[q] = fields[q];
-    k_connect<<<plan.ntasks, 128, 0, c->stream>>>(plan.d_tasks, fs);
+    if (int rc = launch_follow_on(k_connect, dim3(plan.ntasks), 128, 0, c->stream, 1, plan.d_tasks, fs)) return rc;
     MG_LAUNCHED(c);
     return 0;
 }
