@@ -454,8 +454,12 @@ __device__ void boundary_terms(const FluxArgs& a, const DevGrid& G, int k, int j
 
 // One CTA per j-slab of a grid, one thread per interior (k, j) of the slab,
 // marching i.
-template <bool kW>
-__global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
+// kT: threads; up to kFluxNarrow the launch has the registers the fluxes ask for (us a
+// launch with 56 and 85: 8 grids of 24^3 86 / 76, 144 with a model 443 / 409, 210 of
+// 21x26x19 157 / 127, 832 of 16^3 with ghost cells 363 / 341).
+constexpr int kFluxNarrow = 384;
+template <bool kW, int kT>
+__global__ void __launch_bounds__(kT, 2) k_mx_flux(FluxArgs a) {
     extern __shared__ float2 sm[];
     const DevGrid G = a.grids[blockIdx.x / a.nslab];
     const int slab = blockIdx.x % a.nslab;
@@ -563,6 +567,7 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
     const bool wv = (wg || (kW && a.gall)) && !(a.guni && a.guni[2 * (blockIdx.x / a.nslab)] != 0.0);
     for (int i = 3; i <= ii - 2; ++i) {
         float uo = 0.f, vo = 0.f, wo = 0.f;
+        const long long c = o + (long long)(i - 1) * kj + (long long)(j - 1) * kk + (k - 1);
         if (on) {
             if constexpr (kW) {
                 const Visc3 vs = visc_at(a, G, wv, k, j, i);
@@ -582,7 +587,6 @@ __global__ void __launch_bounds__(576, 2) k_mx_flux(FluxArgs a) {
         __syncthreads();   // every thread is done with slot (i-1)%3 and p slot i%2
         if (i + 2 <= ii - 1) load_plane(i + 2, (i + 2) % 3, (i + 2) % 2, true, unx2, vnx2, wnx2);
         if (on) {
-            const long long c = o + (long long)(i - 1) * kj + (long long)(j - 1) * kk + (k - 1);
             if (kW && pgrid) {
                 a.UO[c] = (double)uo; a.VO[c] = (double)vo; a.WO[c] = (double)wo;
             } else {
@@ -791,6 +795,7 @@ __global__ void __launch_bounds__(576, 2)
     const bool wv = (wg || (kW && a.gall)) && !(a.guni && a.guni[2 * gid] != 0.0);
     for (int i = 3; i <= ii - 2; ++i) {
         float uo = 0.f, vo = 0.f, wo = 0.f;
+        const long long c = o + (long long)(i - 1) * kj + (long long)(j - 1) * kk + (k - 1);
         if (on) {
             if constexpr (kW) {
                 const Visc3 vs = visc_at(a, G, wv, k, j, i);
@@ -808,7 +813,6 @@ __global__ void __launch_bounds__(576, 2)
             convert(i + 2, (i + 2) % 3, (i + 2) % 2, unx2, vnx2, wnx2);
         }
         if (on) {
-            const long long c = o + (long long)(i - 1) * kj + (long long)(j - 1) * kk + (k - 1);
             if (kW && pgrid) {
                 a.UO[c] = (double)uo; a.VO[c] = (double)vo; a.WO[c] = (double)wo;
             } else {
@@ -905,6 +909,14 @@ static int encode_plane_map(Ctx* c, const double* base, CUtensorMap* m) {
     return 0;
 }
 
+// lets the plane-load kernels take smem bytes
+static int flux_allow(size_t smem) {
+    for (auto* k : {k_mx_flux<false, kFluxNarrow>, k_mx_flux<true, kFluxNarrow>, k_mx_flux<false, 576>,
+                    k_mx_flux<true, 576>})
+        MG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return 0;
+}
+
 // Checks the launch limits of the flux kernel for this grid shape and opts
 // in to the dynamic shared memory it needs; where a grid's k x j interior
 // fits one CTA and its planes meet the TMA rules (16-byte rows, whole 128-byte
@@ -920,8 +932,7 @@ int mx_flux_prepare(Ctx* c) {
         set_error("mixed form: grid planes too large for the flux kernel's shared memory");
         return MGLET_ERR_UNSUPPORTED;
     }
-    MG_CUDA(cudaFuncSetAttribute(k_mx_flux<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    MG_CUDA(cudaFuncSetAttribute(k_mx_flux<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int rc = flux_allow(smem)) return rc;
     FluxState& fs = g_flux[c];
     fs = FluxState();
     for (const DevGrid& g : c->grids)
@@ -978,11 +989,10 @@ static int launch_variant(Ctx* c, int v, const FluxArgs& a, int threads) {
         k_mx_flux_rows<<<dim3(c->ngrid * 2 * (a.nslab - 1), (G0.ii * G0.kk + 255) / 256), 256, 0, c->stream>>>(a);
         MG_LAUNCHED(c);
     }
-    if (kw) {
-        k_mx_flux<true><<<nb, threads, psm, c->stream>>>(a);
-    } else {
-        k_mx_flux<false><<<nb, threads, psm, c->stream>>>(a);
-    }
+    if (threads <= kFluxNarrow)
+        (kw ? k_mx_flux<true, kFluxNarrow> : k_mx_flux<false, kFluxNarrow>)<<<nb, threads, psm, c->stream>>>(a);
+    else
+        (kw ? k_mx_flux<true, 576> : k_mx_flux<false, 576>)<<<nb, threads, psm, c->stream>>>(a);
     MG_LAUNCHED(c);
     return 0;
 }
@@ -1120,8 +1130,7 @@ int mx_flux_set_pw(Ctx* c, const unsigned char* d_pw) {
         set_error("mixed form: grid planes too large for the ghost-cell flux windows");
         return MGLET_ERR_UNSUPPORTED;
     }
-    MG_CUDA(cudaFuncSetAttribute(k_mx_flux<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return 0;
+    return flux_allow(smem);
 }
 
 }  // namespace mg
