@@ -652,9 +652,9 @@ static size_t march_smem(int rows, int len, int kk) {
 }
 constexpr size_t kMarchSmem = 220 * 1024;
 
-// How k_tstle4_march cuts the grids: as many rows a CTA as its threads hold (the row
-// before the first is computed twice), and planes so that the CTAs fill the SMs
-// evenly (the fluxes through the first i face twice).  Returns the grids it takes:
+// How k_tstle4_march cuts the grids: rows (the row before a CTA's first is computed
+// twice) and planes (the fluxes through its first i face twice) so that the largest
+// share of an SM in FP64 work, whole warps times planes, is least.  Returns the grids it takes:
 // equal dimensions, all six faces connected.
 static int march_shape(Ctx* c, MarchArgs* m) {
     int n = 0;
@@ -666,23 +666,23 @@ static int march_shape(Ctx* c, MarchArgs* m) {
     const DevGrid& G = c->grids[0];
     const int nk1 = G.kk - 3, nj = G.jj - 4, ni = G.ii - 4;
     if (!c->uniform || n == 0 || 2 * nk1 > kMarchThreads) return 0;
-    const int most = kMarchThreads / nk1 - 1;
-    m->nrow = (nj + most - 1) / most;
-    m->rows = (nj + m->nrow - 1) / m->nrow;
+    const int most = std::min(nj, kMarchThreads / nk1 - 1);
     double best = 0.0;
-    for (int len = 1; len <= ni; ++len) {
-        if (march_smem(m->rows, len, G.kk) > kMarchSmem) break;
-        const int nchunk = (ni + len - 1) / len;
-        const long long waves = ((long long)n * m->nrow * nchunk + 151) / 152;
-        const double t = (double)waves * (len + 0.5);
-        if (best == 0.0 || t <= best) {
-            best = t;
-            m->len = len;
-            m->nchunk = nchunk;
+    for (int rows = most; rows >= 1; --rows)
+        for (int len = 1; len <= ni; ++len) {
+            if (march_smem(rows, len, G.kk) > kMarchSmem) break;
+            const int nrow = (nj + rows - 1) / rows, nchunk = (ni + len - 1) / len;
+            const long long waves = ((long long)n * nrow * nchunk + 151) / 152;
+            const double t = (double)waves * (len + 0.5) * (march_threads(rows, G.kk) / 32);
+            if (best == 0.0 || t < best) {
+                best = t;
+                m->rows = rows;
+                m->nrow = nrow;
+                m->len = len;
+                m->nchunk = nchunk;
+            }
         }
-    }
-    // the last rows and planes of the cut may be empty
-    m->nrow = (nj + m->rows - 1) / m->rows;
+    if (best == 0.0) return 0;
     return n;
 }
 

@@ -68,18 +68,25 @@ __device__ __forceinline__ double tile_lap(const TileArgs<double>& a, int cls, c
     return lap - w[1] * n[1] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] - w[5] * n[5] - w[6] * o.h.v[i];
 }
 
+// max(|r|, mx) on the words (an order of non-negative numbers; fmax is two FP64
+// instructions), which like fmax passes over NaN
+__device__ __forceinline__ unsigned long long larger(double r, unsigned long long mx) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+    return b > mx && b <= 0x7ff0000000000000ull ? b : mx;
+}
+
 // laplacephi of hilf, rescal (rhs += res) with maxabscal_grid, accumulate (dp +=
 // hilf): one thread a tile; gridmax takes the maximum over the CTAs of a grid (of
 // non-negative numbers, as integers).
 template <class L, bool kUni>
 __global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOuterArgs a) {
     constexpr int N = L::N;
-    __shared__ double shm[4];
+    __shared__ unsigned long long shm[4];
     const TileShape& s = a.t.s;
     const int g = blockIdx.y, cls = a.t.gcls[g];
     const long long base = (long long)g * s.npp;
     const int tile = blockIdx.x * 128 + threadIdx.x, p = N * tile;
-    double mx = 0.0;
+    unsigned long long mx = 0;
     int4 n0, n1;
     if (tile < s.ntile) {
         n0 = __ldg(s.nbr + 2 * tile);
@@ -99,18 +106,20 @@ __global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOute
             const double r = rh.v[i] + tile_lap<L, kUni>(a.t, cls, o, c, i);
             rh.v[i] = r;
             dp.v[i] = dp.v[i] + o.h.v[i];
-            mx = fmax(fabs(r), mx);
+            mx = larger(r, mx);
         }
         stt(a.RHS + base + p, rh);
         stt(a.DP + base + p, dp);
     }
-    for (int q = 16; q > 0; q >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, q));
+    for (int q = 16; q > 0; q >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, q);
+        mx = y > mx ? y : mx;
+    }
     if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
     __syncthreads();
     if (threadIdx.x == 0) {
-        mx = fmax(fmax(shm[0], shm[1]), fmax(shm[2], shm[3]));
-        atomicMax(reinterpret_cast<unsigned long long*>(a.gridmax) + g,
-                  (unsigned long long)__double_as_longlong(mx));
+        for (int q = 1; q < 4; ++q) mx = shm[q] > mx ? shm[q] : mx;
+        atomicMax(reinterpret_cast<unsigned long long*>(a.gridmax) + g, mx);
     }
 }
 

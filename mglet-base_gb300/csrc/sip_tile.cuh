@@ -533,11 +533,15 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_sweep(const __gri
         return;
     }
     // kD steps of loads in flight: a step issues the loads of kD steps on before it
-    // computes, into the set the step before has left
+    // computes, into the set the step before has left.  FP64: the warps take the chunks
+    // of a hyperplane in turn, one on each step, so that the chunks that every
+    // hyperplane has do not stay on one of the SM's four FP64 pipes.
     TileSet<L, T> q[kD + 1];
+    int lane = tid;
     auto fetch = [&](int t, TileSet<L, T>& c) {
         const int ta = w.tst[t], tb = w.tst[t + 1];
-        w.fetch(c, tid, kFwd ? ta : tb, kFwd ? tb : ta);
+        w.fetch(c, lane, kFwd ? ta : tb, kFwd ? tb : ta);
+        if constexpr (sizeof(T) == 8) lane = lane + 32 < ncomp ? lane + 32 : lane + 32 - ncomp;
     };
 #pragma unroll
     for (int d = 0; d < kD; ++d) fetch(d, q[d]);
