@@ -29,6 +29,7 @@ struct ScaArgs {
     double *qtu, *qtv, *qtw;
     const double *ddx, *ddy, *ddz, *rdx, *rdy, *rdz;
     double gmol, rho, prmol, prturb;
+    double gscamol;             // gmol / rho / prmol
     int kayscrawford, les;
 };
 
@@ -41,7 +42,7 @@ __device__ __forceinline__ double prt(const ScaArgs& A, double gtgmol) {
 }
 
 __device__ __forceinline__ double gsca(const ScaArgs& A, double g0, double g1) {
-    const double gscamol = A.gmol / A.rho / A.prmol;
+    const double gscamol = A.gscamol;
     if (!A.les) return gscamol;
     const double gtgmolp = (g0 - A.gmol) / A.gmol, gtgmoln = (g1 - A.gmol) / A.gmol;
     const double gs = gscamol + (g1 + g0 - 2.0 * A.gmol) / A.rho / (prt(A, gtgmoln) + prt(A, gtgmolp));
@@ -683,6 +684,7 @@ int timeintegrate_scalar(Ctx* c, double dt, int irk, const mglet_rk_scheme* rk) 
         A.ddx = c->L("DDX"); A.ddy = c->L("DDY"); A.ddz = c->L("DDZ");
         A.rdx = c->L("RDX"); A.rdy = c->L("RDY"); A.rdz = c->L("RDZ");
         A.gmol = c->prm.gmol; A.rho = c->prm.rho; A.prmol = sd.prmol; A.prturb = c->prturb;
+        A.gscamol = A.gmol / A.rho / A.prmol;
         A.kayscrawford = sd.kayscrawford; A.les = c->ilesmodel != 0;
         k_tstsca4<<<bg, 256, 0, c->stream>>>(A);
         MG_LAUNCHED(c);

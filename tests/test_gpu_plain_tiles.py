@@ -41,7 +41,7 @@ def _same(gpu_lib, case, form, **kw):
 SHAPES = [
     ((2, 1, 1), (2, 2, 2)), ((1, 1, 1), (2, 3, 5)), ((1, 2, 2), (2, 16, 6)), ((2, 1, 2), (11, 2, 7)),
     ((2, 2, 2), (24, 24, 24)), ((1, 1, 2), (33, 29, 31)), ((1, 1, 1), (40, 36, 44)),
-    ((3, 3, 3), (10, 9, 8)), ((4, 4, 4), (5, 6, 8)), ((6, 6, 5), (8, 10, 12)), ((6, 6, 5), (9, 8, 7))]
+    ((3, 3, 3), (10, 9, 8)), ((4, 4, 4), (5, 6, 8)), ((6, 6, 5), (8, 10, 12)), ((7, 7, 7), (6, 5, 8)), ((7, 7, 7), (5, 6, 7)), ((6, 6, 5), (9, 8, 7))]
 
 
 @pytest.mark.parametrize("tiles,shape", SHAPES)
