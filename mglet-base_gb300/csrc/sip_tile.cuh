@@ -473,8 +473,10 @@ struct TileSweep {
     // the recurrence of a tile's cells in step t
     __device__ __forceinline__ void solve(int t, const TileSet<L, T>& q, Vec<T, L::N>& r) {
         const int x = q.x - back;
-        Face* cur = face + (t & 1) * 3 * s.slots + x;
-        const Face* prv = face + ((t + 1) & 1) * 3 * s.slots + x;
+        solve_at(face + (t & 1) * 3 * s.slots + x, face + ((t + 1) & 1) * 3 * s.slots + x, q, r);
+    }
+    // (cur, prv: the tile's slot in the faces of the step and of the one before)
+    __device__ __forceinline__ void solve_at(Face* cur, const Face* prv, const TileSet<L, T>& q, Vec<T, L::N>& r) {
         const Face fi = prv[W], fj = prv[s.slots + one], fk = prv[2 * s.slots];
 #pragma unroll
         for (int m = 0; m < L::N; ++m) {
@@ -489,15 +491,16 @@ struct TileSweep {
             r.v[i] = q.v.v[i] - q.c[2].v[i] * rk - q.c[1].v[i] * rj - q.c[0].v[i] * ri;
         }
         cur[0] = tile_part<L, 0, kFwd, T, TileFace<L>::M>(r);
-        if constexpr (kRanks) {
-            // the row the next rank starts from
-            const int I = kFwd ? i1 : i0, J = q.x - (I + 1) * s.w - 1;
-            const int h = (kFwd ? t : s.NT - 1 - t) - I;
-            if (down && J >= 0 && J < s.NJ)
-                cluster_put(bndto + (J * s.NK + h - J) * (unsigned)sizeof(Face), mbarto + 8 * h, cur[0]);
-        }
         cur[s.slots] = tile_part<L, 1, kFwd, T, TileFace<L>::M>(r);
         cur[2 * s.slots] = tile_part<L, 2, kFwd, T, TileFace<L>::M>(r);
+    }
+    // the faces of the row the next rank starts from
+    __device__ __forceinline__ void put(int t, const TileSet<L, T>& q, const Vec<T, L::N>& r) {
+        const int I = kFwd ? i1 : i0, J = q.x - (I + 1) * s.w - 1;
+        const int h = (kFwd ? t : s.NT - 1 - t) - I;
+        if (down && J >= 0 && J < s.NJ)
+            cluster_put(bndto + (J * s.NK + h - J) * (unsigned)sizeof(Face), mbarto + 8 * h,
+                        tile_part<L, 0, kFwd, T, TileFace<L>::M>(r));
     }
     template <bool kHz>
     __device__ __forceinline__ void store(int tile, const Vec<T, L::N>& r) {
@@ -624,17 +627,23 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     }
     __syncthreads();
     Vec<T, L::N> r;
+    // (a set's steps have one parity)
+    auto* const cur = w.face + ((t0 + set) & 1) * 3 * s.slots - w.back;
+    auto* const prv = w.face + ((t0 + set + 1) & 1) * 3 * s.slots - w.back;
     if (set) __syncthreads();   // the first step
     for (int t = t0 + set; t < end; t += 2 * kD) {
 #pragma unroll
         for (int d = 0; d < kD; ++d) {
             const int m = t + 2 * d;
             if (m >= end) break;
-            if (q[d].tile >= 0) w.solve(m, q[d], r);
+            if (q[d].tile >= 0) w.solve_at(cur + q[d].x, prv + q[d].x, q[d], r);
             __syncthreads();
-            // while the other set works: the results to memory, the loads of the
-            // step kD turns on
-            if (q[d].tile >= 0) w.template store<kHz>(q[d].tile, r);
+            // while the other set works: the results to the next rank and to memory,
+            // the loads of the step kD turns on
+            if (q[d].tile >= 0) {
+                if constexpr (kRanks) w.put(m, q[d], r);
+                w.template store<kHz>(q[d].tile, r);
+            }
             const int n = min(m + 2 * kD, NT + 1);
             if constexpr (kRanks) {
                 w.fetch(q[d], lane, w.tst[n], w.tend[n]);
