@@ -2019,12 +2019,12 @@ static int launch_tile_sweep(const SipState& st, const TileArgs<float>& a, int n
                    : launch_tile_sweep_of<kFwd, kHz, false>(st, a, ng, s);
 }
 
-template <bool kPad>
+template <bool kPad, bool kHz>
 static int launch_tile_pre(const SipState& st, const TileArgs<float>& a, int ng, cudaStream_t s) {
     const dim3 grid(tile_parts(st, 128), ng);
-    if (st.unicls) return launch_follow_on(k_tile_pre<T8, float, true, 0, 128, 6, kPad>, grid, 128, 0, s, 1, a);
-    if (st.prepk) return launch_follow_on(k_tile_pre<T8, float, false, 0, 128, 4, kPad>, grid, 128, 0, s, 1, a);
-    return launch_follow_on(k_tile_pre<T8, float, false, 1, 128, 4, kPad>, grid, 128, 0, s, 1, a);
+    if (st.unicls) return launch_follow_on(k_tile_pre<T8, float, kHz, true, 0, 128, 6, kPad>, grid, 128, 0, s, 1, a);
+    if (st.prepk) return launch_follow_on(k_tile_pre<T8, float, kHz, false, 0, 128, 4, kPad>, grid, 128, 0, s, 1, a);
+    return launch_follow_on(k_tile_pre<T8, float, kHz, false, 1, 128, 4, kPad>, grid, 128, 0, s, 1, a);
 }
 
 bool sip_on_tiles(const SipState& st) {
@@ -2408,9 +2408,10 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
             a.R = st.rs[rwrite];
             a.LPR = st.tcf + 3 * ts.npp;
             a.lprcls = 4 * ts.npp;
-            a.hzero = hzero ? 1 : 0;
-            if (int rc = ts.pad ? launch_tile_pre<true>(st, a, ng, c->stream)
-                                : launch_tile_pre<false>(st, a, ng, c->stream))
+            if (int rc = ts.pad ? (hzero ? launch_tile_pre<true, true>(st, a, ng, c->stream)
+                                         : launch_tile_pre<true, false>(st, a, ng, c->stream))
+                                : (hzero ? launch_tile_pre<false, true>(st, a, ng, c->stream)
+                                         : launch_tile_pre<false, false>(st, a, ng, c->stream)))
                 return rc;
             MG_LAUNCHED(c);
         }

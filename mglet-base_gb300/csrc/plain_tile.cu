@@ -285,14 +285,14 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
             ++gi;
             const bool hz = il == 1;
             a.R = p.rs[gi % 3];
-            a.hzero = hz;
             a.rev = 0;
             {
                 ProfScope ps_(c, "laplacephi");
-                if (int rc = launch_follow_on(p.unicls ? k_tile_pre<L, double, true, 0, 128, 4>
-                                                       : k_tile_pre<L, double, false, 0, 128, 4>,
-                                              tiles, 128, 0, c->stream, 1, a))
-                    return rc;
+                auto* k = hz ? (p.unicls ? k_tile_pre<L, double, true, true, 0, 128, 4>
+                                         : k_tile_pre<L, double, true, false, 0, 128, 4>)
+                             : (p.unicls ? k_tile_pre<L, double, false, true, 0, 128, 4>
+                                         : k_tile_pre<L, double, false, false, 0, 128, 4>);
+                if (int rc = launch_follow_on(k, tiles, 128, 0, c->stream, 1, a)) return rc;
                 MG_LAUNCHED(c);
             }
             {

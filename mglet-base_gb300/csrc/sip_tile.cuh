@@ -208,7 +208,6 @@ struct TileArgs {
     const int* ctl;                 // [0] converged: nothing to do
     int cfcls, lprcls;              // values between the classes of CF and of LPR
     int* err;                       // set when a rank waited in vain
-    int hzero;                      // hilf is zero
     int rev;                        // walk the grids in reverse block order
 };
 
@@ -757,11 +756,12 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<L, T>& o, int i, T n[6]
 
 // The part of sipiter1 outside the recurrence, (rhs + laplacephi(hilf)) lpr
 // (sip_hyperplane_mod.F90:491, laplacephi_mod.F90:153-160), one thread a tile;
-// the tiles of a grid in gridDim.x CTAs.  kUni: one value of each operator
+// the tiles of a grid in gridDim.x CTAs.  kHz: hilf is zero (a run-time branch had the
+// other side compute this one's two instructions a cell as well).  kUni: one value of each operator
 // coefficient a class.  Of the first two products one rounds by itself and the
 // other is contracted with it: the first in kOrder 0, the second in kOrder 1, as the
 // compiler does it in the packed and in the table-driven cell pre-pass.
-template <class L, typename T, bool kUni, int kOrder, int kThreads, int kMinBlocks, bool kPad = false>
+template <class L, typename T, bool kHz, bool kUni, int kOrder, int kThreads, int kMinBlocks, bool kPad = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_constant__ TileArgs<T> a) {
     constexpr int N = L::N;
     const TileShape& s = a.s;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
     follow_on();
     if (flag_at(a.ctl) || !on) return;
     ldt_co(true, a.RHS + base + p, rh);
-    if (a.hzero) {
+    if constexpr (kHz) {
 #pragma unroll
         for (int i = 0; i < N; ++i) out.v[i] = mul_rounded(rh.v[i] + T(0), lp.v[i]);
     } else {
