@@ -43,14 +43,17 @@ UNIT = "cell-updates/s"
 
 # Algorithmic bytes per interior cell and launch of the kernel families:
 # every operand read once and every result written once (FP64 8 B, FP32 4 B).
+# The plain solver's are those of one level, on tiles: the pre-pass (timed as
+# laplacephi), the sweeps and the outer step (rescal_maxabs); coefficients that the
+# grids of a class share come from L2.
 PLAIN_BYTES = {
     "tstle4": 8 * (5 + 3),          # read u,v,w,p,g; write uo,vo,wo
     "rkstep": 8 * 4,                # read p,dp,rhs; write p,dp (per component) / 1.25 ~ 4+1
-    "laplacephi": 8 * 3,            # read phi, ap; write res (bp is skipped where it is 1.0)
-    "sipiter1": 8 * 7,              # read rhs, res, lw, ls, lb, lpr; write res
-    "sipiter2": 8 * 7,              # read res, ue, un, ut, phi; write res, phi
+    "laplacephi": 8 * 3,            # read hilf, rhs; write res
+    "sipiter1": 8 * 2,              # read and write res
+    "sipiter2": 8 * 3,              # read res, hilf; write hilf
     "divcal": 8 * 4,                # read u, v, w; write rhs
-    "rescal_maxabs": 8 * 3,         # read rhs, res; write rhs
+    "rescal_maxabs": 8 * 5,         # read hilf, rhs, dp; write rhs, dp
     "accumulate": 8 * 4,            # read dp, hilf; write dp, hilf (whole slab)
     "mgpcorr": 8 * 9,               # read dp,u,v,w,p; write u,v,w,p
 }
@@ -68,30 +71,31 @@ MIXED_BYTES = {
 # outer iteration (the first of them starts from hilf = 0); scaled by cells
 # for other tilings.
 NCU_DRAM_4096 = {
-    "mx_sip_pre": (472.8e6, 184.3e6),
-    "mx_sip_fwd": (373.2e6, 168.0e6),
-    "mx_sip_bwd": (509.5e6, 177.3e6),
-    "mx_outer": (1263.3e6, 848.9e6),
+    "mx_sip_pre": (392.4e6, 245.8e6),
+    "mx_sip_fwd": (300.2e6, 177.5e6),
+    "mx_sip_bwd": (377.6e6, 235.7e6),
+    "mx_outer": (1172.7e6, 896.6e6),
 }
 NCU_CELLS = 4096 * 13824
 
 
 # FP64 thread instructions (DADD, DMUL, DFMA and the conversions the FP64 pipe
 # issues) per interior cell and launch of the plain FP64 kernels, measured by
-# ncu (sm__inst_executed_pipe_fp64 x 32 over one launch on 1024 grids of 24^3,
-# parity build without FMA contraction); with the measured FP64 issue rate
-# they give each kernel's fraction of the second roof.
+# ncu (sm__inst_executed_pipe_fp64 x 32 over one launch on 343 grids of 24^3, parity
+# build without FMA contraction; the pre-pass 15 and, from hilf = 0, 2); with the
+# measured FP64 issue rate they give each kernel's fraction of the second roof.
 FP64_INSTR_PER_CELL = {
-    "tstle4": 232650752 * 32 / (1024 * 13824),      # 525.9 (uniform-G shortcut)
-    "laplacephi": 5750784 * 32 / (1024 * 13824),    # 13.0
-    "sipiter1": 3850240 * 32 / (1024 * 13824),      # 8.70
-    "sipiter2": 3330048 * 32 / (1024 * 13824),      # 7.53
+    "tstle4": 28925190 * 32 / (343 * 13824),        # 195.2 (connected grids, one value of G)
+    "laplacephi": (4 * 15 + 2) / 5,                 # 12.4
+    "sipiter1": 1012536 * 32 / (343 * 13824),       # 6.83
+    "sipiter2": 1012536 * 32 / (343 * 13824),
+    "rescal_maxabs": 2370816 * 32 / (343 * 13824),  # 16.0
 }
 
 
 def kernel_bytes(name, case, ninner):
     """Algorithmic bytes of one launch of a kernel family on this case.
-    FP32 plane-order SIP kernels: the pre-pass reads hilf and rhs and writes
+    FP32 SIP kernels: the pre-pass reads hilf and rhs and writes
     (rhs + laplacian) x lpr; the forward recurrence reads that and writes res
     over it; the backward sweep reads res and hilf and writes hilf; the outer
     step reads hilf and the float-float residual and correction and writes

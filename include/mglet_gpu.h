@@ -541,12 +541,16 @@ int mglet_gpu_set_partition(mglet_ctx* ctx, const int32_t* halo, int32_t nsend,
                             mglet_exchange_fn fn, void* user);
 
 /* ---- Launch tuning of the mixed form (no counterpart in the reference) -----
- * mglet_gpu_create times the launch variants of the mixed form's pre-pass
- * (points loaded ahead, CTAs per SM, and the uniform-coefficient variant
- * where every coefficient class allows it) on the case itself and keeps the
- * fastest, cached per grid shape for the process; the environment variable
- * MGLET_TUNE=0 keeps the defaults.  The same holds for the packed sweeps
- * (ranks per thread, CTAs per SM), the flux kernel (plane loads or TMA) and
+ * The pressure solve on 2x2x2 tiles, the default, has no variants to pick;
+ * forcing a variant of "mx_sip_pre", "mx_sip_sweep", "mx_outer" or
+ * "mx_sip_solve" makes the solve run on the cell hyperplane kernels.  For
+ * grids that tiles do not take, mglet_gpu_create times the launch variants
+ * of the cell hyperplane pre-pass (points loaded ahead, CTAs per SM, and the
+ * uniform-coefficient variant where every coefficient class allows it) on
+ * the case itself and keeps the fastest, cached per grid shape for the
+ * process; the environment variable MGLET_TUNE=0 keeps the defaults.  The
+ * same holds for the packed sweeps (ranks per thread, CTAs per SM), for any
+ * grids for the flux kernel (plane loads or TMA), and for
  * the persistent solve of single-level cases (the whole outer loop of
  * mgpoisl as one cooperative launch with grid-wide barriers; timed and
  * reported, run only when forced: the per-phase kernels are faster in the
