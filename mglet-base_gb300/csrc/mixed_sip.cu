@@ -1375,28 +1375,21 @@ __global__ void k_sip_extract(const DevGrid* __restrict__ grids, const int* __re
 using T8 = Tile<2, 2, 2>;
 
 // class coefficients on tiles from the FP64 fields of the representative grids:
-// {lw, ls, lb, lpr}, {ue, un, ut}, the operator's seven (with the couplings BP
-// closes masked) and ap as two floats
+// {lw, ls, lb, lpr}, {ue, un, ut} and ap as two floats
 __global__ void k_tile_extract(const DevGrid* __restrict__ grids, const int* __restrict__ reps, TileShape s,
                                int planeorder, const double* __restrict__ lw, const double* __restrict__ ls,
                                const double* __restrict__ lb, const double* __restrict__ lpr,
                                const double* __restrict__ ue, const double* __restrict__ un,
-                               const double* __restrict__ ut, const double* __restrict__ ap,
-                               const float* __restrict__ AW, const float* __restrict__ AE,
-                               const float* __restrict__ AS, const float* __restrict__ AN,
-                               const float* __restrict__ AB, const float* __restrict__ AT,
-                               const unsigned char* __restrict__ BM, float* CF, float* CB, float* LAP,
-                               float* APX) {
+                               const double* __restrict__ ut, const double* __restrict__ ap, float* CF,
+                               float* CB, float* APX) {
     const long long cls = blockIdx.y;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= s.npp) return;
-    const int rep = reps[cls];
-    const DevGrid G = grids[rep];
+    const DevGrid G = grids[reps[cls]];
     const int id = s.cell[p];
     if (id < 0) {   // a pad
         for (int q = 0; q < 4; ++q) CF[(cls * 4 + q) * s.npp + p] = 0.f;
         for (int q = 0; q < 3; ++q) CB[(cls * 3 + q) * s.npp + p] = 0.f;
-        for (int q = 0; q < 7; ++q) LAP[(cls * 7 + q) * s.npp + p] = 0.f;
         APX[cls * 2 * s.npp + p] = APX[(cls * 2 + 1) * s.npp + p] = 0.f;
         return;
     }
@@ -1406,13 +1399,6 @@ __global__ void k_tile_extract(const DevGrid* __restrict__ grids, const int* __r
     const double apv = ap[G.ip3 + id];
     for (int q = 0; q < 4; ++q) CF[(cls * 4 + q) * s.npp + p] = f[q];
     for (int q = 0; q < 3; ++q) CB[(cls * 3 + q) * s.npp + p] = b[q];
-    const int kk = G.kk, jj = G.jj;
-    const int ix = G.ipx + id / (kk * jj), iy = G.ipy + (id / kk) % jj, iz = G.ipz + id % kk;
-    const unsigned mk = BM ? BM[(long long)rep * s.npp + p] : 0x3Fu;
-    auto on = [mk](int q, float x) { return (mk >> q) & 1u ? x : 0.f; };
-    const float l[7] = {on(0, AW[ix]), on(1, AE[ix]), on(2, AS[iy]), on(3, AN[iy]),
-                        on(4, AB[iz]), on(5, AT[iz]), (float)apv};
-    for (int q = 0; q < 7; ++q) LAP[(cls * 7 + q) * s.npp + p] = l[q];
     APX[cls * 2 * s.npp + p] = (float)apv;
     APX[(cls * 2 + 1) * s.npp + p] = (float)(apv - (double)(float)apv);
 }
@@ -1980,7 +1966,8 @@ static TileArgs<float> tile_args(SipState& st, const int* gcls, const int* ctl, 
     a.H = st.h32;
     a.RHS = st.rhs32;
     a.PG = st.pg;
-    a.LAP = st.tlap;
+    a.AP = st.tap;
+    a.apcls = 2 * st.tile->s.npp;
     a.UNI = st.uni;
     a.ctl = ctl;
     a.rev = next_order(st);
@@ -2284,7 +2271,7 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
     // a second extraction (new classes after the ghost-cell set-up) replaces
     // the records of the first
     for (void** p : {(void**)&st.swf, (void**)&st.swb, (void**)&st.spr, (void**)&st.uni, (void**)&st.tcf,
-                     (void**)&st.tcb, (void**)&st.tlap, (void**)&st.tap}) {
+                     (void**)&st.tcb, (void**)&st.tap}) {
         cudaFree(*p);
         *p = nullptr;
     }
@@ -2298,12 +2285,11 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
         const size_t nt = (size_t)nclass * ts.npp * sizeof(float);
         MG_CUDA(cudaMalloc(&st.tcf, 4 * nt));
         MG_CUDA(cudaMalloc(&st.tcb, 3 * nt));
-        MG_CUDA(cudaMalloc(&st.tlap, 7 * nt));
         MG_CUDA(cudaMalloc(&st.tap, 2 * nt));
         k_tile_extract<<<dim3((ts.npp + 255) / 256, nclass), 256, 0, c->stream>>>(
             c->d_grids, d_reps, ts, planeorder ? 1 : 0, c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"),
-            c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), st.a1[0], st.a1[1],
-            st.a1[2], st.a1[3], st.a1[4], st.a1[5], st.tbm, st.tcf, st.tcb, st.tlap, st.tap);
+            c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), st.tcf, st.tcb,
+            st.tap);
         MG_LAUNCHED(c);
     }
     k_sip_extract<<<grid, 256, 0, c->stream>>>(
@@ -2368,7 +2354,7 @@ void sip_release(SipState& st) {
                     (void*)st.a1[2], (void*)st.a1[3], (void*)st.a1[4], (void*)st.a1[5],
                     (void*)st.a1lo[0], (void*)st.a1lo[1], (void*)st.a1lo[2], (void*)st.a1lo[3],
                     (void*)st.a1lo[4], (void*)st.a1lo[5], (void*)st.pg, (void*)st.bm, (void*)st.d_bar,
-                    (void*)st.tcf, (void*)st.tcb, (void*)st.tlap, (void*)st.tap, (void*)st.tbm})
+                    (void*)st.tcf, (void*)st.tcb, (void*)st.tap, (void*)st.tbm})
         cudaFree(p);
     if (st.tile) {
         tile_free(*st.tile);
@@ -2405,6 +2391,9 @@ int sip_forward(Ctx* c, SipState& st, const float* cf, const int* gcls, int* ctl
         {
             ProfScope ps_(c, "mx_sip_pre");
             TileArgs<float> a = tile_args(st, gcls, ctl, glist);
+            for (int q = 0; q < 6; ++q) a.A1[q] = st.a1[q];
+            a.grids = c->d_grids;
+            a.BM = st.tbm;
             a.R = st.rs[rwrite];
             a.LPR = st.tcf + 3 * ts.npp;
             a.lprcls = 4 * ts.npp;

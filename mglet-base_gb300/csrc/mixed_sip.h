@@ -39,11 +39,11 @@ struct SipState {
     float4* swf = nullptr;      // [ncls][npp]
     float4* swb = nullptr;
     // the solver on 2x2x2 tiles (sip_tile.cuh): tables,
-    // and per class {lw, ls, lb, lpr}, {ue, un, ut}, the seven operator
-    // coefficients and ap in two floats, npp values each; tbm the open couplings of
+    // and per class {lw, ls, lb, lpr}, {ue, un, ut} and ap in two floats, npp values
+    // each; tbm the open couplings of
     // the ghost-cell IB
     TileDev* tile = nullptr;
-    float *tcf = nullptr, *tcb = nullptr, *tlap = nullptr, *tap = nullptr;
+    float *tcf = nullptr, *tcb = nullptr, *tap = nullptr;
     unsigned char* tbm = nullptr;
     // packed pre-pass (npp + 6 fs < 32768): neighbour codes [npp][3] and per
     // class the records [ncls][3][npp]

@@ -47,13 +47,14 @@ struct PtOuterArgs {
     double* gridmax;
 };
 
-// the laplacian coefficients of a tile's cells (kUni: one value each over a class)
+// the laplacian coefficients of a tile's cells (kUni: one value each over a class; the
+// diagonal AP is the last of a class's seven arrays)
 template <class L, bool kUni>
 __device__ __forceinline__ void tile_lap_coefs(const TileArgs<double>& a, int cls, int p,
                                                Vec<double, L::N> (&c)[kUni ? 1 : 7]) {
     if constexpr (!kUni)
 #pragma unroll
-        for (int f = 0; f < 7; ++f) ldt(true, a.LAP + ((long long)cls * 7 + f) * a.s.npp + p, c[f]);
+        for (int f = 0; f < 7; ++f) ldt(true, a.AP + ((long long)cls * 7 + f - 6) * a.s.npp + p, c[f]);
 }
 
 // laplacephi at cell i of a tile
@@ -267,7 +268,11 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     a.RHS = p.rhs;
     a.LPR = p.cf + 3 * s.npp;
     a.lprcls = 4 * s.npp;
-    a.LAP = p.lap;
+    a.AP = p.lap + 6 * s.npp;
+    a.apcls = 7 * s.npp;
+    const char* const a1[6] = {"GSAW", "GSAE", "GSAS", "GSAN", "GSAB", "GSAT"};
+    for (int q = 0; q < 6; ++q) a.A1[q] = c->L(a1[q]);
+    a.grids = c->d_grids;
     a.UNI = p.uni;
     a.ctl = ctl;
     a.err = ctl + 2;

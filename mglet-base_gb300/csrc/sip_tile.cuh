@@ -203,10 +203,13 @@ struct TileArgs {
     const T* PG;                    // [ngrid][6][fs] hilf ghosts of PAR faces (null: zero)
     const T* CF;                    // sweeps: per class three coefficients (i, j, k), npp each
     const T* LPR;                   // per class lpr
-    const T* LAP;                   // per class [aw | ae | as | an | ab | at | ap], npp each
+    const T* AP;                    // per class the operator's diagonal
+    const T* A1[6];                 // pre-pass: its other coefficients aw, ae, as, an, ab, at by coordinate
+    const DevGrid* grids;
+    const unsigned char* BM;        // [ngrid][npp] open couplings (null: all)
     const T* UNI;                   // [ncls][8] operator coefficients of uniform classes
     const int* ctl;                 // [0] converged: nothing to do
-    int cfcls, lprcls;              // values between the classes of CF and of LPR
+    int cfcls, lprcls, apcls;       // values between the classes of CF, LPR and AP
     int* err;                       // set when a rank waited in vain
     int rev;                        // walk the grids in reverse block order
 };
@@ -756,7 +759,10 @@ __device__ __forceinline__ void tile_nbrs(const TileHalo<L, T>& o, int i, T n[6]
 
 // The part of sipiter1 outside the recurrence, (rhs + laplacephi(hilf)) lpr
 // (sip_hyperplane_mod.F90:491, laplacephi_mod.F90:153-160), one thread a tile;
-// the tiles of a grid in gridDim.x CTAs.  kHz: hilf is zero (a run-time branch had the
+// the tiles of a grid in gridDim.x CTAs.  Coefficients that differ from cell to cell come
+// by coordinate from the grids' one-dimensional arrays, with the couplings a body closes
+// masked (as arrays of a class's cells, which a grid with a body does not share, they were
+// 28 bytes a cell: 144 grids of 24^3 13.1 -> 11.6 us a launch).  kHz: hilf is zero (a run-time branch had the
 // other side compute this one's two instructions a cell as well).  kUni: one value of each operator
 // coefficient a class.  Of the first two products one rounds by itself and the
 // other is contracted with it: the first in kOrder 0, the second in kOrder 1, as the
@@ -771,7 +777,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
     const long long base = (long long)g * s.npp;
     const int tile = blockIdx.x * kThreads + threadIdx.x, p = N * tile;
     const bool on = tile < s.ntile;
-    const T* LAP = a.LAP + (long long)cls * 7 * s.npp;
     Vec<T, N> rh, lp, out;
     T u[7];
 #pragma unroll
@@ -782,6 +787,29 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
         n0 = __ldg(s.nbr + 2 * tile);
         n1 = __ldg(s.nbr + 2 * tile + 1);
     }
+    // the operator's coefficients by coordinate, and the diagonal
+    T ci[2][L::TI], cj[2][L::TJ], ck[2][L::TK];
+    Vec<T, N> ap;
+    uint2 bm = make_uint2(0x3f3f3f3fu, 0x3f3f3f3fu);
+    if constexpr (!kUni && !kHz) {
+        if (on) {
+            const DevGrid* G = a.grids + g;
+            const int x = G->ipx + 2 + (n1.z & 1023), y = G->ipy + 2 + ((n1.z >> 10) & 1023),
+                      z = G->ipz + 2 + (n1.z >> 20);
+#pragma unroll
+            for (int f = 0; f < 2; ++f) {
+#pragma unroll
+                for (int d = 0; d < L::TI; ++d) ci[f][d] = __ldg(a.A1[f] + x + d);
+#pragma unroll
+                for (int d = 0; d < L::TJ; ++d) cj[f][d] = __ldg(a.A1[2 + f] + y + d);
+#pragma unroll
+                for (int d = 0; d < L::TK; ++d) ck[f][d] = __ldg(a.A1[4 + f] + z + d);
+            }
+            if constexpr (N == 8)
+                if (a.BM) bm = __ldg(reinterpret_cast<const uint2*>(a.BM + base + p));
+        }
+        ldt(on, a.AP + (long long)cls * a.apcls + p, ap);
+    }
     follow_on();
     if (flag_at(a.ctl) || !on) return;
     ldt_co(true, a.RHS + base + p, rh);
@@ -791,16 +819,18 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
     } else {
         TileHalo<L, T> o;
         tile_halo<kPad>(a, g, tile, n0, n1, o);
-        Vec<T, N> c[kUni ? 1 : 7];
-        if constexpr (!kUni)
-#pragma unroll
-            for (int f = 0; f < 7; ++f) ldt(true, LAP + f * s.npp + p, c[f]);
 #pragma unroll
         for (int i = 0; i < N; ++i) {
             T n[6], w[7];
             tile_nbrs<L>(o, i, n);
+            const unsigned mk = ((i < 4 ? bm.x : bm.y) >> (8 * (i & 3))) & 0xffu;
+            const int di = i / (L::TJ * L::TK), dj = (i / L::TK) % L::TJ, dk = i % L::TK;
 #pragma unroll
-            for (int f = 0; f < 7; ++f) w[f] = kUni ? u[f] : c[kUni ? 0 : f].v[i];
+            for (int f = 0; f < 6; ++f) {
+                const T x = f < 2 ? ci[f][di] : (f < 4 ? cj[f - 2][dj] : ck[f - 4][dk]);
+                w[f] = kUni ? u[f] : (N < 8 || (mk >> f & 1u) ? x : T(0));
+            }
+            w[6] = kUni ? u[6] : ap.v[i];
             T lap = mul_rounded(-w[kOrder], n[kOrder]);
             lap = lap - w[1 - kOrder] * n[1 - kOrder] - w[2] * n[2] - w[3] * n[3] - w[4] * n[4] - w[5] * n[5] -
                   w[6] * o.h.v[i];
