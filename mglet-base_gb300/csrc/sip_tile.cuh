@@ -428,15 +428,16 @@ struct TileSweep {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // one warp, in step t: stages the faces the rank before has put in step t.  The wait
-    // for them ends after kSpin looks: then the error flag is set and nothing waits
+    // for them ends after about a second: then the error flag is set and nothing waits
     // any more.
-    static constexpr int kSpin = 1 << 20;
+    static constexpr long long kWait = 2000000000LL;   // SM clocks
     __device__ __forceinline__ void boundary(int t, bool& lost) {
         if (!up) return;
         const int I = kFwd ? i0 - 1 : i1 + 1, h = (kFwd ? t : s.NT - 1 - t) - I;
         const int lo = row_lo(h), hi = row_hi(h);
         if (lo > hi) return;
-        for (int n = 0; !lost; ++n) {
+        const long long since = clock64();
+        while (!lost) {
             int ok;
             asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
                          " selp.s32 %0, 1, 0, p;\n}"
@@ -444,7 +445,7 @@ struct TileSweep {
                          : "r"(mbar + 8 * h)
                          : "memory");
             if (__all_sync(0xffffffffu, ok)) break;
-            if (n >= kSpin) {
+            if (__any_sync(0xffffffffu, clock64() - since > kWait)) {
                 lost = true;
                 if ((threadIdx.x & 31) == 0) *a.err = 1;
             }
