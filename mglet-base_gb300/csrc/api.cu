@@ -556,6 +556,13 @@ static double* field_ptr(mglet_ctx* c, const char* name) {
     return it == c->f3.end() ? nullptr : it->second;
 }
 
+// Every entry point that writes a field by its name reports it here: the plain form's
+// solve on tiles keeps copies of BP's and the Poisson coefficients' values.
+static void field_written(mglet_ctx* c, const char* name) {
+    if (name && (!std::strcmp(name, "BP") || !std::strcmp(name, "GSAP") || !std::strncmp(name, "SIP", 3)))
+        c->coef_user = true;
+}
+
 extern "C" {
 
 int32_t mglet_gpu_abi_version(void) { return MGLET_GPU_ABI_VERSION; }
@@ -845,9 +852,7 @@ int mglet_gpu_set_field(mglet_ctx* c, const char* name, const double* host, int6
     MG_CUDA(cudaMemcpyAsync(p, host, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     MG_CUDA(cudaStreamSynchronize(c->stream));
     if (std::strcmp(name, "G") == 0) c->g_user = true;
-    // the solve on tiles keeps copies of these
-    if (!std::strcmp(name, "BP") || !std::strcmp(name, "GSAP") || !std::strncmp(name, "SIP", 3))
-        c->coef_user = true;
+    field_written(c, name);
     if (c->prm.form == MGLET_FORM_MIXED) mixed_field_changed(c, name);
     return 0;
 }
@@ -898,6 +903,8 @@ int mglet_gpu_rkstep(mglet_ctx* c, const char* p, const char* dp, const char* rh
     double *a = field_ptr(c, p), *b = field_ptr(c, dp), *r = field_ptr(c, rhsp);
     if (!a || !b || !r) return fail(MGLET_ERR_NAME, "rkstep: unknown field");
     cudaSetDevice(c->device);
+    field_written(c, p);
+    field_written(c, dp);
     return MG_PLAIN_FN(c, launch_rkstep)(c, a, b, r, frhs, dtfu);
 }
 
@@ -912,6 +919,7 @@ int mglet_gpu_connect(mglet_ctx* c, int32_t ilevel, int32_t layers, const char* 
         if (names[q] && !f[q]) return fail(MGLET_ERR_NAME, std::string("connect: unknown field ") + names[q]);
     }
     cudaSetDevice(c->device);
+    for (const char* nm : names) field_written(c, nm);
     return connect(c, ilevel, layers, f[0], f[1], f[2], f[3], f[4], f[5], corners != 0,
                    normal != 0, forward);
 }
@@ -921,6 +929,7 @@ int mglet_gpu_divcal(mglet_ctx* c, const char* div, double fak) {
     double* d = field_ptr(c, div);
     if (!d) return fail(MGLET_ERR_NAME, "divcal: unknown field");
     cudaSetDevice(c->device);
+    field_written(c, div);
     return MG_PLAIN_FN(c, launch_divcal)(c, d, c->F("U"), c->F("V"), c->F("W"), fak);
 }
 
@@ -929,6 +938,7 @@ int mglet_gpu_laplacephi(mglet_ctx* c, const char* res, const char* phi) {
     double *r = field_ptr(c, res), *p = field_ptr(c, phi);
     if (!r || !p) return fail(MGLET_ERR_NAME, "laplacephi: unknown field");
     cudaSetDevice(c->device);
+    field_written(c, res);
     if (int rc = launch_bp_ones(c)) return rc;
     return MG_PLAIN_FN(c, launch_laplacephi)(c, 0, r, p);
 }
@@ -973,6 +983,7 @@ int mglet_gpu_ftoc(mglet_ctx* c, int32_t ilevel, const char* ff, const char* fc,
     if (!flag || !std::strchr("UVWPRST", flag))
         return fail(MGLET_ERR_ARG, "ftoc: flag is one of U V W P R S T");
     cudaSetDevice(c->device);
+    field_written(c, fc);
     return launch_ftoc(c, ilevel, f, g, flag);
 }
 
@@ -1072,6 +1083,7 @@ int mglet_gpu_par_ftoc_norm(mglet_ctx* c, int32_t ilevel, const char* v1, const 
     double *u = field_ptr(c, v1), *v = field_ptr(c, v2), *w = field_ptr(c, v3);
     if (!u || !v || !w) return fail(MGLET_ERR_NAME, "par_ftoc_norm: unknown field");
     cudaSetDevice(c->device);
+    for (const char* nm : {v1, v2, v3}) field_written(c, nm);
     return launch_par_ftoc_norm(c, ilevel, u, v, w, sum != 0);
 }
 
@@ -1083,6 +1095,7 @@ int mglet_gpu_ftoc_multiple(mglet_ctx* c, int32_t ilevel, const char* v1, const 
     for (int q = 0; q < 6; ++q)
         if (n[q] && !field_ptr(c, n[q])) return fail(MGLET_ERR_NAME, "ftoc: unknown field");
     cudaSetDevice(c->device);
+    for (const char* nm : n) field_written(c, nm);
     for (int q = 0; q < 6; ++q)
         if (n[q])
             if (int rc = launch_ftoc(c, ilevel, field_ptr(c, n[q]), field_ptr(c, n[q]), fl[q])) return rc;
@@ -1094,6 +1107,7 @@ int mglet_gpu_ctof(mglet_ctx* c, int32_t ilevel, const char* ff, const char* fc)
     double *f = field_ptr(c, ff), *g = field_ptr(c, fc);
     if (!f || !g) return fail(MGLET_ERR_NAME, "ctof: unknown field");
     cudaSetDevice(c->device);
+    field_written(c, ff);
     return launch_ctof(c, ilevel, f, g);
 }
 
@@ -1102,6 +1116,7 @@ int mglet_gpu_bound_pressure(mglet_ctx* c, int32_t ilevel, const char* dp, int32
     double* p = field_ptr(c, dp);
     if (!p) return fail(MGLET_ERR_NAME, "bound_pressure: unknown field");
     cudaSetDevice(c->device);
+    field_written(c, dp);
     double* b = field_buffer(c, dp);
     if (!b) return fail(MGLET_ERR_CUDA, "bound_pressure: buffer allocation");
     return launch_bound_pressure(c, ilevel, p, b, with_bp != 0);

@@ -126,7 +126,7 @@ struct Ctx {
     MixedState* mx = nullptr;
     Part* part = nullptr;      // grid partition over ranks (null: one rank)
     PlainTile* ptile = nullptr;   // plain form: the pressure solve on tiles (null: not for these grids)
-    bool coef_user = false;    // the caller set BP or a Poisson coefficient field
+    bool coef_user = false;    // the caller wrote BP or a Poisson coefficient field
     int device = 0;
     cudaStream_t stream = nullptr;
     int ngrid = 0;
