@@ -588,7 +588,7 @@ int mixed_test_barrier_timeout(Ctx* c) {
     return 0;
 }
 
-int mixed_force_variant(Ctx* c, const char* kernel, int v) {
+static int force_variant(Ctx* c, const char* kernel, int v) {
     MixedState* m = c->mx;
     if (m && std::strcmp(kernel, "mx_outer") == 0) {
         if (v < -1 || v >= sip_outer_variants()) {
@@ -683,6 +683,12 @@ int mixed_force_variant(Ctx* c, const char* kernel, int v) {
         m->graph = nullptr;
     }
     return 0;
+}
+
+int mixed_force_variant(Ctx* c, const char* kernel, int v) {
+    const bool tiles = c->mx && sip_on_tiles(c->mx->sip);
+    if (int rc = force_variant(c, kernel, v)) return rc;
+    return sip_on_tiles(c->mx->sip) != tiles ? sip_clear(c, c->mx->sip) : 0;
 }
 
 void mixed_release(Ctx* c) {

@@ -2019,6 +2019,12 @@ bool sip_on_tiles(const SipState& st) {
            !st.fuse_pre && st.solve_variant < 0;
 }
 
+int sip_clear(Ctx* c, SipState& st) {
+    for (float* p : {st.rs[0], st.rs[1], st.rs[2], st.h32, st.rhs32, st.rhsl, st.dph, st.dpl})
+        MG_CUDA(zero_on(c->stream, p, (size_t)c->ngrid * sip_npp(st) * sizeof(float)));
+    return 0;
+}
+
 PosMap sip_posmap(const SipState& st) {
     if (sip_on_tiles(st)) {
         const TileShape& s = st.tile->s;

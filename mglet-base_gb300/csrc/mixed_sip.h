@@ -100,8 +100,11 @@ struct SipState {
 // The layout of the solver's arrays (hilf, res, rhs, dp): on tiles, unless the
 // shape or a forced variant asks for the cell hyperplane order.  The arrays are
 // written and read within one pressure solve, so the layout may change between
-// solves.
+// solves; the pads of the last tiles, which no kernel but the solver's writes, are
+// cleared then (a zero coefficient does not clear what the other order left there
+// when that is not finite).
 bool sip_on_tiles(const SipState& st);
+int sip_clear(Ctx* c, SipState& st);
 // position of a cell in the layout in use
 struct PosMap {
     const int* tpos;            // [planes][ni or NI], see mixed_sip.cu and sip_tile.cuh
