@@ -45,6 +45,8 @@ struct PtOuterArgs {
     TileArgs<double> t;
     double *RHS, *DP;
     double* gridmax;
+    const double* RS[3];   // scatter: the res slots
+    int ninner;
 };
 
 // the laplacian coefficients of a tile's cells (kUni: one value each over a class; the
@@ -124,8 +126,35 @@ __global__ void __launch_bounds__(128) k_pt_outer(const __grid_constant__ PtOute
     }
 }
 
+// The ghosts of RES next to face kF (-i, +i, -j, +j, -k, +k) of a tile, as the last
+// exchange of res left them: the facing cells of the grid across, from slot R
+// (tile -1 - nb there; org: the tile's first cell, see TileShape::nbr).
+template <class L, int kF>
+__device__ __forceinline__ void res_ghosts(const TileArgs<double>& a, int g, int nb, int org, const double* R,
+                                           double* RES) {
+    constexpr int ax = kF / 2;
+    const TileShape& s = a.s;
+    if (nb >= 0 || !R) return;
+    const int n = a.fnbr[6 * g + kF];
+    if (n < 0) return;
+    Vec<double, L::N> v;
+    ldt_co(true, R + ((long long)n * s.npp + L::N * (-1 - nb)), v);
+    const auto f = tile_part<L, ax, kF % 2 == 0>(v);
+    const int out = kF % 2 == 0 ? -1 : (ax == 0 ? s.ni : (ax == 1 ? s.nj : s.nk));
+    const int kk = s.nk + 4, jj = s.nj + 4;
+#pragma unroll
+    for (int q = 0; q < L::template F<ax>; ++q) {
+        int io = org & 1023, jo = (org >> 10) & 1023, ko = org >> 20;
+        if (ax == 0) io = out, jo += q / L::TK, ko += q % L::TK;
+        else if (ax == 1) jo = out, io += q / L::TK, ko += q % L::TK;
+        else ko = out, io += q / L::TJ, jo += q % L::TJ;
+        RES[(ko + 2) + (jo + 2) * kk + (io + 2) * kk * jj] = f.v[q];
+    }
+}
+
 // the residual and the accumulated correction back into RHS and DP, and the
-// laplacian of the last correction into RES
+// laplacian of the last correction into RES; its ghosts hold what the last two inner
+// iterations exchanged (the last one only from the high side)
 template <class L, bool kUni>
 __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOuterArgs a,
                                                     const DevGrid* __restrict__ grids,
@@ -138,7 +167,16 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
     if (tile >= s.ntile) return;
     const long long base = (long long)g * s.npp, ip3 = grids[g].ip3;
     TileHalo<L, double> o;
-    tile_halo(a.t, g, tile, __ldg(s.nbr + 2 * tile), __ldg(s.nbr + 2 * tile + 1), o);
+    const int4 n0 = __ldg(s.nbr + 2 * tile), n1 = __ldg(s.nbr + 2 * tile + 1);
+    tile_halo(a.t, g, tile, n0, n1, o);
+    const int last = a.t.ctl[1] * a.ninner;   // inner iterations done
+    const double *low = a.ninner > 1 ? a.RS[(last - 1) % 3] : nullptr, *high = a.RS[last % 3];
+    res_ghosts<L, 0>(a.t, g, n0.x, n1.z, low, RES + ip3);
+    res_ghosts<L, 1>(a.t, g, n0.y, n1.z, high, RES + ip3);
+    res_ghosts<L, 2>(a.t, g, n0.z, n1.z, low, RES + ip3);
+    res_ghosts<L, 3>(a.t, g, n0.w, n1.z, high, RES + ip3);
+    res_ghosts<L, 4>(a.t, g, n1.x, n1.z, low, RES + ip3);
+    res_ghosts<L, 5>(a.t, g, n1.y, n1.z, high, RES + ip3);
     Vec<double, N> c[kUni ? 1 : 7];
     tile_lap_coefs<L, kUni>(a.t, cls, p, c);
 #pragma unroll
@@ -280,6 +318,8 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     o.RHS = p.rhs;
     o.DP = p.dp;
     o.gridmax = p.gridmax;
+    o.ninner = c->prm.ninner;
+    for (int q = 0; q < 3; ++q) o.RS[q] = p.rs[q];
     const int ninner = c->prm.ninner;
     // inner iteration gi writes res slot gi % 3 and takes its low ghosts from the
     // last iteration whose exchange covered every face (every inner iteration but
