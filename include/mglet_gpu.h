@@ -582,6 +582,13 @@ int mglet_gpu_test_wait_timeout(mglet_ctx* ctx);
  * returns MGLET_ERR_CUDA ("timed out").  Needs the persistent solve in use
  * (mglet_gpu_force_variant "mx_sip_solve").  The context stays usable. */
 int mglet_gpu_test_barrier_timeout(mglet_ctx* ctx);
+/* Test switch for the waits of the plain form's sweeps where a few grids are
+ * shared by several SMs each: in the next solve the forward sweeps take one row of
+ * faces for not arrived, although it is, so their wait gives up (after about 50 ms
+ * here, about a second otherwise) and raises the error flag; the solve ends
+ * and returns MGLET_ERR_CUDA ("timed out").  MGLET_ERR_UNSUPPORTED where no grid is
+ * shared.  The context stays usable. */
+int mglet_gpu_test_sweep_timeout(mglet_ctx* ctx);
 
 /* ---- Misc ----------------------------------------------------------------- */
 int mglet_gpu_synchronize(mglet_ctx* ctx);

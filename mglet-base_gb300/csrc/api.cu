@@ -1380,6 +1380,11 @@ int mglet_gpu_test_wait_timeout(mglet_ctx* c) {
     return mixed_test_wait_timeout(c);
 }
 
+int mglet_gpu_test_sweep_timeout(mglet_ctx* c) {
+    if (!c) return fail(MGLET_ERR_ARG, "test_sweep_timeout: null context");
+    return plain_tile_test_timeout(c);
+}
+
 int mglet_gpu_test_barrier_timeout(mglet_ctx* c) {
     if (!c) return fail(MGLET_ERR_ARG, "test_barrier_timeout: null context");
     return mixed_test_barrier_timeout(c);

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
     TileHalo<L, double> o;
     const int4 n0 = __ldg(s.nbr + 2 * tile), n1 = __ldg(s.nbr + 2 * tile + 1);
     tile_halo(a.t, g, tile, n0, n1, o);
-    const int last = a.t.ctl[1] * a.ninner;   // inner iterations done
+    const int last = max(a.t.ctl[1], 1) * a.ninner;   // inner iterations done (none: the solve was lost)
     const double *low = a.ninner > 1 ? a.RS[(last - 1) % 3] : nullptr, *high = a.RS[last % 3];
     res_ghosts<L, 0>(a.t, g, n0.x, n1.z, low, RES + ip3);
     res_ghosts<L, 1>(a.t, g, n0.y, n1.z, high, RES + ip3);
@@ -313,7 +313,12 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     a.grids = c->d_grids;
     a.UNI = p.uni;
     a.ctl = ctl;
-    a.err = ctl + 2;
+    if (s.nc > 1) {
+        a.err = ctl + 2;
+        a.stop = ctl;
+        a.lose = p.lose_once;
+        p.lose_once = false;
+    }
     PtOuterArgs o{};
     o.RHS = p.rhs;
     o.DP = p.dp;
@@ -390,7 +395,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
         return rc;
     MG_CUDA(cudaStreamSynchronize(c->stream));
     if (reinterpret_cast<const int*>(p.h_stat + 2)[0]) {
-        set_error("mgpoisl: a sweep waited for another CTA in vain");
+        set_error("mgpoisl: a sweep timed out waiting for another CTA");
         return MGLET_ERR_CUDA;
     }
     if (st) {
@@ -567,6 +572,15 @@ void plain_tile_release(Ctx* c) {
     if (p->h_stat) cudaFreeHost(p->h_stat);
     delete p;
     c->ptile = nullptr;
+}
+
+int plain_tile_test_timeout(Ctx* c) {
+    if (!c->ptile || !plain_tile_ready(c) || c->ptile->t.s.nc == 1) {
+        set_error("test_sweep_timeout: needs the plain form's solve on tiles with grids shared by SMs");
+        return MGLET_ERR_UNSUPPORTED;
+    }
+    c->ptile->lose_once = true;
+    return 0;
 }
 
 bool plain_tile_ready(const Ctx* c) {

@@ -19,6 +19,7 @@ struct PlainTile {
     double* gridmax = nullptr;  // [ngrid]
     double* stat = nullptr;     // device {max |rhs|, ints: converged, outer iterations, error}
     double* h_stat = nullptr;   // pinned copy
+    bool lose_once = false;     // test switch: a wait of the next solve's forward sweeps runs out
 };
 
 // Set up when the context's grids take it: one level, equal dimensions, SIP in
@@ -27,5 +28,7 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d);
 void plain_tile_release(Ctx* c);
 // May the solve run on tiles now (the coefficients are still the library's own)?
 bool plain_tile_ready(const Ctx* c);
+// mglet_gpu_test_sweep_timeout
+int plain_tile_test_timeout(Ctx* c);
 
 }  // namespace mg

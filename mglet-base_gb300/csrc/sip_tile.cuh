@@ -210,7 +210,9 @@ struct TileArgs {
     const T* UNI;                   // [ncls][8] operator coefficients of uniform classes
     const int* ctl;                 // [0] converged: nothing to do
     int cfcls, lprcls, apcls;       // values between the classes of CF, LPR and AP
-    int* err;                       // set when a rank waited in vain
+    int* err;                       // set when a rank waited in vain (null: no ranks)
+    int* stop;                      // pre-pass: ctl[0], which it sets when err is
+    int lose;                       // test switch: forward, rank 1 misses the first faces of every grid
     int rev;                        // walk the grids in reverse block order
 };
 
@@ -427,31 +429,47 @@ struct TileSweep {
             }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // has row hyperplane h arrived?  (one warp)
+    __device__ __forceinline__ bool arrived(int h) const {
+        int ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+                     " selp.s32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(mbar + 8 * h)
+                     : "memory");
+        return __all_sync(0xffffffffu, ok);
+    }
+    static __device__ __forceinline__ bool expired(long long since, long long limit) {
+        return __any_sync(0xffffffffu, clock64() - since > limit);
+    }
     // one warp, in step t: stages the faces the rank before has put in step t.  The wait
-    // for them ends after about a second: then the error flag is set and nothing waits
-    // any more.
-    static constexpr long long kWait = 2000000000LL;   // SM clocks
+    // for them ends after about a second: then the error flag is set and this launch
+    // waits no more.  The next pre-pass sees the flag and ends the solve.
+    static constexpr long long kWait = 2000000000LL, kWaitTest = 100000000LL;   // SM clocks
     __device__ __forceinline__ void boundary(int t, bool& lost) {
         if (!up) return;
         const int I = kFwd ? i0 - 1 : i1 + 1, h = (kFwd ? t : s.NT - 1 - t) - I;
         const int lo = row_lo(h), hi = row_hi(h);
         if (lo > hi) return;
+        const bool lose = kFwd && a.lose && rank == 1 && h == 0;
         const long long since = clock64();
         while (!lost) {
-            int ok;
-            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
-                         " selp.s32 %0, 1, 0, p;\n}"
-                         : "=r"(ok)
-                         : "r"(mbar + 8 * h)
-                         : "memory");
-            if (__all_sync(0xffffffffu, ok)) break;
-            if (__any_sync(0xffffffffu, clock64() - since > kWait)) {
+            if (arrived(h) && !lose) break;
+            if (expired(since, lose ? kWaitTest : kWait)) {
                 lost = true;
                 if ((threadIdx.x & 31) == 0) *a.err = 1;
             }
         }
         Face* f = face + (t & 1) * 3 * s.slots + (kFwd ? (I + 1) * s.w + 1 : I * s.w);
         for (int J = lo + (threadIdx.x & 31); J <= hi; J += 32) f[J] = bnd[J * s.NK + h - J];
+    }
+    // one warp of a rank that gave up, behind the last cluster barrier: every face has been
+    // put by now, and the CTA stays until they are here (or another second is over)
+    __device__ __forceinline__ void drain() {
+        const long long since = clock64();
+        for (int h = 0; h < s.NJ + s.NK - 1; ++h)
+            while (!arrived(h))
+                if (expired(since, kWait)) return;
     }
     // thread lane's loads of a step whose tiles are t0 .. t1
     __device__ __forceinline__ void fetch(TileSet<L, T>& q, int lane, int t0, int t1) {
@@ -625,7 +643,10 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
                 if (t < t1 - 1) w.boundary(t, lost);
             __syncthreads();
         }
-        if constexpr (kRanks) cluster_barrier();   // no rank ends while another may put into it
+        if constexpr (kRanks) {
+            cluster_barrier();   // no rank ends while another may put into it
+            if (lost) w.drain();
+        }
         return;
     }
     __syncthreads();
@@ -812,6 +833,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
         ldt(on, a.AP + (long long)cls * a.apcls + p, ap);
     }
     follow_on();
+    // (the sweeps read ctl, which has to be one value for the ranks of a cluster, so they
+    // cannot set it)
+    if (a.err && tile == 0 && blockIdx.y == 0 && flag_at(a.err)) *a.stop = 1;
     if (flag_at(a.ctl) || !on) return;
     ldt_co(true, a.RHS + base + p, rh);
     if constexpr (kHz) {
