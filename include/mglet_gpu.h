@@ -560,7 +560,7 @@ int mglet_gpu_set_partition(mglet_ctx* ctx, const int32_t* halo, int32_t nsend,
  * mgpoisl as one cooperative launch with grid-wide barriers; timed and
  * reported, run only when forced: the per-phase kernels are faster in the
  * stage graph).  mglet_gpu_tuning describes the
- * choices ("" for the plain form); mglet_gpu_force_variant overrides one
+ * kernels in use ("" for the plain form); mglet_gpu_force_variant overrides one
  * (kernel "mx_sip_pre" 0..9, "mx_sip_sweep" 0..4, "mx_flux" 0..1,
  * "mx_sip_solve" 0..5, "mx_outer_pre" 0..1 -- 1: on one level the outer step
  * writes the next hilf-zero pre-pass itself; -1 = default, for

@@ -538,6 +538,10 @@ std::string mixed_tuning(Ctx* c) {
     MixedState* m = c->mx;
     if (!m) return "";
     const SipState& s = m->sip;
+    if (sip_on_tiles(s))   // one form of each kernel, by the number of grids and their shape
+        return std::string("mx_sip_pre: 2x2x2 tiles; uniform classes: ") + (s.unicls ? "yes" : "no") +
+               "; sweeps: 2x2x2 tiles; mx_sip_solve: " + sip_solve_variant_name(s.solve_variant) +
+               "; mx_outer: 2x2x2 tiles; " + mx_flux_tuning(c);
     char buf[512];
     std::snprintf(buf, sizeof buf,
                   "mx_sip_pre: %s%s (%.4f ms); uniform classes: %s; sweeps: %s%s (%.4f ms per "
