@@ -589,6 +589,11 @@ int mglet_gpu_test_barrier_timeout(mglet_ctx* ctx);
  * and returns MGLET_ERR_CUDA ("timed out").  MGLET_ERR_UNSUPPORTED where no grid is
  * shared.  The context stays usable. */
 int mglet_gpu_test_sweep_timeout(mglet_ctx* ctx);
+/* Test switch for a device that runs out of memory: of the allocations a context can
+ * do without (tables and arrays of the solves on tiles, the table of the PAR
+ * blocks) this thread's calls get n more and are then refused, as by
+ * cudaMalloc; the context takes the path without them.  -1: no limit. */
+int mglet_gpu_test_scratch_limit(int32_t n);
 
 /* ---- Misc ----------------------------------------------------------------- */
 int mglet_gpu_synchronize(mglet_ctx* ctx);

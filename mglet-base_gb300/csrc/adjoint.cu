@@ -651,9 +651,8 @@ int energy_gradient(Ctx* c, int nsteps, int ncheck, double dt, const mglet_rk_sc
         cudaFree(stg);
         cudaFree(fin);
     };
-    if (cudaMalloc(&ck, (size_t)nck * 7 * fb) != cudaSuccess ||
-        cudaMalloc(&stg, (size_t)seg * nrk * 3 * fb) != cudaSuccess ||
-        cudaMalloc(&fin, 7 * fb) != cudaSuccess) {
+    auto take = [&](double** p, size_t n) { return need_alloc(c, reinterpret_cast<void**>(p), n) == cudaSuccess; };
+    if (!take(&ck, (size_t)nck * 7 * fb) || !take(&stg, (size_t)seg * nrk * 3 * fb) || !take(&fin, 7 * fb)) {
         release();
         return fail(MGLET_ERR_CUDA, "energy_gradient: checkpoint memory");
     }

@@ -37,6 +37,27 @@ static int fail(int code, const std::string& msg) {
     return code;
 }
 
+// test switch (mglet_gpu_test_scratch_limit): allocations this thread still gets, -1: any
+static thread_local int t_scratch_left = -1;
+
+int scratch_alloc(void** p, size_t n) {
+    *p = nullptr;
+    if (t_scratch_left == 0) return kNoScratch;
+    if (t_scratch_left > 0) --t_scratch_left;
+    const cudaError_t e = cudaMalloc(p, n);
+    if (e == cudaSuccess) return 0;
+    cudaGetLastError();   // (not the next launch's)
+    return e == cudaErrorMemoryAllocation ? kNoScratch : cuda_fail(e, "scratch memory");
+}
+
+cudaError_t need_alloc(Ctx* c, void** p, size_t n) {
+    cudaError_t e = t_scratch_left == 0 && c->ptile ? cudaErrorMemoryAllocation : cudaMalloc(p, n);
+    if (e != cudaErrorMemoryAllocation || !c->ptile) return e;
+    cudaGetLastError();
+    plain_tile_release(c);
+    return cudaMalloc(p, n);
+}
+
 
 namespace {
 
@@ -246,7 +267,7 @@ __global__ void k_fill(double* a, double v, long long n) {
 
 int alloc3(Ctx* c, const char* name) {
     double* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, (size_t)c->idim3d * sizeof(double));
+    cudaError_t e = need_alloc(c, reinterpret_cast<void**>(&p), (size_t)c->idim3d * sizeof(double));
     if (e != cudaSuccess) return fail(MGLET_ERR_NOMEM, std::string("cudaMalloc ") + name);
     MG_CUDA(cudaMemsetAsync(p, 0, (size_t)c->idim3d * sizeof(double), c->stream));
     c->f3[name] = p;
@@ -557,10 +578,10 @@ static double* field_ptr(mglet_ctx* c, const char* name) {
 }
 
 // Every entry point that writes a field by its name reports it here: the plain form's
-// solve on tiles keeps copies of BP's and the Poisson coefficients' values.
+// solve on tiles has copies of BP's and the Poisson coefficients' values, and ends.
 static void field_written(mglet_ctx* c, const char* name) {
     if (name && (!std::strcmp(name, "BP") || !std::strcmp(name, "GSAP") || !std::strncmp(name, "SIP", 3)))
-        c->coef_user = true;
+        plain_tile_release(c);
 }
 
 extern "C" {
@@ -1214,6 +1235,7 @@ int mglet_gpu_set_ghostcell(mglet_ctx* c) {
         if (int rc = hierarchy_ready(c)) return rc;
     if (c->gch.empty()) c->gch.resize(c->ngrid);
     c->ibtype = 1;
+    plain_tile_release(c);
     if (int rc = launch_giteig(c)) return rc;
     MG_CUDA(cudaStreamSynchronize(c->stream));
     int rc = c->prm.psolver == MGLET_PSOLVER_CLASSIC ? launch_sip_lu_classic(c) : launch_sip_lu_hp(c);
@@ -1388,6 +1410,11 @@ int mglet_gpu_test_sweep_timeout(mglet_ctx* c) {
 int mglet_gpu_test_barrier_timeout(mglet_ctx* c) {
     if (!c) return fail(MGLET_ERR_ARG, "test_barrier_timeout: null context");
     return mixed_test_barrier_timeout(c);
+}
+
+int mglet_gpu_test_scratch_limit(int32_t n) {
+    t_scratch_left = n < 0 ? -1 : n;
+    return 0;
 }
 
 int mglet_gpu_force_variant(mglet_ctx* c, const char* kernel, int32_t variant) {

@@ -128,6 +128,7 @@ int set_partition(Ctx* c, const int32_t* halo, int nsend, const int32_t* send, i
         return MGLET_ERR_ARG;
     }
     part_release(c);
+    plain_tile_release(c);
     Part* p = new Part();
     c->part = p;
     p->fn = fn;

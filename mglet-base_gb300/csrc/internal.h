@@ -125,8 +125,7 @@ struct PlainTile;    // plain_tile.h
 struct Ctx {
     MixedState* mx = nullptr;
     Part* part = nullptr;      // grid partition over ranks (null: one rank)
-    PlainTile* ptile = nullptr;   // plain form: the pressure solve on tiles (null: not for these grids)
-    bool coef_user = false;    // the caller wrote BP or a Poisson coefficient field
+    PlainTile* ptile = nullptr;   // plain form: the pressure solve on tiles (null: not there, or no more)
     int device = 0;
     cudaStream_t stream = nullptr;
     int ngrid = 0;
@@ -262,6 +261,19 @@ inline cudaError_t copy_on(cudaStream_t s, void* dst, const void* src, size_t n,
 }
 inline cudaError_t zero_on(cudaStream_t s, void* p, size_t n) { return cudaMemsetAsync(p, 0, n, s); }
 
+// Device memory for a path that a context can do without: kNoScratch when there is none,
+// and the caller takes the path that needs less.
+constexpr int kNoScratch = -1;
+int scratch_alloc(void** p, size_t n);
+// Memory that the context itself needs: the plain form's solve on tiles gives its own
+// back before this fails.
+struct Ctx;
+cudaError_t need_alloc(Ctx* c, void** p, size_t n);
+template <class T>
+int scratch(T** p, size_t n) {
+    return scratch_alloc(reinterpret_cast<void**>(p), n * sizeof(T));
+}
+
 #define MG_LAUNCHED(ctx)                                              \
     do {                                                              \
         (ctx)->launches++;                                            \
@@ -380,5 +392,8 @@ int part_allreduce(Ctx* c, double* v, int n, int op);
 int set_partition(Ctx* c, const int32_t* halo, int nsend, const int32_t* send, int nrecv,
                   const int32_t* recv, mglet_exchange_fn fn, void* user);
 void part_release(Ctx* c);
+// the plain form's pressure solve on tiles goes for good and gives its memory back
+// (plain_tile.cu): a partition, a body, coefficients of the caller's
+void plain_tile_release(Ctx* c);
 
 }  // namespace mg

@@ -530,8 +530,13 @@ int mx_level_prepare(Ctx* c, SipState& st, LevelState& lv) {
             int* d = nullptr;
             if (int rc = upload(c, gf, &d)) return rc;
             lv.d_faces = reinterpret_cast<int2*>(d);
-            MG_CUDA(cudaMalloc(&lv.bpw, 10 * n * sizeof(double)));
-            MG_CUDA(cudaMalloc(&lv.bpidx, 2 * n * sizeof(long long)));
+            int rc = scratch(&lv.bpw, 10 * n);
+            if (!rc) rc = scratch(&lv.bpidx, 2 * n);
+            if (rc && rc != kNoScratch) return rc;
+            if (rc) {   // the weights in every launch
+                cudaFree(lv.bpw);
+                lv.bpw = nullptr;
+            }
         }
     }
     if (!lv.ibflag.empty()) {

@@ -2019,10 +2019,28 @@ bool sip_on_tiles(const SipState& st) {
            !st.fuse_pre && st.solve_variant < 0;
 }
 
+static void drop_tiles(SipState& st) {
+    if (!st.tile) return;
+    tile_free(*st.tile);
+    delete st.tile;
+    st.tile = nullptr;
+    for (void** p : {(void**)&st.tcf, (void**)&st.tcb, (void**)&st.tap, (void**)&st.tbm}) {
+        cudaFree(*p);
+        *p = nullptr;
+    }
+}
+
 int sip_clear(Ctx* c, SipState& st) {
     for (float* p : {st.rs[0], st.rs[1], st.rs[2], st.h32, st.rhs32, st.rhsl, st.dph, st.dpl})
         MG_CUDA(zero_on(c->stream, p, (size_t)c->ngrid * sip_npp(st) * sizeof(float)));
     return 0;
+}
+
+// from tiles to the cell hyperplane order for good
+static int sip_leave_tiles(Ctx* c, SipState& st) {
+    MG_CUDA(cudaStreamSynchronize(c->stream));
+    drop_tiles(st);
+    return sip_clear(c, st);
 }
 
 PosMap sip_posmap(const SipState& st) {
@@ -2214,12 +2232,8 @@ int sip_init(Ctx* c, SipState& st) {
                        cudaMemcpyHostToDevice));
     // the tables of the solver on tiles, for the shapes it takes
     st.tile = new TileDev();
-    if (int rc = tile_init(c, st.ni, st.nj, st.nk, 1, 1, 1, 1, 512, *st.tile)) return rc;
-    if (!st.tile->ok || tile_layout<T8, float>(st.tile->s).bytes > 200 * 1024) {
-        tile_free(*st.tile);
-        delete st.tile;
-        st.tile = nullptr;
-    }
+    if (int rc = tile_init(c, st.ni, st.nj, st.nk, 1, 1, 1, 1, 512, *st.tile); rc && rc != kNoScratch) return rc;
+    if (!st.tile->ok || tile_layout<T8, float>(st.tile->s).bytes > 200 * 1024) drop_tiles(st);
     // face neighbours from the connection table (regular periodic tiling)
     std::vector<int> fn((size_t)6 * c->ngrid, -1);
     for (size_t r = 0; r < c->conns.size(); r += 4) {
@@ -2286,18 +2300,6 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
     MG_CUDA(cudaMalloc(cb, 3 * n * sizeof(float)));
     MG_CUDA(cudaMalloc(apx, 2 * n * sizeof(float)));
     dim3 grid((st.npp + 255) / 256, nclass);
-    if (st.tile) {
-        const TileShape& ts = st.tile->s;
-        const size_t nt = (size_t)nclass * ts.npp * sizeof(float);
-        MG_CUDA(cudaMalloc(&st.tcf, 4 * nt));
-        MG_CUDA(cudaMalloc(&st.tcb, 3 * nt));
-        MG_CUDA(cudaMalloc(&st.tap, 2 * nt));
-        k_tile_extract<<<dim3((ts.npp + 255) / 256, nclass), 256, 0, c->stream>>>(
-            c->d_grids, d_reps, ts, planeorder ? 1 : 0, c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"),
-            c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), st.tcf, st.tcb,
-            st.tap);
-        MG_LAUNCHED(c);
-    }
     k_sip_extract<<<grid, 256, 0, c->stream>>>(
         c->d_grids, d_reps, st.d_qmap, d_idx, st.d_pst, st.nm, st.npp, planeorder ? 1 : 0,
         c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"), c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"),
@@ -2345,6 +2347,25 @@ int sip_extract(Ctx* c, SipState& st, int nclass, const int* d_reps, const int* 
             MG_CUDA(copy_on(c->stream, st.uni, uni.data(), uni.size() * sizeof(float),
                             cudaMemcpyHostToDevice));
         }
+    }
+    // the tiles' coefficients, where there is room for them beside the records of the cell
+    // hyperplane order
+    if (st.tile) {
+        const size_t nt = (size_t)nclass * st.tile->s.npp;
+        int rc = scratch(&st.tcf, 4 * nt);
+        if (!rc) rc = scratch(&st.tcb, 3 * nt);
+        if (!rc) rc = scratch(&st.tap, 2 * nt);
+        if (rc && rc != kNoScratch) return rc;
+        if (rc)
+            if (int rc2 = sip_leave_tiles(c, st)) return rc2;
+    }
+    if (st.tile) {
+        const TileShape& ts = st.tile->s;
+        k_tile_extract<<<dim3((ts.npp + 255) / 256, nclass), 256, 0, c->stream>>>(
+            c->d_grids, d_reps, ts, planeorder ? 1 : 0, c->F("SIPLW"), c->F("SIPLS"), c->F("SIPLB"),
+            c->F("SIPLPR"), c->F("SIPUE"), c->F("SIPUN"), c->F("SIPUT"), c->F("GSAP"), st.tcf, st.tcb,
+            st.tap);
+        MG_LAUNCHED(c);
     }
     return 0;
 }
@@ -2558,9 +2579,14 @@ int sip_bpmask(Ctx* c, SipState& st) {
     dim3 grid((st.npp + 255) / 256, c->ngrid);
     k_sip_bpmask<<<grid, 256, 0, c->stream>>>(c->d_grids, st.npp, st.d_idxp, c->F("BP"), st.bm);
     MG_LAUNCHED(c);
+    if (st.tile && !st.tbm) {
+        const int rc = scratch(&st.tbm, (size_t)c->ngrid * st.tile->s.npp);
+        if (rc && rc != kNoScratch) return rc;
+        if (rc)
+            if (int rc2 = sip_leave_tiles(c, st)) return rc2;
+    }
     if (st.tile) {
         const TileShape& ts = st.tile->s;
-        if (!st.tbm) MG_CUDA(cudaMalloc(&st.tbm, (size_t)c->ngrid * ts.npp));
         k_sip_bpmask<<<dim3((ts.npp + 255) / 256, c->ngrid), 256, 0, c->stream>>>(c->d_grids, ts.npp, ts.cell,
                                                                                   c->F("BP"), st.tbm);
         MG_LAUNCHED(c);

@@ -455,7 +455,7 @@ __global__ void k_pt_uniform(TileShape s, const double* __restrict__ LAP, double
     if (threadIdx.x == 0) UNI[8 * cls + 7] = bad ? 0.0 : 1.0;
 }
 
-int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
+static int set_up(Ctx* c, const mglet_grid_desc* d) {
     if (c->minlevel != c->maxlevel || !c->uniform || c->prm.psolver == MGLET_PSOLVER_CLASSIC ||
         c->prm.form != MGLET_FORM_PLAIN || c->prm.ninner < 1 || c->prm.nouter < 1)
         return 0;
@@ -522,7 +522,7 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
     }
     p->ncls = (int)reps.size();
     auto up = [&](int** q, const std::vector<int>& h) -> int {
-        MG_CUDA(cudaMalloc(q, h.size() * sizeof(int)));
+        if (int rc = scratch(q, h.size())) return rc;
         MG_CUDA(copy_on(c->stream, *q, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
         return 0;
     };
@@ -533,7 +533,7 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
     const size_t n = pad((size_t)c->ngrid * s.npp), m = (size_t)p->ncls * s.npp;
     const size_t cls[3] = {pad(4 * m), pad(3 * m), pad(7 * m)};
     const size_t all = 6 * n + cls[0] + cls[1] + cls[2] + pad(8 * p->ncls) + pad(c->ngrid) + pad(3);
-    MG_CUDA(cudaMalloc(&p->mem, all * sizeof(double)));
+    if (int rc = scratch(&p->mem, all)) return rc;
     double* q = p->mem;
     auto take = [&](double** d, size_t len) {
         *d = q;
@@ -564,9 +564,17 @@ int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
     return 0;
 }
 
+int plain_tile_init(Ctx* c, const mglet_grid_desc* d) {
+    const int rc = set_up(c, d);
+    if (rc != kNoScratch) return rc;
+    plain_tile_release(c);   // the per-operator kernels need no more than the fields
+    return 0;
+}
+
 void plain_tile_release(Ctx* c) {
     PlainTile* p = c->ptile;
     if (!p) return;
+    cudaStreamSynchronize(c->stream);
     tile_free(p->t);
     for (void* q : {(void*)p->gcls, (void*)p->fnbr, (void*)p->mem}) cudaFree(q);
     if (p->h_stat) cudaFreeHost(p->h_stat);
@@ -575,7 +583,7 @@ void plain_tile_release(Ctx* c) {
 }
 
 int plain_tile_test_timeout(Ctx* c) {
-    if (!c->ptile || !plain_tile_ready(c) || c->ptile->t.s.nc == 1) {
+    if (!c->ptile || c->ptile->t.s.nc == 1) {
         set_error("test_sweep_timeout: needs the plain form's solve on tiles with grids shared by SMs");
         return MGLET_ERR_UNSUPPORTED;
     }
@@ -583,9 +591,7 @@ int plain_tile_test_timeout(Ctx* c) {
     return 0;
 }
 
-bool plain_tile_ready(const Ctx* c) {
-    return c->ptile && !c->part && c->ibtype == 0 && !c->coef_user;
-}
+bool plain_tile_ready(const Ctx* c) { return c->ptile != nullptr; }
 #endif
 
 }  // namespace mg

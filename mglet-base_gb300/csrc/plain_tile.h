@@ -23,10 +23,11 @@ struct PlainTile {
 };
 
 // Set up when the context's grids take it: one level, equal dimensions, SIP in
-// plane order, face neighbours on opposite faces.  c->ptile stays null otherwise.
+// plane order, face neighbours on opposite faces, and the memory for it (6 FP64 arrays,
+// 14 more of every class of grids with equal faces and spacing).  c->ptile stays null
+// otherwise.
 int plain_tile_init(Ctx* c, const mglet_grid_desc* d);
-void plain_tile_release(Ctx* c);
-// May the solve run on tiles now (the coefficients are still the library's own)?
+// Does the solve run on tiles?
 bool plain_tile_ready(const Ctx* c);
 // mglet_gpu_test_sweep_timeout
 int plain_tile_test_timeout(Ctx* c);

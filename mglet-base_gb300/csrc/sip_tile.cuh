@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
 template <typename V>
 int tile_up(Ctx* c, TileDev& d, const V** p, const std::vector<V>& h) {
     V* m = nullptr;
-    MG_CUDA(cudaMalloc(&m, h.size() * sizeof(V)));
+    if (int rc = scratch(&m, h.size())) return rc;
     d.mem.push_back(m);
     MG_CUDA(copy_on(c->stream, m, h.data(), h.size() * sizeof(V), cudaMemcpyHostToDevice));
     *p = m;
@@ -878,7 +878,7 @@ int tile_up(Ctx* c, TileDev& d, const V** p, const std::vector<V>& h) {
 
 // Tables of a grid of ni x nj x nk cells in tiles of 2^si x 2^sj x 2^sk.  d.ok
 // stays false for hyperplanes of more than maxtiles tiles and shapes beyond the
-// 10-bit cells or 16-bit slots.
+// 10-bit cells or 16-bit slots; kNoScratch where the device has no room for them.
 inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int nc, int maxtiles, TileDev& d) {
     TileShape& s = d.s;
     s.nc = nc;

@@ -37,6 +37,7 @@ EXPORTS = [
     "mglet_gpu_force_variant", "mglet_create_flowstencils", "mglet_flowstencils_size",
     "mglet_flowstencils_copy", "mglet_flowstencils_free", "mglet_gpu_set_partition",
     "mglet_gpu_test_wait_timeout", "mglet_gpu_test_barrier_timeout", "mglet_gpu_test_sweep_timeout",
+    "mglet_gpu_test_scratch_limit",
     "mglet_gpu_set_scastencils",
     "mglet_gpu_set_scalar_geometry", "mglet_create_scastencils", "mglet_scastencils_size",
     "mglet_scastencils_copy", "mglet_scastencils_free", "mglet_mesh_create",
@@ -125,6 +126,7 @@ def load(path=None):
     L.mglet_gpu_test_wait_timeout.argtypes = [vp]
     L.mglet_gpu_test_barrier_timeout.argtypes = [vp]
     L.mglet_gpu_test_sweep_timeout.argtypes = [vp]
+    L.mglet_gpu_test_scratch_limit.argtypes = [C.c_int32]
     L.mglet_gpu_set_scastencils.argtypes = [vp, C.c_int32, C.c_int32, vp, vp, vp]
     L.mglet_gpu_set_scalar_geometry.argtypes = [vp, C.c_int32, C.c_int32, vp, vp]
     L.mglet_create_scastencils.argtypes = [vp, vp, C.POINTER(vp)]
