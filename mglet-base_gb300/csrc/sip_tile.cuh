@@ -893,22 +893,32 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
     s.fs = (std::max(nj * nk, std::max(ni * nk, ni * nj)) + 3) & ~3;
     s.w = NJ + 1;
     s.slots = (NI + 1) * (NJ + 1);
+    // (before any table: one grid of 256^3, whose hyperplanes are too long, would be
+    // listed cell by cell for nothing, 115 of 862 ms of its context)
+    auto jlo = [&](int t, int I) { return std::max(0, t - I - (NK - 1)); };
+    auto jhi = [&](int t, int I) { return std::min(NJ - 1, t - I); };
+    for (int t = 0; t < s.NT; ++t)
+        for (int r = 0; r < nc; ++r) {
+            int n = 0;
+            for (int I = (r * NI + nc - 1) / nc; I < ((r + 1) * NI + nc - 1) / nc; ++I)
+                n += std::max(0, jhi(t, I) - jlo(t, I) + 1);
+            s.maxt = std::max(s.maxt, n);
+        }
+    if (s.maxt > maxtiles || s.slots > 0xffff || (s.pad && s.ntile > 0xffff)) return 0;
     std::vector<int> tst(1, 0), tpos((size_t)s.NT * NI, 0);
     std::vector<unsigned short> slot((s.ntile + 3) & ~3, 0);
     std::vector<int> ti(s.ntile), tj(s.ntile), tk(s.ntile);
     for (int t = 0, p = 0; t < s.NT; ++t) for (int r = 0; r < nc; ++r) {
         for (int I = (r * NI + nc - 1) / nc; I < ((r + 1) * NI + nc - 1) / nc; ++I) {
-            const int jlo = std::max(0, t - I - (NK - 1)), jhi = std::min(NJ - 1, t - I);
-            tpos[(size_t)t * NI + I] = p - jlo;
-            for (int J = jlo; J <= jhi; ++J, ++p) {
+            tpos[(size_t)t * NI + I] = p - jlo(t, I);
+            for (int J = jlo(t, I); J <= jhi(t, I); ++J, ++p) {
                 ti[p] = I; tj[p] = J; tk[p] = t - I - J;
                 slot[p] = (unsigned short)((I + 1) * s.w + J + 1);
             }
         }
-        s.maxt = std::max(s.maxt, p - tst.back());
         tst.push_back(p);
     }
-    if (tst.back() != s.ntile || s.maxt > maxtiles || s.slots > 0xffff || (s.pad && s.ntile > 0xffff)) return 0;
+    if (tst.back() != s.ntile) return 0;
     auto tile = [&](int I, int J, int K) { return tpos[(size_t)(I + J + K) * NI + I] + J; };
     std::vector<int4> nbr((size_t)2 * s.ntile);
     for (int p = 0; p < s.ntile; ++p) {
