@@ -60,7 +60,6 @@ struct BpArgs {
     const int4* hier;
     const int* list;            // grids of the level with a PAR face
     const int* fnbr;            // [ngrid][6] face neighbours
-    const int* facepos;         // [6][fs]
     PlaneMap m;
     const float* H;
     float* PG;                  // [ngrid][6][fs]
@@ -594,7 +593,6 @@ static BpArgs bp_args(Ctx* c, const SipState& st, const int* ctl) {
     A.grids = c->d_grids;
     A.hier = c->d_hier;
     A.fnbr = st.d_fnbr;
-    A.facepos = sip_facepos(st);
     A.m = plane_map(st);
     A.H = st.h32;
     A.PG = st.pg;

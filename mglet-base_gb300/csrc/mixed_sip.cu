@@ -2051,8 +2051,6 @@ PosMap sip_posmap(const SipState& st) {
     return PosMap{st.d_tpos, st.ni, st.nj, st.nk, st.npp, st.fs, 0};
 }
 
-const int* sip_facepos(const SipState& st) { return sip_on_tiles(st) ? st.tile->s.facepos : st.d_facepos; }
-
 int sip_npp(const SipState& st) { return st.tile ? std::max(st.npp, st.tile->s.npp) : st.npp; }
 
 int sip_init(Ctx* c, SipState& st) {

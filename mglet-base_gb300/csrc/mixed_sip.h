@@ -119,7 +119,6 @@ struct PosMap {
     }
 };
 PosMap sip_posmap(const SipState& st);
-const int* sip_facepos(const SipState& st);
 int sip_npp(const SipState& st);   // length of a grid's array, for either order
 int sip_init(Ctx* c, SipState& st);
 // Class coefficients: FP32 blocks [lw|ls|lb|lpr|ap] and [ue|un|ut] per padded

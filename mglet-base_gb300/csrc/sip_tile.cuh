@@ -61,7 +61,6 @@ struct TileShape {
     const int* tpos;                // [NT][NI] tile (I, J) of hyperplane T is tpos[T*NI+I] + J
     const int* cell;                // [npp] natural local index of each position, -1 in pads
     const int* plane;               // [npp] its position in the cell hyperplane order, -1 in pads
-    const int* facepos;             // [6][fs] position of the boundary cell of each face index
 };
 
 // position of a cell
@@ -993,30 +992,12 @@ inline int tile_init(Ctx* c, int ni, int nj, int nk, int si, int sj, int sk, int
                 }
             }
     }
-    std::vector<int> facepos((size_t)6 * s.fs, -1);
-    auto pos = [&](int io, int jo, int ko) { return tile_pos(s, tpos.data(), io, jo, ko); };
-    for (int jo = 0; jo < nj; ++jo)
-        for (int ko = 0; ko < nk; ++ko) {
-            facepos[0 * s.fs + ko + jo * nk] = pos(0, jo, ko);
-            facepos[1 * s.fs + ko + jo * nk] = pos(ni - 1, jo, ko);
-        }
-    for (int io = 0; io < ni; ++io)
-        for (int ko = 0; ko < nk; ++ko) {
-            facepos[2 * s.fs + ko + io * nk] = pos(io, 0, ko);
-            facepos[3 * s.fs + ko + io * nk] = pos(io, nj - 1, ko);
-        }
-    for (int io = 0; io < ni; ++io)
-        for (int jo = 0; jo < nj; ++jo) {
-            facepos[4 * s.fs + jo + io * nj] = pos(io, jo, 0);
-            facepos[5 * s.fs + jo + io * nj] = pos(io, jo, nk - 1);
-        }
     if (int rc = tile_up(c, d, &s.tst, tst)) return rc;
     if (int rc = tile_up(c, d, &s.tpos, tpos)) return rc;
     if (int rc = tile_up(c, d, &s.slot, slot)) return rc;
     if (int rc = tile_up(c, d, &s.nbr, nbr)) return rc;
     if (int rc = tile_up(c, d, &s.cell, cell)) return rc;
     if (int rc = tile_up(c, d, &s.plane, plane)) return rc;
-    if (int rc = tile_up(c, d, &s.facepos, facepos)) return rc;
     d.ok = true;
     return 0;
 }
