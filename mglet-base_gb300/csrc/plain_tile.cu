@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
     TileHalo<L, double> o;
     const int4 n0 = __ldg(s.nbr + 2 * tile), n1 = __ldg(s.nbr + 2 * tile + 1);
     tile_halo(a.t, g, tile, n0, n1, o);
-    const int last = max(a.t.ctl[1], 1) * a.ninner;   // inner iterations done (none: the solve was lost)
+    const int last = a.t.ctl[2] * a.ninner;   // inner iterations done
     const double *low = a.ninner > 1 ? a.RS[(last - 1) % 3] : nullptr, *high = a.RS[last % 3];
     res_ghosts<L, 0>(a.t, g, n0.x, n1.z, low, RES + ip3);
     res_ghosts<L, 1>(a.t, g, n0.y, n1.z, high, RES + ip3);
@@ -189,8 +189,7 @@ __global__ void __launch_bounds__(128) k_pt_scatter(const __grid_constant__ PtOu
 }
 
 // maxabscal over the grids (one level: no level scale) and the stopping test; the
-// maxima are cleared for the next outer iteration.  stat: {max |rhs|, converged,
-// outer iterations done}.
+// maxima are cleared for the next outer iteration.  stat: see PlainTile.
 __global__ void k_pt_conv(int ngrid, double* __restrict__ gridmax, double* stat, double prefak, double epcorr,
                           int nouter_min) {
     int* ctl = reinterpret_cast<int*>(stat + 1);
@@ -210,8 +209,8 @@ __global__ void k_pt_conv(int ngrid, double* __restrict__ gridmax, double* stat,
         m = l < (int)(blockDim.x >> 5) ? sh[l] : 0.0;
         for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
         if (l == 0) {
-            const int done = ctl[1] + 1;
-            ctl[1] = done;
+            const int done = ctl[2] + 1;
+            ctl[2] = done;
             stat[0] = m;
             if (done >= nouter_min && m / prefak < epcorr) ctl[0] = 1;
         }
@@ -313,12 +312,9 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     a.grids = c->d_grids;
     a.UNI = p.uni;
     a.ctl = ctl;
-    if (s.nc > 1) {
-        a.err = ctl + 2;
-        a.stop = ctl;
-        a.lose = p.lose_once;
-        p.lose_once = false;
-    }
+    a.err = ctl + 1;
+    a.lose = p.lose_once;
+    p.lose_once = false;
     PtOuterArgs o{};
     o.RHS = p.rhs;
     o.DP = p.dp;
@@ -347,6 +343,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
             }
             {
                 ProfScope ps_(c, "sipiter1");
+                a.stamp = 2 * gi;
                 a.G = lastfull > 0 ? p.rs[lastfull % 3] : nullptr;
                 a.CF = p.cf;
                 a.cfcls = 4 * s.npp;
@@ -355,6 +352,7 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
             }
             {
                 ProfScope ps_(c, "sipiter2");
+                a.stamp = 2 * gi + 1;
                 a.G = a.R;
                 a.CF = p.cb;
                 a.cfcls = 3 * s.npp;
@@ -380,7 +378,8 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
         if (ip % 12 == 0 && ip < c->prm.nouter) {
             MG_CUDA(cudaMemcpyAsync(p.h_stat, p.stat, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
             MG_CUDA(cudaStreamSynchronize(c->stream));
-            if (reinterpret_cast<const int*>(p.h_stat + 1)[0]) break;
+            const int* h = reinterpret_cast<const int*>(p.h_stat + 1);
+            if (h[0] || h[1]) break;
         }
     }
     o.t = a;
@@ -394,12 +393,12 @@ int solve(Ctx* c, double prefak, mglet_stage_stats* st) {
     if (int rc = connect(c, 0, 1, nullptr, nullptr, nullptr, c->F("DP"), nullptr, nullptr, false, false, 0))
         return rc;
     MG_CUDA(cudaStreamSynchronize(c->stream));
-    if (reinterpret_cast<const int*>(p.h_stat + 2)[0]) {
+    if (reinterpret_cast<const int*>(p.h_stat + 1)[1]) {
         set_error("mgpoisl: a sweep timed out waiting for another CTA");
         return MGLET_ERR_CUDA;
     }
     if (st) {
-        st->nouter_done = reinterpret_cast<const int*>(p.h_stat + 1)[1];
+        st->nouter_done = reinterpret_cast<const int*>(p.h_stat + 1)[2];
         st->ipc = st->nouter_done * ninner;
         st->maxrhs = p.h_stat[0];
         st->prefak = prefak;

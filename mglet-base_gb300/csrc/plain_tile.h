@@ -17,7 +17,7 @@ struct PlainTile {
     double *cf = nullptr, *cb = nullptr, *lap = nullptr, *uni = nullptr;   // 4, 3, 7 arrays; [ncls][8]
     double *h = nullptr, *rhs = nullptr, *dp = nullptr, *rs[3] = {nullptr, nullptr, nullptr};
     double* gridmax = nullptr;  // [ngrid]
-    double* stat = nullptr;     // device {max |rhs|, ints: converged, outer iterations, error}
+    double* stat = nullptr;     // device {max |rhs|, ints: converged, error, outer iterations}
     double* h_stat = nullptr;   // pinned copy
     bool lose_once = false;     // test switch: a wait of the next solve's forward sweeps runs out
 };

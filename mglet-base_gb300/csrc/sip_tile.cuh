@@ -207,11 +207,11 @@ struct TileArgs {
     const DevGrid* grids;
     const unsigned char* BM;        // [ngrid][npp] open couplings (null: all)
     const T* UNI;                   // [ncls][8] operator coefficients of uniform classes
-    const int* ctl;                 // [0] converged: nothing to do
+    const int* ctl;                 // [0] converged: nothing to do; ranks: [1] err
     int cfcls, lprcls, apcls;       // values between the classes of CF, LPR and AP
-    int* err;                       // set when a rank waited in vain (null: no ranks)
-    int* stop;                      // pre-pass: ctl[0], which it sets when err is
-    int lose;                       // test switch: forward, rank 1 misses the first faces of every grid
+    int* err;                       // takes stamp when a rank waited in vain
+    int stamp;                      // the sweep's, not 0, another one in each launch of a solve
+    int lose;                       // test switch: forward, rank 1 of every grid misses its first faces
     int rev;                        // walk the grids in reverse block order
 };
 
@@ -442,21 +442,22 @@ struct TileSweep {
         return __any_sync(0xffffffffu, clock64() - since > limit);
     }
     // one warp, in step t: stages the faces the rank before has put in step t.  The wait
-    // for them ends after about a second: then the error flag is set and this launch
-    // waits no more.  The next pre-pass sees the flag and ends the solve.
+    // for them ends after about a second: then the error flag takes the launch's stamp
+    // and this rank waits no more.  Later sweeps find a stamp that is not theirs and
+    // return at once; what this launch writes stops none of its own CTAs, so that of a
+    // cluster all return or none.
     static constexpr long long kWait = 2000000000LL, kWaitTest = 100000000LL;   // SM clocks
-    __device__ __forceinline__ void boundary(int t, bool& lost) {
+    __device__ __forceinline__ void boundary(int t, bool& lost, bool lose = false) {
         if (!up) return;
         const int I = kFwd ? i0 - 1 : i1 + 1, h = (kFwd ? t : s.NT - 1 - t) - I;
         const int lo = row_lo(h), hi = row_hi(h);
         if (lo > hi) return;
-        const bool lose = kFwd && a.lose && rank == 1 && h == 0;
         const long long since = clock64();
         while (!lost) {
             if (arrived(h) && !lose) break;
             if (expired(since, lose ? kWaitTest : kWait)) {
                 lost = true;
-                if ((threadIdx.x & 31) == 0) *a.err = 1;
+                if ((threadIdx.x & 31) == 0) *a.err = a.stamp;
             }
         }
         Face* f = face + (t & 1) * 3 * s.slots + (kFwd ? (I + 1) * s.w + 1 : I * s.w);
@@ -618,7 +619,14 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     w.tables();
     if constexpr (kRanks) w.arm();
     follow_on();
-    const int converged = flag_at(a.ctl);
+    int converged;
+    if constexpr (kRanks) {
+        int err;
+        asm volatile("ld.global.v2.s32 {%0, %1}, [%2];" : "=r"(converged), "=r"(err) : "l"(a.ctl) : "memory");
+        converged |= err && err != a.stamp;
+    } else {
+        converged = flag_at(a.ctl);
+    }
     auto start = [&]() {
         if (tid < 2 * ncomp)
 #pragma unroll
@@ -634,7 +642,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_sweep_few(const __grid_consta
     if (tid >= 2 * ncomp) {
         bool lost = false;
         w.stage(t0 - 1);
-        if constexpr (kRanks) w.boundary(t0 - 1, lost);
+        if constexpr (kRanks) w.boundary(t0 - 1, lost, kFwd && a.lose && w.rank == 1);
         __syncthreads();
         for (int t = t0; t < end; ++t) {
             if (t < t1) w.stage(t);
@@ -832,9 +840,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_tile_pre(const __grid_
         ldt(on, a.AP + (long long)cls * a.apcls + p, ap);
     }
     follow_on();
-    // (the sweeps read ctl, which has to be one value for the ranks of a cluster, so they
-    // cannot set it)
-    if (a.err && tile == 0 && blockIdx.y == 0 && flag_at(a.err)) *a.stop = 1;
     if (flag_at(a.ctl) || !on) return;
     ldt_co(true, a.RHS + base + p, rh);
     if constexpr (kHz) {
