@@ -345,7 +345,8 @@ __global__ void __launch_bounds__(256) k_tstle4(const DevGrid* __restrict__ grid
 // term st*0 is zero for finite fields and falls away; a grid with a result that is not
 // finite is left to k_tstle4, as one with several values of G is.
 // Bound by the FP64 pipe (ncu: busy all the time on the SMs with a CTA): 526
-// instructions a point and its faces in k_tstle4, about 150 here.  512 grids of 24^3
+// instructions a cell in k_tstle4, 195 here (343 grids of 24^3, with the faces that two
+// CTAs compute and the idle lanes of partial warps).  512 grids of 24^3
 // contracted 6.15 -> 2.72 ms, 64 grids uncontracted 0.95 -> 0.45, 216 of 20^3 1.84 ->
 // 0.74.
 

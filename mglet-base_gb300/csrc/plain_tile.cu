@@ -11,7 +11,7 @@
 // stays in L2), and the host round trip of every outer iteration: the stopping
 // test sets a flag the following kernels return on.  A time step of three stages
 // (per-operator kernels before): one grid of 32^3 10.6 ms (50.3), 64 of 24^3 15.4
-// (38.5), 512 of 24^3 contracted 52.8 (103).  What bounds the sweeps is the FP64 pipe
+// (38.5), 512 of 24^3 contracted 53-57 (103).  What bounds the sweeps is the FP64 pipe
 // (432 warps of points of 24^3, 6 instructions a point uncontracted, 64 clocks each
 // on four pipes: 20 us on one SM) and, with fewer grids than SMs, the chain of the
 // hyperplanes.
