@@ -179,9 +179,10 @@ int64_t mglet_gpu_idim3d(const mglet_ctx* ctx);
  * equal idim3d.  Host memory may be pageable or pinned.
  * The plain form's pressure solve on one level keeps its own copies of the
  * Poisson coefficients, which mglet_gpu_create makes.  Once BP, GSAP or one of
- * SIP* is written, here or by an entry point that takes a field's name, and
- * whatever the values are, the context reads the fields instead and solves
- * with one kernel per operator: the same bits, at half the speed or less. */
+ * SIP* is written, here or by an entry point that takes a field's name (other
+ * than a connect of BP or GSAP), and whatever the values are, the context reads
+ * the fields instead and solves with one kernel per operator: the same bits,
+ * at half the speed or less. */
 int mglet_gpu_set_field(mglet_ctx* ctx, const char* name, const double* host, int64_t n);
 int mglet_gpu_get_field(mglet_ctx* ctx, const char* name, double* host, int64_t n);
 

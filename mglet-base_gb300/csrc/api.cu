@@ -940,7 +940,10 @@ int mglet_gpu_connect(mglet_ctx* c, int32_t ilevel, int32_t layers, const char* 
         if (names[q] && !f[q]) return fail(MGLET_ERR_NAME, std::string("connect: unknown field ") + names[q]);
     }
     cudaSetDevice(c->device);
-    for (const char* nm : names) field_written(c, nm);
+    // (of BP and GSAP it writes ghosts: equal ones while the solve on tiles is there, and
+    // such as no operator reads; SIP* are in hyperplane order)
+    for (const char* nm : names)
+        if (nm && std::strcmp(nm, "BP") && std::strcmp(nm, "GSAP")) field_written(c, nm);
     return connect(c, ilevel, layers, f[0], f[1], f[2], f[3], f[4], f[5], corners != 0,
                    normal != 0, forward);
 }

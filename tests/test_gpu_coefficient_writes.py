@@ -32,7 +32,9 @@ def _stage(gpu_lib, g):
     ("GSAP", lambda g: g.rkstep("DU", "GSAP", "UO", 0.5, 1.0)),
     ("BP", lambda g: g.rkstep("BP", "DU", "UO", 0.5, 1.0)),
     ("GSAP", lambda g: g.divcal("GSAP", -100.0)),
-    ("GSAP", lambda g: g.laplacephi("GSAP", "VO"))])
+    ("GSAP", lambda g: g.laplacephi("GSAP", "VO")),
+    ("SIPLPR", lambda g: g.connect(0, 2, s1="SIPLPR")), ("GSAP", lambda g: g.connect(0, 2, s1="GSAP")),
+    ("BP", lambda g: g.connect(0, 2, s1="BP", corners=True))])
 def test_a_written_coefficient_is_used(gpu_lib, name, call):
     case = cases.periodic_box(2, 1, 1, n=8)
     a = _solver(gpu_lib, case)
@@ -45,3 +47,18 @@ def test_a_written_coefficient_is_used(gpu_lib, name, call):
         assert np.array_equal(x, y, equal_nan=True)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("name,kept", [("BP", True), ("GSAP", True), ("SIPLPR", False), ("P", True)])
+def test_connecting_ghosts_keeps_the_solve_on_tiles(gpu_lib, name, kept):
+    case = cases.periodic_box(2, 1, 1, n=8)
+    n = []
+    for call in (False, True):
+        g = _solver(gpu_lib, case)
+        if call:
+            g.connect(0, 2, s1=name)
+        n0 = g.launches
+        _stage(gpu_lib, g)
+        n.append(g.launches - n0)
+        g.close()
+    assert (n[0] == n[1]) == kept
